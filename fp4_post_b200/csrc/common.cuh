@@ -170,16 +170,47 @@ __device__ __forceinline__ float folded_index(float q) {
   return min3(q, __fmaf_rn(q, 0.5f, 2.0f), __fmaf_rn(q, 0.25f, 4.0f));
 }
 
+// Two floats in one 64-bit register pair and the packed fp32 instructions on them (each half rounds as the scalar
+// instruction does).  One issue slot serves two elements; the pipe rate per element is the scalar one (measured: 2.1
+// cycles per warp instruction against 1.07), so they pay off where a kernel is bound by issue, as the quantizers are.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void split2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// v - m element by element (as v + (-m): the same single rounding, the same sign of a zero)
+__device__ __forceinline__ void subtract16(float (&v)[16], const float (&m)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 2) split2(add2(pack2(v[i], v[i + 1]), pack2(-m[i], -m[i + 1])), v[i], v[i + 1]);
+}
+
 // Correctly rounded a / h for |a| <= 12.1 h from a refined reciprocal r of h: one
-// multiplication, the exact remainder and one correction (Markstein).  A remainder that
-// underflows only occurs for quotients far below the first rounding boundary.
+// multiplication, the exact remainder and one correction (Markstein), two elements at a time.
+// A remainder that underflows only occurs for quotients far below the first rounding boundary.
 __device__ __forceinline__ float refine_reciprocal(float h) {
   const float r = rcp_approx(h);
   return __fmaf_rn(__fmaf_rn(-h, r, 1.0f), r, r);
 }
-__device__ __forceinline__ float divide_exact(float a, float h, float r) {
-  const float q0 = __fmul_rn(a, r);
-  return __fmaf_rn(__fmaf_rn(-h, q0, a), r, q0);
+__device__ __forceinline__ f32x2 divide_exact2(f32x2 a, f32x2 minus_h, f32x2 r) {
+  const f32x2 q0 = mul2(a, r);
+  return fma2(fma2(minus_h, q0, a), r, q0);
 }
 
 // 8 values -> 8 e2m1 nibbles, element 0 in the low nibble: round to nearest, ties to the even code,
@@ -205,9 +236,9 @@ __device__ __forceinline__ uint32_t pack_e2m1x8(const float (&v)[8]) {
 // and 4 on [4, 8) (round to nearest even in the binade of the sum, as the reference's addition does),
 // makes them agree everywhere.  t comes from the exponent bits of v: 0x40000000 is 2.0, 0x40800000 is
 // 4.0; below 2, bit 30 is clear and what is left (0 or 2^-126) changes nothing; the sign is kept.
-__device__ __forceinline__ float round_like_folded(float v) {
-  const float t = __uint_as_float(__float_as_uint(v) & 0xC0800000u);
-  return __fsub_rn(__fadd_rn(v, t), t);
+__device__ __forceinline__ f32x2 round_like_folded2(f32x2 v) {
+  const f32x2 t = v & 0xC0800000C0800000ull;
+  return fma2(t, 0xBF800000BF800000ull /* -1, -1 */, add2(v, t));
 }
 
 // Round-to-nearest codes of kGroups*8 consecutive values sharing the block scale `s`
@@ -215,21 +246,23 @@ __device__ __forceinline__ float round_like_folded(float v) {
 // the low nibble.  Every element goes through the reference's own arithmetic: the correctly
 // rounded quotient x/s (half the reference's |x|/(s/2), exactly), its second rounding, and round
 // half to even onto the e2m1 grid by the hardware conversion, which packs two codes with their
-// sign bits per instruction.  (The conversion runs on the special-function unit at about 26 cycles
-// per warp; sending half of every block down an FMA/ALU-only path of the folded index, magic-number
-// rounding and shifted adds instead was measured slower: 4 more instructions per element cost more
-// than the relieved unit gives back.)  There is no approximate fast path because with bf16
+// sign bits per instruction (4 cycles per warp instruction and scheduler, i.e. 2 per element; packing the codes by
+// integer arithmetic instead was measured slower).  Division and second rounding run on the packed fp32
+// instructions, two elements per issue slot: these kernels are bound by issue, not by a pipe.
+// There is no approximate fast path because with bf16
 // inputs exact ties (an element equal to amax/8, 5/24 amax, ...) are common.  The division is
 // signed: -0.0 comes out as +0.0 (the remainder +0 wins the final sum), any negative x keeps its
 // sign down to -0.0, which is the reference's sign bit (x < 0).
 template <int kGroups>
 __device__ __forceinline__ void quantize_rn(const float (&x)[8 * kGroups], float s, uint32_t (&out)[kGroups]) {
   const float r = refine_reciprocal(s);
+  const f32x2 rr = pack2(r, r), minus_s = pack2(-s, -s);
 #pragma unroll
   for (int g = 0; g < kGroups; ++g) {
     float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = round_like_folded(divide_exact(x[8 * g + i], s, r));
+    for (int i = 0; i < 8; i += 2)
+      split2(round_like_folded2(divide_exact2(pack2(x[8 * g + i], x[8 * g + i + 1]), minus_s, rr)), v[i], v[i + 1]);
     out[g] = pack_e2m1x8(v);
   }
 }
@@ -305,11 +338,16 @@ __device__ __forceinline__ uint32_t cvt_rs_e2m1x4(float e0, float e1, float e2, 
 }
 __device__ __forceinline__ void quantize16_sr_hw(const float (&x)[16], float s, uint4 rnd, uint32_t (&out)[2]) {
   const float inv = rcp_approx(s);
+  const f32x2 inv2 = pack2(inv, inv);
   const uint32_t rw[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
   uint32_t h[4];
 #pragma unroll
-  for (int w = 0; w < 4; ++w)
-    h[w] = cvt_rs_e2m1x4(x[4 * w] * inv, x[4 * w + 1] * inv, x[4 * w + 2] * inv, x[4 * w + 3] * inv, rw[w]);
+  for (int w = 0; w < 4; ++w) {
+    float q[4];
+    split2(mul2(pack2(x[4 * w], x[4 * w + 1]), inv2), q[0], q[1]);
+    split2(mul2(pack2(x[4 * w + 2], x[4 * w + 3]), inv2), q[2], q[3]);
+    h[w] = cvt_rs_e2m1x4(q[0], q[1], q[2], q[3], rw[w]);
+  }
   out[0] = h[0] | (h[1] << 16);
   out[1] = h[2] | (h[3] << 16);
 }

@@ -46,10 +46,7 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
     if (kMean) Load16<float>::load(col_mean + (int64_t)bc * 16, m);
     const Philox rng(seed);
     auto quantize_block = [&](float (&v)[16], int r) {
-      if (kMean) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __fsub_rn(v[i], m[i]);
-      }
+      if (kMean) subtract16(v, m);
       const float a = abs_max16(v);
       const float s = block_scale_from_amax(a);
       const int64_t b = (int64_t)r * blocks_per_row + bc;
@@ -96,6 +93,10 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
 // r sits at chunk c ^ (r & 7)).  One __syncthreads per tile: staging and the column means are double
 // buffered.  A tile load that does not arrive within the wait limit raises the error word of the
 // workspace header (the scale pass then publishes NaN as the unit) instead of hanging.
+// What bounds it: instruction issue (24 warps per SM; the rows-only form runs at 85 % of the copy bandwidth).
+// Measured at 16384 x 4096 bf16, this pass alone, rows / transposed / both / both centred and stochastic: 37.1 / 48.2 /
+// 76.9 / 91.5 us with scalar fp32 arithmetic and 64-bit divisions in the tile walk, 32.9 / 39.6 / 63.8 / 80.2 us with
+// packed fp32 (3-6 us of it) and the walk by additions with every thread's offsets inside a tile kept (the rest).
 template <typename T> struct TileCfg {
   static constexpr int kRows = 128;
   static constexpr int kCols = 128 / sizeof(T);            // 64 (bf16) or 32 (fp32): 128 bytes per row
@@ -119,6 +120,12 @@ constexpr uint64_t kColumnStream = 1ull << 63;             // Philox counter spa
 // then the block maxima of Q and of Qt.
 constexpr int kDualMaxCtas = 640;
 constexpr int kDualHeaderBytes = 256 + ((kDualMaxCtas * 3 * 4 + 255) / 256) * 256;
+
+// How a CTA walks the tiles: their number, those along a row of x, and gridDim.x split into whole rows of tiles
+// and a remainder.
+struct TileWalk {
+  uint32_t tiles, col_tiles, step_rows, step_cols;
+};
 
 struct TileOutputs {
   uint8_t* codes_t;  float* amax_t;  unsigned int* gmax_t;        // Qt [cols, rows]
@@ -163,7 +170,7 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 
 template <typename T, bool kMean, bool kSR, bool kRowsOut, bool kColsOut>
 __global__ void __launch_bounds__(kQuantThreads, 3)
-quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, int64_t rows, int64_t cols,
+quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk walk, int64_t rows, int64_t cols,
                      const float* __restrict__ col_mean, uint64_t seed, uint64_t offset,
                      const uint64_t* __restrict__ offset_ctr, const TileOutputs out) {
   using TC = TileCfg<T>;
@@ -178,11 +185,17 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, int64_t rows, in
   if (kSR && offset_ctr) offset += *offset_ctr;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int64_t row_tiles = (rows + TC::kRows - 1) / TC::kRows;
-  const int64_t col_tiles = (cols + TC::kCols - 1) / TC::kCols;
-  const int64_t tiles = row_tiles * col_tiles;       // tile id = row tile * col_tiles + column tile
   const int64_t bpr = cols >> 4;                     // blocks per row of Q
   const int64_t bpc = rows >> 4;                     // blocks per row of Qt
+  // Tile id = row tile * col_tiles + column tile; the CTA takes the ids blockIdx.x + i * gridDim.x.  The two
+  // coordinates advance by additions (walk.step_* = gridDim.x in mixed radix): a 64-bit division per thread and tile
+  // costs as much as three elements' arithmetic.
+  const uint32_t tiles = walk.tiles, col_tiles = walk.col_tiles;
+  auto advance = [&](uint32_t& rt, uint32_t& ct) {
+    ct += walk.step_cols;
+    rt += walk.step_rows;
+    if (ct >= col_tiles) { ct -= col_tiles; ++rt; }
+  };
 
   if (tid == 0) {
     for (int s = 0; s < TC::kStages; ++s) mbar_init(&full[s], 1);
@@ -190,42 +203,58 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, int64_t rows, in
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  auto fill_mean = [&](int64_t tile, int buf) {
+  auto fill_mean = [&](uint32_t ct, int buf) {
     if (kMean && tid < TC::kCols) {
-      const int64_t c = (tile % col_tiles) * TC::kCols + tid;
+      const int64_t c = (int64_t)ct * TC::kCols + tid;
       s_mean[buf * TC::kCols + tid] = c < cols ? __ldg(col_mean + c) : 0.0f;
     }
   };
-  if ((int64_t)blockIdx.x < tiles) fill_mean(blockIdx.x, 0);
+  uint32_t rt = blockIdx.x / col_tiles, ct = blockIdx.x - rt * col_tiles;
+  if (blockIdx.x < tiles) fill_mean(ct, 0);
   __syncthreads();
 
-  auto issue = [&](int64_t tile, int stage) {
-    const int64_t rt = tile / col_tiles, ct = tile - rt * col_tiles;
-    mbar_expect_tx(&full[stage], TC::kStageBytes);
-    tma_load_2d(smem + stage * TC::kStageBytes, &map_x, (int32_t)(ct * TC::kCols), (int32_t)(rt * TC::kRows), &full[stage]);
+  uint32_t ahead_rt = rt, ahead_ct = ct, ahead = blockIdx.x;       // the next tile to be requested
+  auto issue = [&](int stage) {
+    if (ahead < tiles) {
+      mbar_expect_tx(&full[stage], TC::kStageBytes);
+      tma_load_2d(smem + stage * TC::kStageBytes, &map_x, (int32_t)(ahead_ct * TC::kCols), (int32_t)(ahead_rt * TC::kRows), &full[stage]);
+      ahead += gridDim.x;
+      advance(ahead_rt, ahead_ct);
+    }
   };
   if (tid == 0) {
-    for (int s = 0; s < TC::kStages; ++s) {
-      const int64_t t = (int64_t)blockIdx.x + (int64_t)s * gridDim.x;
-      if (t < tiles) issue(t, s);
-    }
+    for (int s = 0; s < TC::kStages; ++s) issue(s);
   }
 
   const Philox rng(seed);
   float running_t = 0.0f, running_r = 0.0f;
   const uint32_t smem_base = smem_u32(smem);
+  // Where this thread's work lies inside a tile does not change from tile to tile: per tile only the tile's own
+  // position is added.
   // column phase: this lane's word of a row, as chunk and offset inside the chunk
   const uint32_t word_chunk = (uint32_t)lane >> 2, word_in_chunk = ((uint32_t)lane & 3u) * 4u;
+  const uint32_t col_smem = (uint32_t)(warp * 16) * 128u + word_in_chunk;
+  const int64_t col_ctr = (int64_t)(lane * TC::kColsPerWord) * bpc + warp;      // Philox counter of its first block
+  // row phase: block (row_r + u * kRowStep, row_b)
+  constexpr int kRowStep = kQuantThreads / TC::kBlocksPerRow;
+  const int row_b = tid & (TC::kBlocksPerRow - 1), row_r = tid / TC::kBlocksPerRow;
+  const int64_t row_blk = (int64_t)row_r * bpr + row_b;
+  // write-out of Qt: 8-byte piece out_piece of the out rows out_j, out_j + 32, ...
+  const int out_j = tid >> 3, out_piece = tid & 7;
+  const int64_t pitch_t = rows >> 1;
+  const int64_t out_off = out_j * pitch_t + out_piece * 8;
+  const uint32_t out_staged = (uint32_t)((out_j % TC::kColsPerWord) * TC::kCodeArray + (out_j / TC::kColsPerWord) * TC::kCodePitch + out_piece * 8);
   volatile int* failed = &s_failed;
   int stage = 0;
   uint32_t it = 0;
-  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
     const int buf = it & 1;
     if (!mbar_wait(&full[stage], (it / TC::kStages) & 1u, failed)) *failed = 1;
     if (*failed) break;                               // every thread sees the same outcome of the barrier, or the flag
 
-    const int64_t rt = tile / col_tiles, ct = tile - rt * col_tiles;
-    const int64_t row0 = rt * TC::kRows, col0 = ct * TC::kCols;
+    const int64_t row0 = (int64_t)rt * TC::kRows, col0 = (int64_t)ct * TC::kCols;
+    const int live_rows = (int)min((int64_t)TC::kRows, rows - row0);            // of this tile
+    const int live_cols = (int)min((int64_t)TC::kCols, cols - col0);            // both multiples of 16 where that output exists
     const uint32_t tile_smem = smem_base + stage * TC::kStageBytes;
     uint8_t* staging = s_staging + buf * TC::kStagingBytes;
     float* s_amax = reinterpret_cast<float*>(staging + TC::kColsPerWord * TC::kCodeArray);   // [kRowBlocks][kCols]
@@ -233,91 +262,88 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, int64_t rows, in
 
     // ---- column phase: warp = row block, lane = 32-bit word of the row ----
     if (kColsOut) {
-      const int rb = warp;
       float v[TC::kColsPerWord][16];
-      float m[TC::kColsPerWord];
-#pragma unroll
-      for (int c = 0; c < TC::kColsPerWord; ++c) m[c] = kMean ? mean[lane * TC::kColsPerWord + c] : 0.0f;
-      const uint32_t row_base = tile_smem + (uint32_t)(rb * 16) * 128u + word_in_chunk;
+      const uint32_t row_base = tile_smem + col_smem;
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
         const uint32_t w = lds32(row_base + r * 128 + ((word_chunk ^ (uint32_t)(r & 7)) << 4));
         if constexpr (sizeof(T) == 2) { v[0][r] = bf16_lo(w); v[1][r] = bf16_hi(w); }
         else                          { v[0][r] = __uint_as_float(w); }
-        if (kMean) {
+      }
+      if (kMean) {
 #pragma unroll
-          for (int c = 0; c < TC::kColsPerWord; ++c) v[c][r] = __fsub_rn(v[c][r], m[c]);
+        for (int c = 0; c < TC::kColsPerWord; ++c) {
+          const float m = mean[lane * TC::kColsPerWord + c];
+          const f32x2 minus_m = pack2(-m, -m);
+#pragma unroll
+          for (int r = 0; r < 16; r += 2) split2(add2(pack2(v[c][r], v[c][r + 1]), minus_m), v[c][r], v[c][r + 1]);
         }
       }
-      const bool rows_live = row0 + rb * 16 < rows;
+      const bool rows_live = warp * 16 < live_rows;
       float amax[TC::kColsPerWord];
 #pragma unroll
       for (int c = 0; c < TC::kColsPerWord; ++c) {
         if (out.hadamard) hadamard16(v[c], out.hadamard & 0xFFFFu);           // uniform over the grid
-        const int64_t out_row = col0 + lane * TC::kColsPerWord + c;           // row of Qt = column of x
         const float a = abs_max16(v[c]);
         const float s = block_scale_from_amax(a);
         uint32_t packed[2];
         if (kSR) {
-          const uint64_t b = (uint64_t)out_row * (uint64_t)bpc + (uint64_t)((row0 >> 4) + rb);
+          const uint64_t b = (uint64_t)(col0 * bpc + (row0 >> 4) + col_ctr + c * bpc);            // block index in Qt
           const uint4 bits = rng(b, kRowsOut ? (offset ^ kColumnStream) : offset);                // alone: the transposed call's own stream
           if (out.sr16) quantize16_sr(v[c], s, bits, packed);
           else quantize16_sr_hw(v[c], s, bits, packed);
         } else {
           quantize_rn<2>(v[c], s, packed);
         }
-        *reinterpret_cast<uint2*>(staging + c * TC::kCodeArray + lane * TC::kCodePitch + rb * 8) = make_uint2(packed[0], packed[1]);
+        *reinterpret_cast<uint2*>(staging + c * TC::kCodeArray + lane * TC::kCodePitch + warp * 8) = make_uint2(packed[0], packed[1]);
         amax[c] = a;
-        if (rows_live && out_row < cols) running_t = fmaxf(running_t, a);
+        if (rows_live && lane * TC::kColsPerWord + c < live_cols) running_t = fmaxf(running_t, a);
       }
-      if constexpr (sizeof(T) == 2) *reinterpret_cast<float2*>(s_amax + rb * TC::kCols + 2 * lane) = make_float2(amax[0], amax[1]);
-      else                          s_amax[rb * TC::kCols + lane] = amax[0];
+      if constexpr (sizeof(T) == 2) *reinterpret_cast<float2*>(s_amax + warp * TC::kCols + 2 * lane) = make_float2(amax[0], amax[1]);
+      else                          s_amax[warp * TC::kCols + lane] = amax[0];
     }
 
     // ---- row phase: a thread owns blocks (row, b) with b fixed, straight to global memory ----
     if (kRowsOut) {
-      const int b = tid & (TC::kBlocksPerRow - 1);
-      const bool cols_live = col0 + b * 16 < cols;
+      const bool cols_live = row_b * 16 < live_cols;
+      const int64_t tile_blk = row0 * bpr + (col0 >> 4);
       float mb[16];
       if (kMean) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 f = *reinterpret_cast<const float4*>(mean + b * 16 + 4 * i);
+          const float4 f = *reinterpret_cast<const float4*>(mean + row_b * 16 + 4 * i);
           mb[4 * i] = f.x; mb[4 * i + 1] = f.y; mb[4 * i + 2] = f.z; mb[4 * i + 3] = f.w;
         }
       }
 #pragma unroll
       for (int u = 0; u < TC::kRowUnits; ++u) {
-        const int r = (tid + u * kQuantThreads) / TC::kBlocksPerRow;
+        const int r = row_r + u * kRowStep;
         const uint32_t row_addr = tile_smem + (uint32_t)r * 128u;
         const uint32_t swz = (uint32_t)(r & 7);
         RawBlock<T> raw;
         if constexpr (sizeof(T) == 2) {
-          raw.a = lds128(row_addr + (((uint32_t)(2 * b) ^ swz) << 4));
-          raw.b = lds128(row_addr + (((uint32_t)(2 * b + 1) ^ swz) << 4));
+          raw.a = lds128(row_addr + (((uint32_t)(2 * row_b) ^ swz) << 4));
+          raw.b = lds128(row_addr + (((uint32_t)(2 * row_b + 1) ^ swz) << 4));
         } else {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const uint4 w = lds128(row_addr + (((uint32_t)(4 * b + k) ^ swz) << 4));
+            const uint4 w = lds128(row_addr + (((uint32_t)(4 * row_b + k) ^ swz) << 4));
             raw.q[k] = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
           }
         }
         float v[16];
         raw.unpack(v);
-        if (kMean) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __fsub_rn(v[i], mb[i]);
-        }
+        if (kMean) subtract16(v, mb);
         const float a = abs_max16(v);
         const float s = block_scale_from_amax(a);
-        const int64_t blk = (row0 + r) * bpr + (col0 >> 4) + b;
+        const int64_t blk = tile_blk + row_blk + u * (kRowStep * bpr);
         uint32_t packed[2];
         if (kSR) {
           if (out.sr16) quantize16_sr(v, s, rng((uint64_t)blk, offset), packed);
           else quantize16_sr_hw(v, s, rng((uint64_t)blk, offset), packed);
         }
         else     quantize_rn<2>(v, s, packed);
-        if (cols_live && row0 + r < rows) {
+        if (cols_live && r < live_rows) {
           reinterpret_cast<uint2*>(out.codes_r)[blk] = make_uint2(packed[0], packed[1]);
           out.amax_r[blk] = a;
           running_r = fmaxf(running_r, a);
@@ -325,48 +351,48 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, int64_t rows, in
       }
     }
 
-    const int64_t next = tile + gridDim.x;
-    if (next < tiles) fill_mean(next, buf ^ 1);        // its last readers passed the previous barrier
+    uint32_t next_rt = rt, next_ct = ct;
+    advance(next_rt, next_ct);
+    if (tile + gridDim.x < tiles) fill_mean(next_ct, buf ^ 1);        // its last readers passed the previous barrier
     __syncthreads();                                   // staging complete; this tile's stage is free
-    if (tid == 0) {
-      const int64_t ahead = tile + (int64_t)TC::kStages * gridDim.x;
-      if (ahead < tiles) issue(ahead, stage);
-    }
+    if (tid == 0) issue(stage);
 
     // ---- write-out of Qt: out row j owns 64 contiguous code bytes and 8 maxima of this tile ----
-    const int64_t valid_rows = min((int64_t)TC::kRows, rows - row0);            // multiple of 16
+    if (kColsOut) {
+      uint8_t* tile_codes = out.codes_t + (col0 * pitch_t + (row0 >> 1));
+      const bool piece_live = out_piece * 16 < live_rows;
 #pragma unroll
-    for (int k = 0; kColsOut && k < TC::kCols * 8 / kQuantThreads; ++k) {                   // 8-byte pieces: 8 per out row
-      const int i = tid + k * kQuantThreads;
-      const int j = i >> 3, piece = i & 7;
-      const int64_t orow = col0 + j;
-      if (orow < cols && piece * 16 < valid_rows)
-        *reinterpret_cast<uint2*>(out.codes_t + orow * (rows >> 1) + (row0 >> 1) + piece * 8) =
-            *reinterpret_cast<const uint2*>(staging + (j % TC::kColsPerWord) * TC::kCodeArray + (j / TC::kColsPerWord) * TC::kCodePitch + piece * 8);
-    }
-    if (kColsOut && tid < TC::kCols * 2) {
-      const int j = tid & (TC::kCols - 1), h = tid / TC::kCols;                 // half h: row blocks 4h .. 4h+3
-      const int64_t orow = col0 + j;
-      if (orow < cols) {
-        float* dst = out.amax_t + orow * bpc + (row0 >> 4) + 4 * h;
-        float a4[4];
+      for (int k = 0; k < TC::kCols * 8 / kQuantThreads; ++k) {                 // 8-byte pieces: 8 per out row, 32 rows a trip
+        static_assert((kQuantThreads / 8) % TC::kColsPerWord == 0, "the staged array of a thread's pieces does not change");
+        if (piece_live && out_j + 32 * k < live_cols)
+          *reinterpret_cast<uint2*>(tile_codes + (out_off + 32 * k * pitch_t)) =
+              *reinterpret_cast<const uint2*>(staging + out_staged + (32 / TC::kColsPerWord) * TC::kCodePitch * k);
+      }
+      if (tid < TC::kCols * 2) {
+        const int j = tid & (TC::kCols - 1), h = tid / TC::kCols;               // half h: row blocks 4h .. 4h+3
+        if (j < live_cols) {
+          float* dst = out.amax_t + ((col0 + j) * bpc + (row0 >> 4) + 4 * h);
+          float a4[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) a4[k] = s_amax[(4 * h + k) * TC::kCols + j];
-        if (valid_rows == TC::kRows && (bpc & 3) == 0) {
-          *reinterpret_cast<float4*>(dst) = make_float4(a4[0], a4[1], a4[2], a4[3]);
-        } else {
+          for (int k = 0; k < 4; ++k) a4[k] = s_amax[(4 * h + k) * TC::kCols + j];
+          if (live_rows == TC::kRows && (bpc & 3) == 0) {
+            *reinterpret_cast<float4*>(dst) = make_float4(a4[0], a4[1], a4[2], a4[3]);
+          } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) if ((4 * h + k) * 16 < valid_rows) dst[k] = a4[k];
+            for (int k = 0; k < 4; ++k) if ((4 * h + k) * 16 < live_rows) dst[k] = a4[k];
+          }
         }
       }
     }
+    rt = next_rt;
+    ct = next_ct;
     if (++stage == TC::kStages) stage = 0;
   }
   if (s_failed) {
     // loads of this CTA may still be in flight: give each a bounded chance to land before the CTA leaves
     if (tid == 0) {
       int st = stage;
-      for (int64_t t = blockIdx.x + (int64_t)it * gridDim.x, k = 0; t < tiles && k < TC::kStages; t += gridDim.x, ++k) {
+      for (uint32_t t = blockIdx.x + it * gridDim.x, k = 0; t < tiles && k < TC::kStages; t += gridDim.x, ++k) {
         const uint64_t t0 = global_ns();
         while (!mbar_try(&full[st], ((it + k) / TC::kStages) & 1u) && global_ns() - t0 < kWaitLimitNs) {}
         if (++st == TC::kStages) st = 0;
@@ -631,8 +657,7 @@ quantize_small_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int
         const int r = b / blocks_per_row, c = b - r * blocks_per_row;
         float m[16];
         Load16<float>::load(col_mean + (int64_t)c * 16, m);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = __fsub_rn(v[e], m[e]);
+        subtract16(v, m);
       }
       const float a = abs_max16(v);
       uint32_t pk[2];
@@ -823,16 +848,18 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
   const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   if (int32_t rc = make_map(&map, dt, sizeof(T), x, cols, rows, ld * (int64_t)sizeof(T), TC::kCols, TC::kRows, "x", 128))
     return rc;
-  const int64_t tiles = ceil_div(cols, TC::kCols) * ceil_div(rows, TC::kRows);
+  const int64_t col_tiles = ceil_div(cols, TC::kCols), tiles = col_tiles * ceil_div(rows, TC::kRows);
+  if (tiles >= (int64_t)1 << 31) return fail(METIS_ERR_TOO_LARGE, "tensor of more than 2^31 tiles");
   int64_t grid = (int64_t)sm_count() * 3;          // three CTAs of ~63 KiB per SM
   if (grid > tiles) grid = tiles;
   if (out.records && grid > kDualMaxCtas) grid = kDualMaxCtas;
+  const TileWalk walk = {(uint32_t)tiles, (uint32_t)col_tiles, (uint32_t)(grid / col_tiles), (uint32_t)(grid % col_tiles)};
   const bool with_rows = out.codes_r != nullptr, with_cols = out.codes_t != nullptr;
 #define METIS_LAUNCH_TILE(MEAN, SR, ROWS, COLS)                                                             \
   do {                                                                                                      \
     auto kern = quantize_tile_kernel<T, MEAN, SR, ROWS, COLS>;                                              \
     METIS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC::kSmemBytes)); \
-    METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)grid), dim3(kQuantThreads), TC::kSmemBytes, st, map, rows, cols, \
+    METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)grid), dim3(kQuantThreads), TC::kSmemBytes, st, map, walk, rows, cols, \
                                     mean, seed, offset, ctr, out));                                         \
   } while (0)
 #define METIS_LAUNCH_TILE_MS(MEAN, SR)                                  \

@@ -102,10 +102,13 @@ rmsnorm_quantize_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, 
         RawBlock<__nv_bfloat16> graw;
         graw.load(reinterpret_cast<const __nv_bfloat16*>(gamma) + (int64_t)bc * 16);
         const uint32_t gw[8] = {graw.a.x, graw.a.y, graw.a.z, graw.a.w, graw.b.x, graw.b.y, graw.b.z, graw.b.w};
+        const f32x2 rs2 = pack2(rs, rs);
         __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const __nv_bfloat162 n2 = __floats2bfloat162_rn(__fmul_rn(v[j][2 * i], rs), __fmul_rn(v[j][2 * i + 1], rs));
+          float n0, n1;
+          split2(mul2(pack2(v[j][2 * i], v[j][2 * i + 1]), rs2), n0, n1);
+          const __nv_bfloat162 n2 = __floats2bfloat162_rn(n0, n1);
           const __nv_bfloat162 p2 = __hmul2(n2, *reinterpret_cast<const __nv_bfloat162*>(&gw[i]));
           amax2 = __hmax2(amax2, __habs2(p2));
           const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
