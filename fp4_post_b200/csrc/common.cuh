@@ -507,7 +507,8 @@ constexpr int kSmallCtas = 8;                      // portable cluster size
 // Sum of the 16 signed codes of one block, in half units.  prmt looks four codes up at once in the
 // 8-entry magnitude table {0,1,2,3,4,6,8,12}; a selector nibble with bit 3 set yields the sign
 // replica of the table byte, i.e. zero, so the first look-up keeps the positive codes and the second
-// (sign bits flipped) the negative ones.  Byte sums stay below 256, one dp4a adds the four bytes.
+// (sign bits flipped) the negative ones.  Byte sums stay below 49, so their difference plus 48 fits a byte and
+// one dp4a adds the four.
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   uint32_t d;
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
@@ -518,7 +519,7 @@ __device__ __forceinline__ int block_code_sum(uint2 w) {
   const uint32_t nx = w.x ^ 0x88888888u, ny = w.y ^ 0x88888888u;
   const uint32_t pos = prmt(kLo, kHi, w.x) + prmt(kLo, kHi, w.x >> 16) + prmt(kLo, kHi, w.y) + prmt(kLo, kHi, w.y >> 16);
   const uint32_t neg = prmt(kLo, kHi, nx) + prmt(kLo, kHi, nx >> 16) + prmt(kLo, kHi, ny) + prmt(kLo, kHi, ny >> 16);
-  return __dp4a(pos, 0x01010101u, 0u) - __dp4a(neg, 0x01010101u, 0u);
+  return (int)__dp4a(pos + 0x30303030u - neg, 0x01010101u, (uint32_t)-192);
 }
 
 constexpr int64_t kSmallMaxPaddedWords = 16384;    // words of the tiled scale array, zero-filled padding included

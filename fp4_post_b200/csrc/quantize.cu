@@ -426,15 +426,14 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
 }
 
 // ---- pass 2: block maxima -> E4M3 bytes + unit ------------------------------------------------------
-// One thread per group of 4 scale columns (one 128-bit read of maxima, one 32-bit write).
-// For METIS_SF_MMA the loop runs over the padded extent and pads with zero bytes.  blockIdx.y picks
-// the job: the dual quantizer finishes both orientations in one launch.
+// blockIdx.y picks the job: the dual quantizer finishes both orientations in one launch.  For METIS_SF_MMA the
+// walk covers the padded extent and pads with zero bytes.
 struct FinalizeJob {
   const float* amax;  const unsigned int* gmax;  const unsigned int* error;
   int64_t R, sf_cols;
   int32_t sf_layout;
   uint8_t* scales;  float* unit;
-  int32_t bx;                 // threads along a row of groups (a power of two up to the CTA size)
+  int32_t log_tx;             // log2 of the threads along the tiles of a row
   // optional by-product: row_sums[r] = the sum of the quantized values of row r (unit included), from the
   // codes the first pass wrote.  A weight-gradient product needs these sums of its operands when they
   // were centred; here they cost one extra read of codes that are still in L2 instead of a pass of their own.
@@ -447,21 +446,34 @@ struct FinalizeJobs { FinalizeJob job[2]; };
 // E4M3 bytes of 4 neighbouring blocks from their maxima (quant.py:23): RN_e4m3(RN_fp32(s / unit)), two packed
 // conversions.  The division is replaced by a product with RN(1 / unit), which lies within 3 fp32 steps of the
 // correctly rounded quotient; the E4M3 byte of a normal value changes only where the 20 dropped mantissa bits
-// pass 0x80000 (the tie), so a product further than that from a tie converts to the same byte.  The others,
-// everything in E4M3's subnormal range (other tie positions) and NaN take the division itself.
-__device__ __forceinline__ uint32_t scale_bytes4(const float (&a)[4], int live, float unit, float inv_unit) {
-  float ratio[4];
+// pass 0x80000 (the tie), so a product further than that from a tie converts to the same byte.  The others and
+// everything in E4M3's subnormal range (other tie positions) take the division itself; a NaN (of s or of the unit) is
+// a NaN either way.  Whether any of the four needs it is one test: the smallest distance and the smallest product.
+// Returns whether the bytes stand (else: scale_bytes4_exact).
+__device__ __forceinline__ bool scale_bytes4(const float4 a, f32x2 inv_unit2, uint32_t& bytes) {
+  const f32x2 r6 = pack2(0x1.555556p-3f, 0x1.555556p-3f), minus6 = pack2(-6.0f, -6.0f), tiny = pack2(1e-9f, 1e-9f);
+  const f32x2 a2[2] = {pack2(a.x, a.y), pack2(a.z, a.w)};
+  float q[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float s = block_scale_from_amax(a[j]);
-    float q = __fmul_rn(s, inv_unit);
-    const uint32_t low = __float_as_uint(q) & 0xFFFFFu;
-    if (low - 0x7FFF8u <= 16u || !(q >= 0.0157f)) q = __fdiv_rn(s, unit);
-    ratio[j] = j < live ? q : 0.0f;
+  for (int h = 0; h < 2; ++h) {                            // block_scale_from_amax, two at a time
+    const f32x2 q0 = mul2(a2[h], r6);
+    split2(mul2(add2(fma2(fma2(minus6, q0, a2[h]), r6, q0), tiny), inv_unit2), q[2 * h], q[2 * h + 1]);
   }
-  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(ratio[0], ratio[1]), __NV_SATFINITE, __NV_E4M3);
-  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(ratio[2], ratio[3]), __NV_SATFINITE, __NV_E4M3);
-  return lo | (hi << 16);
+  uint32_t nearest = 0xFFFFFFFFu;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) nearest = min(nearest, (__float_as_uint(q[j]) & 0xFFFFFu) - 0x7FFF8u);
+  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), __NV_SATFINITE, __NV_E4M3);
+  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), __NV_SATFINITE, __NV_E4M3);
+  bytes = lo | (hi << 16);
+  return nearest > 16u && fminf(fminf(q[0], q[1]), fminf(q[2], q[3])) >= 0.0157f;
+}
+// Not inlined: four divisions at each of its uses would push the loop out of the instruction cache.
+__device__ __noinline__ uint32_t scale_bytes4_exact(float4 a, float unit) {
+  const float v[4] = {a.x, a.y, a.z, a.w};
+  uint32_t bytes = 0;
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) bytes |= (uint32_t)float_to_e4m3(__fdiv_rn(block_scale_from_amax(v[j]), unit)) << (8 * j);
+  return bytes;
 }
 
 // the four E4M3 bytes of a word as floats (exact)
@@ -472,38 +484,37 @@ __device__ __forceinline__ void e4m3x4_to_float(uint32_t packed, float (&f)[4]) 
   f[0] = l.x; f[1] = l.y; f[2] = h.x; f[3] = h.y;
 }
 
-// Thread (tx, ty) of a bx x by CTA (bx per job) walks the groups tx, tx + bx, ... of the rows ty,
-// ty + by * gridDim.x, ...: no index divisions, and two rows are in flight per thread.
-__global__ void __launch_bounds__(kQuantThreads)
+// A thread finishes one 16-byte piece of the tiled layout at a time: the scales of the rows l, l + 32, l + 64, l + 96 of
+// a 128-row block for 4 scale columns, i.e. four 16-byte reads of maxima and one 16-byte store (row-major scales: four
+// words of four rows).  Two neighbouring lanes take two neighbouring l, the next ones the tiles to the right, so a warp
+// reads runs of up to 256 bytes and stores whole 32-byte sectors.  An item is such a pair of l (8 rows) over the whole
+// row; a CTA takes 64 / tx items at once.  With one 4-column group of two rows per thread, scalar arithmetic and 64-bit
+// index arithmetic this pass took 62 instructions per block and was bound by issue; what counts beside the arithmetic is
+// that edges, padding and divisions stay out of the unrolled path (with them inside it 27 instructions per block and
+// waits for instruction fetch).  Measured at 16384 x 4096, one output / both / both with token sums: 11.2 / 21.0 / 28.2
+// us then, 5.6 / 10.0 / 21.1 now; at 65536 x 4096 32 / 62 / 79 -> 16 / 30 / 67 (the bytes alone take 13 / 26 / 46).
+constexpr int kFinThreads = 128;
+template <bool kSums>                                            // some job of the launch wants row sums (twice the registers)
+__global__ void __launch_bounds__(kFinThreads)
 finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t* __restrict__ offset_ctr) {
-  __shared__ float2 s_sum[kQuantThreads / 32];
+  __shared__ unsigned int s_top[kFinThreads / 32], s_bad[kFinThreads / 32];
+  __shared__ float s_sum[kFinThreads / 32][2][4];
   grid_dependency_wait();
   const FinalizeJob& J = blockIdx.y == 0 ? job0 : job1;
-  const int bx = J.bx, by = kQuantThreads / bx;
-  const int tx = threadIdx.x & (bx - 1), ty = threadIdx.x / bx;
-  const float* __restrict__ amax = J.amax;
-  uint8_t* __restrict__ scales = J.scales;
-  const int64_t R = J.R, sf_cols = J.sf_cols;
-  const bool tiled = J.sf_layout == METIS_SF_MMA;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned int top = 0u, bad = 0u;                 // bits of the largest block maximum (>= 0: they order like the value)
   if (J.records) {
-    __shared__ unsigned int s_top[2];
-    if (threadIdx.x < 32) {                        // one warp reads the few KiB of records (L2) for the CTA
-      const int n = (int)J.records[-1];
-      for (int i = threadIdx.x; i < n; i += 32) {
-        top = max(top, J.records[3 * i + J.which]);
-        bad |= J.records[3 * i + 2];
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-      }
-      if (threadIdx.x == 0) { s_top[0] = top; s_top[1] = bad; }
+    const int n = (int)J.records[-1];
+    for (int i = tid; i < n; i += kFinThreads) {
+      top = max(top, J.records[3 * i + J.which]);
+      bad |= J.records[3 * i + 2];
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (lane == 0) { s_top[warp] = top; s_bad[warp] = bad; }
     __syncthreads();
-    top = s_top[0];
-    bad = s_top[1];
+#pragma unroll
+    for (int w = 0; w < kFinThreads / 32; ++w) { top = max(top, s_top[w]); bad |= s_bad[w]; }
   } else {
     top = *J.gmax;
     bad = *J.error;
@@ -511,100 +522,123 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
   const float smax = block_scale_from_amax(__uint_as_float(top));
   // quant.py:21-22; a pass-1 kernel that gave up on a load raises the error word: publish NaN so that it shows
   const float unit = bad ? __uint_as_float(0x7FC00000u) : __fdiv_rn(smax, 448.0f);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && tid == 0) {
     *J.unit = unit;
     if (offset_ctr && blockIdx.y == 0) *offset_ctr += 1;       // pass 1 of this call has finished: the next call draws fresh bits
   }
-  const int64_t tiles = sf_tiles_per_row(sf_cols * 16);
-  const int groups_per_row = (int)(tiled ? tiles : (sf_cols + 3) / 4);
-  const int64_t R_out = tiled ? ((R + 127) / 128) * 128 : R;
-  const bool vec = (sf_cols & 3) == 0;
-  const int64_t row_step = (int64_t)gridDim.x * by;
-  const bool sums = J.row_sums != nullptr;                       // the host asks for them only when vec holds
-
-  auto load = [&](int64_t r, int g, float (&a)[4]) -> int {       // maxima of group g of row r; returns how many are real
-    a[0] = a[1] = a[2] = a[3] = 0.0f;
-    const int64_t k0 = (int64_t)g * 4;
-    if (r >= R || k0 >= sf_cols) return 0;
-    const float* src = amax + r * sf_cols + k0;
-    if (vec) {
-      const float4 w = *reinterpret_cast<const float4*>(src);
-      a[0] = w.x; a[1] = w.y; a[2] = w.z; a[3] = w.w;
-      return 4;
-    }
-    const int live = (int)(sf_cols - k0 < 4 ? sf_cols - k0 : 4);
-    for (int j = 0; j < live; ++j) a[j] = src[j];
-    return live;
-  };
-  auto store = [&](int64_t r, int g, uint32_t packed, int live) {
-    const int64_t k0 = (int64_t)g * 4;
-    if (tiled) {
-      *reinterpret_cast<uint32_t*>(scales + sf_mma_offset(r, k0, tiles)) = packed;      // padding bytes are zero
-    } else if (vec) {
-      *reinterpret_cast<uint32_t*>(scales + r * sf_cols + k0) = packed;
-    } else {
-      for (int j = 0; j < live; ++j) scales[r * sf_cols + k0 + j] = (uint8_t)(packed >> (8 * j));
-    }
-  };
-  // codes of the 4 blocks of group g of row r, and their sum of code values x scale in half units of `unit`
-  auto load_codes = [&](int64_t r, int g, uint4 (&c)[2]) {
-    const uint4* src = reinterpret_cast<const uint4*>(J.codes + r * sf_cols + (int64_t)g * 4);
-    c[0] = src[0];
-    c[1] = src[1];
-  };
-  auto group_sum = [&](const uint4 (&c)[2], uint32_t packed) -> float {
-    float f[4];
-    e4m3x4_to_float(packed, f);
-    float acc = (float)block_code_sum(make_uint2(c[0].x, c[0].y)) * f[0];
-    acc = fmaf((float)block_code_sum(make_uint2(c[0].z, c[0].w)), f[1], acc);
-    acc = fmaf((float)block_code_sum(make_uint2(c[1].x, c[1].y)), f[2], acc);
-    return fmaf((float)block_code_sum(make_uint2(c[1].z, c[1].w)), f[3], acc);
-  };
   const float inv_unit = __fdiv_rn(1.0f, unit);
-  // the row loop is uniform over the CTA (the reduction below meets at a barrier)
-  for (int64_t r0 = (int64_t)blockIdx.x * by; r0 < R_out; r0 += 2 * row_step) {
-    const int64_t r = r0 + ty, r2 = r + row_step;
-    float sum_a = 0.0f, sum_b = 0.0f;
-    if (r < R_out) {
-      const bool second = r2 < R_out;
-      for (int g = tx; g < groups_per_row; g += bx) {
-        float a[4], b[4];
-        uint4 ca[2], cb[2];
-        // every load of the two rows is issued before the first use
-        const int la = load(r, g, a);
-        const int lb = second ? load(r2, g, b) : 0;
-        if (sums && la) load_codes(r, g, ca);
-        if (sums && lb) load_codes(r2, g, cb);
-        const uint32_t pa = scale_bytes4(a, la, unit, inv_unit);
-        store(r, g, pa, la);
-        if (sums && la) sum_a += group_sum(ca, pa);
-        if (second) {
-          const uint32_t pb = scale_bytes4(b, lb, unit, inv_unit);
-          store(r2, g, pb, lb);
-          if (sums && lb) sum_b += group_sum(cb, pb);
+  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+
+  const bool tiled = J.sf_layout == METIS_SF_MMA;
+  const int64_t R = J.R, sf_cols = J.sf_cols;
+  const int tiles = (int)sf_tiles_per_row(sf_cols * 16);       // padded to whole stages (METIS_SF_MMA)
+  const int groups = tiled ? tiles : (int)((sf_cols + 3) >> 2);
+  const bool vec = (sf_cols & 3) == 0;
+  const bool sums = kSums && J.row_sums != nullptr;              // the host asks for them only when vec holds
+  const int tx = 1 << J.log_tx, per_cta = 64 >> J.log_tx;        // threads along a row, items per CTA
+  const int k_lane = (tid >> 1) & (tx - 1), sub = tid >> (1 + J.log_tx);
+  const int64_t items = ((R + 127) / 128) * 16;
+  const int64_t row_pitch = 32 * sf_cols;                        // between a thread's four rows
+  // the item loop is uniform over the CTA (the sums of a row meet at a barrier)
+  for (int64_t first = (int64_t)blockIdx.x * per_cta; first < items; first += (int64_t)gridDim.x * per_cta) {
+    const int64_t item = first + sub;
+    const bool live = item < items;
+    const int64_t row0 = (item >> 4) * 128 + (item & 15) * 2 + (tid & 1);       // this thread's rows: row0 + 32 c
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const float* src = J.amax + row0 * sf_cols;
+    const uint2* codes = J.codes + row0 * sf_cols;
+    uint8_t* dst = tiled ? J.scales + (item >> 4) * tiles * 512 + ((item & 15) * 2 + (tid & 1)) * 16 : J.scales + row0 * sf_cols;
+    const bool whole = live && (vec || tiled) && row0 + 96 < R;    // all four rows are there: no bounds inside a piece
+    for (int k = k_lane; live && k < groups; k += tx) {
+      if (whole && 4 * k + 4 <= sf_cols) {
+        float4 a[4];
+        uint4 cd[4][2];
+        uint32_t out[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {                             // every load before the first use
+          const float* from = src + c * row_pitch + 4 * k;
+          if (vec) a[c] = *reinterpret_cast<const float4*>(from);
+          else     a[c] = make_float4(from[0], from[1], from[2], from[3]);
+        }
+        if (sums) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint4* w = reinterpret_cast<const uint4*>(codes + c * row_pitch + 4 * k);
+            cd[c][0] = w[0];
+            cd[c][1] = w[1];
+          }
+        }
+        bool stands[4], all = true;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) all &= stands[c] = scale_bytes4(a[c], inv_unit2, out[c]);
+        if (!all) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) if (!stands[c]) out[c] = scale_bytes4_exact(a[c], unit);
+        }
+        if (sums) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float f[4];
+            e4m3x4_to_float(out[c], f);
+            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].x, cd[c][0].y)), f[0], acc[c]);
+            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].z, cd[c][0].w)), f[1], acc[c]);
+            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].x, cd[c][1].y)), f[2], acc[c]);
+            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].z, cd[c][1].w)), f[3], acc[c]);
+          }
+        }
+        if (tiled) {
+          *reinterpret_cast<uint4*>(dst + (int64_t)k * 512) = make_uint4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) *reinterpret_cast<uint32_t*>(dst + c * row_pitch + 4 * k) = out[c];
+        }
+      } else {                                                      // an edge of the tensor, or padding: kept short
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          const int64_t r = row0 + 32 * c;
+          uint32_t word = 0u;
+          if (r < R) {
+#pragma unroll 1
+            for (int j = 0; j < 4 && 4 * (int64_t)k + j < sf_cols; ++j) {
+              const int64_t b = r * sf_cols + 4 * k + j;
+              const uint8_t byte = float_to_e4m3(__fdiv_rn(block_scale_from_amax(J.amax[b]), unit));
+              word |= (uint32_t)byte << (8 * j);
+              if (!tiled) J.scales[b] = byte;
+              if (sums) {
+                const float part = (float)block_code_sum(J.codes[b]) * e4m3_to_float(byte);
+                if (c == 0) acc[0] += part; else if (c == 1) acc[1] += part; else if (c == 2) acc[2] += part; else acc[3] += part;
+              }
+            }
+          }
+          if (tiled) *reinterpret_cast<uint32_t*>(dst + (int64_t)k * 512 + 4 * c) = word;
         }
       }
     }
     if (sums) {
-      // fixed order: lanes of a row by butterfly, then the row's warps one after the other
-      for (int o = (bx < 32 ? bx : 32) >> 1; o > 0; o >>= 1) {
-        sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
-        sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
+      // fixed order: lanes of an item by butterfly, then its warps one after the other
+      for (int o = tx < 16 ? tx : 16; o >= 2; o >>= 1) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
       }
-      if (bx > 32) {
-        const int warp = threadIdx.x >> 5, per_row = bx >> 5;
-        if ((threadIdx.x & 31) == 0) s_sum[warp] = make_float2(sum_a, sum_b);
+      if (tx > 16) {
+        if (lane < 2) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) s_sum[warp][lane][c] = acc[c];
+        }
         __syncthreads();
-        if (tx == 0) {
-          sum_a = sum_b = 0.0f;
-          for (int w = 0; w < per_row; ++w) { sum_a += s_sum[ty * per_row + w].x; sum_b += s_sum[ty * per_row + w].y; }
+        const int warps = tx >> 4;                              // per item
+        if (k_lane == 0) {
+          for (int w = 1; w < warps; ++w) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[c] += s_sum[warp + w][tid & 1][c];
+          }
         }
         __syncthreads();
       }
-      if (tx == 0) {
+      if (live && k_lane == 0) {
         const float half_unit = 0.5f * unit;
-        if (r < R) J.row_sums[r] = sum_a * half_unit;
-        if (r2 < R) J.row_sums[r2] = sum_b * half_unit;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) if (row0 + 32 * c < R) J.row_sums[row0 + 32 * c] = acc[c] * half_unit;
       }
     }
   }
@@ -879,19 +913,18 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
   int64_t blocks = 1;
   for (int j = 0; j < njobs; ++j) {
     FinalizeJob& J = jobs.job[j];
-    const bool tiled = J.sf_layout == METIS_SF_MMA;
-    const int64_t groups = tiled ? sf_tiles_per_row(J.sf_cols * 16) : ceil_div(J.sf_cols, 4);
-    const int64_t rows = tiled ? ceil_div(J.R, 128) * 128 : J.R;
-    int bx = 1;
-    while (bx < groups && bx < kQuantThreads) bx <<= 1;
-    J.bx = bx;
-    const int64_t need = ceil_div(rows, 2 * (kQuantThreads / bx));           // two rows per thread
+    const int64_t groups = J.sf_layout == METIS_SF_MMA ? sf_tiles_per_row(J.sf_cols * 16) : ceil_div(J.sf_cols, 4);
+    J.log_tx = 2;                                             // a warp holds at most 8 rows' lanes of 4 tiles
+    while (J.log_tx < 6 && (1 << J.log_tx) < groups) ++J.log_tx;
+    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16, 64 >> J.log_tx);
     if (need > blocks) blocks = need;
   }
   if (njobs == 1) jobs.job[1] = jobs.job[0];
-  const int64_t cap = (int64_t)sm_count() * 8 / njobs;
+  const bool sums = jobs.job[0].row_sums || jobs.job[1].row_sums;
+  auto kern = sums ? finalize_scales_kernel<true> : finalize_scales_kernel<false>;
+  const int64_t cap = (int64_t)sm_count() * (sums ? 10 : 8) / njobs;     // resident at once: 5 (sums) and 8 per SM
   if (blocks > cap) blocks = ceil_div(blocks, ceil_div(blocks, cap));    // the fewest CTAs that need no more rounds than `cap` would
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, finalize_scales_kernel, dim3((unsigned)blocks, (unsigned)njobs), dim3(kQuantThreads), 0, st,
+  METIS_CUDA_OK(launch_overlapped(kLaunchShort, kern, dim3((unsigned)blocks, (unsigned)njobs), dim3(kFinThreads), 0, st,
                                   jobs.job[0], jobs.job[1], offset_ctr));
   return METIS_OK;
 }

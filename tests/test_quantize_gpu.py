@@ -463,3 +463,24 @@ def test_deferred_scale_pass_writes_what_the_undeferred_call_writes(defer, stoch
     assert torch.equal(qt.token_sums, want_t.token_sums)
     with pytest.raises(ValueError):
         ops.nvfp4_quantize_dual(x, defer="both")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
+@pytest.mark.parametrize("rows,cols", [(16, 16), (1120, 208), (144, 2064), (320, 4112), (2112, 1040)])
+def test_scale_pass_at_the_edges_of_its_walk(rows, cols, layout):
+    """Rows that end inside a 128-row block, scale columns that no group of four and no stage of the GEMM divides
+    (1120 / 16 = 70, 2064 / 16 = 129), several trips along a row (4112 / 64 > 64 tiles), both layouts; the token sums
+    (where rows allow them) against float64 sums of the values the bytes stand for."""
+    x = synthetic(rows, cols, "outliers", rows + cols, torch.float32)
+    x[:, 3] = 0.0                                         # scales in E4M3's subnormal range
+    dev = x.cuda()
+    sums = rows % 64 == 0
+    q, qt = ops.nvfp4_quantize_dual(dev, sf_layout=layout, token_sums=sums)
+    assert_packed_equal(q, x.numpy(), layout, what="row-major")
+    assert_packed_equal(qt, np.ascontiguousarray(x.numpy().T), layout, what="transposed")
+    if sums:
+        want = qt.dequantize(torch.float32).double().sum(1)
+        # fp32 sum of `rows` terms, each exact up to its scale product
+        bound = 2.0 ** -23 * (rows / 16 + 8) * qt.dequantize(torch.float32).double().abs().sum(1) + 1e-30
+        assert bool(((qt.token_sums.double() - want).abs() <= bound).all())
