@@ -38,7 +38,7 @@ struct PanelParams {
   const __nv_bfloat16* yv;  int64_t ldyv;
   const void* s;  int32_t s_is_f32;
   __nv_bfloat16* d_yv;  int64_t ldd;
-  float* block_sums;  unsigned int* ticket;  float* ds;
+  float* block_sums;
   int32_t r;
 };
 
@@ -265,90 +265,134 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
   }
   if constexpr (kDts) {
-    // this CTA's column sums (its four 32-row groups in a fixed order), then the last CTA to arrive adds all
-    // CTAs' sums in CTA order: ds does not depend on timing
+    // this CTA's column sums, its four 32-row groups in a fixed order (lowrank_ds_kernel adds the CTAs')
     for (int c = threadIdx.x; c < p.r; c += kPanelThreads)
       p.block_sums[(int64_t)blockIdx.x * p.r + c] = (s_colsum[c] + s_colsum[256 + c]) + (s_colsum[512 + c] + s_colsum[768 + c]);
-    __threadfence();
-    __syncthreads();
-    __shared__ unsigned int s_last;
-    if (threadIdx.x == 0) s_last = (atomicAdd(p.ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
-    __syncthreads();
-    if (s_last) {
-      __threadfence();
-      for (int c = threadIdx.x; c < p.r; c += kPanelThreads) {
-        float total = 0.0f;
-        for (unsigned b = 0; b < gridDim.x; ++b) total += __ldcg(p.block_sums + (int64_t)b * p.r + c);
-        p.ds[c] = total;
-      }
-      if (threadIdx.x == 0) *p.ticket = 0u;
-    }
   }
 }
 
 // ---- finish kernels -------------------------------------------------------------------------------------------
 
 // d_ts = bf16(sum over splits); d_yv = bf16(d_ts * bf16(s)); per-CTA column sums of bf16(d_ts * y_v)
-// go to block_sums [gridDim.x, r]; the last CTA to finish adds them in block order into ds.
-constexpr int kFinishThreads = 256;
-__global__ void __launch_bounds__(kFinishThreads)
+// go to block_sums [gridDim.x, r], which lowrank_ds_kernel adds into ds.
+// A thread takes four columns of a row and has the partial sums of all splits in flight before it adds them; a CTA
+// takes 512 / r rows at a time and the grid as many CTAs as there are such groups (up to kDtsFinishCtas).  Bound by
+// the read of the partial sums.  The CTAs are small (128 threads of up to 64 registers) because they run beside a
+// weight-gradient product, whose CTA leaves 22 K registers of an SM: CTAs of 256 threads and 128 registers waited
+// for that product to end (58 us in a step of 8192 x 1536 x 8960), and a CTA per 64 rows with one column per thread
+// and one load in flight took 52 us by itself (1120 x 128, 7 splits).
+constexpr int kFinishThreads = 128;
+constexpr int kPanelMaxSplits = 16;
+// v += the partial sums at src of all splits, in split order, eight loads in flight
+__device__ __forceinline__ void add_splits(const float* __restrict__ src, int splits, int64_t split_pitch, float (&v)[4]) {
+  for (int sp0 = 0; sp0 < splits; sp0 += 8) {
+    float4 part[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (sp0 + i < splits) part[i] = *reinterpret_cast<const float4*>(src + (int64_t)(sp0 + i) * split_pitch);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (sp0 + i < splits) { v[0] += part[i].x; v[1] += part[i].y; v[2] += part[i].z; v[3] += part[i].w; }
+  }
+}
+__global__ void __launch_bounds__(kFinishThreads, 7)
 lowrank_dts_finish_kernel(const float* __restrict__ partial, int splits, int64_t M, int r, int64_t ldp,
                           const __nv_bfloat16* __restrict__ yv, int64_t ldyv, const void* __restrict__ s, int s_is_f32,
-                          __nv_bfloat16* __restrict__ d_yv, int64_t ldd, float* __restrict__ block_sums,
-                          unsigned int* __restrict__ ticket, float* __restrict__ ds) {
+                          __nv_bfloat16* __restrict__ d_yv, int64_t ldd, float* __restrict__ block_sums) {
   grid_dependency_wait();
-  // thread (cx, ry): columns cx, cx + 64, ... ; rows ry, ry + 4, ... of this CTA's row range
-  const int cx = threadIdx.x & 63, ry = threadIdx.x >> 6;
-  const int64_t rows_per_cta = (M + gridDim.x - 1) / gridDim.x;
-  const int64_t r_begin = (int64_t)blockIdx.x * rows_per_cta;
-  const int64_t r_end = r_begin + rows_per_cta < M ? r_begin + rows_per_cta : M;
-  __shared__ float s_sum[4][256];
-  for (int c = cx; c < r; c += 64) {
-    const float sc = s_is_f32 ? __bfloat162float(__float2bfloat16_rn(static_cast<const float*>(s)[c]))
-                              : __bfloat162float(static_cast<const __nv_bfloat16*>(s)[c]);
-    float acc = 0.0f;
-    for (int64_t row = r_begin + ry; row < r_end; row += 4) {
-      float v = 0.0f;
-      for (int sp = 0; sp < splits; ++sp) v += partial[((int64_t)sp * M + row) * ldp + c];
-      const float dts = __bfloat162float(__float2bfloat16_rn(v));                   // the product's bf16 output
-      d_yv[row * ldd + c] = __float2bfloat16_rn(dts * sc);
-      acc += __bfloat162float(__float2bfloat16_rn(dts * __bfloat162float(yv[row * ldyv + c])));
+  const int groups = r >> 2, lanes = kFinishThreads / groups;      // threads of a row, rows at a time
+  const int cg = threadIdx.x % groups, ry = threadIdx.x / groups;
+  const int c = cg * 4;
+  __shared__ float4 s_sum[kFinishThreads];                         // [lanes][groups]
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (ry < lanes) {
+    float sc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      sc[j] = s_is_f32 ? __bfloat162float(__float2bfloat16_rn(static_cast<const float*>(s)[c + j]))
+                       : __bfloat162float(static_cast<const __nv_bfloat16*>(s)[c + j]);
+    for (int64_t row = (int64_t)blockIdx.x * lanes + ry; row < M; row += (int64_t)gridDim.x * lanes) {
+      const float* src = partial + row * ldp + c;
+      const uint2 yw = *reinterpret_cast<const uint2*>(yv + row * ldyv + c);
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      add_splits(src, splits, M * ldp, v);
+      const float y[4] = {bf16_lo(yw.x), bf16_hi(yw.x), bf16_lo(yw.y), bf16_hi(yw.y)};
+      __nv_bfloat16 o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float dts = __bfloat162float(__float2bfloat16_rn(v[j]));                   // the product's bf16 output
+        o[j] = __float2bfloat16_rn(dts * sc[j]);
+        acc[j] += __bfloat162float(__float2bfloat16_rn(dts * y[j]));
+      }
+      *reinterpret_cast<uint2*>(d_yv + row * ldd + c) = *reinterpret_cast<const uint2*>(o);
     }
-    s_sum[ry][c] = acc;
+    s_sum[ry * groups + cg] = make_float4(acc[0], acc[1], acc[2], acc[3]);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < r; c += kFinishThreads)
-    block_sums[(int64_t)blockIdx.x * r + c] = (s_sum[0][c] + s_sum[1][c]) + (s_sum[2][c] + s_sum[3][c]);
-  // the last CTA adds the block sums in block order: the result does not depend on timing
-  __threadfence();
-  __syncthreads();
-  __shared__ unsigned int s_last;
-  if (threadIdx.x == 0) s_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    for (int c = threadIdx.x; c < r; c += kFinishThreads) {
-      float total = 0.0f;
-      for (unsigned b = 0; b < gridDim.x; ++b) total += __ldcg(block_sums + (int64_t)b * r + c);
-      ds[c] = total;
+  if (threadIdx.x < groups) {
+    float4 t = s_sum[threadIdx.x];
+    for (int l = 1; l < lanes; ++l) {
+      const float4 u = s_sum[l * groups + threadIdx.x];
+      t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
     }
-    if (threadIdx.x == 0) *ticket = 0u;                // ready for the next call
+    *reinterpret_cast<float4*>(block_sums + (int64_t)blockIdx.x * r + 4 * threadIdx.x) = t;
   }
 }
 
-template <typename TU>
-__global__ void __launch_bounds__(kFinishThreads)
-lowrank_du_finish_kernel(const float* __restrict__ partial, int splits, int64_t N, int r, int64_t ldp,
-                         TU* __restrict__ grad_u, int64_t ldu) {
+// ds[c] = sum of block_sums[b][c] over the blocks, in a fixed order: a warp takes 32 columns and every eighth block, the
+// eight warps' sums are added in order.  A launch of its own: the last CTA of the kernel that writes block_sums could add
+// them too, but the fence and the ticket that takes cost that kernel 12-17 us, and nothing on the step's critical
+// path waits for ds.
+__global__ void __launch_bounds__(256)
+lowrank_ds_kernel(const float* __restrict__ block_sums, int blocks, int r, float* __restrict__ ds) {
   grid_dependency_wait();
-  const int64_t total = N * r;
-  for (int64_t i = (int64_t)blockIdx.x * kFinishThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kFinishThreads) {
-    const int64_t n = i / r;
-    const int c = (int)(i - n * r);
-    float v = 0.0f;
-    for (int sp = 0; sp < splits; ++sp) v += partial[((int64_t)sp * N + n) * ldp + c];
-    if constexpr (sizeof(TU) == 2) grad_u[n * ldu + c] = __float2bfloat16_rn(v);
-    else grad_u[n * ldu + c] = v;
+  __shared__ float s_part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  float acc = 0.0f;
+  if (c < r) {
+#pragma unroll 16
+    for (int b = warp; b < blocks; b += 8) acc += block_sums[(int64_t)b * r + c];
+  }
+  s_part[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0 && c < r) {
+    float total = s_part[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) total += s_part[w][lane];
+    ds[c] = total;
+  }
+}
+
+// Sum over the splits, four columns per thread (`vec`: they can be stored at once).
+template <typename TU>
+__global__ void __launch_bounds__(kFinishThreads, 7)
+lowrank_du_finish_kernel(const float* __restrict__ partial, int splits, int64_t N, int r, int64_t ldp,
+                         TU* __restrict__ grad_u, int64_t ldu, bool vec) {
+  grid_dependency_wait();
+  const uint32_t groups = (uint32_t)(r + 3) >> 2, lanes = kFinishThreads / groups;
+  const uint32_t cg = threadIdx.x % groups, ry = threadIdx.x / groups;
+  if (ry >= lanes) return;
+  const int c = (int)cg * 4;
+  for (int64_t n = (int64_t)blockIdx.x * lanes + ry; n < N; n += (int64_t)gridDim.x * lanes) {
+    const float* src = partial + n * ldp + c;                     // the partial sums fill whole 64-column panels
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    add_splits(src, splits, N * ldp, v);
+    TU* dst = grad_u + n * ldu + c;
+    if constexpr (sizeof(TU) == 2) {
+      __nv_bfloat162 o[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+      if (vec) {
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+      } else {
+        for (int j = 0; j < 4 && c + j < r; ++j) dst[j] = reinterpret_cast<const __nv_bfloat16*>(o)[j];
+      }
+    } else {
+      if (vec) {
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        for (int j = 0; j < 4 && c + j < r; ++j) dst[j] = v[j];
+      }
+    }
   }
 }
 
@@ -368,7 +412,7 @@ static PanelPlan plan_panel(int64_t Mg, int64_t Ng, int64_t Kg) {
   // enough work items to fill the SMs once, never fewer than 8 K stages per split
   int64_t s = device_sm_count() / pl.tiles_m;
   if (s > k_iters / 8) s = k_iters / 8;
-  if (s > 16) s = 16;
+  if (s > kPanelMaxSplits) s = kPanelMaxSplits;
   if (s < 1) s = 1;
   pl.k_per_split = (int)ceil_div(k_iters, s);
   pl.splits = (int)ceil_div(k_iters, pl.k_per_split);
@@ -411,6 +455,16 @@ static int32_t launch_panel(const void* a, bool a_mn, int64_t lda, const void* b
   return METIS_OK;
 }
 
+template <typename TU>
+static int32_t launch_sum(const float* partial, const PanelPlan& pl, int64_t rows, int64_t r, TU* out, int64_t ld, cudaStream_t st) {
+  int64_t blocks = ceil_div(rows, kFinishThreads / ceil_div(r, 4));
+  if (blocks > (int64_t)device_sm_count() * 8) blocks = (int64_t)device_sm_count() * 8;
+  const bool vec = r % 4 == 0 && ld % 4 == 0 && aligned16(out);
+  METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_du_finish_kernel<TU>, dim3((unsigned)blocks), dim3(kFinishThreads), 0, st,
+                                  partial, pl.splits, rows, (int)r, pl.ldp, out, ld, vec));
+  return METIS_OK;
+}
+
 static int32_t check_bf16_matrix(const void* p, int64_t ld, int64_t cols, const char* what) {
   if (!p) return fail(METIS_ERR_BAD_ARGUMENT, "%s is null", what);
   if (!aligned16(p) || ld < cols || ld % 8 != 0) return fail(METIS_ERR_BAD_ALIGNMENT, "%s must be 16-byte aligned with a leading dimension that is a multiple of 8", what);
@@ -418,10 +472,10 @@ static int32_t check_bf16_matrix(const void* p, int64_t ld, int64_t cols, const 
 }
 
 constexpr int kDtsFinishCtas = 256;
-// ticket word + per-CTA column sums: the finish kernel's CTAs, or one per 128 rows when the finish is fused
+// per-CTA column sums: the finish kernel's CTAs, or one per 128 rows when the finish is fused
 static int64_t dts_tail_bytes(int64_t M, int64_t r) {
   const int64_t ctas = ceil_div(M, 128) > kDtsFinishCtas ? ceil_div(M, 128) : kDtsFinishCtas;
-  return 256 + ctas * r * (int64_t)sizeof(float);
+  return ctas * r * (int64_t)sizeof(float);
 }
 
 }  // namespace metis
@@ -446,11 +500,7 @@ extern "C" int32_t metis_bf16_panel_gemm(const void* a, int32_t a_mn_major, int6
   const PanelPlan pl = plan_panel(Mg, Ng, Kg);
   float* partial = static_cast<float*>(workspace);
   if (int32_t rc = launch_panel(a, a_mn_major != 0, lda, b, b_mn_major != 0, ldb, Mg, Ng, Kg, pl, partial, status, st)) return rc;
-  int64_t blocks = ceil_div(Mg * Ng, kFinishThreads);
-  if (blocks > (int64_t)device_sm_count() * 8) blocks = (int64_t)device_sm_count() * 8;
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_du_finish_kernel<float>, dim3((unsigned)blocks), dim3(kFinishThreads), 0, st,
-                                  (const float*)partial, pl.splits, Mg, (int)Ng, pl.ldp, d, ldd));
-  return METIS_OK;
+  return launch_sum(partial, pl, Mg, Ng, d, ldd, st);
 }
 
 extern "C" int64_t metis_lowrank_dts_workspace_bytes(int64_t M, int64_t N, int64_t r) {
@@ -473,23 +523,26 @@ extern "C" int32_t metis_lowrank_dts(const void* g, int64_t ldg, int64_t M, int6
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const PanelPlan pl = plan_panel(M, r, N);
   float* partial = static_cast<float*>(workspace);
-  unsigned int* ticket = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + pl.partial_bytes);
-  float* block_sums = reinterpret_cast<float*>(static_cast<char*>(workspace) + pl.partial_bytes + 256);
-  METIS_CUDA_OK(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), st));
+  float* block_sums = reinterpret_cast<float*>(static_cast<char*>(workspace) + pl.partial_bytes);
+  int64_t blocks;
   // d_ts = G U: G [M, N] is K-major (contraction over its columns), U [N, r] holds the contraction in its rows
   if (pl.splits == 1) {
     // one split (many tokens): d_yv and ds come straight from the accumulator, no partial sums in memory
     PanelParams f = {};
     f.yv = static_cast<const __nv_bfloat16*>(yv); f.ldyv = ldyv; f.s = s; f.s_is_f32 = (s_dtype == METIS_DTYPE_F32);
-    f.d_yv = static_cast<__nv_bfloat16*>(d_yv); f.ldd = ldd; f.block_sums = block_sums; f.ticket = ticket; f.ds = ds; f.r = (int32_t)r;
-    return launch_panel(g, false, ldg, u, true, ldu, M, r, N, pl, partial, status, st, &f);
+    f.d_yv = static_cast<__nv_bfloat16*>(d_yv); f.ldd = ldd; f.block_sums = block_sums; f.r = (int32_t)r;
+    if (int32_t rc = launch_panel(g, false, ldg, u, true, ldu, M, r, N, pl, partial, status, st, &f)) return rc;
+    blocks = pl.tiles_m;
+  } else {
+    if (int32_t rc = launch_panel(g, false, ldg, u, true, ldu, M, r, N, pl, partial, status, st)) return rc;
+    blocks = ceil_div(M, kFinishThreads / (r / 4));
+    if (blocks > kDtsFinishCtas) blocks = kDtsFinishCtas;
+    METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_dts_finish_kernel, dim3((unsigned)blocks), dim3(kFinishThreads), 0, st,
+                                    (const float*)partial, pl.splits, M, (int)r, pl.ldp, static_cast<const __nv_bfloat16*>(yv), ldyv, s,
+                                    (int)(s_dtype == METIS_DTYPE_F32), static_cast<__nv_bfloat16*>(d_yv), ldd, block_sums));
   }
-  if (int32_t rc = launch_panel(g, false, ldg, u, true, ldu, M, r, N, pl, partial, status, st)) return rc;
-  int64_t ctas = ceil_div(M, 64);
-  if (ctas > kDtsFinishCtas) ctas = kDtsFinishCtas;
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_dts_finish_kernel, dim3((unsigned)ctas), dim3(kFinishThreads), 0, st,
-                                  (const float*)partial, pl.splits, M, (int)r, pl.ldp, static_cast<const __nv_bfloat16*>(yv), ldyv, s,
-                                  (int)(s_dtype == METIS_DTYPE_F32), static_cast<__nv_bfloat16*>(d_yv), ldd, block_sums, ticket, ds));
+  METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_ds_kernel, dim3((unsigned)ceil_div(r, 32)), dim3(256), 0, st,
+                                  (const float*)block_sums, (int)blocks, (int)r, ds));
   return METIS_OK;
 }
 
@@ -514,13 +567,6 @@ extern "C" int32_t metis_lowrank_du(const void* g, int64_t ldg, int64_t M, int64
   float* partial = static_cast<float*>(workspace);
   // dU = G^T ts: both operands hold the contraction (the tokens) in their rows
   if (int32_t rc = launch_panel(g, true, ldg, ts, true, ldts, N, r, M, pl, partial, status, st)) return rc;
-  int64_t blocks = ceil_div(N * r, kFinishThreads);
-  if (blocks > (int64_t)device_sm_count() * 8) blocks = (int64_t)device_sm_count() * 8;
-  if (u_dtype == METIS_DTYPE_BF16)
-    METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_du_finish_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(kFinishThreads), 0, st,
-                                    (const float*)partial, pl.splits, N, (int)r, pl.ldp, static_cast<__nv_bfloat16*>(grad_u), ldgu));
-  else
-    METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_du_finish_kernel<float>, dim3((unsigned)blocks), dim3(kFinishThreads), 0, st,
-                                    (const float*)partial, pl.splits, N, (int)r, pl.ldp, static_cast<float*>(grad_u), ldgu));
-  return METIS_OK;
+  if (u_dtype == METIS_DTYPE_BF16) return launch_sum(partial, pl, N, r, static_cast<__nv_bfloat16*>(grad_u), ldgu, st);
+  return launch_sum(partial, pl, N, r, static_cast<float*>(grad_u), ldgu, st);
 }

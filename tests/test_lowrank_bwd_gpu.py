@@ -49,7 +49,8 @@ def test_panel_product_reads_strided_operands_as_they_lie():
     assert rel_l2(got.double().cpu().numpy(), (a.double().t() @ b.double().t()).cpu().numpy()) <= 1e-5
 
 
-@pytest.mark.parametrize("M,N,r", [(256, 384, 32), (512, 1536, 64), (2048, 4096, 128), (1000, 520, 256), (16384, 4096, 128)])
+@pytest.mark.parametrize("M,N,r", [(256, 384, 32), (512, 1536, 64), (2048, 4096, 128), (1000, 520, 256), (16384, 4096, 128),
+                                   (1120, 3584, 96), (33, 1024, 8), (9472, 640, 200)])
 @pytest.mark.parametrize("s_dtype", [torch.bfloat16, torch.float32])
 def test_gradient_through_ulinear_and_the_scaling(M, N, r, s_dtype):
     g = _randn(M, N, seed=M + N)
