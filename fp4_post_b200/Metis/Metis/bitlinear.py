@@ -392,7 +392,13 @@ class LinearLowbitFunction(torch.autograd.Function):
             done = None
             if defer is not None:
                 q, qt, finish = res
-                done = _finish_beside(finish, flat.device)
+
+                def finish_with_tail():
+                    finish()
+                    if defer == "transposed" and qt.token_sums is not None and LinearLowbitFunction._backward_centred():
+                        qt._tail = _add_mean(qt.token_sums, mean, flat.shape[0])     # here it is off every critical path
+                done = _finish_beside(finish_with_tail, flat.device)
+                qt._tail_event = done
             else:
                 q, qt = res
             if getattr(qt, "token_sums", None) is not None:
@@ -685,6 +691,31 @@ def _row_sums(q, rotate=None):
     return cached
 
 
+def _add_mean(sums, mean, rows: int):
+    return torch.add(sums, mean, alpha=float(rows))               # one kernel
+
+
+def _token_tail(x_t, rotate, rows: int):
+    """Qx^T 1 + M mu_x of a transposed activation (one of the two row vectors of a centred weight gradient), once per
+    activation: formed behind the deferred scale pass where there is one, else by whichever branch of the backward
+    comes first; the other waits for its event."""
+    cached = getattr(x_t, "_tail", None)
+    if cached is None:
+        sums = _row_sums(x_t, rotate)
+        if x_t.col_vec is None:
+            return sums
+        cached = x_t._tail = _add_mean(sums, x_t.col_vec, rows)
+        x_t._tail_event = None
+        if cached.is_cuda:
+            x_t._tail_event = torch.cuda.Event()
+            x_t._tail_event.record()
+    elif x_t._tail_event is not None:
+        cur = torch.cuda.current_stream(cached.device)
+        cur.wait_event(x_t._tail_event)
+        cached.record_stream(cur)
+    return cached
+
+
 def _row_sums_beside(op: "PackedOperand"):
     """The token sums of an activation's transposed quantization are needed by the backward pass only: issue
     them on the second stream, after what the current stream has queued so far (the quantization), so that
@@ -701,7 +732,9 @@ def _row_sums_beside(op: "PackedOperand"):
         _row_sums(x_t, op.rotate)
         done = torch.cuda.Event()
         done.record(aux)
-    x_t._row_sums_event = done
+        x_t._row_sums_event = done
+        if x_t.col_vec is not None:
+            _token_tail(x_t, op.rotate, op.q.shape[0])
 
 
 def _packed_dx(da: PackedOperand, wq: PackedOperand, out_dtype, addend=None, side=None, mean_row=None, sm_limit=0):
@@ -714,12 +747,12 @@ def _packed_dx(da: PackedOperand, wq: PackedOperand, out_dtype, addend=None, sid
     if row is None and da.mean is not None:
         row = ops.nvfp4_gemv(w_t, da.mean)
     lowrank = None
+    rank1 = [(None, row)] if row is not None else []
     if side is not None:
         t_acc, u, extra = side
         lowrank = (t_acc, u)
         if extra is not None:
-            row = extra if row is None else row + extra
-    rank1 = [(None, row)] if row is not None else []
+            rank1.append((None, extra))                     # the epilogue adds both rows
     return _packed_matmul(da.rowmajor(), w_t, rank1=rank1, lowrank=lowrank, c=addend, out_dtype=out_dtype, sm_limit=sm_limit)
 
 
@@ -736,10 +769,7 @@ def _packed_dw(da: PackedOperand, xa: PackedOperand, M: int, out_dtype=torch.flo
     if mu_x is not None:
         rank1.append((_row_sums(d_t, da.rotate), mu_x))
     if mu_d is not None:
-        tail = _row_sums(x_t, xa.rotate)
-        if mu_x is not None:
-            tail = torch.add(tail, mu_x, alpha=float(M))          # one kernel: Qx^T 1 + M mu_x
-        rank1.append((mu_d, tail))
+        rank1.append((mu_d, _token_tail(x_t, xa.rotate, M)))
     # rotated operands: (H s)^T (H s) = 16 I
     return ops.nvfp4_gemm(d_t, x_t, rank1=rank1, out_dtype=out_dtype, sm_limit=sm_limit, alpha=1.0 / 16 if da.rotate is not None else 1.0)
 
@@ -946,6 +976,7 @@ class MetisFusedFunction(torch.autograd.Function):
         def low_rank_branch(before_weight_gradient=None):
             # ulinear: plain linear on ts = s . yv; vlinear: quantized backward with grad_output = d_yv
             v_t = u_side = None
+            d_yv_mean = []
             if fuse_dx:
                 # operand of the bf16 side product of the fused dX launch; it needs nothing of this pass
                 v_t = vq.transposed()
@@ -957,8 +988,11 @@ class MetisFusedFunction(torch.autograd.Function):
                 ts = ops.lowrank_scale(yv, s, one, one)
                 out_dtype = u_weight.dtype if u_weight.dtype in (torch.bfloat16, torch.float32) else torch.float32
                 grad_u = ops.lowrank_du(g, ts, out_dtype=out_dtype).to(u_weight.dtype)
-                d_yv, ds32 = ops.lowrank_dts(g, u_weight.detach().to(torch.bfloat16), yv, s)
-                grad_s = ds32.to(s.dtype)
+                # ds in s's dtype, and the column mean of d_yv that its quantization starts from, out of the same launches
+                ds_dtype = s.dtype if s.dtype in (torch.bfloat16, torch.float32) else torch.float32
+                d_yv, grad_s, *d_yv_mean = ops.lowrank_dts(g, u_weight.detach().to(torch.bfloat16), yv, s, ds_dtype=ds_dtype,
+                                                           want_mean=centred)
+                grad_s = grad_s.to(s.dtype)
             else:
                 ts = yv * s.to(act)
                 u = u_weight.to(act)
@@ -966,7 +1000,7 @@ class MetisFusedFunction(torch.autograd.Function):
                 d_ts = g @ u                                                            # [M, r]
                 grad_s = (d_ts * yv).sum(dim=0).to(s.dtype)
                 d_yv = d_ts * s.to(act)
-            dv = F._pack_centred(d_yv, quantizer, centred, both=True)
+            dv = F._pack_centred(d_yv, quantizer, centred, both=True, fresh_mean=d_yv_mean[0] if d_yv_mean else None)
             side = None
             if fuse_dx:
                 side = (u_side, ops.nvfp4_gemv(v_t, dv.mean) if dv.mean is not None else None)
@@ -994,8 +1028,8 @@ class MetisFusedFunction(torch.autograd.Function):
         def side_operand(dv, dg):
             # D^v in the units the fused dX launch accumulates in.  e2m1 x e4m3 is exact in bf16; the ratio of the
             # two products' units goes into T, rounded once to bf16 (the unfused dX_v would be rounded there too).
-            ratio = (dv.q.unit * vq.transposed().unit) / (dg.rowmajor().unit * rq.transposed().unit)
-            return ops.nvfp4_dequantize(dv.q, torch.bfloat16, add_mean=False, unit=ratio)
+            return ops.nvfp4_dequantize_ratio(dv.q, torch.bfloat16, dv.q.unit, vq.transposed().unit,
+                                              dg.rowmajor().unit, rq.transposed().unit)
 
         mean_row = t_acc = None
         concurrent = MetisFusedFunction.concurrent_branches and g.is_cuda

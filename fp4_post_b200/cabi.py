@@ -26,13 +26,13 @@ STATUS_TEXT = {
 EXPORTS = (
     "metis_query", "metis_last_error_string", "metis_nvfp4_sf_bytes",
     "metis_nvfp4_quantize_workspace_bytes", "metis_nvfp4_quantize", "metis_rmsnorm_nvfp4_quantize",
-    "metis_nvfp4_dequantize", "metis_col_mean_workspace_bytes", "metis_col_mean", "metis_nvfp4_gemv",
+    "metis_nvfp4_dequantize", "metis_nvfp4_dequantize_ratio", "metis_col_mean_workspace_bytes", "metis_col_mean", "metis_nvfp4_gemv",
     "metis_nvfp4_gemm", "metis_nvfp4_quantize_static", "metis_nvfp4_gemm_workspace_bytes",
     "metis_lowrank_scale",
     "metis_nvfp4_quantize_dual_workspace_bytes", "metis_nvfp4_quantize_dual", "metis_nvfp4_quantize_dual_finish",
     "metis_rmsnorm_mean_workspace_bytes", "metis_rmsnorm_mean",
     "metis_bf16_panel_gemm_workspace_bytes", "metis_bf16_panel_gemm",
-    "metis_lowrank_dts_workspace_bytes", "metis_lowrank_dts", "metis_lowrank_du_workspace_bytes", "metis_lowrank_du",
+    "metis_lowrank_dts_workspace_bytes", "metis_lowrank_dts", "metis_lowrank_dts_mean", "metis_lowrank_du_workspace_bytes", "metis_lowrank_du",
 )
 
 
@@ -100,6 +100,8 @@ def lib() -> C.CDLL:
     L.metis_rmsnorm_mean.restype = i32
     L.metis_nvfp4_dequantize.argtypes = [vp, vp, vp, i32, i64, i64, vp, vp, i32, i64, vp]
     L.metis_nvfp4_dequantize.restype = i32
+    L.metis_nvfp4_dequantize_ratio.argtypes = [vp, vp, vp, vp, vp, vp, i32, i64, i64, vp, i32, i64, vp]
+    L.metis_nvfp4_dequantize_ratio.restype = i32
     L.metis_col_mean_workspace_bytes.argtypes = [i64, i64]
     L.metis_col_mean_workspace_bytes.restype = i64
     L.metis_col_mean.argtypes = [vp, i32, i64, i64, i64, vp, vp, i64, vp]
@@ -117,6 +119,8 @@ def lib() -> C.CDLL:
     L.metis_bf16_panel_gemm.restype = i32
     L.metis_lowrank_dts.argtypes = [vp, i64, i64, i64, vp, i64, i64, vp, i64, vp, i32, vp, i64, vp, vp, i64, vp, vp]
     L.metis_lowrank_dts.restype = i32
+    L.metis_lowrank_dts_mean.argtypes = [vp, i64, i64, i64, vp, i64, i64, vp, i64, vp, i32, vp, i64, vp, i32, vp, vp, i64, vp, vp]
+    L.metis_lowrank_dts_mean.restype = i32
     L.metis_lowrank_du.argtypes = [vp, i64, i64, i64, vp, i64, i64, vp, i32, i64, vp, i64, vp, vp]
     L.metis_lowrank_du.restype = i32
     L.metis_nvfp4_gemm_workspace_bytes.argtypes = [i64, i64, i64]

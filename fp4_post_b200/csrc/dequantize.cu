@@ -11,20 +11,29 @@ __device__ __forceinline__ float scale_at(const uint8_t* scales, int32_t sf_layo
   return e4m3_to_float(__ldg(scales + off));
 }
 
+// The unit the values are expressed in: *u0, or (*u0 * *u1) / (*d0 * *d1) (a ratio of two products' units, formed here
+// instead of by three one-element kernels in front of this one).
+struct UnitPtrs {
+  const float* u0;  const float* u1;  const float* d0;  const float* d1;
+};
+
 // One thread per 8 elements (4 code bytes).
 template <typename TO>
 __global__ void __launch_bounds__(256)
 dequantize_kernel(const uint32_t* __restrict__ codes, const uint8_t* __restrict__ scales,
-                  const float* __restrict__ unit_ptr, int32_t sf_layout, int64_t R, int64_t C,
+                  const UnitPtrs units, int32_t sf_layout, int64_t R, int64_t C,
                   const float* __restrict__ add_row_vec, TO* __restrict__ out, int64_t ld) {
   grid_dependency_wait();
-  const float unit = __ldg(unit_ptr);
+  float unit = __ldg(units.u0);
+  if (units.u1) unit = __fdiv_rn(__fmul_rn(unit, __ldg(units.u1)), __fmul_rn(__ldg(units.d0), __ldg(units.d1)));
   const int64_t chunks_per_row = C >> 3;
   const int64_t total = R * chunks_per_row;
+  const bool small = total < ((int64_t)1 << 31);
   const int64_t sf_cols = C >> 4;
   const int64_t tiles = sf_tiles_per_row(C);
   for (int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x; c < total; c += (int64_t)gridDim.x * 256) {
-    const int64_t r = c / chunks_per_row;
+    // 32-bit index arithmetic where it fits (a 64-bit division is a subroutine of ~100 instructions)
+    const int64_t r = small ? (int64_t)((uint32_t)c / (uint32_t)chunks_per_row) : c / chunks_per_row;
     const int64_t ch = c - r * chunks_per_row;
     const uint32_t w = __ldg(codes + c);
     // value = e2m1 * (e4m3 * unit): the same two roundings as quant.py:23-35
@@ -364,11 +373,9 @@ extern "C" int32_t metis_lowrank_scale(const void* yv, int64_t M, int64_t r, int
   return METIS_OK;
 }
 
-extern "C" int32_t metis_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales, const float* unit,
-                                          int32_t sf_layout, int64_t R, int64_t C,
-                                          const float* add_row_vec, void* out, int32_t out_dtype,
-                                          int64_t ld, void* stream) {
-  if (!codes || !scales || !unit || !out) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
+static int32_t dequantize(const uint8_t* codes, const uint8_t* scales, const UnitPtrs unit, int32_t sf_layout, int64_t R, int64_t C,
+                          const float* add_row_vec, void* out, int32_t out_dtype, int64_t ld, void* stream) {
+  if (!codes || !scales || !unit.u0 || !out) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
   if (R <= 0 || C <= 0 || C % 16 != 0) return fail(METIS_ERR_BAD_SHAPE, "bad shape [%lld, %lld]", (long long)R, (long long)C);
   if (sf_layout != METIS_SF_ROWMAJOR && sf_layout != METIS_SF_MMA) return fail(METIS_ERR_BAD_ARGUMENT, "unknown sf_layout %d", sf_layout);
   if (out_dtype != METIS_DTYPE_BF16 && out_dtype != METIS_DTYPE_F32) return fail(METIS_ERR_BAD_ARGUMENT, "unknown out_dtype %d", out_dtype);
@@ -386,6 +393,20 @@ extern "C" int32_t metis_nvfp4_dequantize(const uint8_t* codes, const uint8_t* s
     launch_overlapped(kLaunchShort, dequantize_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, st, c32, scales, unit, sf_layout, R, C, add_row_vec, static_cast<float*>(out), ld);
   METIS_CUDA_OK(cudaGetLastError());
   return METIS_OK;
+}
+
+extern "C" int32_t metis_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales, const float* unit,
+                                          int32_t sf_layout, int64_t R, int64_t C,
+                                          const float* add_row_vec, void* out, int32_t out_dtype,
+                                          int64_t ld, void* stream) {
+  return dequantize(codes, scales, UnitPtrs{unit, nullptr, nullptr, nullptr}, sf_layout, R, C, add_row_vec, out, out_dtype, ld, stream);
+}
+
+extern "C" int32_t metis_nvfp4_dequantize_ratio(const uint8_t* codes, const uint8_t* scales, const float* unit0, const float* unit1,
+                                                const float* over0, const float* over1, int32_t sf_layout, int64_t R, int64_t C,
+                                                void* out, int32_t out_dtype, int64_t ld, void* stream) {
+  if (!unit1 || !over0 || !over1) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
+  return dequantize(codes, scales, UnitPtrs{unit0, unit1, over0, over1}, sf_layout, R, C, nullptr, out, out_dtype, ld, stream);
 }
 
 extern "C" int32_t metis_nvfp4_gemv(const uint8_t* codes, const uint8_t* scales, const float* unit,

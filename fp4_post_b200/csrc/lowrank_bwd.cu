@@ -34,7 +34,8 @@ struct PanelParams {
   int32_t splits, k_per_split;      // K stages per split
   float* partial;  int64_t ldp;     // [splits, Mg, ldp] fp32
   int32_t* status;
-  // fused finish of d_ts = G U (one split only): d_yv, and the column sums of bf16(d_ts * y_v) for ds
+  // fused finish of d_ts = G U (one split only): d_yv, and per CTA the column sums of bf16(d_ts * y_v) for ds, then
+  // those of d_yv for its mean: block_sums [tiles, 2, r]
   const __nv_bfloat16* yv;  int64_t ldyv;
   const void* s;  int32_t s_is_f32;
   __nv_bfloat16* d_yv;  int64_t ldd;
@@ -43,7 +44,7 @@ struct PanelParams {
 };
 
 static inline int panel_stage_bytes(int bn) { return kPanelABytes + bn * 128; }
-static inline int panel_smem_bytes(int bn, int stages) { return stages * panel_stage_bytes(bn) + 1024 + 256 + 4 * 256 * 4; }
+static inline int panel_smem_bytes(int bn, int stages) { return stages * panel_stage_bytes(bn) + 1024 + 256 + 2 * 4 * 256 * 4; }
 
 // Column sums of a 32 x 32 block held one row per lane: after five exchange-and-add steps lane l holds
 // the sum of column l (31 shuffles instead of 160).
@@ -74,7 +75,7 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   uint64_t* drain = bars + 2 * p.stages + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * p.stages + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_colsum = reinterpret_cast<float*>(smem + p.stages * stage_bytes + 256);     // [4][256], fused finish only
+  float* s_colsum = reinterpret_cast<float*>(smem + p.stages * stage_bytes + 256);     // [2][4][256], fused finish only
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -208,7 +209,7 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               }
             }
             tc_wait_ld(acc);
-            float prod[32];
+            float prod[32], dyv[32];
             uint32_t ow[16];
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
@@ -226,6 +227,8 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
               const uint32_t pw = *reinterpret_cast<const uint32_t*>(&p2);
               prod[i] = live ? bf16_lo(pw) : 0.0f;
               prod[i + 1] = live ? bf16_hi(pw) : 0.0f;
+              dyv[i] = live ? bf16_lo(ow[i >> 1]) : 0.0f;
+              dyv[i + 1] = live ? bf16_hi(ow[i >> 1]) : 0.0f;
             }
             if (live) {
 #pragma unroll
@@ -234,6 +237,7 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                   reinterpret_cast<uint4*>(p.d_yv + row * p.ldd + ch * 32)[i] = make_uint4(ow[4 * i], ow[4 * i + 1], ow[4 * i + 2], ow[4 * i + 3]);
             }
             s_colsum[q * 256 + ch * 32 + lane] = column_sums32(prod, lane);
+            s_colsum[1024 + q * 256 + ch * 32 + lane] = column_sums32(dyv, lane);
           }
         } else {
           float* dst = p.partial + ((int64_t)split * p.Mg + row) * p.ldp;
@@ -266,15 +270,20 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   }
   if constexpr (kDts) {
     // this CTA's column sums, its four 32-row groups in a fixed order (lowrank_ds_kernel adds the CTAs')
-    for (int c = threadIdx.x; c < p.r; c += kPanelThreads)
-      p.block_sums[(int64_t)blockIdx.x * p.r + c] = (s_colsum[c] + s_colsum[256 + c]) + (s_colsum[512 + c] + s_colsum[768 + c]);
+    for (int c = threadIdx.x; c < p.r; c += kPanelThreads) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float* part = s_colsum + 1024 * k + c;
+        p.block_sums[((int64_t)blockIdx.x * 2 + k) * p.r + c] = (part[0] + part[256]) + (part[512] + part[768]);
+      }
+    }
   }
 }
 
 // ---- finish kernels -------------------------------------------------------------------------------------------
 
-// d_ts = bf16(sum over splits); d_yv = bf16(d_ts * bf16(s)); per-CTA column sums of bf16(d_ts * y_v)
-// go to block_sums [gridDim.x, r], which lowrank_ds_kernel adds into ds.
+// d_ts = bf16(sum over splits); d_yv = bf16(d_ts * bf16(s)); per-CTA column sums of bf16(d_ts * y_v) and of d_yv
+// go to block_sums [gridDim.x, 2, r], which lowrank_ds_kernel adds into ds and the column mean of d_yv.
 // A thread takes four columns of a row and has the partial sums of all splits in flight before it adds them; a CTA
 // takes 512 / r rows at a time and the grid as many CTAs as there are such groups (up to kDtsFinishCtas).  Bound by
 // the read of the partial sums.  The CTAs are small (128 threads of up to 64 registers) because they run beside a
@@ -303,8 +312,8 @@ lowrank_dts_finish_kernel(const float* __restrict__ partial, int splits, int64_t
   const int groups = r >> 2, lanes = kFinishThreads / groups;      // threads of a row, rows at a time
   const int cg = threadIdx.x % groups, ry = threadIdx.x / groups;
   const int c = cg * 4;
-  __shared__ float4 s_sum[kFinishThreads];                         // [lanes][groups]
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  __shared__ float4 s_sum[2][kFinishThreads];                      // [lanes][groups]
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc_o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (ry < lanes) {
     float sc[4];
 #pragma unroll
@@ -323,36 +332,40 @@ lowrank_dts_finish_kernel(const float* __restrict__ partial, int splits, int64_t
         const float dts = __bfloat162float(__float2bfloat16_rn(v[j]));                   // the product's bf16 output
         o[j] = __float2bfloat16_rn(dts * sc[j]);
         acc[j] += __bfloat162float(__float2bfloat16_rn(dts * y[j]));
+        acc_o[j] += __bfloat162float(o[j]);
       }
       *reinterpret_cast<uint2*>(d_yv + row * ldd + c) = *reinterpret_cast<const uint2*>(o);
     }
-    s_sum[ry * groups + cg] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    s_sum[0][ry * groups + cg] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    s_sum[1][ry * groups + cg] = make_float4(acc_o[0], acc_o[1], acc_o[2], acc_o[3]);
   }
   __syncthreads();
-  if (threadIdx.x < groups) {
-    float4 t = s_sum[threadIdx.x];
+  for (int i = threadIdx.x; i < 2 * groups; i += kFinishThreads) {
+    const int k = i >= groups, col = i - k * groups;
+    float4 t = s_sum[k][col];
     for (int l = 1; l < lanes; ++l) {
-      const float4 u = s_sum[l * groups + threadIdx.x];
+      const float4 u = s_sum[k][l * groups + col];
       t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
     }
-    *reinterpret_cast<float4*>(block_sums + (int64_t)blockIdx.x * r + 4 * threadIdx.x) = t;
+    *reinterpret_cast<float4*>(block_sums + ((int64_t)blockIdx.x * 2 + k) * r + 4 * col) = t;
   }
 }
 
-// ds[c] = sum of block_sums[b][c] over the blocks, in a fixed order: a warp takes 32 columns and every eighth block, the
-// eight warps' sums are added in order.  A launch of its own: the last CTA of the kernel that writes block_sums could add
-// them too, but the fence and the ticket that takes cost that kernel 12-17 us, and nothing on the step's critical
-// path waits for ds.
+// ds[c] (blockIdx.y 0) and the column mean of d_yv (1): sums of block_sums[b][y][c] over the blocks, in a fixed order: a
+// warp takes 32 columns and every eighth block, the eight warps' sums are added in order.  A launch of its own: the last
+// CTA of the kernel that writes block_sums could add them too, but the fence and the ticket that takes cost that
+// kernel 12-17 us.  The mean replaces a pass over d_yv of two launches (8 us of the step's critical chain).
+template <typename TS>
 __global__ void __launch_bounds__(256)
-lowrank_ds_kernel(const float* __restrict__ block_sums, int blocks, int r, float* __restrict__ ds) {
+lowrank_ds_kernel(const float* __restrict__ block_sums, int blocks, int r, float rows, TS* __restrict__ ds, float* __restrict__ mean) {
   grid_dependency_wait();
   __shared__ float s_part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  const int c = blockIdx.x * 32 + lane, y = blockIdx.y;
   float acc = 0.0f;
   if (c < r) {
 #pragma unroll 16
-    for (int b = warp; b < blocks; b += 8) acc += block_sums[(int64_t)b * r + c];
+    for (int b = warp; b < blocks; b += 8) acc += block_sums[((int64_t)b * 2 + y) * r + c];
   }
   s_part[warp][lane] = acc;
   __syncthreads();
@@ -360,7 +373,9 @@ lowrank_ds_kernel(const float* __restrict__ block_sums, int blocks, int r, float
     float total = s_part[0][lane];
 #pragma unroll
     for (int w = 1; w < 8; ++w) total += s_part[w][lane];
-    ds[c] = total;
+    if (y == 1) mean[c] = __fdiv_rn(total, rows);
+    else if constexpr (sizeof(TS) == 2) ds[c] = __float2bfloat16_rn(total);
+    else ds[c] = total;
   }
 }
 
@@ -475,7 +490,7 @@ constexpr int kDtsFinishCtas = 256;
 // per-CTA column sums: the finish kernel's CTAs, or one per 128 rows when the finish is fused
 static int64_t dts_tail_bytes(int64_t M, int64_t r) {
   const int64_t ctas = ceil_div(M, 128) > kDtsFinishCtas ? ceil_div(M, 128) : kDtsFinishCtas;
-  return ctas * r * (int64_t)sizeof(float);
+  return 2 * ctas * r * (int64_t)sizeof(float);
 }
 
 }  // namespace metis
@@ -508,9 +523,11 @@ extern "C" int64_t metis_lowrank_dts_workspace_bytes(int64_t M, int64_t N, int64
   return plan_panel(M, r, N).partial_bytes + dts_tail_bytes(M, r);
 }
 
-extern "C" int32_t metis_lowrank_dts(const void* g, int64_t ldg, int64_t M, int64_t N, const void* u, int64_t ldu, int64_t r,
-                                     const void* yv, int64_t ldyv, const void* s, int32_t s_dtype, void* d_yv, int64_t ldd,
-                                     float* ds, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
+extern "C" int32_t metis_lowrank_dts_mean(const void* g, int64_t ldg, int64_t M, int64_t N, const void* u, int64_t ldu, int64_t r,
+                                          const void* yv, int64_t ldyv, const void* s, int32_t s_dtype, void* d_yv, int64_t ldd,
+                                          void* ds, int32_t ds_dtype, float* d_yv_mean, void* workspace, int64_t workspace_bytes,
+                                          int32_t* status, void* stream) {
+  if (ds_dtype != METIS_DTYPE_BF16 && ds_dtype != METIS_DTYPE_F32) return fail(METIS_ERR_BAD_ARGUMENT, "unknown ds_dtype %d", ds_dtype);
   if (M <= 0 || N <= 0 || r <= 0) return fail(METIS_ERR_BAD_SHAPE, "empty product %lld x %lld x %lld", (long long)M, (long long)N, (long long)r);
   if (r > 256 || r % 8 != 0 || N % 8 != 0) return fail(METIS_ERR_BAD_SHAPE, "rank %lld must be a multiple of 8 up to 256 and N = %lld a multiple of 8", (long long)r, (long long)N);
   if (int32_t rc = check_bf16_matrix(g, ldg, N, "g")) return rc;
@@ -541,9 +558,21 @@ extern "C" int32_t metis_lowrank_dts(const void* g, int64_t ldg, int64_t M, int6
                                     (const float*)partial, pl.splits, M, (int)r, pl.ldp, static_cast<const __nv_bfloat16*>(yv), ldyv, s,
                                     (int)(s_dtype == METIS_DTYPE_F32), static_cast<__nv_bfloat16*>(d_yv), ldd, block_sums));
   }
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_ds_kernel, dim3((unsigned)ceil_div(r, 32)), dim3(256), 0, st,
-                                  (const float*)block_sums, (int)blocks, (int)r, ds));
+  const dim3 grid((unsigned)ceil_div(r, 32), d_yv_mean ? 2 : 1);
+  if (ds_dtype == METIS_DTYPE_BF16)
+    METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_ds_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const float*)block_sums,
+                                    (int)blocks, (int)r, (float)M, static_cast<__nv_bfloat16*>(ds), d_yv_mean));
+  else
+    METIS_CUDA_OK(launch_overlapped(kLaunchShort, lowrank_ds_kernel<float>, grid, dim3(256), 0, st, (const float*)block_sums,
+                                    (int)blocks, (int)r, (float)M, static_cast<float*>(ds), d_yv_mean));
   return METIS_OK;
+}
+
+extern "C" int32_t metis_lowrank_dts(const void* g, int64_t ldg, int64_t M, int64_t N, const void* u, int64_t ldu, int64_t r,
+                                     const void* yv, int64_t ldyv, const void* s, int32_t s_dtype, void* d_yv, int64_t ldd,
+                                     float* ds, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
+  return metis_lowrank_dts_mean(g, ldg, M, N, u, ldu, r, yv, ldyv, s, s_dtype, d_yv, ldd, ds, METIS_DTYPE_F32, nullptr, workspace,
+                                workspace_bytes, status, stream);
 }
 
 extern "C" int64_t metis_lowrank_du_workspace_bytes(int64_t M, int64_t N, int64_t r) {

@@ -332,6 +332,20 @@ def nvfp4_dequantize(q: NVFP4Tensor, dtype: torch.dtype = torch.float32, add_mea
     return out
 
 
+def nvfp4_dequantize_ratio(q: NVFP4Tensor, dtype: torch.dtype, unit0, unit1, over0, over1) -> torch.Tensor:
+    """Dense [R, C] tensor of q with (unit0 * unit1) / (over0 * over1) in place of its unit (device fp32 [1] each); the
+    mean vectors of q are left out."""
+    R, Cc = q.shape
+    with _on_device(q.device):
+        out = torch.empty((R, Cc), dtype=dtype, device=q.device)
+        rc = cabi.lib().metis_nvfp4_dequantize_ratio(q.codes.data_ptr(), q.scales.data_ptr(), unit0.data_ptr(), unit1.data_ptr(),
+                                                     over0.data_ptr(), over1.data_ptr(), q.sf_layout, R, Cc, out.data_ptr(),
+                                                     _DTYPES[dtype], out.stride(0), _stream())
+    cabi.check(rc, "metis_nvfp4_dequantize_ratio")
+    LAUNCHES["dequantize"] += 1
+    return out
+
+
 def nvfp4_gemv(q: NVFP4Tensor, v: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[r] = sum_c v[c] * value(q)[r, c] (v None: row sums), fp32; the mean vectors of q are ignored."""
     R, Cc = q.shape
@@ -468,9 +482,11 @@ def bf16_panel_gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = Fals
     return out
 
 
-def lowrank_dts(g: torch.Tensor, u: torch.Tensor, yv: torch.Tensor, s: torch.Tensor, status: Optional[torch.Tensor] = None):
+def lowrank_dts(g: torch.Tensor, u: torch.Tensor, yv: torch.Tensor, s: torch.Tensor, status: Optional[torch.Tensor] = None,
+                *, ds_dtype: torch.dtype = torch.float32, want_mean: bool = False):
     """(d_yv, ds) of the low-rank branch from one pass over g [M, N]: d_ts = bf16(g @ u), d_yv = bf16(d_ts * s),
-    ds = sum over rows of bf16(d_ts * yv) in fp32.  u [N, r], yv [M, r] bf16; s [r] bf16 or fp32."""
+    ds = sum over rows of bf16(d_ts * yv), summed in fp32 and returned in ds_dtype.  u [N, r], yv [M, r] bf16; s [r]
+    bf16 or fp32.  want_mean: a third value, the column mean of d_yv (fp32 [r])."""
     g, u, yv = _bf16_rows(g, "g"), _bf16_rows(u, "u"), _bf16_rows(yv, "yv")
     M, N = g.shape
     r = u.shape[1]
@@ -482,14 +498,15 @@ def lowrank_dts(g: torch.Tensor, u: torch.Tensor, yv: torch.Tensor, s: torch.Ten
     L = cabi.lib()
     with _on_device(g.device):
         d_yv = torch.empty((M, r), dtype=torch.bfloat16, device=g.device)
-        ds = torch.empty(r, dtype=torch.float32, device=g.device)
+        ds = torch.empty(r, dtype=ds_dtype, device=g.device)
+        mean = torch.empty(r, dtype=torch.float32, device=g.device) if want_mean else None
         ws = torch.empty(L.metis_lowrank_dts_workspace_bytes(M, N, r), dtype=torch.uint8, device=g.device)
-        rc = L.metis_lowrank_dts(g.data_ptr(), g.stride(0), M, N, u.data_ptr(), u.stride(0), r, yv.data_ptr(), yv.stride(0),
-                                 s.data_ptr(), _dtype_code(s, "s"), d_yv.data_ptr(), d_yv.stride(0), ds.data_ptr(),
-                                 ws.data_ptr(), ws.numel(), _ptr(status), _stream())
-    cabi.check(rc, "metis_lowrank_dts")
+        rc = L.metis_lowrank_dts_mean(g.data_ptr(), g.stride(0), M, N, u.data_ptr(), u.stride(0), r, yv.data_ptr(), yv.stride(0),
+                                      s.data_ptr(), _dtype_code(s, "s"), d_yv.data_ptr(), d_yv.stride(0), ds.data_ptr(),
+                                      _DTYPES[ds_dtype], _ptr(mean), ws.data_ptr(), ws.numel(), _ptr(status), _stream())
+    cabi.check(rc, "metis_lowrank_dts_mean")
     LAUNCHES["lowrank_bwd"] += 2
-    return d_yv, ds
+    return (d_yv, ds, mean) if want_mean else (d_yv, ds)
 
 
 def lowrank_du(g: torch.Tensor, ts: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,

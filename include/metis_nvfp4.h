@@ -258,6 +258,15 @@ int32_t metis_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales, cons
                                void* out, int32_t out_dtype, int64_t ld, void* stream);
 
 /*
+ * The same values expressed in another unit: (*unit0 * *unit1) / (*over0 * *over1) takes the place of the unit
+ * (the left operand of a side product in the accumulator units of the product it is added to).
+ */
+int32_t metis_nvfp4_dequantize_ratio(const uint8_t* codes, const uint8_t* scales, const float* unit0,
+                                     const float* unit1, const float* over0, const float* over1,
+                                     int32_t sf_layout, int64_t R, int64_t C, void* out, int32_t out_dtype,
+                                     int64_t ld, void* stream);
+
+/*
  * Column means of x [rows, cols]: mean[c] = (sum_r x[r][c]) / rows in fp32
  * (input_flat.mean(dim=0), bitlinear.py:326).  Deterministic summation order.
  * workspace: at least metis_col_mean_workspace_bytes(rows, cols) bytes (unused, one launch, up to 128 rows).
@@ -370,6 +379,12 @@ int64_t metis_lowrank_dts_workspace_bytes(int64_t M, int64_t N, int64_t r);
 int32_t metis_lowrank_dts(const void* g, int64_t ldg, int64_t M, int64_t N, const void* u, int64_t ldu, int64_t r,
                           const void* yv, int64_t ldyv, const void* s, int32_t s_dtype, void* d_yv, int64_t ldd,
                           float* ds, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
+/* The same with ds in bf16 or fp32 (rounded once) and, where d_yv_mean is given, the column mean of d_yv (fp32 [r], the
+ * sum of the rounded values over M): what the mean-centred quantization of d_yv starts from (bitlinear.py:462-474). */
+int32_t metis_lowrank_dts_mean(const void* g, int64_t ldg, int64_t M, int64_t N, const void* u, int64_t ldu, int64_t r,
+                               const void* yv, int64_t ldyv, const void* s, int32_t s_dtype, void* d_yv, int64_t ldd,
+                               void* ds, int32_t ds_dtype, float* d_yv_mean, void* workspace, int64_t workspace_bytes,
+                               int32_t* status, void* stream);
 
 /*
  * Weight gradient of ulinear: dU = G^T ts [N, r] with ts = bf16(s * y_v) [M, r] (bitlinear.py:756-757

@@ -90,3 +90,25 @@ def test_bad_shapes_are_rejected_on_the_host():
         ops.lowrank_dts(g, u, yv, torch.ones(12, device=DEV))          # rank 12: not a multiple of 8
     with pytest.raises(ValueError):
         ops.bf16_panel_gemm(_randn(64, 64, 4), _randn(300, 64, 5))     # more than 256 columns
+
+
+@pytest.mark.parametrize("M,N,r", [(33, 1024, 8), (1120, 3584, 96), (9472, 640, 200), (12800, 520, 128)])
+def test_ds_in_bf16_and_the_column_mean_of_d_yv(M, N, r):
+    """Both finishes (sums over splits; straight from the accumulator from 9600 tokens on): ds rounded once, the mean
+    that of the rounded d_yv.  Bound: fp32 sums of M terms in blocks, 2^-24 times the sum of magnitudes times the depth."""
+    g, u, yv = _randn(M, N, seed=M), _randn(N, r, seed=N, scale=N ** -0.5), _randn(M, r, seed=r)
+    s = torch.linspace(0.5, 1.5, r, device=DEV).to(torch.bfloat16)
+    d_yv, ds32 = ops.lowrank_dts(g, u, yv, s)
+    d_yv2, ds16, mean = ops.lowrank_dts(g, u, yv, s, ds_dtype=torch.bfloat16, want_mean=True)
+    assert torch.equal(d_yv, d_yv2) and torch.equal(ds16, ds32.to(torch.bfloat16))
+    want = d_yv.double().mean(0)
+    bound = 2.0 ** -24 * 64 * d_yv.double().abs().mean(0) + 1e-30
+    assert bool(((mean.double() - want).abs() <= bound).all())
+
+
+def test_dequantized_in_a_ratio_of_units():
+    q = ops.nvfp4_quantize(_randn(96, 272, seed=9))
+    units = [torch.full((1,), v, device=DEV) for v in (0.37, 1.9, 0.011, 5.3)]
+    got = ops.nvfp4_dequantize_ratio(q, torch.bfloat16, *units)
+    want = ops.nvfp4_dequantize(q, torch.bfloat16, unit=(units[0] * units[1]) / (units[2] * units[3]))
+    assert torch.equal(got, want)
