@@ -104,8 +104,8 @@ class PackedOperand:
         return self._dense[dtype]
 
 
-def _packed_matmul(a, b, rank1=(), lowrank=None, c=None, out_dtype=torch.bfloat16, sm_limit=0):
-    return ops.nvfp4_gemm(a, b, rank1=rank1, lowrank=lowrank, c=c, out_dtype=out_dtype, sm_limit=sm_limit)
+def _packed_matmul(a, b, rank1=(), lowrank=None, c=None, out_dtype=torch.bfloat16, sm_limit=0, scaled=None):
+    return ops.nvfp4_gemm(a, b, rank1=rank1, lowrank=lowrank, c=c, out_dtype=out_dtype, sm_limit=sm_limit, scaled=scaled)
 
 
 def _backward_can_pack(shared) -> bool:
@@ -893,7 +893,7 @@ class MetisFusedFunction(torch.autograd.Function):
         N = rq.q.shape[0]
         act = xa.dtype if xa.dtype in (torch.bfloat16, torch.float32) else torch.float32
         rank1_v, rank1_r = [], []
-        join_residual = None
+        join_residual = bias_row = None
 
         def ready(op):
             if op.ready_event is not None:             # quantized on another stream: order this stream after it, once
@@ -921,20 +921,31 @@ class MetisFusedFunction(torch.autograd.Function):
                 if overlap and rq.ready_event is not None:
                     torch.cuda.current_stream(xa.mean.device).wait_event(rq.ready_event)
                 row_r = ops.nvfp4_gemv(rq.q, xa.mean)
+                # a parameter is complete whatever stream this is (a cast of one is ordered on the current stream only)
+                if isinstance(bias, torch.nn.Parameter):
+                    bias_row = bias.float()
             if v_ready is not None:
                 torch.cuda.current_stream(xa.mean.device).wait_event(v_ready)
                 row_v.record_stream(torch.cuda.current_stream(xa.mean.device))
-                join_residual = lambda: join(row_r)
+                join_residual = lambda: join(row_r, bias_row)
             rank1_v.append((None, row_v))
             rank1_r.append((None, row_r))
         if bias is not None:
-            rank1_r.append((None, bias.float()))
+            rank1_r.append((None, bias.float() if bias_row is None else bias_row))
         ready(vq)
-        yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act)                 # [M, r]
         # torch.mul(self.s, y), in the units the side product accumulates in: 1/(unit_x * unit_R)
         if act == torch.bfloat16:
-            lowrank = (ops.lowrank_scale(yv, s, xa.q.unit, rq.q.unit), u_weight.detach().to(torch.bfloat16))
+            if M <= 128:                            # decode-sized: the scaling comes out of the product's own last launch
+                ready(rq)                           # its unit
+                yv, t_acc = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, scaled=(s, xa.q.unit, rq.q.unit))     # [M, r]
+            else:
+                yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act)
+                ready(rq)
+                t_acc = ops.lowrank_scale(yv, s, xa.q.unit, rq.q.unit)
+            lowrank = (t_acc, u_weight.detach().to(torch.bfloat16))
         else:
+            yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act)
+            ready(rq)
             ts = yv * s.to(act)
             lowrank = _bf16_factors(ts.float() / (xa.q.unit * rq.q.unit), u_weight.detach(), act)
         if join_residual is not None:

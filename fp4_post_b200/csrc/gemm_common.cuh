@@ -83,7 +83,13 @@ struct GemmParams {
   int32_t k_per_split = 1 << 30;
   float* partial = nullptr;
   int64_t ldp = 0;
+  // scaled copy of a bf16 D, written by the split-K finish: scaled[m][n] = bf16(float(bf16(D * s[n])) /
+  // (*s_unit_a * *s_unit_b)), row pitch N: the rank-r factor that the next product takes as its side operand
+  const void* s = nullptr;  int32_t s_is_f32 = 0;
+  const float* s_unit_a = nullptr;  const float* s_unit_b = nullptr;
+  __nv_bfloat16* scaled = nullptr;
 };
+
 
 // Tile order: bands of `group` row tiles; inside a band the row tile runs fastest, then the column
 // tile.  The CTAs that run at the same time then share a few A row panels and walk the B column

@@ -350,23 +350,38 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
 // ---- split-K: sum of the partial products + the epilogue terms -----------------------------------------
 
+constexpr int kMaxSplits = 8;
 template <typename TD>
 __global__ void __launch_bounds__(256)
 splitk_finish_kernel(const GemmParams p) {
   grid_dependency_wait();
   grid_launch_dependents();
   const int64_t groups_per_row = (p.N + 3) / 4;
+  const bool small = p.M * groups_per_row < ((int64_t)1 << 31);
   const float g = p.alpha * __ldg(p.a_unit) * __ldg(p.b_unit);
+  const float units = p.scaled ? __fmul_rn(__ldg(p.s_unit_a), __ldg(p.s_unit_b)) : 1.0f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.M * groups_per_row; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / groups_per_row, col = (i - row * groups_per_row) * 4;
+    // 32-bit index arithmetic where it fits (a 64-bit division is a subroutine of ~100 instructions)
+    const int64_t row = small ? (int64_t)((uint32_t)i / (uint32_t)groups_per_row) : i / groups_per_row, col = (i - row * groups_per_row) * 4;
+    const float* src = p.partial + row * p.ldp + col;
+    float4 v[kMaxSplits];
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s)            // every load in flight before the first addition
+      if (s < p.splits) v[s] = *reinterpret_cast<const float4*>(src + (int64_t)s * p.M * p.ldp);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < p.splits; ++s) {            // fixed order: the result does not depend on timing
-      const float4 v = *reinterpret_cast<const float4*>(p.partial + ((int64_t)s * p.M + row) * p.ldp + col);
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-    }
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s)            // fixed order: the result does not depend on timing
+      if (s < p.splits) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
     float o[4] = {acc.x * g, acc.y * g, acc.z * g, acc.w * g};
     const float c0 = p.rvec0 ? (p.cvec0 ? __ldg(p.cvec0 + row) : 1.0f) : 0.0f;
     const float c1 = p.rvec1 ? (p.cvec1 ? __ldg(p.cvec1 + row) : 1.0f) : 0.0f;
+    __nv_bfloat16 sv[4];
+    if (p.scaled) {                                 // N is a multiple of 8 then
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        sv[j] = p.s_is_f32 ? __float2bfloat16_rn(__ldg(static_cast<const float*>(p.s) + col + j))
+                           : __ushort_as_bfloat16(__ldg(static_cast<const unsigned short*>(p.s) + col + j));
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (col + j >= p.N) break;
@@ -376,8 +391,14 @@ splitk_finish_kernel(const GemmParams p) {
         if constexpr (sizeof(TD) == 2) o[j] += __bfloat162float(static_cast<const __nv_bfloat16*>(p.c)[row * p.ldc + col + j]);
         else o[j] += static_cast<const float*>(p.c)[row * p.ldc + col + j];
       }
-      if constexpr (sizeof(TD) == 2) static_cast<__nv_bfloat16*>(p.d)[row * p.ldd + col + j] = __float2bfloat16_rn(o[j]);
-      else static_cast<float*>(p.d)[row * p.ldd + col + j] = o[j];
+      if constexpr (sizeof(TD) == 2) {
+        const __nv_bfloat16 y = __float2bfloat16_rn(o[j]);
+        static_cast<__nv_bfloat16*>(p.d)[row * p.ldd + col + j] = y;
+        // torch.mul(s, y) in bf16 (the product is exact in fp32: one rounding), in the side product's accumulator units
+        if (p.scaled) p.scaled[row * p.N + col + j] = __float2bfloat16_rn(__fdiv_rn(__bfloat162float(__hmul(y, sv[j])), units));
+      } else {
+        static_cast<float*>(p.d)[row * p.ldd + col + j] = o[j];
+      }
     }
   }
 }
@@ -390,7 +411,7 @@ static int choose_splits(int64_t M, int64_t N, int64_t K, int bn, int sms) {
   const int64_t k_iters = ceil_div(K, 256);
   int64_t s = sms / tiles;
   if (s > k_iters / 2) s = k_iters / 2;
-  if (s > 8) s = 8;
+  if (s > kMaxSplits) s = kMaxSplits;
   return s < 2 ? 1 : (int)s;
 }
 static int tile_width(int64_t M, int64_t N, int sms) {
@@ -439,7 +460,16 @@ extern "C" int64_t metis_nvfp4_gemm_workspace_bytes(int64_t M, int64_t N, int64_
   return splits > 1 ? (int64_t)splits * M * (ceil_div(N, 32) * 32) * (int64_t)sizeof(float) : 0;
 }
 
-extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) {
+namespace {
+// The second output of metis_nvfp4_gemm_scaled.
+struct ScaledOutput {
+  const void* s;  int32_t s_dtype;
+  const float* unit_a;  const float* unit_b;
+  void* t;
+};
+}  // namespace
+
+static int32_t run_gemm(const metis_gemm_args* a, const ScaledOutput* scaled) {
   if (!a) return fail(METIS_ERR_BAD_ARGUMENT, "args is null");
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return fail(METIS_ERR_BAD_SHAPE, "empty GEMM %lld x %lld x %lld", (long long)a->M, (long long)a->N, (long long)a->K);
   if (a->K % 32 != 0) return fail(METIS_ERR_BAD_SHAPE, "K = %lld must be a multiple of 32 (16-byte rows of packed codes)", (long long)a->K);
@@ -493,6 +523,18 @@ extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) {
     p.partial = static_cast<float*>(a->workspace);
     p.ldp = ceil_div(a->N, 32) * 32;
   }
+  if (scaled) {
+    // Only the split-K finish of a decode-sized product writes the scaled copy itself (one launch of 4 us less in the
+    // chain).  In the epilogue of the unsplit kernel it was measured slower than the launch it saves: 15.5 + 7.0 us ->
+    // 24.4 at 16384 x 128 x 4096, where four warps per SM do all the divisions.
+    if (p.splits == 1) {
+      if (int32_t rc = run_gemm(a, nullptr)) return rc;
+      return metis_lowrank_scale(a->d, a->M, a->N, a->ldd, scaled->s, scaled->s_dtype, scaled->unit_a, scaled->unit_b, scaled->t, a->stream);
+    }
+    p.s = scaled->s; p.s_is_f32 = scaled->s_dtype == METIS_DTYPE_F32;
+    p.s_unit_a = scaled->unit_a; p.s_unit_b = scaled->unit_b;
+    p.scaled = static_cast<__nv_bfloat16*>(scaled->t);
+  }
   if (pair) return launch_gemm_pair(a, ma, mb, mt, mu, p);
   if (bn == 256) {
     if (a->d_dtype == METIS_DTYPE_BF16) return launch_gemm<256, __nv_bfloat16>(a, ma, mb, mt, mu, p);
@@ -500,4 +542,16 @@ extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) {
   }
   if (a->d_dtype == METIS_DTYPE_BF16) return launch_gemm<128, __nv_bfloat16>(a, ma, mb, mt, mu, p);
   return launch_gemm<128, float>(a, ma, mb, mt, mu, p);
+}
+
+extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) { return run_gemm(a, nullptr); }
+
+extern "C" int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* a, const void* s, int32_t s_dtype, const float* unit_a,
+                                           const float* unit_b, void* t) {
+  if (!a || !s || !unit_a || !unit_b || !t) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
+  if (s_dtype != METIS_DTYPE_BF16 && s_dtype != METIS_DTYPE_F32) return fail(METIS_ERR_BAD_ARGUMENT, "unknown s_dtype %d", s_dtype);
+  if (a->d_dtype != METIS_DTYPE_BF16 || a->N % 8 != 0 || a->ldd % 8 != 0) return fail(METIS_ERR_BAD_ARGUMENT, "the scaled copy is of a bf16 D whose width is a multiple of 8");
+  if (!aligned16(t) || (reinterpret_cast<uintptr_t>(s) & 3u)) return fail(METIS_ERR_BAD_ALIGNMENT, "t must be 16-byte aligned");
+  const ScaledOutput scaled = {s, s_dtype, unit_a, unit_b, t};
+  return run_gemm(a, &scaled);
 }

@@ -385,13 +385,14 @@ def lowrank_scale(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_
 def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Optional[torch.Tensor] = None,
                out_dtype: torch.dtype = torch.bfloat16, alpha: float = 1.0,
                status: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-               sm_limit: int = 0, _debug: int = 0) -> torch.Tensor:
+               sm_limit: int = 0, scaled=None, _debug: int = 0):
     """D = alpha*ua*ub * (A @ B^T + T @ U^T) + sum_i cvec_i (x) rvec_i (+ c), see metis_nvfp4_gemm.
 
     a: [M, K], b: [N, K] (both METIS_SF_MMA).  lowrank = (T [M, r] bf16, U [N, r] bf16), already in
     accumulator units.  rank1 = up to two (cvec or None, rvec) pairs of fp32 vectors.
     Only the packed parts of a and b enter the product; their mean vectors do not.
-    sm_limit > 0 caps the SMs this launch occupies (room for a collective's kernel beside it)."""
+    sm_limit > 0 caps the SMs this launch occupies (room for a collective's kernel beside it).
+    scaled = (s, unit_a, unit_b), for a bf16 D: returns (D, lowrank_scale(D, s, unit_a, unit_b)) from the same launch."""
     M, K = a.shape
     N, K2 = b.shape
     if K != K2:
@@ -447,10 +448,20 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
             keep.append(ws)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws_bytes
-        rc = cabi.lib().metis_nvfp4_gemm(C.byref(args))
+        if scaled is None:
+            rc = cabi.lib().metis_nvfp4_gemm(C.byref(args))
+        else:
+            s, unit_a, unit_b = scaled
+            if s.dtype not in (torch.bfloat16, torch.float32):
+                s = s.float()
+            s = s.reshape(-1).contiguous()
+            assert s.numel() == N and s.device == dev
+            t = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
+            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), s.data_ptr(), _dtype_code(s, "s"), unit_a.data_ptr(),
+                                                    unit_b.data_ptr(), t.data_ptr())
     cabi.check(rc, "metis_nvfp4_gemm")
     LAUNCHES["gemm"] += 2 if ws_bytes > 0 else 1
-    return out
+    return out if scaled is None else (out, t)
 
 
 def _bf16_rows(t: torch.Tensor, what: str) -> torch.Tensor:

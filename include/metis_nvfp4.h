@@ -343,6 +343,14 @@ typedef struct metis_gemm_args {
 int32_t metis_nvfp4_gemm(const metis_gemm_args* args);
 
 /*
+ * metis_nvfp4_gemm with a bf16 D [M, N] (N a multiple of 8), and metis_lowrank_scale of it in the same launch:
+ * t[m][n] = bf16( float(bf16(D[m][n] * s[n])) / (unit_a * unit_b) ), row pitch N: the product with V and the
+ * scaling behind it (bitlinear.py:752-756).
+ */
+int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* args, const void* s, int32_t s_dtype, const float* unit_a,
+                                const float* unit_b, void* t);
+
+/*
  * Scratch that lets a decode-sized product (M <= 128: the rollout path, bitlinear.py:704-751,
  * and the weight gradients of the rank-r factors) split its K loop over otherwise idle SMs:
  * bytes of fp32 partial sums, 0 when the shape is not split.  Without the scratch the same

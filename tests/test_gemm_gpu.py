@@ -232,3 +232,19 @@ def test_argument_errors():
     qk = ops.nvfp4_quantize(torch.zeros(128, 128, device=DEV))
     with pytest.raises(ValueError):
         ops.nvfp4_gemm(qa, qk)                 # inner dimensions differ
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 128, 4096), (100, 48, 1024), (300, 128, 512), (129, 16, 256), (5, 256, 2048), (256, 192, 256)])
+@pytest.mark.parametrize("s_dtype", [torch.bfloat16, torch.float32])
+def test_scaled_copy_of_the_output_is_lowrank_scale_of_it(M, N, K, s_dtype):
+    """In the split-K finish and, where the product is not split, behind it."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = ops.nvfp4_quantize(torch.randn(M, K, device="cuda", generator=g))
+    b = ops.nvfp4_quantize(torch.randn(N, K, device="cuda", generator=g))
+    s = (torch.rand(N, device="cuda", generator=g) + 0.5).to(s_dtype)
+    row = torch.randn(N, device="cuda", generator=g)
+    ua, ub = torch.full((1,), 0.013, device="cuda"), torch.full((1,), 0.7, device="cuda")
+    plain = ops.nvfp4_gemm(a, b, rank1=[(None, row)])
+    out, t = ops.nvfp4_gemm(a, b, rank1=[(None, row)], scaled=(s, ua, ub))
+    assert torch.equal(out, plain)
+    assert torch.equal(t, ops.lowrank_scale(plain, s, ua, ub))
