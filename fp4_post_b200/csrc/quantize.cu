@@ -11,6 +11,7 @@
 #include "tma.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace metis {
 
@@ -487,12 +488,12 @@ __device__ __forceinline__ void e4m3x4_to_float(uint32_t packed, float (&f)[4]) 
 // A thread finishes one 16-byte piece of the tiled layout at a time: the scales of the rows l, l + 32, l + 64, l + 96 of
 // a 128-row block for 4 scale columns, i.e. four 16-byte reads of maxima and one 16-byte store (row-major scales: four
 // words of four rows).  Two neighbouring lanes take two neighbouring l, the next ones the tiles to the right, so a warp
-// reads runs of up to 256 bytes and stores whole 32-byte sectors.  An item is such a pair of l (8 rows) over the whole
-// row; a CTA takes 64 / tx items at once.  With one 4-column group of two rows per thread, scalar arithmetic and 64-bit
+// reads runs of up to 256 bytes and stores whole 32-byte sectors.  An item is such a pair of l (8 rows) over a segment of
+// the row (the whole of it where its sum is wanted); a CTA takes 64 / tx items at once.  With one 4-column group of two rows per thread, scalar arithmetic and 64-bit
 // index arithmetic this pass took 62 instructions per block and was bound by issue; what counts beside the arithmetic is
 // that edges, padding and divisions stay out of the unrolled path (with them inside it 27 instructions per block and
 // waits for instruction fetch).  Measured at 16384 x 4096, one output / both / both with token sums: 11.2 / 21.0 / 28.2
-// us then, 5.6 / 10.0 / 21.1 now; at 65536 x 4096 32 / 62 / 79 -> 16 / 30 / 67 (the bytes alone take 13 / 26 / 46).
+// us then, 5.8 / 10.4 / 21.2 now; at 65536 x 4096 32 / 62 / 79 -> 16 / 30 / 67 (the bytes alone take 13 / 26 / 46); 64 x 18944, fewer rows than a block has: 4.0 -> 2.8.
 constexpr int kFinThreads = 128;
 template <bool kSums>                                            // some job of the launch wants row sums (twice the registers)
 __global__ void __launch_bounds__(kFinThreads)
@@ -538,60 +539,83 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
   const int tx = 1 << J.log_tx, per_cta = 64 >> J.log_tx;        // threads along a row, items per CTA
   const int k_lane = (tid >> 1) & (tx - 1), sub = tid >> (1 + J.log_tx);
   const int64_t items = ((R + 127) / 128) * 16;
+  // without row sums a row is cut into segments of tx tiles, so that a few wide rows still fill the SMs
+  const int segments = sums ? 1 : (groups + tx - 1) >> J.log_tx;
+  const int64_t work = items * segments;
   const int64_t row_pitch = 32 * sf_cols;                        // between a thread's four rows
   // the item loop is uniform over the CTA (the sums of a row meet at a barrier)
-  for (int64_t first = (int64_t)blockIdx.x * per_cta; first < items; first += (int64_t)gridDim.x * per_cta) {
-    const int64_t item = first + sub;
-    const bool live = item < items;
+  for (int64_t first = (int64_t)blockIdx.x * per_cta; first < work; first += (int64_t)gridDim.x * per_cta) {
+    const bool live = first + sub < work;
+    const int64_t item = segments == 1 ? first + sub : (first + sub) / segments;
+    const int k_first = segments == 1 ? 0 : (int)((first + sub) - item * segments) << J.log_tx;
+    const int k_end = segments == 1 ? groups : min(groups, k_first + tx);
     const int64_t row0 = (item >> 4) * 128 + (item & 15) * 2 + (tid & 1);       // this thread's rows: row0 + 32 c
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const float* src = J.amax + row0 * sf_cols;
     const uint2* codes = J.codes + row0 * sf_cols;
     uint8_t* dst = tiled ? J.scales + (item >> 4) * tiles * 512 + ((item & 15) * 2 + (tid & 1)) * 16 : J.scales + row0 * sf_cols;
-    const bool whole = live && (vec || tiled) && row0 + 96 < R;    // all four rows are there: no bounds inside a piece
-    for (int k = k_lane; live && k < groups; k += tx) {
-      if (whole && 4 * k + 4 <= sf_cols) {
-        float4 a[4];
-        uint4 cd[4][2];
-        uint32_t out[4];
+    const int rows = row0 >= R ? 0 : (int)min((int64_t)4, (R - row0 + 31) >> 5);      // of this thread's four: the first ones
+    // the piece of tile k (all four blocks of it exist); kWhole: of four rows, else of the first `rows`
+    auto piece = [&](auto whole, int k) {
+      constexpr bool kWhole = decltype(whole)::value;
+      float4 a[4];
+      uint4 cd[4][2];
+      uint32_t out[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {                             // every load before the first use
-          const float* from = src + c * row_pitch + 4 * k;
+      for (int c = 0; c < 4; ++c) {                             // every load before the first use
+        const float* from = src + c * row_pitch + 4 * k;
+        a[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (kWhole || c < rows) {
           if (vec) a[c] = *reinterpret_cast<const float4*>(from);
           else     a[c] = make_float4(from[0], from[1], from[2], from[3]);
         }
-        if (sums) {
+      }
+      if (sums) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4* w = reinterpret_cast<const uint4*>(codes + c * row_pitch + 4 * k);
-            cd[c][0] = w[0];
-            cd[c][1] = w[1];
-          }
+        for (int c = 0; c < 4; ++c) {
+          cd[c][0] = cd[c][1] = make_uint4(0u, 0u, 0u, 0u);
+          if (!kWhole && c >= rows) continue;
+          const uint4* w = reinterpret_cast<const uint4*>(codes + c * row_pitch + 4 * k);
+          cd[c][0] = w[0];
+          cd[c][1] = w[1];
         }
-        bool stands[4], all = true;
+      }
+      bool stands[4], all = true;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) all &= stands[c] = scale_bytes4(a[c], inv_unit2, out[c]);
-        if (!all) {
+      for (int c = 0; c < 4; ++c) {
+        stands[c] = scale_bytes4(a[c], inv_unit2, out[c]) || (!kWhole && c >= rows);
+        all &= stands[c];
+      }
+      if (!all) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) if (!stands[c]) out[c] = scale_bytes4_exact(a[c], unit);
+        for (int c = 0; c < 4; ++c) if (!stands[c]) out[c] = scale_bytes4_exact(a[c], unit);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) if (!kWhole && c >= rows) out[c] = 0u;            // padding
+      if (sums) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float f[4];
+          e4m3x4_to_float(out[c], f);
+          acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].x, cd[c][0].y)), f[0], acc[c]);
+          acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].z, cd[c][0].w)), f[1], acc[c]);
+          acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].x, cd[c][1].y)), f[2], acc[c]);
+          acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].z, cd[c][1].w)), f[3], acc[c]);
         }
-        if (sums) {
+      }
+      if (tiled) {
+        *reinterpret_cast<uint4*>(dst + (int64_t)k * 512) = make_uint4(out[0], out[1], out[2], out[3]);
+      } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            float f[4];
-            e4m3x4_to_float(out[c], f);
-            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].x, cd[c][0].y)), f[0], acc[c]);
-            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][0].z, cd[c][0].w)), f[1], acc[c]);
-            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].x, cd[c][1].y)), f[2], acc[c]);
-            acc[c] = fmaf((float)block_code_sum(make_uint2(cd[c][1].z, cd[c][1].w)), f[3], acc[c]);
-          }
-        }
-        if (tiled) {
-          *reinterpret_cast<uint4*>(dst + (int64_t)k * 512) = make_uint4(out[0], out[1], out[2], out[3]);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) *reinterpret_cast<uint32_t*>(dst + c * row_pitch + 4 * k) = out[c];
-        }
+        for (int c = 0; c < 4; ++c) if (kWhole || c < rows) *reinterpret_cast<uint32_t*>(dst + c * row_pitch + 4 * k) = out[c];
+      }
+    };
+    for (int k = k_first + k_lane; live && k < k_end; k += tx) {
+      const bool full = (vec || tiled) && 4 * k + 4 <= sf_cols;
+      if (full && rows == 4) {
+        piece(std::true_type{}, k);
+      } else if (!kSums && full) {                                  // decode: fewer than 128 rows (a second copy beside the sums costs a third more registers)
+        piece(std::false_type{}, k);
       } else {                                                      // an edge of the tensor, or padding: kept short
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
@@ -916,7 +940,8 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
     const int64_t groups = J.sf_layout == METIS_SF_MMA ? sf_tiles_per_row(J.sf_cols * 16) : ceil_div(J.sf_cols, 4);
     J.log_tx = 2;                                             // a warp holds at most 8 rows' lanes of 4 tiles
     while (J.log_tx < 6 && (1 << J.log_tx) < groups) ++J.log_tx;
-    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16, 64 >> J.log_tx);
+    const int64_t segments = J.row_sums ? 1 : ceil_div(groups, (int64_t)1 << J.log_tx);
+    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16 * segments, 64 >> J.log_tx);
     if (need > blocks) blocks = need;
   }
   if (njobs == 1) jobs.job[1] = jobs.job[0];

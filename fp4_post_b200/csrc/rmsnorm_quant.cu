@@ -526,14 +526,31 @@ rmsnorm_colsum_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, in
   }
 }
 
-__global__ void rmsnorm_mean_finish_kernel(const float* __restrict__ partial, int64_t slots, int64_t rows, int64_t cols,
-                                           float* __restrict__ mean) {
+// A CTA takes 32 columns: each of its eight warps adds every eighth row slot (coalesced, eight loads in flight), then their
+// sums are added in warp order: a fixed order.  One thread per column that walks all slots is a chain of loads: 13.4 us
+// for 256 slots, 15.5 for 296 (hidden 4096), 4.6 and 5.9 here (64 slots 4.5 -> 2.3).
+__global__ void __launch_bounds__(256)
+rmsnorm_mean_finish_kernel(const float* __restrict__ partial, int64_t slots, int64_t rows, int64_t cols, float* __restrict__ mean) {
+  __shared__ float s_part[8][32];
   grid_dependency_wait();
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t c = (int64_t)blockIdx.x * 32 + lane;
   float sum = 0.0f;
-  for (int64_t s = 0; s < slots; ++s) sum += partial[s * cols + c];        // fixed order
-  mean[c] = __fdiv_rn(sum, (float)rows);
+  if (c < cols) {
+    const float* src = partial + warp * cols + c;
+    const int mine = ((int)slots - warp + 7) >> 3;
+    const int64_t step = 8 * cols;
+#pragma unroll 8
+    for (int i = 0; i < mine; ++i) sum += src[i * step];
+  }
+  s_part[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0 && c < cols) {
+    float total = s_part[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) total += s_part[w][lane];
+    mean[c] = __fdiv_rn(total, (float)rows);
+  }
 }
 
 struct NormShape { int bx, by, per_thread; };
@@ -650,7 +667,7 @@ extern "C" int32_t metis_rmsnorm_mean(const void* x, int32_t x_dtype, int64_t ro
   if (rc) return rc;
   const NormShape sh = norm_shape((int)(cols >> 4));
   const int64_t slots = colsum_ctas(rows, sh.by) * sh.by;
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, rmsnorm_mean_finish_kernel, dim3((unsigned)ceil_div(cols, 256)), dim3(256), 0, st,
+  METIS_CUDA_OK(launch_overlapped(kLaunchShort, rmsnorm_mean_finish_kernel, dim3((unsigned)ceil_div(cols, 32)), dim3(256), 0, st,
                                   (const float*)partial, slots, rows, cols, mean));
   return METIS_OK;
 }
