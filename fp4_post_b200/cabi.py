@@ -14,6 +14,7 @@ DTYPE_BF16, DTYPE_F32 = 0, 1
 SF_ROWMAJOR, SF_MMA = 0, 1
 Q_TRANSPOSE, Q_STOCHASTIC, Q_OFFSET_ON_DEVICE, Q_HADAMARD = 1, 2, 4, 8
 Q_DEFER_ROWMAJOR, Q_DEFER_TRANSPOSED, Q_SR16 = 16, 32, 64
+QUANTIZE_EXTRA_WORKSPACE = 8192
 STATIC_MAX_ELEMENTS = 16 * 1024 * 1024
 
 STATUS_TEXT = {

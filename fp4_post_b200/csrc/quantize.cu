@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kQuantThreads)
 quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
                      const float* __restrict__ col_mean, uint64_t seed, uint64_t offset,
                      const uint64_t* __restrict__ offset_ctr, uint2* __restrict__ codes, float* __restrict__ amax_out,
-                     unsigned int* __restrict__ gmax, uint32_t sr16) {
+                     unsigned int* __restrict__ gmax, unsigned int* __restrict__ records, uint32_t sr16) {
   grid_dependency_wait();
   if (kSR && offset_ctr) offset += *offset_ctr;             // per-device call counter (graph-safe stream of offsets)
   const int bc = blockIdx.x * blockDim.x + threadIdx.x;     // column block of this thread
@@ -76,7 +76,25 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
     }
   }
   // whole warps reach this point together: a warp never spans the bc bound unevenly in y
-  fold_global_max(gmax, running);
+  if (!records) {
+    fold_global_max(gmax, running);
+    return;
+  }
+  // a record per CTA (see TileOutputs): nobody has to zero a shared maximum first
+  __shared__ unsigned int s_max[kQuantThreads / 32];
+  const unsigned tid = threadIdx.y * blockDim.x + threadIdx.x;
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(running));
+  if ((tid & 31u) == 0) s_max[tid >> 5] = m;
+  __syncthreads();
+  if (tid == 0) {
+    unsigned top = 0u;
+    for (unsigned w = 0; w < blockDim.x * blockDim.y / 32; ++w) top = max(top, s_max[w]);
+    const unsigned cta = blockIdx.y * gridDim.x + blockIdx.x;
+    records[3 * cta] = top;
+    records[3 * cta + 1] = 0u;
+    records[3 * cta + 2] = 0u;
+    if (cta == 0) records[-1] = gridDim.x * gridDim.y;
+  }
 }
 
 // ---- pass 1 on shared-memory tiles: the transposed quantization, alone or together with the row-major one ----
@@ -679,6 +697,7 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
 // 8.0, 32 x 4096 5.2, 64 x 4096 6.8 against 8.1.
 constexpr int kSmallThreads = 512;
 constexpr int kSmallBlocks = 4;                    // blocks per thread
+constexpr int64_t kClusterMaxBlocksWithRecords = 4096;
 constexpr int64_t kSmallMaxBlocks = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks;
 
 template <typename T, bool kMean>
@@ -866,7 +885,7 @@ static int sm_count() { return device_sm_count(); }
 template <typename T>
 static void launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, const float* mean, bool sr,
                         uint64_t seed, uint64_t offset, const uint64_t* ctr, uint32_t* codes, const WorkspaceView& ws,
-                        cudaStream_t st, uint32_t sr16 = 0) {
+                        cudaStream_t st, uint32_t sr16 = 0, unsigned int* records = nullptr) {
   const int bpr = (int)(cols >> 4);
   // threads along the row: the power of two that pads the row least (hidden 1536 = 96 blocks runs
   // as 3 x 32, not as 128 with a quarter of the lanes idle); ties go to the wider shape
@@ -885,6 +904,7 @@ static void launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, cons
 #undef METIS_OCC_ROWS
   if (per_sm < 1) per_sm = 1;
   int64_t cap = (int64_t)sm_count() * per_sm * 4 / gx;
+  if (records && cap > kDualMaxCtas / gx) cap = kDualMaxCtas / gx;
   if (cap < 1) cap = 1;
   if (gy > cap) gy = cap;
   if (gy > 65535) gy = 65535;
@@ -892,7 +912,7 @@ static void launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, cons
   const dim3 g((unsigned)gx, (unsigned)gy), b((unsigned)bx, (unsigned)by);
 #define METIS_LAUNCH_ROWS(MEAN, SR)                                                              \
   launch_overlapped(kLaunchStream, quantize_rows_kernel<T, MEAN, SR>, g, b, 0, st, x, (int)rows, bpr, ld, mean, seed, offset, ctr, \
-                    reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, sr16)
+                    reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, records, sr16)
   if (mean) { if (sr) METIS_LAUNCH_ROWS(true, true); else METIS_LAUNCH_ROWS(true, false); }
   else      { if (sr) METIS_LAUNCH_ROWS(false, true); else METIS_LAUNCH_ROWS(false, false); }
 #undef METIS_LAUNCH_ROWS
@@ -954,10 +974,10 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
   return METIS_OK;
 }
 
-int32_t launch_finalize(const WorkspaceView& ws, int64_t R, int64_t C, int32_t sf_layout,
-                        uint8_t* scales, float* unit, cudaStream_t st, uint64_t* offset_ctr) {
+int32_t launch_finalize(const WorkspaceView& ws, int64_t R, int64_t C, int32_t sf_layout, uint8_t* scales, float* unit,
+                        cudaStream_t st, uint64_t* offset_ctr, const unsigned int* records, int32_t which) {
   FinalizeJobs jobs = {};
-  jobs.job[0] = {ws.amax, ws.gmax, ws.gmax + 1, R, C / 16, sf_layout, scales, unit, 0, nullptr, nullptr, nullptr, 0};
+  jobs.job[0] = {ws.amax, ws.gmax, ws.gmax + 1, R, C / 16, sf_layout, scales, unit, 0, nullptr, nullptr, records, which};
   return launch_finalize_jobs(jobs, 1, st, offset_ctr);
 }
 
@@ -1027,19 +1047,28 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
   if (rows >= ((int64_t)1 << 31) || cols >= ((int64_t)1 << 31)) return fail(METIS_ERR_TOO_LARGE, "tensor too large");
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // With METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than it needs the workspace also holds a record per CTA of the first
+  // pass, as in the dual quantizer; without them the running maximum and the error word are zeroed in front of it, and
+  // that memset node costs 3-4 us (16 x 14336: 8.2 us with it, 4.9 without; 1120 x 3584: 12.4, 8.1).
+  const int64_t records_at = (metis_nvfp4_quantize_workspace_bytes(R, C) + 15) / 16 * 16;
+  unsigned int* records = workspace_bytes >= records_at + 16 + kDualMaxCtas * 12
+      ? reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + records_at) + 4 : nullptr;
+  // One cluster for the whole tensor: with records, only where two launches over many SMs are not faster (16 x 4096:
+  // 4.3 us against 4.5; 64 x 3584 on the cluster's 8 SMs: 7.1 against 5.0).
   int64_t tiles = 0, padded_words = 0;
-  if (!transpose && !sr && aligned16(scales) && small_path(R, C, sf_layout, &tiles, &padded_words)) {
+  if (!transpose && !sr && aligned16(scales) && small_path(R, C, sf_layout, &tiles, &padded_words) &&
+      (!records || R * (C / 16) <= kClusterMaxBlocksWithRecords)) {
     return x_dtype == METIS_DTYPE_BF16
         ? launch_small(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st)
         : launch_small(static_cast<const float*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st);
   }
   const WorkspaceView ws = view_workspace(workspace);
-  METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
+  if (!records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));
   // Large row-major tensors take the tile kernel too (row phase only): its TMA ring keeps two tiles in
   // flight per CTA, where the register-fed kernel waits on its loads.  Same arithmetic, same bytes.
   const bool rows_by_tiles = !transpose && rows * cols >= kTileRowsMinElements && (ld * esz) % 16 == 0;
   if (rows_by_tiles) {
-    const TileOutputs out = {nullptr, nullptr, nullptr, codes, ws.amax, ws.gmax, ws.gmax + 1, nullptr, 0u, sr16};
+    const TileOutputs out = {nullptr, nullptr, nullptr, codes, ws.amax, ws.gmax, ws.gmax + 1, records, 0u, sr16};
     const int32_t rc = x_dtype == METIS_DTYPE_BF16
         ? launch_tile(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st)
         : launch_tile(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st);
@@ -1047,19 +1076,19 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
   } else if (!transpose) {
     if (x_dtype == METIS_DTYPE_BF16)
       launch_rows(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
-                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16);
+                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16, records);
     else
       launch_rows(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
-                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16);
+                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16, records);
   } else {
-    const TileOutputs out = {codes, ws.amax, ws.gmax, nullptr, nullptr, nullptr, ws.gmax + 1, nullptr, rht, sr16};
+    const TileOutputs out = {codes, ws.amax, ws.gmax, nullptr, nullptr, nullptr, ws.gmax + 1, records, rht, sr16};
     const int32_t rc = x_dtype == METIS_DTYPE_BF16
         ? launch_tile(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st)
         : launch_tile(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st);
     if (rc) return rc;
   }
   METIS_CUDA_OK(cudaGetLastError());
-  return launch_finalize(ws, R, C, sf_layout, scales, unit, st, ctr);
+  return launch_finalize(ws, R, C, sf_layout, scales, unit, st, ctr, records, transpose ? 1 : 0);
 }
 
 // Scale pass of the dual quantizer's outputs (either or both) from the block maxima in its workspace.

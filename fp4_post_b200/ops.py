@@ -168,7 +168,7 @@ def nvfp4_quantize(x: torch.Tensor, *, transpose: bool = False, stochastic: bool
         assert mean.numel() == cols
     with _on_device(dev):
         codes, scales, unit = _packed_buffers(L, R, Cc, sf_layout, dev)
-        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(R, Cc), dtype=torch.uint8, device=dev)
+        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(R, Cc) + cabi.QUANTIZE_EXTRA_WORKSPACE, dtype=torch.uint8, device=dev)
         rc = L.metis_nvfp4_quantize(x2.data_ptr(), _dtype_code(x2, "x"), rows, cols, x2.stride(0), _ptr(mean),
                                     flags, seed & (2**64 - 1), offset & (2**64 - 1), sf_layout,
                                     codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), ws.data_ptr(),

@@ -6,7 +6,7 @@ import torch
 
 from fp4_post_b200 import cabi, ops
 from oracle import nvfp4_oracle as O
-from gpu_helpers import assert_packed_equal, packed_to_numpy, synthetic
+from gpu_helpers import assert_packed_equal, oracle_packed, packed_to_numpy, synthetic
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -501,3 +501,30 @@ def test_vector_product_along_the_tiled_scales(rows, cols):
     bound = 2.0 ** -24 * (cols / 32 + 40) * (deq.abs() @ v.double().abs().cuda())
     assert got.shape == (rows,) and bool(((got - want).abs() <= bound).all())
     assert torch.equal(got, ops.nvfp4_gemv(q, v.cuda()).double())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,transpose", [(16, 4096, False), (17, 4112, False), (64, 3584, False), (16, 14336, False), (300, 4096, False),
+                                                 (1, 81920, False), (48, 1040, True), (512, 4096, True)])
+@pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
+def test_a_workspace_with_room_for_records_gives_the_same_bytes(rows, cols, transpose, layout):
+    """Both forms of the workspace, on either side of the one-cluster limit, over a workspace full of old bytes."""
+    x = synthetic(rows, cols, "normal", rows + cols, torch.bfloat16).to(DEV)
+    L = cabi.lib()
+    R, C = (cols, rows) if transpose else (rows, cols)
+    got = []
+    for extra in (0, cabi.QUANTIZE_EXTRA_WORKSPACE):
+        codes = torch.empty(R, C // 2, dtype=torch.uint8, device=DEV)
+        scales = torch.full((L.metis_nvfp4_sf_bytes(R, C, layout),), 0xA5, dtype=torch.uint8, device=DEV)
+        unit = torch.empty(1, device=DEV)
+        ws = torch.full((L.metis_nvfp4_quantize_workspace_bytes(R, C) + extra,), 0xFF, dtype=torch.uint8, device=DEV)
+        rc = L.metis_nvfp4_quantize(x.data_ptr(), cabi.DTYPE_BF16, rows, cols, cols, None, cabi.Q_TRANSPOSE if transpose else 0, 0, 0, layout,
+                                    codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), ws.data_ptr(), ws.numel(),
+                                    torch.cuda.current_stream().cuda_stream)
+        cabi.check(rc, "metis_nvfp4_quantize")
+        got.append((codes, scales, unit))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    xs = x.float().cpu().numpy()
+    ocodes, oscales, ounit = oracle_packed(np.ascontiguousarray(xs.T) if transpose else xs, layout)
+    assert np.array_equal(got[1][0].cpu().numpy(), ocodes) and np.array_equal(got[1][1].cpu().numpy(), oscales)
