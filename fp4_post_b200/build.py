@@ -25,7 +25,7 @@ CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_lib"
 LIB = OUT_DIR / "libmetis_nvfp4.so"
 KNOBS_LIB = OUT_DIR / "libmetis_nvfp4_knobs.so"
-SOURCES = ["api.cu", "quantize.cu", "rmsnorm_quant.cu", "dequantize.cu", "gemm_tcgen05.cu", "gemm_tcgen05_pair.cu", "lowrank_bwd.cu"]
+SOURCES = ["api.cu", "quantize.cu", "rmsnorm_quant.cu", "dequantize.cu", "gemm_tcgen05.cu", "gemm_tcgen05_pair.cu", "lowrank_bwd.cu", "decoder_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",

@@ -34,6 +34,7 @@ EXPORTS = (
     "metis_rmsnorm_mean_workspace_bytes", "metis_rmsnorm_mean",
     "metis_bf16_panel_gemm_workspace_bytes", "metis_bf16_panel_gemm",
     "metis_lowrank_dts_workspace_bytes", "metis_lowrank_dts", "metis_lowrank_dts_mean", "metis_lowrank_du_workspace_bytes", "metis_lowrank_du",
+    "metis_rope_pair", "metis_silu_mul",
 )
 
 
@@ -128,6 +129,10 @@ def lib() -> C.CDLL:
     L.metis_lowrank_du.restype = i32
     L.metis_nvfp4_gemm_workspace_bytes.argtypes = [i64, i64, i64]
     L.metis_nvfp4_gemm_workspace_bytes.restype = i64
+    L.metis_rope_pair.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, vp]
+    L.metis_rope_pair.restype = i32
+    L.metis_silu_mul.argtypes = [vp, vp, vp, i64, vp]
+    L.metis_silu_mul.restype = i32
     _lib = L
     return L
 

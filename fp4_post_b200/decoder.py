@@ -21,6 +21,7 @@ import torch
 import torch.nn.functional as Fn
 from torch import nn
 
+from fp4_post_b200 import ops
 from fp4_post_b200.Metis.Metis.bitlinear import forward_group
 from fp4_post_b200.Metis.models.llama import RMSNorm
 
@@ -56,6 +57,11 @@ def _rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor
     return x * cos + torch.cat((-x2, x1), dim=-1) * sin
 
 
+def _native(*tensors) -> bool:
+    """Inference on bf16 CUDA tensors: the elementwise pieces run as one launch each, with the same roundings."""
+    return not torch.is_grad_enabled() and all(t.is_cuda and t.dtype == torch.bfloat16 and t.device == tensors[0].device for t in tensors)
+
+
 class Attention(nn.Module):
     def __init__(self, cfg: DecoderConfig):
         super().__init__()
@@ -69,10 +75,13 @@ class Attention(nn.Module):
         B, T, _ = h.shape
         c = self.cfg
         q, k, v = forward_group((self.q_proj, self.k_proj, self.v_proj), h)     # one shared activation, three branches
-        q = q.view(B, T, c.heads, c.head_dim).transpose(1, 2)
-        k = k.view(B, T, c.kv_heads, c.head_dim).transpose(1, 2)
+        q = q.view(B, T, c.heads, c.head_dim)
+        k = k.view(B, T, c.kv_heads, c.head_dim)
         v = v.view(B, T, c.kv_heads, c.head_dim).transpose(1, 2)
-        q, k = _rope(q, cos, sin), _rope(k, cos, sin)
+        if _native(q, k, cos, sin) and c.head_dim % 8 == 0 and cos.numel() == sin.numel() == T * c.head_dim:
+            q, k = (t.transpose(1, 2) for t in ops.rope_pair(q, k, cos, sin))
+        else:
+            q, k = _rope(q.transpose(1, 2), cos, sin), _rope(k.transpose(1, 2), cos, sin)
         a = Fn.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
         return self.o_proj(a.transpose(1, 2).reshape(B, T, c.heads * c.head_dim))
 
@@ -86,6 +95,8 @@ class MLP(nn.Module):
 
     def forward(self, h):
         gate, up = forward_group((self.gate_proj, self.up_proj), h)
+        if _native(gate, up) and gate.numel() % 8 == 0:
+            return self.down_proj(ops.silu_mul(gate, up))
         return self.down_proj(Fn.silu(gate) * up)
 
 

@@ -16,7 +16,7 @@ _DTYPES = {torch.bfloat16: cabi.DTYPE_BF16, torch.float32: cabi.DTYPE_F32}
 
 # Kernels of this library launched since import, by entry point (two per quantizer call: the
 # streaming pass and the scale pass; the memset between them is not a kernel).
-LAUNCHES = {"quantize": 0, "rmsnorm_quantize": 0, "dequantize": 0, "col_mean": 0, "gemv": 0, "gemm": 0, "lowrank_bwd": 0}
+LAUNCHES = {"quantize": 0, "rmsnorm_quantize": 0, "dequantize": 0, "col_mean": 0, "gemv": 0, "gemm": 0, "lowrank_bwd": 0, "decoder": 0}
 
 
 def launch_count() -> int:
@@ -536,4 +536,41 @@ def lowrank_du(g: torch.Tensor, ts: torch.Tensor, out_dtype: torch.dtype = torch
                                 out.stride(0), ws.data_ptr(), ws.numel(), _ptr(status), _stream())
     cabi.check(rc, "metis_lowrank_du")
     LAUNCHES["lowrank_bwd"] += 2
+    return out
+
+
+def rope_pair(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
+    """Rotary embedding (rotate-half convention) of q [B, T, Hq, D] and k [B, T, Hk, D], bf16 and contiguous, in one
+    launch, with every rounding of `x * cos + cat(-x2, x1) * sin` on bf16 tensors.  cos, sin: bf16, T rows of D elements
+    (any leading ones).  Returns tensors shaped like q and k.  No autograd."""
+    for name, t in (("q", q), ("k", k), ("cos", cos), ("sin", sin)):
+        _need_cuda(t, name)
+        if t.dtype != torch.bfloat16:
+            raise TypeError(f"{name} must be bfloat16")
+    B, T, Hq, D = q.shape
+    Hk = k.shape[2]
+    if k.shape != (B, T, Hk, D) or cos.numel() != T * D or sin.numel() != T * D:
+        raise ValueError(f"shapes do not fit: q {tuple(q.shape)}, k {tuple(k.shape)}, cos {tuple(cos.shape)}, sin {tuple(sin.shape)}")
+    q, k, cos, sin = q.contiguous(), k.contiguous(), cos.contiguous(), sin.contiguous()
+    with _on_device(q.device):
+        qo, ko = torch.empty_like(q), torch.empty_like(k)
+        rc = cabi.lib().metis_rope_pair(q.data_ptr(), k.data_ptr(), cos.data_ptr(), sin.data_ptr(), qo.data_ptr(), ko.data_ptr(),
+                                        B * T, T, Hq, Hk, D, _stream())
+    cabi.check(rc, "metis_rope_pair")
+    LAUNCHES["decoder"] += 1
+    return qo, ko
+
+
+def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up for bf16 tensors of one shape, with the rounding of silu's output, in one launch.  No autograd."""
+    _need_cuda(gate, "gate")
+    _need_cuda(up, "up")
+    if gate.dtype != torch.bfloat16 or up.dtype != torch.bfloat16 or gate.shape != up.shape:
+        raise TypeError("gate and up must be bfloat16 tensors of one shape")
+    gate, up = gate.contiguous(), up.contiguous()
+    with _on_device(gate.device):
+        out = torch.empty_like(gate)
+        rc = cabi.lib().metis_silu_mul(gate.data_ptr(), up.data_ptr(), out.data_ptr(), gate.numel(), _stream())
+    cabi.check(rc, "metis_silu_mul")
+    LAUNCHES["decoder"] += 1
     return out

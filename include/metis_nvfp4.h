@@ -407,6 +407,18 @@ int32_t metis_lowrank_du(const void* g, int64_t ldg, int64_t M, int64_t N, const
                          void* grad_u, int32_t u_dtype, int64_t ldgu, void* workspace, int64_t workspace_bytes,
                          int32_t* status, void* stream);
 
+/* ---- elementwise pieces of a decoder block (inference) ------------------------------------------------- */
+
+/*
+ * Rotary embedding of q [tokens, heads_q, head_dim] and k [tokens, heads_k, head_dim] (bf16, contiguous) in one launch:
+ * bf16(bf16(x cos) + bf16((-x2, x1) sin)) with cos and sin bf16 [positions, head_dim]; token t takes row t % positions.
+ */
+int32_t metis_rope_pair(const void* q, const void* k, const void* cos, const void* sin, void* q_out, void* k_out,
+                        int64_t tokens, int64_t positions, int32_t heads_q, int32_t heads_k, int32_t head_dim,
+                        void* stream);
+/* out = bf16(bf16(silu(gate)) * up) for n bf16 elements (a multiple of 8). */
+int32_t metis_silu_mul(const void* gate, const void* up, void* out, int64_t n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

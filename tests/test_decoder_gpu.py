@@ -124,3 +124,31 @@ def test_a_projection_group_on_parallel_streams_equals_the_calls_one_after_the_o
         torch.cuda.synchronize()
         assert torch.equal(replayed, want_logits)
         graphed.release()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hk,D", [(1, 64, 28, 4, 128), (2, 7, 12, 2, 128), (3, 1, 2, 2, 8), (1, 33, 5, 1, 40)])
+def test_rotary_embedding_in_one_launch_is_the_torch_expression(B, T, Hq, Hk, D):
+    from fp4_post_b200 import decoder, ops
+    g = torch.Generator(device="cuda").manual_seed(T * D)
+    q = torch.randn(B, T, Hq, D, device="cuda", generator=g).to(torch.bfloat16)
+    k = torch.randn(B, T, Hk, D, device="cuda", generator=g).to(torch.bfloat16)
+    ang = torch.rand(1, 1, T, D, device="cuda", generator=g) * 6.3
+    cos, sin = ang.cos().to(torch.bfloat16), ang.sin().to(torch.bfloat16)
+    got = ops.rope_pair(q, k, cos, sin)
+    for x, y in zip((q, k), got):
+        want = decoder._rope(x.transpose(1, 2), cos, sin).transpose(1, 2)
+        assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 18944), (3, 7, 40), (8,)])
+def test_silu_times_up_in_one_launch_is_the_torch_expression(shape):
+    from fp4_post_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(shape[-1])
+    gate = (4 * torch.randn(*shape, device="cuda", generator=g)).to(torch.bfloat16)
+    gate.view(-1)[0], gate.view(-1)[1] = float("-inf"), 200.0
+    up = torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+    got, want = ops.silu_mul(gate, up), torch.nn.functional.silu(gate) * up
+    # one bf16 ulp: the two compilations of exp and the division agree, but nothing promises it
+    ok = (got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7
+    assert bool((ok | (got.isnan() & want.isnan())).all())
+    assert float(((got == want) | want.isnan()).float().mean()) > 0.99
