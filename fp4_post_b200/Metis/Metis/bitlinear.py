@@ -30,6 +30,7 @@ import torch.nn as nn
 import torch.nn.init as init
 
 from fp4_post_b200 import ops
+from fp4_post_b200.ops import current_stream, on_stream, recorded_event
 from .quant import *  # noqa: F401,F403  (the reference re-exports its quantizers the same way)
 from .quant import is_native, quant_func, random_lane
 
@@ -79,13 +80,13 @@ class PackedOperand:
             self._qt = self.quantizer.quantize_packed(self.source, transpose=True, mean=self.q.row_vec,
                                                       hadamard_signs=self.rotate)
         if self._qt_event is not None:
-            torch.cuda.current_stream(self._qt.codes.device).wait_event(self._qt_event)
+            current_stream(self._qt.codes.device).wait_event(self._qt_event)
         return self._qt
 
     def rowmajor(self):
         """`q`, once its scale pass has run (see _q_event)."""
         if self._q_event is not None:
-            torch.cuda.current_stream(self.q.codes.device).wait_event(self._q_event)
+            current_stream(self.q.codes.device).wait_event(self._q_event)
         return self.q
 
     def join_deferred(self):
@@ -94,7 +95,7 @@ class PackedOperand:
         finished, and a stream capture that ends there sees the other stream joined."""
         for ev in (self._q_event, self._qt_event):
             if ev is not None:
-                torch.cuda.current_stream(self.q.codes.device).wait_event(ev)
+                current_stream(self.q.codes.device).wait_event(ev)
 
     def dense(self, dtype):
         """The dequantized tensor the reference would have produced (mean added back)."""
@@ -380,8 +381,7 @@ class LinearLowbitFunction(torch.autograd.Function):
                     mean_cache[cache_key] = (fresh.detach().reshape(1, -1), rows)
         mean_event = None
         if mean is not None and flat.is_cuda:
-            mean_event = torch.cuda.Event()
-            mean_event.record()             # work that needs only the mean may overlap the quantization
+            mean_event = recorded_event(current_stream(flat.device))             # work that needs only the mean may overlap the quantization
         rotate = LinearLowbitFunction._wgrad_rotation()
         if both and _dual_ok(flat):
             # a centred operand's weight-gradient product needs the token sums of the transposed quantization
@@ -551,14 +551,12 @@ def _finish_beside(finish, device, index=2):
     for such passes (index 2: activations and gradients, 4: weights, which are quantized on the second stream and
     would otherwise hold up the activation's pass queued behind theirs), after everything issued so far on the
     current stream.  Returns the event that marks it done."""
-    here, beside = torch.cuda.current_stream(device), _aux_stream(device, index)
-    issued = torch.cuda.Event()
-    issued.record(here)
+    here, beside = current_stream(device), _aux_stream(device, index)
+    issued = recorded_event(here)
     beside.wait_event(issued)
-    with torch.cuda.stream(beside):
+    with on_stream(beside):
         finish()
-        done = torch.cuda.Event()
-        done.record(beside)
+        done = recorded_event(beside)
     return done
 
 
@@ -599,22 +597,20 @@ def forward_group(layers, x: torch.Tensor):
     if not parallel:
         return [layer(x) for layer in layers]
     dev = x.device
-    main = torch.cuda.current_stream(dev)
+    main = current_stream(dev)
     if getattr(layers[0], "activation_group", None) is not None:
         LinearLowbitFunction.mean_cache = layers[0].mean_cache
         layers[0]._get_shared_quantized_input(x)      # a grouped activation is quantized here, once, in front of the fork
-    fork = torch.cuda.Event()
-    fork.record(main)
+    fork = recorded_event(main)
     outs = [None] * len(layers)
     try:
         for i in range(1, len(layers)):
             _BRANCH = i
             st = _aux_stream(dev, 3)
             st.wait_event(fork)
-            with torch.cuda.stream(st):
+            with on_stream(st):
                 outs[i] = layers[i](x)
-                done = torch.cuda.Event()
-                done.record(st)
+                done = recorded_event(st)
             outs[i].record_stream(main)
             outs[i] = (outs[i], done)
     finally:
@@ -638,9 +634,9 @@ class _beside:
     def __enter__(self):
         if self.event is None:
             return lambda *tensors: None
-        self.main, self.aux = torch.cuda.current_stream(self.device), _aux_stream(self.device)
+        self.main, self.aux = current_stream(self.device), _aux_stream(self.device)
         self.aux.wait_event(self.event)
-        self.ctx = torch.cuda.stream(self.aux)
+        self.ctx = on_stream(self.aux)
         self.ctx.__enter__()
 
         def join(*tensors):
@@ -685,7 +681,7 @@ def _row_sums(q, rotate=None):
     else:
         done = getattr(q, "_row_sums_event", None)
         if done is not None:                        # computed on the second stream (_row_sums_beside)
-            cur = torch.cuda.current_stream(cached.device)
+            cur = current_stream(cached.device)
             cur.wait_event(done)
             cached.record_stream(cur)
     return cached
@@ -707,10 +703,9 @@ def _token_tail(x_t, rotate, rows: int):
         cached = x_t._tail = _add_mean(sums, x_t.col_vec, rows)
         x_t._tail_event = None
         if cached.is_cuda:
-            x_t._tail_event = torch.cuda.Event()
-            x_t._tail_event.record()
+            x_t._tail_event = recorded_event(current_stream(cached.device))
     elif x_t._tail_event is not None:
-        cur = torch.cuda.current_stream(cached.device)
+        cur = current_stream(cached.device)
         cur.wait_event(x_t._tail_event)
         cached.record_stream(cur)
     return cached
@@ -724,14 +719,12 @@ def _row_sums_beside(op: "PackedOperand"):
     if getattr(x_t, "_row_sums", None) is not None:
         return
     dev = x_t.codes.device
-    main, aux = torch.cuda.current_stream(dev), _aux_stream(dev)
-    queued = torch.cuda.Event()
-    queued.record(main)
+    main, aux = current_stream(dev), _aux_stream(dev)
+    queued = recorded_event(main)
     aux.wait_event(queued)
-    with torch.cuda.stream(aux):
+    with on_stream(aux):
         _row_sums(x_t, op.rotate)
-        done = torch.cuda.Event()
-        done.record(aux)
+        done = recorded_event(aux)
         x_t._row_sums_event = done
         if x_t.col_vec is not None:
             _token_tail(x_t, op.rotate, op.q.shape[0])
@@ -898,7 +891,7 @@ class MetisFusedFunction(torch.autograd.Function):
 
         def ready(op):
             if op.ready_event is not None:             # quantized on another stream: order this stream after it, once
-                torch.cuda.current_stream(xa.q.device).wait_event(op.ready_event)
+                current_stream(xa.q.device).wait_event(op.ready_event)
                 op.ready_event = None
         if xa.mean is not None:
             # mu_x V^T and mu_x R^T need the mean only: on the second stream they run beside the
@@ -912,32 +905,29 @@ class MetisFusedFunction(torch.autograd.Function):
                 ready(rq)
             with _beside(xa.mean_event if overlap else None, xa.mean.device) as join:
                 if overlap and vq.ready_event is not None:      # quantized on a stream of their own: order this one after each
-                    torch.cuda.current_stream(xa.mean.device).wait_event(vq.ready_event)
+                    current_stream(xa.mean.device).wait_event(vq.ready_event)
                 row_v = ops.nvfp4_gemv(vq.q, xa.mean)
                 # the product with V needs only this one: the pass over the (much larger) residual
                 # weight stays off the critical path until the residual product
-                v_ready = torch.cuda.Event() if overlap else None
-                if v_ready is not None:
-                    v_ready.record()
+                v_ready = recorded_event(current_stream(xa.mean.device)) if overlap else None
                 # a parameter is complete whatever stream this is (a cast of one is ordered on the current stream only)
                 if isinstance(bias, torch.nn.Parameter):
                     bias_row = bias.float()
                 late = overlap and M <= 128
                 if overlap and rq.ready_event is not None:
-                    torch.cuda.current_stream(xa.mean.device).wait_event(rq.ready_event)
+                    current_stream(xa.mean.device).wait_event(rq.ready_event)
                 if not late:
                     row_r = ops.nvfp4_gemv(rq.q, xa.mean)
             if v_ready is not None:
-                torch.cuda.current_stream(xa.mean.device).wait_event(v_ready)
-                row_v.record_stream(torch.cuda.current_stream(xa.mean.device))
+                current_stream(xa.mean.device).wait_event(v_ready)
+                row_v.record_stream(current_stream(xa.mean.device))
                 if not late:
                     join_residual = lambda: join(row_r, bias_row)
             rank1_v.append((None, row_v))
             if late:
                 # At decode sizes the pass over the residual weight fills every SM for longer than the quantization takes;
                 # issued in front of the product with V it would make that one (a few CTAs that need an SM each) wait.
-                quantized = torch.cuda.Event()
-                quantized.record()
+                quantized = recorded_event(current_stream(xa.mean.device))
 
                 def row_of_residual():
                     with _beside(quantized, xa.mean.device) as join_late:
@@ -1069,12 +1059,11 @@ class MetisFusedFunction(torch.autograd.Function):
             x_t = xa.transposed()
             if centred and getattr(x_t, "_row_sums", None) is None:
                 _row_sums(x_t, xa.rotate)   # cached on x_t and read by both branches
-            main, aux = torch.cuda.current_stream(), _aux_stream(g.device)
+            main, aux = current_stream(g.device), _aux_stream(g.device)
             aux.wait_stream(main)
             # the weight-gradient product comes first and reads the transposed output only
             dg = F._pack_centred(g, quantizer, centred, both=True, defer="rowmajor" if F.defer_scale_pass else None)
-            dg_done = torch.cuda.Event()
-            dg_done.record(main)
+            dg_done = recorded_event(main)
             for_dx = {}
 
             if dg.mean is not None:
@@ -1082,10 +1071,9 @@ class MetisFusedFunction(torch.autograd.Function):
                 # belongs to neither chain, so it gets a stream of its own and runs wherever there is room
                 third = _aux_stream(g.device, 1)
                 third.wait_event(dg.mean_event)
-                with torch.cuda.stream(third):
+                with on_stream(third):
                     mean_row = ops.nvfp4_gemv(rq.transposed(), dg.mean)
-                    mean_row_done = torch.cuda.Event()
-                    mean_row_done.record(third)
+                    mean_row_done = recorded_event(third)
 
             def input_gradient_operands(dv):
                 # What the input-gradient product needs from this stream goes out ahead of this branch's own
@@ -1093,10 +1081,9 @@ class MetisFusedFunction(torch.autograd.Function):
                 if fuse_dx:
                     aux.wait_event(dg_done)                # the unit of Q(g)
                     for_dx["t_acc"] = side_operand(dv, dg)
-                for_dx["ready"] = torch.cuda.Event()
-                for_dx["ready"].record(aux)
+                for_dx["ready"] = recorded_event(aux)
 
-            with torch.cuda.stream(aux), random_lane(1):
+            with on_stream(aux), random_lane(1):
                 grad_u, grad_s, dv, grad_v, side = low_rank_branch(input_gradient_operands)
             grad_r = residual_weight_gradient(dg)
             main.wait_event(for_dx["ready"])
@@ -1323,16 +1310,14 @@ class BitLinear(nn.Module):
             return                                        # (probably) cache hits: nothing to overlap
         # a stream of their own (not the one the mean's row vectors run on: those would queue behind the residual
         # weight's quantization although the first of them needs V only)
-        main, aux = torch.cuda.current_stream(x.device), _aux_stream(x.device, 5)
+        main, aux = current_stream(x.device), _aux_stream(x.device, 5)
         aux.wait_stream(main)
-        with torch.cuda.stream(aux):
+        with on_stream(aux):
             # the small one first: the product with V is the first consumer on the forward's critical path
             vq = v._get_quantized_weight(v.weight.to(v.compute_dtype))
-            v_done = torch.cuda.Event()
-            v_done.record(aux)
+            v_done = recorded_event(aux)
             rq = w._get_quantized_weight(w.weight.to(w.compute_dtype))
-            r_done = torch.cuda.Event()
-            r_done.record(aux)
+            r_done = recorded_event(aux)
         for op, done in ((vq, v_done), (rq, r_done)):
             if isinstance(op, PackedOperand) and op.fresh:
                 op.ready_event = done

@@ -42,10 +42,17 @@ static inline WorkspaceView view_workspace(void* ws) {
 int32_t launch_finalize(const WorkspaceView& ws, int64_t R, int64_t C, int32_t sf_layout,
                         uint8_t* scales, float* unit, cudaStream_t st, uint64_t* offset_ctr = nullptr,
                         const unsigned int* records = nullptr, int32_t which = 0);
+// Where a workspace that holds METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than [R, C] needs has its per-CTA records
+// (nullptr: it does not).  Word -1 is their number, three words each: largest maximum (of the row-major, of the
+// transposed output), error.
+constexpr int kMaxRecords = 640;
+unsigned int* workspace_records(void* workspace, int64_t workspace_bytes, int64_t R, int64_t C);
 int32_t check_quant_outputs(int64_t R, int64_t C, int32_t sf_layout, const void* codes,
                             const void* scales, const void* unit, const void* workspace,
                             int64_t workspace_bytes);
 int device_sm_count();
+// cudaOccupancyMaxActiveBlocksPerMultiprocessor, asked once per kernel, shape and device (at least 1)
+int resident_ctas(const void* kernel, int threads, size_t smem);
 int gemm_sm_budget(int32_t limit);   // device_sm_count(), capped by a positive per-call limit
 
 // ---- overlapped launches ------------------------------------------------------------------------

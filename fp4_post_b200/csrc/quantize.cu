@@ -10,7 +10,10 @@
 #include "common.cuh"
 #include "tma.cuh"
 
+#include <atomic>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 
 namespace metis {
@@ -137,7 +140,7 @@ constexpr uint64_t kColumnStream = 1ull << 63;             // Philox counter spa
 
 // Workspace of the dual quantizer: word 63 = number of CTA records, records from word 64 on (3 words per CTA),
 // then the block maxima of Q and of Qt.
-constexpr int kDualMaxCtas = 640;
+constexpr int kDualMaxCtas = kMaxRecords;
 constexpr int kDualHeaderBytes = 256 + ((kDualMaxCtas * 3 * 4 + 255) / 256) * 256;
 
 // How a CTA walks the tiles: their number, those along a row of x, and gridDim.x split into whole rows of tiles
@@ -874,11 +877,31 @@ static int64_t col_mean_splits(int64_t rows) {
 // ---- launch helpers ------------------------------------------------------------------------------------------
 
 int device_sm_count() {
+  static std::atomic<int> known[64] = {};                // by device; 0: not asked yet
   int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
-    return n;
-  return 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  const bool keep = dev >= 0 && dev < 64;
+  if (keep && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+  if (keep) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+int resident_ctas(const void* kernel, int threads, size_t smem) {
+  static std::mutex mutex;
+  static std::map<std::tuple<const void*, int, size_t, int>, int> known;
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto key = std::make_tuple(kernel, threads, smem, dev);
+  const auto hit = known.find(key);
+  if (hit != known.end()) return hit->second;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1) return 1;
+  known[key] = n;
+  return n;
+}
+unsigned int* workspace_records(void* workspace, int64_t workspace_bytes, int64_t R, int64_t C) {
+  const int64_t at = (metis_nvfp4_quantize_workspace_bytes(R, C) + 15) / 16 * 16;
+  return workspace_bytes >= at + 16 + kMaxRecords * 12 ? reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + at) + 4 : nullptr;
 }
 static int sm_count() { return device_sm_count(); }
 
@@ -898,7 +921,7 @@ static void launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, cons
   int64_t gy = ceil_div(rows, by);
   // four waves of resident CTAs (grid-stride over the rows): whole waves leave no tail
   int per_sm = 0;
-#define METIS_OCC_ROWS(MEAN, SR) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_rows_kernel<T, MEAN, SR>, kQuantThreads, 0)
+#define METIS_OCC_ROWS(MEAN, SR) per_sm = resident_ctas(reinterpret_cast<const void*>(quantize_rows_kernel<T, MEAN, SR>), kQuantThreads, 0)
   if (mean) { if (sr) METIS_OCC_ROWS(true, true); else METIS_OCC_ROWS(true, false); }
   else      { if (sr) METIS_OCC_ROWS(false, true); else METIS_OCC_ROWS(false, false); }
 #undef METIS_OCC_ROWS
@@ -1050,9 +1073,7 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
   // With METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than it needs the workspace also holds a record per CTA of the first
   // pass, as in the dual quantizer; without them the running maximum and the error word are zeroed in front of it, and
   // that memset node costs 3-4 us (16 x 14336: 8.2 us with it, 4.9 without; 1120 x 3584: 12.4, 8.1).
-  const int64_t records_at = (metis_nvfp4_quantize_workspace_bytes(R, C) + 15) / 16 * 16;
-  unsigned int* records = workspace_bytes >= records_at + 16 + kDualMaxCtas * 12
-      ? reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + records_at) + 4 : nullptr;
+  unsigned int* records = workspace_records(workspace, workspace_bytes, R, C);
   // One cluster for the whole tensor: with records, only where two launches over many SMs are not faster (16 x 4096:
   // 4.3 us against 4.5; 64 x 3584 on the cluster's 8 SMs: 7.1 against 5.0).
   int64_t tiles = 0, padded_words = 0;

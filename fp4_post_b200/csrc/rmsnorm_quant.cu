@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_quantize_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
                         const TG* __restrict__ gamma, float eps, uint2* __restrict__ codes,
                         float* __restrict__ amax_out, unsigned int* __restrict__ gmax,
-                        void* __restrict__ norm_out) {
+                        unsigned int* __restrict__ records, void* __restrict__ norm_out) {
   grid_dependency_wait();
   // The product normalised(x) * gamma has the promoted dtype: bf16 only if both are bf16.
   constexpr bool kProductBf16 = (sizeof(TX) == 2) && (sizeof(TG) == 2);
@@ -153,7 +153,22 @@ rmsnorm_quantize_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, 
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) running = fmaxf(running, __shfl_xor_sync(0xffffffffu, running, o));
-  if (lane == 0 && running > 0.0f) atomicMax(gmax, __float_as_uint(running));
+  if (!records) {
+    if (lane == 0 && running > 0.0f) atomicMax(gmax, __float_as_uint(running));
+    return;
+  }
+  // a record per CTA: nobody has to zero a shared maximum first
+  __shared__ float s_top[kNormThreads / 32];
+  if (lane == 0) s_top[warp] = running;
+  __syncthreads();
+  if (tid == 0) {
+    float top = 0.0f;
+    for (int w = 0; w < (bx * by + 31) / 32; ++w) top = fmaxf(top, s_top[w]);
+    records[3 * blockIdx.x] = __float_as_uint(top);
+    records[3 * blockIdx.x + 1] = 0u;
+    records[3 * blockIdx.x + 2] = 0u;
+    if (blockIdx.x == 0) records[-1] = gridDim.x;
+  }
 }
 
 // ---- decode-sized inputs: one launch ---------------------------------------------------------------
@@ -374,31 +389,33 @@ static int32_t try_small(const TX* x, int64_t rows, int64_t cols, int64_t ld, co
   return METIS_OK;
 }
 
+// *records: in: where the per-CTA records may go (or nullptr); out: nullptr if the running maximum was used instead
 template <typename TX, typename TG, int kBlocks>
-static void launch_norm(const TX* x, int64_t rows, int bpr, int bx, int64_t ld, const TG* gamma, float eps,
-                        uint32_t* codes, const WorkspaceView& ws, void* norm_out, int sms, cudaStream_t st) {
+static int32_t launch_norm(const TX* x, int64_t rows, int bpr, int bx, int64_t ld, const TG* gamma, float eps,
+                           uint32_t* codes, const WorkspaceView& ws, unsigned int** records, void* norm_out, int sms, cudaStream_t st) {
   const int by = kNormThreads / bx;
   // persistent CTAs: exactly as many as are resident at once, so that all of them finish together
-  int per_sm = 0;
-  if (norm_out) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rmsnorm_quantize_kernel<TX, TG, kBlocks, true>, bx * by, 0);
-  else          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rmsnorm_quantize_kernel<TX, TG, kBlocks, false>, bx * by, 0);
-  if (per_sm < 1) per_sm = 1;
-  int64_t blocks = (int64_t)sms * per_sm;
+  const void* kern = norm_out ? reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, true>)
+                              : reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, false>);
+  int64_t blocks = (int64_t)sms * resident_ctas(kern, bx * by, 0);
   const int64_t need = ceil_div(rows, by);
   if (blocks > need) blocks = need;
+  if (blocks > kMaxRecords) *records = nullptr;
+  if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
   const dim3 b((unsigned)bx, (unsigned)by);
   uint2* c2 = reinterpret_cast<uint2*>(codes);
   if (norm_out)
-    launch_overlapped(kLaunchStream, rmsnorm_quantize_kernel<TX, TG, kBlocks, true>, dim3((unsigned)blocks), b, 0, st,
-                      x, (int)rows, bpr, ld, gamma, eps, c2, ws.amax, ws.gmax, norm_out);
+    METIS_CUDA_OK(launch_overlapped(kLaunchStream, rmsnorm_quantize_kernel<TX, TG, kBlocks, true>, dim3((unsigned)blocks), b, 0, st,
+                                    x, (int)rows, bpr, ld, gamma, eps, c2, ws.amax, ws.gmax, *records, norm_out));
   else
-    launch_overlapped(kLaunchStream, rmsnorm_quantize_kernel<TX, TG, kBlocks, false>, dim3((unsigned)blocks), b, 0, st,
-                      x, (int)rows, bpr, ld, gamma, eps, c2, ws.amax, ws.gmax, norm_out);
+    METIS_CUDA_OK(launch_overlapped(kLaunchStream, rmsnorm_quantize_kernel<TX, TG, kBlocks, false>, dim3((unsigned)blocks), b, 0, st,
+                                    x, (int)rows, bpr, ld, gamma, eps, c2, ws.amax, ws.gmax, *records, norm_out));
+  return METIS_OK;
 }
 
 template <typename TX, typename TG>
 static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t ld, const TG* gamma,
-                               float eps, uint32_t* codes, const WorkspaceView& ws, void* norm_out,
+                               float eps, uint32_t* codes, const WorkspaceView& ws, unsigned int** records, void* norm_out,
                                int sms, cudaStream_t st) {
   const int bpr = (int)(cols >> 4);
   // threads along the row: whole warps, as many as the row has 32-block groups (hidden 1536 runs
@@ -412,13 +429,12 @@ static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t 
     while (bx < bpr) bx <<= 1;
   }
   const int per_thread = (bpr + bx - 1) / bx;
-  if (per_thread <= 1) launch_norm<TX, TG, 1>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, norm_out, sms, st);
-  else if (per_thread <= 2) launch_norm<TX, TG, 2>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, norm_out, sms, st);
-  else if (per_thread <= 3) launch_norm<TX, TG, 3>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, norm_out, sms, st);
-  else if (per_thread <= 5) launch_norm<TX, TG, 5>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, norm_out, sms, st);
-  else if (per_thread <= 8) launch_norm<TX, TG, 8>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, norm_out, sms, st);
-  else return fail(METIS_ERR_TOO_LARGE, "rmsnorm rows longer than %d elements are not supported", 8 * kNormThreads * 16);
-  return METIS_OK;
+  if (per_thread <= 1) return launch_norm<TX, TG, 1>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+  if (per_thread <= 2) return launch_norm<TX, TG, 2>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+  if (per_thread <= 3) return launch_norm<TX, TG, 3>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+  if (per_thread <= 5) return launch_norm<TX, TG, 5>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+  if (per_thread <= 8) return launch_norm<TX, TG, 8>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+  return fail(METIS_ERR_TOO_LARGE, "rmsnorm rows longer than %d elements are not supported", 8 * kNormThreads * 16);
 }
 
 // ---- RMSNorm with the column sums of its output (the mean-centred path) ------------------------------------
@@ -619,20 +635,20 @@ extern "C" int32_t metis_rmsnorm_nvfp4_quantize(const void* x, int32_t x_dtype, 
     rc = try_small(static_cast<const float*>(x), rows, cols, ld, static_cast<const float*>(gamma), eps, codes, sf_layout, scales, unit, norm_out, st, &taken);
   if (rc || taken) return rc;
   const WorkspaceView ws = view_workspace(workspace);
-  METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
+  unsigned int* records = workspace_records(workspace, workspace_bytes, rows, cols);
   const int sms = device_sm_count();
   uint32_t* c32 = reinterpret_cast<uint32_t*>(codes);
   if (x_dtype == METIS_DTYPE_BF16 && gamma_dtype == METIS_DTYPE_BF16)
-    rc = dispatch_chunks(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, static_cast<const __nv_bfloat16*>(gamma), eps, c32, ws, norm_out, sms, st);
+    rc = dispatch_chunks(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, static_cast<const __nv_bfloat16*>(gamma), eps, c32, ws, &records, norm_out, sms, st);
   else if (x_dtype == METIS_DTYPE_BF16)
-    rc = dispatch_chunks(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, static_cast<const float*>(gamma), eps, c32, ws, norm_out, sms, st);
+    rc = dispatch_chunks(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, static_cast<const float*>(gamma), eps, c32, ws, &records, norm_out, sms, st);
   else if (gamma_dtype == METIS_DTYPE_BF16)
-    rc = dispatch_chunks(static_cast<const float*>(x), rows, cols, ld, static_cast<const __nv_bfloat16*>(gamma), eps, c32, ws, norm_out, sms, st);
+    rc = dispatch_chunks(static_cast<const float*>(x), rows, cols, ld, static_cast<const __nv_bfloat16*>(gamma), eps, c32, ws, &records, norm_out, sms, st);
   else
-    rc = dispatch_chunks(static_cast<const float*>(x), rows, cols, ld, static_cast<const float*>(gamma), eps, c32, ws, norm_out, sms, st);
+    rc = dispatch_chunks(static_cast<const float*>(x), rows, cols, ld, static_cast<const float*>(gamma), eps, c32, ws, &records, norm_out, sms, st);
   if (rc) return rc;
   METIS_CUDA_OK(cudaGetLastError());
-  return launch_finalize(ws, rows, cols, sf_layout, scales, unit, st);
+  return launch_finalize(ws, rows, cols, sf_layout, scales, unit, st, nullptr, records, 0);
 }
 
 

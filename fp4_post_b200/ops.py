@@ -35,8 +35,11 @@ def _need_cuda(t: torch.Tensor, what: str) -> None:
         raise RuntimeError(f"{what} must be a CUDA tensor: the NVFP4 path has no CPU fallback")
 
 
+_current_device = torch._C._cuda_getDevice            # torch.cuda.current_device() without its checks: a CUDA tensor exists
+
+
 def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(_current_device())
 
 
 class _on_device:
@@ -44,7 +47,7 @@ class _on_device:
     __slots__ = ("guard",)
 
     def __init__(self, dev: torch.device):
-        self.guard = None if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+        self.guard = None if dev.index == _current_device() else torch.cuda.device(dev)
 
     def __enter__(self):
         if self.guard is not None:
@@ -55,14 +58,72 @@ class _on_device:
             self.guard.__exit__(*exc)
 
 
+_STREAMS = {}          # (stream id, device index, device type) -> torch.cuda.Stream: handles only, rebuilt when dropped
+
+
+def _stream_object(key) -> "torch.cuda.Stream":
+    st = _STREAMS.get(key)
+    if st is None:
+        if len(_STREAMS) >= 256:
+            _STREAMS.clear()
+        st = _STREAMS[key] = torch.cuda.Stream(stream_id=key[0], device_index=key[1], device_type=key[2])
+    return st
+
+
+def current_stream(dev: torch.device) -> "torch.cuda.Stream":
+    """torch.cuda.current_stream(dev) for a device with an index, without building a new handle on every call."""
+    return _stream_object(torch._C._cuda_getCurrentStream(_current_device() if dev.index is None else dev.index))
+
+
+class on_stream:
+    """torch.cuda.stream(st) at a tenth of its cost where st's device is the current one (elsewhere: the same)."""
+    __slots__ = ("st", "prev", "full")
+
+    def __init__(self, st: "torch.cuda.Stream"):
+        self.st = st
+
+    def __enter__(self):
+        st = self.st
+        self.full = None
+        if st.device_index != _current_device():
+            self.full = torch.cuda.stream(st)
+            self.full.__enter__()
+            return
+        self.prev = torch._C._cuda_getCurrentStream(st.device_index)
+        torch._C._cuda_setStream(stream_id=st.stream_id, device_index=st.device_index, device_type=st.device_type)
+
+    def __exit__(self, *exc):
+        if self.full is not None:
+            self.full.__exit__(*exc)
+            return
+        prev = self.prev
+        torch._C._cuda_setStream(stream_id=prev[0], device_index=prev[1], device_type=prev[2])
+
+
+def recorded_event(st: "torch.cuda.Stream") -> "torch.cuda.Event":
+    ev = torch.cuda.Event()
+    ev.record(st)
+    return ev
+
+
+def _sf_bytes(R: int, Cc: int, sf_layout: int) -> int:
+    """metis_nvfp4_sf_bytes: one byte per 16 elements, or whole tiles of 128 rows x 256 elements."""
+    if sf_layout == cabi.SF_MMA:
+        return ((R + 127) // 128) * ((Cc + 255) // 256) * 2048
+    if sf_layout == cabi.SF_ROWMAJOR:
+        return R * (Cc // 16)
+    return cabi.lib().metis_nvfp4_sf_bytes(R, Cc, sf_layout)
+
+
 def _packed_buffers(L, R: int, Cc: int, sf_layout: int, dev):
     """codes, scales and unit of one quantized tensor as views of a single allocation."""
-    n_codes = R * (Cc // 2)
-    n_scales = L.metis_nvfp4_sf_bytes(R, Cc, sf_layout)
+    half = Cc // 2
+    n_codes, n_scales = R * half, _sf_bytes(R, Cc, sf_layout)
     o_scales = (n_codes + 255) & ~255
     o_unit = (o_scales + n_scales + 255) & ~255
     buf = torch.empty(o_unit + 16, dtype=torch.uint8, device=dev)
-    return buf[:n_codes].view(R, Cc // 2), buf[o_scales:o_scales + n_scales], buf[o_unit:o_unit + 4].view(torch.float32)
+    return (torch.as_strided(buf, (R, half), (half, 1)), torch.as_strided(buf, (n_scales,), (1,), o_scales),
+            torch.as_strided(buf, (4,), (1,), o_unit).view(torch.float32))
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -247,7 +308,7 @@ def nvfp4_quantize_dual(x: torch.Tensor, *, stochastic: bool = False, seed: int 
                                                      ws.data_ptr(), ws.numel(), _stream())
         cabi.check(rc2, "metis_nvfp4_quantize_dual_finish")
         # the buffers were allocated on the quantizing call's stream and are now also used on this one
-        cur = torch.cuda.current_stream(dev)
+        cur = current_stream(dev)
         for t in (ws, scales, unit, codes_t, scales_t, unit_t, sums):
             if t is not None:
                 t.record_stream(cur)
@@ -271,7 +332,7 @@ def rmsnorm_nvfp4_quantize(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e
     dev = x2.device
     with _on_device(dev):
         codes, scales, unit = _packed_buffers(L, rows, cols, sf_layout, dev)
-        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(rows, cols), dtype=torch.uint8, device=dev)
+        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(rows, cols) + cabi.QUANTIZE_EXTRA_WORKSPACE, dtype=torch.uint8, device=dev)
         norm = None
         if return_norm:
             out_dtype = torch.bfloat16 if (x2.dtype == torch.bfloat16 and gamma.dtype == torch.bfloat16) else torch.float32

@@ -98,8 +98,9 @@ int64_t metis_nvfp4_sf_bytes(int64_t R, int64_t C, int32_t sf_layout);
 /* Bytes of scratch metis_nvfp4_quantize / metis_rmsnorm_nvfp4_quantize need for a
  * quantized [R, C] tensor (per-block fp32 amax + a 256-byte header). */
 int64_t metis_nvfp4_quantize_workspace_bytes(int64_t R, int64_t C);
-/* With this many bytes more than metis_nvfp4_quantize_workspace_bytes, metis_nvfp4_quantize issues kernels only (no
- * memset in front of them); the result is the same either way. */
+/* With this many bytes more than metis_nvfp4_quantize_workspace_bytes, metis_nvfp4_quantize and
+ * metis_rmsnorm_nvfp4_quantize issue kernels only (no memset in front of them) wherever their first pass has at most 640
+ * CTAs; the result is the same either way. */
 #define METIS_QUANTIZE_EXTRA_WORKSPACE 8192
 
 /* ---- quantizers ----------------------------------------------------------------------- */

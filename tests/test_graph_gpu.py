@@ -90,3 +90,18 @@ def test_stochastic_quantizer_counter_advances_once_per_call():
     assert torch.equal(a.codes, c.codes) and torch.equal(a.scales, c.scales)
     with pytest.raises(ValueError):
         ops.nvfp4_quantize(x, stochastic=True, offset_counter=torch.zeros(1, dtype=torch.int32, device=DEV))
+
+
+def test_light_stream_helpers_agree_with_torch():
+    from fp4_post_b200 import ops
+    dev = torch.device("cuda", torch.cuda.current_device())
+    st, before = torch.cuda.Stream(device=dev), torch.cuda.current_stream(dev)
+    assert ops.current_stream(dev) == before
+    with pytest.raises(KeyError):
+        with ops.on_stream(st):
+            assert torch.cuda.current_stream(dev) == st == ops.current_stream(dev)
+            with ops.on_stream(before):
+                assert ops.current_stream(dev) == before
+            assert ops.current_stream(dev) == st
+            raise KeyError
+    assert torch.cuda.current_stream(dev) == before
