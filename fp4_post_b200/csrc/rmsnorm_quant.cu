@@ -186,10 +186,13 @@ __device__ __forceinline__ float norm_block(const float (&v)[16], float rs, cons
     RawBlock<__nv_bfloat16> graw;
     graw.load(reinterpret_cast<const __nv_bfloat16*>(gamma16));
     const uint32_t gw[8] = {graw.a.x, graw.a.y, graw.a.z, graw.a.w, graw.b.x, graw.b.y, graw.b.z, graw.b.w};
+    const f32x2 rs2 = pack2(rs, rs);
     __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const __nv_bfloat162 n2 = __floats2bfloat162_rn(__fmul_rn(v[2 * i], rs), __fmul_rn(v[2 * i + 1], rs));
+      float n0, n1;
+      split2(mul2(pack2(v[2 * i], v[2 * i + 1]), rs2), n0, n1);
+      const __nv_bfloat162 n2 = __floats2bfloat162_rn(n0, n1);
       const __nv_bfloat162 p2 = __hmul2(n2, *reinterpret_cast<const __nv_bfloat162*>(&gw[i]));
       amax2 = __hmax2(amax2, __habs2(p2));
       const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
@@ -209,6 +212,113 @@ __device__ __forceinline__ float norm_block(const float (&v)[16], float rs, cons
       y[i + 1] = __fmul_rn(n1, g[i + 1]);
     }
     return abs_max16(y);
+  }
+}
+
+// ---- long inputs, bf16 rows of up to 4096 elements: a warp per row --------------------------------------------
+// With a CTA per row two barriers stand between its parts (3.1 of 10.5 stalled warps waited there, issue slots 66 % busy,
+// 18 instructions per element).  A warp that owns its row needs none: the row stays in registers as loaded
+// (kM blocks of 16 elements per lane, block lane + 32 j), the sum of squares goes through shuffles.  The sums are added
+// in the order of the CTA-per-row kernel (16 squares of a block one after the other, lanes by butterfly, then the groups
+// of 32 blocks in order), so the results are its results; two blocks' chains share one packed instruction.  Measured at
+// 65536 x 3584 this pass 172 -> 150 us, 65536 x 1536 80 -> 64, 2048 x 2048 6.8 -> 4.8.  Loads that leave L2 first (to keep
+// the block maxima there for the scale pass) change nothing here and cost the tile kernels of quantize.cu 20 %; a prefetch
+// of the next row into L2 changes nothing either.
+constexpr int kNormRowThreads = 256;
+constexpr int64_t kNormRowsMinRows = 1024;                  // fewer rows do not fill the SMs: 512 x 4096 6.8 us against 3.8
+template <typename TG, int kM, bool kWriteNorm>
+__global__ void __launch_bounds__(kNormRowThreads, kM <= 3 ? 3 : 2)
+rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
+                             const TG* __restrict__ gamma, float eps, uint2* __restrict__ codes,
+                             float* __restrict__ amax_out, unsigned int* __restrict__ gmax,
+                             unsigned int* __restrict__ records, void* __restrict__ norm_out) {
+  grid_dependency_wait();
+  constexpr bool kProductBf16 = sizeof(TG) == 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float n_cols = (float)(blocks_per_row * 16);
+  float running = 0.0f;
+  const int row_step = gridDim.x * (kNormRowThreads / 32);
+  for (int r = blockIdx.x * (kNormRowThreads / 32) + warp; r < rows; r += row_step) {
+    const __nv_bfloat16* row = x + (int64_t)r * ld;
+    RawBlock<__nv_bfloat16> raw[kM];
+#pragma unroll
+    for (int j = 0; j < kM; ++j) {
+      raw[j].a = raw[j].b = make_uint4(0u, 0u, 0u, 0u);
+      if (lane + 32 * j < blocks_per_row) raw[j].load(row + (lane + 32 * j) * 16);
+    }
+    float ss[kM];
+#pragma unroll
+    for (int j = 0; j < kM; j += 2) {
+      float v[16], w[16];
+      raw[j].unpack(v);
+      if (j + 1 < kM) {
+        raw[j + 1 < kM ? j + 1 : j].unpack(w);
+        f32x2 acc = 0ull;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const f32x2 e = pack2(v[i], w[i]);
+          acc = fma2(e, e, acc);
+        }
+        split2(acc, ss[j], ss[j + 1 < kM ? j + 1 : j]);
+      } else {
+        ss[j] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) ss[j] = __fmaf_rn(v[i], v[i], ss[j]);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int j = 0; j < kM; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], o);
+    }
+    float tot = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kM; ++j) tot += ss[j];
+    const float rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, n_cols), eps)));   // llama.py:23-24
+#pragma unroll
+    for (int j = 0; j < kM; ++j) {
+      const int bc = lane + 32 * j;
+      if (bc >= blocks_per_row) continue;
+      float v[16], y[16];
+      raw[j].unpack(v);
+      const float a = norm_block<__nv_bfloat16, TG>(v, rs, gamma + bc * 16, y);
+      uint32_t packed[2];
+      quantize_rn<2>(y, block_scale_from_amax(a), packed);
+      const int64_t b = (int64_t)r * blocks_per_row + bc;
+      codes[b] = make_uint2(packed[0], packed[1]);
+      amax_out[b] = a;
+      running = fmaxf(running, a);
+      if (kWriteNorm) {
+        if (kProductBf16) {
+          __nv_bfloat162 o[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);   // exact: already bf16 values
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(norm_out) + b * 16);
+          dst[0] = reinterpret_cast<uint4*>(o)[0];
+          dst[1] = reinterpret_cast<uint4*>(o)[1];
+        } else {
+          float4* dst = reinterpret_cast<float4*>(static_cast<float*>(norm_out) + b * 16);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) dst[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+        }
+      }
+    }
+  }
+  const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(running));       // >= 0: the bits order like the value
+  if (!records) {
+    if (lane == 0 && top > 0u) atomicMax(gmax, top);
+    return;
+  }
+  __shared__ unsigned s_top[kNormRowThreads / 32];
+  if (lane == 0) s_top[warp] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned m = 0u;
+    for (int w = 0; w < kNormRowThreads / 32; ++w) m = max(m, s_top[w]);
+    records[3 * blockIdx.x] = m;
+    records[3 * blockIdx.x + 1] = 0u;
+    records[3 * blockIdx.x + 2] = 0u;
+    if (blockIdx.x == 0) records[-1] = gridDim.x;
   }
 }
 
@@ -413,11 +523,36 @@ static int32_t launch_norm(const TX* x, int64_t rows, int bpr, int bx, int64_t l
   return METIS_OK;
 }
 
+// The warp-per-row kernel for [rows, 16 bpr] bf16, 32 <= bpr <= 256 (512 to 4096 columns).
+template <typename TG, int kM>
+static int32_t launch_norm_rows(const __nv_bfloat16* x, int64_t rows, int bpr, int64_t ld, const TG* gamma, float eps, uint32_t* codes,
+                                const WorkspaceView& ws, unsigned int** records, void* norm_out, int sms, cudaStream_t st) {
+  auto kern = norm_out ? rmsnorm_quantize_rows_kernel<TG, kM, true> : rmsnorm_quantize_rows_kernel<TG, kM, false>;
+  int64_t blocks = (int64_t)sms * resident_ctas(reinterpret_cast<const void*>(kern), kNormRowThreads, 0);
+  const int64_t need = ceil_div(rows, kNormRowThreads / 32);
+  if (blocks > need) blocks = need;
+  if (blocks > kMaxRecords) *records = nullptr;
+  if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
+  METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)blocks), dim3(kNormRowThreads), 0, st, x, (int)rows, bpr, ld, gamma, eps,
+                                  reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, *records, norm_out));
+  return METIS_OK;
+}
+
 template <typename TX, typename TG>
 static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t ld, const TG* gamma,
                                float eps, uint32_t* codes, const WorkspaceView& ws, unsigned int** records, void* norm_out,
                                int sms, cudaStream_t st) {
   const int bpr = (int)(cols >> 4);
+  if constexpr (sizeof(TX) == 2) {
+    if (bpr >= 32 && bpr <= 256 && rows >= kNormRowsMinRows) {
+      switch ((bpr + 31) / 32) {
+#define METIS_NORM_ROWS(M) case M: return launch_norm_rows<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
+        METIS_NORM_ROWS(1); METIS_NORM_ROWS(2); METIS_NORM_ROWS(3); METIS_NORM_ROWS(4);
+        METIS_NORM_ROWS(5); METIS_NORM_ROWS(6); METIS_NORM_ROWS(7); METIS_NORM_ROWS(8);
+#undef METIS_NORM_ROWS
+      }
+    }
+  }
   // threads along the row: whole warps, as many as the row has 32-block groups (hidden 1536 runs
   // with 96 threads per row and two rows per CTA instead of 128 with a quarter of them idle);
   // rows shorter than a warp take the next power of two
