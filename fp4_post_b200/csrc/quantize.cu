@@ -56,8 +56,8 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
       const int64_t b = (int64_t)r * blocks_per_row + bc;
       uint32_t packed[2];
       if (kSR) {
-        if (sr16) quantize16_sr(v, s, rng((uint64_t)b, offset), packed);      // one counter per block
-        else quantize16_sr_hw(v, s, rng((uint64_t)b, offset), packed);
+        if (sr16) quantize16_sr(v, s, rng((uint32_t)b, offset), packed);      // one counter per block
+        else quantize16_sr_hw(v, s, rng((uint32_t)b, offset), packed);
       } else {
         quantize_rn<2>(v, s, packed);
       }
@@ -310,7 +310,7 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
         const float s = block_scale_from_amax(a);
         uint32_t packed[2];
         if (kSR) {
-          const uint64_t b = (uint64_t)(col0 * bpc + (row0 >> 4) + col_ctr + c * bpc);            // block index in Qt
+          const uint32_t b = (uint32_t)(col0 * bpc + (row0 >> 4)) + (uint32_t)(col_ctr + c * bpc);          // block index in Qt
           const uint4 bits = rng(b, kRowsOut ? (offset ^ kColumnStream) : offset);                // alone: the transposed call's own stream
           if (out.sr16) quantize16_sr(v[c], s, bits, packed);
           else quantize16_sr_hw(v[c], s, bits, packed);
@@ -361,8 +361,8 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
         const int64_t blk = tile_blk + row_blk + u * (kRowStep * bpr);
         uint32_t packed[2];
         if (kSR) {
-          if (out.sr16) quantize16_sr(v, s, rng((uint64_t)blk, offset), packed);
-          else quantize16_sr_hw(v, s, rng((uint64_t)blk, offset), packed);
+          if (out.sr16) quantize16_sr(v, s, rng((uint32_t)blk, offset), packed);
+          else quantize16_sr_hw(v, s, rng((uint32_t)blk, offset), packed);
         }
         else     quantize_rn<2>(v, s, packed);
         if (cols_live && r < live_rows) {
