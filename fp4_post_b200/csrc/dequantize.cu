@@ -136,7 +136,7 @@ __device__ __forceinline__ float2 e2m1x2_to_float2(uint32_t byte) {
 }
 
 // The eight codes of a word as floats, exact.
-__device__ __forceinline__ void e2m1x8_to_f32x2(uint32_t w, f32x2 (&f)[4]) {
+__device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
   uint32_t h[4];
   asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
       "cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1; cvt.rn.f16x2.e2m1x2 %2, b2; cvt.rn.f16x2.e2m1x2 %3, b3; }"
@@ -144,112 +144,95 @@ __device__ __forceinline__ void e2m1x8_to_f32x2(uint32_t w, f32x2 (&f)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float2 e = __half22float2(*reinterpret_cast<const __half2*>(&h[i]));
-    f[i] = pack2(e.x, e.y);
+    f[2 * i] = e.x;
+    f[2 * i + 1] = e.y;
   }
 }
 
-// The same product along the tiled scale layout, for matrices with enough rows to fill the SMs.  A 16-byte piece of that
-// layout holds the scales of the rows l, l + 32, l + 64, l + 96 of a 128-row block for 4 blocks (64 columns): a lane takes
-// that unit, i.e. one 16-byte read of scales and 32 bytes of codes of each of four rows, all in flight at once, and
-// the 64 floats of v it needs from shared memory (chunk-major with an odd pitch: no bank conflicts) serve all four
-// rows.  A half-warp takes one l and every 16th group of 64 columns, the eight half-warps of a CTA eight neighbouring l, so
-// 128-byte lines of scales are used whole.  (Reading one scale byte per block and row instead costs a 32-byte sector per
-// 4 blocks, i.e. the bytes of the codes once more.)  The columns are split over the CTAs of a cluster, each of which
-// stages its slice of v only, so that one wave of CTAs shares the work evenly; the slices' sums meet in distributed
-// shared memory in a fixed order.  Two e2m1 codes become two halves with one conversion (exact), products and sums are
-// fp32, two elements per instruction.  Bound by issue and by the conversions (the bytes alone take 6 us at 18944 x 3584).
+// The same product along the tiled scale layout.  A 16-byte piece of that layout holds the scales of the rows l, l + 32,
+// l + 64, l + 96 of a 128-row block for 4 blocks of 16 columns: a warp takes these four rows, lane k of it every 32nd block
+// from k on, so that one 16-byte read of scales (shared by four lanes) and the 16 floats of v (which stay in L1) serve four
+// rows.  (Reading one scale byte per block and row instead costs a 32-byte sector per 4 blocks, i.e. the bytes of the codes
+// once more.)  The additions are those of the other kernels, in the same order: 16 products of a block one after the other,
+// a lane's blocks one after the other, then the lanes pairwise, so which kernel runs does not show in the result (a sum that
+// differs in its last bit can flip the rounding of an activation, and a block of decoder layers makes 1 % of that).
+// With too few rows to fill the SMs that way, `split` warps share the four rows: each takes every split-th round of
+// 32 blocks and parks the block sums in shared memory, and the lanes' sums are then formed from there in order.
+// Two e2m1 codes become two halves with one conversion (exact).  Bound by issue and by the conversions (the bytes alone
+// take 6 us at 18944 x 3584).
 // Measured, gemv_staged_kernel (or, below 2048 columns, gemv_kernel) before and this one after, six weights in turn:
-// 18944 x 3584 20.6 -> 13.5 us, 3584 x 18944 23.8 -> 16.3, 14336 x 4096 21.4 -> 13.6, 4096 x 14336 18.5 -> 14.2,
-// 8960 x 1536 10.4 -> 5.9, 1536 x 8960 7.9 -> 5.7, 4096 x 4096 6.6 -> 5.7; 512 x 3584 3.6 -> 4.3 (too few CTAs: not taken).
-constexpr int kGemvThreads = 128, kGemvLanes = 16, kGemvCtasPerSm = 6;
-constexpr int kGemvMaxSlice = 384;                        // groups of 64 columns a CTA stages: 96 KiB of v
-__global__ void __launch_bounds__(kGemvThreads, kGemvCtasPerSm)
-gemv_tile_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, const float* __restrict__ unit_ptr,
-                 int64_t R, int64_t C, int groups, int slice, const float* __restrict__ v, float* __restrict__ out) {
-  extern __shared__ float4 s_v[];                         // [16][pitch]: chunk j of group g at j * pitch + g
-  __shared__ float s_out[32];
+// 18944 x 3584 20.6 -> 14.1 us, 3584 x 18944 23.8 -> 19.0, 14336 x 4096 21.4 -> 15.3, 4096 x 14336 18.5 -> 16.5,
+// 8960 x 1536 10.4 -> 5.9, 1536 x 8960 7.9 -> 5.9, 4096 x 4096 6.6 -> 6.4.  A form that split the columns over a cluster,
+// with packed multiply-adds and another order of the additions, took 14.6, 16.9, 13.3, 14.7, 5.8, 5.8 and 5.9.
+constexpr int kGemvRowsCtasPerSm = 4;
+template <bool kSplit>
+__global__ void __launch_bounds__(256, kGemvRowsCtasPerSm)
+gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, const float* __restrict__ unit_ptr,
+                 int64_t R, int64_t C, int trips, int split, const float* __restrict__ v, float* __restrict__ out) {
+  extern __shared__ uint32_t s_sums[];                    // kSplit, per four rows: [5][trips][32], the sums of four rows and their scales
   grid_dependency_wait();
-  const int lane = threadIdx.x & (kGemvLanes - 1), unit_l = threadIdx.x / kGemvLanes;
-  const int ranks = (int)cluster_cta_count(), rank = (int)cluster_cta_rank();
-  const int row_group = blockIdx.x / ranks;               // 32 rows: eight l of a 128-row block
-  const int pitch = slice | 1;
-  const int g0 = rank * slice;
-  const int mine = groups - g0 < slice ? groups - g0 : slice;           // may be negative for the last CTAs of a cluster
-  for (int i = threadIdx.x; i < mine * 16; i += kGemvThreads) {
-    const int64_t c = (int64_t)g0 * 64 + i * 4;
-    s_v[(i & 15) * pitch + (i >> 4)] = c < C ? __ldg(reinterpret_cast<const float4*>(v + c)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  }
-  __syncthreads();
-  const int l = (row_group & 3) * 8 + unit_l;
-  const int64_t row0 = (int64_t)(row_group >> 2) * 128 + l;             // this half-warp's rows: row0 + 32 c
-  const int64_t pitch_codes = C >> 1;
-  const uint8_t* row_codes[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int local = kSplit ? warp / split : warp, share = kSplit ? warp - local * split : 0;
+  const int64_t quad = (int64_t)blockIdx.x * (kSplit ? 8 / split : 8) + local;
+  const int64_t row0 = (quad >> 5) * 128 + (quad & 31);   // this warp's rows: row0 + 32 c
+  if (!kSplit && row0 >= R) return;
+  const int sf_cols = (int)(C >> 4);
+  const uint2* row_codes[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) row_codes[c] = codes + (row0 + 32 * c < R ? row0 + 32 * c : R - 1) * pitch_codes + (int64_t)g0 * 32;
-  const uint8_t* row_scales = scales + ((int64_t)(row_group >> 2) * sf_tiles_per_row(C) + g0) * 512 + l * 16;
+  for (int c = 0; c < 4; ++c) row_codes[c] = reinterpret_cast<const uint2*>(codes) + (row0 + 32 * c < R ? row0 + 32 * c : R - 1) * sf_cols;
+  const uint8_t* row_scales = scales + (row0 < R ? quad >> 5 : 0) * sf_tiles_per_row(C) * 512 + (quad & 31) * 16 + (lane >> 2) * 512;
+  uint32_t* sums = s_sums + (kSplit ? local * 5 * trips * 32 : 0) + lane;
+  const int byte = 8 * (lane & 3);
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  for (int g = lane; g < mine; g += kGemvLanes) {
-    const uint4 sw = __ldg(reinterpret_cast<const uint4*>(row_scales + (int64_t)g * 512));
-    const bool half = ((int64_t)(g0 + g) * 64 + 32) >= C;                // the last group of a width that is no multiple of 64
-    uint4 w[4][2];
+#pragma unroll 2
+  for (int t = share; t < trips; t += kSplit ? split : 1) {
+    const int k = t * 32 + lane;
+    if (k < sf_cols) {
+      const uint4 sw = __ldg(reinterpret_cast<const uint4*>(row_scales + (int64_t)t * 8 * 512));
+      uint2 w[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint4* src = reinterpret_cast<const uint4*>(row_codes[c] + g * 32);
-      w[c][0] = __ldg(src);
-      w[c][1] = half ? make_uint4(0u, 0u, 0u, 0u) : __ldg(src + 1);
-    }
-    const uint32_t s4[4] = {sw.x, sw.y, sw.z, sw.w};
+      for (int c = 0; c < 4; ++c) w[c] = __ldg(row_codes[c] + k);
+      float f[16];
+      const float4* v4 = reinterpret_cast<const float4*>(v) + 4 * (int64_t)k;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {                         // the four blocks of the group
-      f32x2 f[8];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 q = s_v[(4 * b + j) * pitch + g];
-        f[2 * j] = pack2(q.x, q.y);
-        f[2 * j + 1] = pack2(q.z, q.w);
+      for (int i = 0; i < 4; ++i) {
+        const float4 q = __ldg(v4 + i);
+        f[4 * i] = q.x; f[4 * i + 1] = q.y; f[4 * i + 2] = q.z; f[4 * i + 3] = q.w;
       }
+      const uint32_t s4[4] = {sw.x >> byte, sw.y >> byte, sw.z >> byte, sw.w >> byte};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const uint4 q = w[c][b >> 1];
-        f32x2 lo[4], hi[4];
-        e2m1x8_to_f32x2((b & 1) ? q.z : q.x, lo);
-        e2m1x8_to_f32x2((b & 1) ? q.w : q.y, hi);
-        f32x2 part = mul2(lo[0], f[0]);
+        float e[16];
+        e2m1x8_to_float(w[c].x, e);
+        e2m1x8_to_float(w[c].y, e + 8);
+        float part = 0.0f;
 #pragma unroll
-        for (int j = 1; j < 4; ++j) part = fma2(lo[j], f[j], part);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) part = fma2(hi[j], f[4 + j], part);
-        float p0, p1;
-        split2(part, p0, p1);
-        acc[c] = fmaf(p0 + p1, e4m3_to_float((uint8_t)(s4[c] >> (8 * b))), acc[c]);
+        for (int i = 0; i < 16; ++i) part = fmaf(e[i], f[i], part);
+        if (kSplit) sums[(c * trips + t) * 32] = __float_as_uint(part);
+        else acc[c] = fmaf(part, e4m3_to_float((uint8_t)s4[c]), acc[c]);
       }
+      if (kSplit) sums[(4 * trips + t) * 32] = __byte_perm(__byte_perm(s4[0], s4[1], 0x0040), __byte_perm(s4[2], s4[3], 0x0040), 0x5410);
     }
   }
+  const float unit = __ldg(unit_ptr);
+  if (kSplit) __syncthreads();
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int o = kGemvLanes / 2; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    if (lane == 0) s_out[c * 8 + unit_l] = acc[c];
-  }
-  __syncthreads();
-  if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (rank == 0 && threadIdx.x < 32) {
-    float sum = s_out[threadIdx.x];
-    for (int k = 1; k < ranks; ++k) {
-      uint32_t remote;
-      float f;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(&s_out[threadIdx.x])), "r"(k));
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(remote) : "memory");
-      sum += f;
+    if (kSplit) {
+      if (c % split != share) continue;                   // with more than four warps, four of them have a row each
+#pragma unroll 8
+      for (int t = 0; t < trips; ++t) {
+        if (t * 32 + lane < sf_cols)
+          acc[c] = fmaf(__uint_as_float(sums[(c * trips + t) * 32]), e4m3_to_float((uint8_t)(sums[(4 * trips + t) * 32] >> (8 * c))), acc[c]);
+      }
     }
-    const int64_t row = (int64_t)(row_group >> 2) * 128 + (row_group & 3) * 8 + (threadIdx.x & 7) + 32 * (threadIdx.x >> 3);
-    if (row < R) out[row] = sum * __ldg(unit_ptr);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (lane == 0 && row0 + 32 * c < R) out[row0 + 32 * c] = acc[c] * unit;
   }
-  // no CTA leaves while the first may still read its sums
-  if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The same product for a tall matrix (12288 rows and more) that gemv_tile_kernel does not take (row-major scales).  Two e2m1 codes become two
+// The same product for a tall matrix (12288 rows and more) that gemv_quad_kernel does not take (row-major scales).  Two e2m1 codes become two
 // halves with one cvt (exact), and the 16 floats of v for a lane's block stay in registers across the
 // 4 rows of the warp (v otherwise costs 8 times the bytes of the codes in L1 traffic).  Shorter
 // matrices keep gemv_kernel: with four rows per warp they would not fill the SMs.
@@ -429,38 +412,22 @@ static cudaError_t launch_gemv_staged(const uint2* codes, const uint8_t* scales,
                            codes, scales, unit, sf_layout, R, C, v, out);
 }
 
-// The split of the columns: the one with the fewest rounds of 16 groups per half-warp over all waves of CTAs (a wave's
-// start counts as one more round).
-static cudaError_t launch_gemv_tile(const uint8_t* codes, const uint8_t* scales, const float* unit, int64_t R, int64_t C,
+// How many warps share four rows: enough to give every scheduler six warps, as long as each has two rounds, and no fewer than
+// keep the block sums of a CTA within 24 KiB (v has to stay in what that leaves of L1).
+constexpr int64_t kGemvSumBytes = 24 << 10, kGemvSumBytesMax = 96 << 10;
+static cudaError_t launch_gemv_quad(const uint8_t* codes, const uint8_t* scales, const float* unit, int64_t R, int64_t C,
                                     const float* v, float* out, cudaStream_t st) {
-  const int64_t row_groups = ceil_div(R, 128) * 4, groups = ceil_div(C, 64), slots = (int64_t)device_sm_count() * kGemvCtasPerSm;
-  int ranks = 1;
-  int64_t best = INT64_MAX;
-  for (int k = 1; k <= 8; ++k) {
-    const int64_t slice = ceil_div(groups, k);
-    if (slice > kGemvMaxSlice) continue;
-    const int64_t cost = ceil_div(row_groups * k, slots) * (ceil_div(slice, kGemvLanes) + 1);
-    if (cost < best) { best = cost; ranks = k; }
-  }
-  const int64_t slice = ceil_div(groups, ranks);
-  const size_t smem = (size_t)(slice | 1) * 16 * sizeof(float4);
-  cudaError_t e = cudaFuncSetAttribute(gemv_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int64_t quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512), bytes = trips * 5 * 32 * sizeof(float);
+  int split = 1;
+  while (split < 8 && quads * split < (int64_t)device_sm_count() * 24 && trips >= 2 * split) split *= 2;
+  while (split > 1 && split < 8 && 8 / split * bytes > kGemvSumBytes) split *= 2;
+  if (8 / split * bytes > kGemvSumBytesMax) split = 1;
+  const dim3 grid((unsigned)ceil_div(quads * split, 8));
+  if (split == 1) return launch_overlapped(kLaunchShort, gemv_quad_kernel<false>, grid, dim3(256), 0, st, codes, scales, unit, R, C, (int)trips, 1, v, out);
+  const size_t smem = (size_t)(8 / split * bytes);
+  cudaError_t e = cudaFuncSetAttribute(gemv_quad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSumBytesMax);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(row_groups * ranks));
-  cfg.blockDim = dim3(kGemvThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ranks;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = launch_overlap_enabled(kLaunchShort) ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemv_tile_kernel, codes, scales, unit, R, C, (int)groups, (int)slice, v, out);
+  return launch_overlapped(kLaunchShort, gemv_quad_kernel<true>, grid, dim3(256), smem, st, codes, scales, unit, R, C, (int)trips, split, v, out);
 }
 
 // t = bf16( float(bf16(yv * s)) / (unit_a * unit_b) ), 8 elements per thread
@@ -567,14 +534,13 @@ extern "C" int32_t metis_nvfp4_gemv(const uint8_t* codes, const uint8_t* scales,
   if (v && !aligned16(v)) return fail(METIS_ERR_BAD_ALIGNMENT, "v must be 16-byte aligned");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const uint2* c4 = reinterpret_cast<const uint2*>(codes);
-  // The kernel along the tiled scales where the layout and the alignment of the rows allow it (widths that are multiples
-  // of 32: every operand of a product) and there are rows enough for it.
-  const bool tiled = sf_layout == METIS_SF_MMA && C % 32 == 0 && aligned16(scales) && C >= kGemvTileMinCols && C <= (int64_t)8 * kGemvMaxSlice * 64;
+  // The kernel along the tiled scales where that is the layout and there are rows enough for it.
+  const bool tiled = sf_layout == METIS_SF_MMA && aligned16(scales) && C >= kGemvTileMinCols && C < ((int64_t)1 << 31);
   // Otherwise, rows of 2048 elements and more: the kernel that stages v in shared memory; too few rows for it: a CTA per
   // row.  Every CTA stages the whole of v, so with very wide rows fewer CTAs of more rows win although they
   // fill the SMs less evenly (3584 x 18944: 16 rows per CTA 19.6 us, 8 rows 28.2).
   if (v && tiled && R >= (C < kGemvStagedMinCols ? 512 : kGemvTileMinRows)) {
-    METIS_CUDA_OK(launch_gemv_tile(codes, scales, unit, R, C, v, out, st));
+    METIS_CUDA_OK(launch_gemv_quad(codes, scales, unit, R, C, v, out, st));
   } else if (v && C >= kGemvStagedMinCols && C <= kGemvStagedMaxCols) {
     const int64_t sms = device_sm_count();
     const bool wide = C >= 8192;

@@ -4,9 +4,10 @@
 // The work is split in two launches because of one global dependency: the E4M3 block
 // scales are expressed relative to the tensor-wide maximum block scale, while the 4-bit
 // codes only depend on their own block.  Pass 1 streams x once, writes the packed codes and
-// the fp32 block maxima, and folds the global maximum with one atomicMax per warp.  Pass 2
-// touches 1/16 of the elements: it turns the block maxima into E4M3 bytes in the layout the
-// consumer wants and publishes the per-tensor unit.
+// the fp32 block maxima, and leaves the tensor-wide maximum either in a record per CTA (nothing
+// to clear beforehand) or, where the scratch holds no records, in one word by an atomicMax per
+// warp.  Pass 2 touches 1/16 of the elements: it turns the block maxima into E4M3 bytes in the
+// layout the consumer wants and publishes the per-tensor unit.
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -118,7 +119,8 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
 // What bounds it: instruction issue (24 warps per SM; the rows-only form runs at 85 % of the copy bandwidth).
 // Measured at 16384 x 4096 bf16, this pass alone, rows / transposed / both / both centred and stochastic: 37.1 / 48.2 /
 // 76.9 / 91.5 us with scalar fp32 arithmetic and 64-bit divisions in the tile walk, 32.9 / 39.6 / 63.8 / 80.2 us with
-// packed fp32 (3-6 us of it) and the walk by additions with every thread's offsets inside a tile kept (the rest).
+// packed fp32 (3-6 us of it) and the walk by additions with every thread's offsets inside a tile kept (the rest); the last
+// figure is 78.6 with 32-bit block counters in the random number generator.
 template <typename T> struct TileCfg {
   static constexpr int kRows = 128;
   static constexpr int kCols = 128 / sizeof(T);            // 64 (bf16) or 32 (fp32): 128 bytes per row
@@ -694,8 +696,8 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
 // holds the whole tensor: a thread quantizes up to 4 blocks and keeps their maxima in registers, the
 // tensor-wide maximum goes through the cluster's shared memory (hardware cluster barrier: nothing to
 // zero, no spinning, no scratch in global memory), and the same thread then writes its E4M3 bytes.
-// Replaces the zero-fill + pass 1 + scale pass of the streaming path where launch latency is all there
-// is to save; with more blocks (or more padding words to clear) the 8 SMs of a cluster lose to the
+// Replaces pass 1 + scale pass of the streaming path (and the zero-fill in front of them where the
+// scratch holds no records) where launch latency is all there is to save; with more blocks (or more padding words to clear) the 8 SMs of a cluster lose to the
 // streaming kernels on 148.  Measured back to back inside a CUDA graph: 16 x 4096 bf16 4.3 us against
 // 8.0, 32 x 4096 5.2, 64 x 4096 6.8 against 8.1.
 constexpr int kSmallThreads = 512;

@@ -175,7 +175,7 @@ rmsnorm_quantize_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, 
 // The same row arithmetic for a handful of rows, run as ONE thread-block cluster of up to 8 CTAs: a CTA
 // of bx x by = 512 threads takes up to kNormSmallPasses groups of `by` rows, every block maximum stays in a
 // register, the tensor-wide maximum crosses the cluster through shared memory, and the threads write
-// their own E4M3 bytes: no zero-fill node, no scale pass, no scratch in global memory.
+// their own E4M3 bytes: no scale pass, no scratch in global memory.
 
 // normalised(x) * gamma for one 16-element block, with the reference's roundings (llama.py:28, 31);
 // returns the block maximum.
@@ -677,31 +677,32 @@ rmsnorm_colsum_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, in
   }
 }
 
-// A CTA takes 32 columns: each of its eight warps adds every eighth row slot (coalesced, eight loads in flight), then their
-// sums are added in warp order: a fixed order.  One thread per column that walks all slots is a chain of loads: 13.4 us
-// for 256 slots, 15.5 for 296 (hidden 4096), 4.6 and 5.9 here (64 slots 4.5 -> 2.3).
+// A CTA takes 32 columns: its eight warps fetch the row slots' sums into shared memory (coalesced, eight loads of a
+// warp in flight), the first warp adds them up slot by slot: a fixed order.  One thread per column that walks all slots in global memory
+// is a chain of loads: 13.4 us for 256 slots, 15.5 for 296 (hidden 4096),
+// 5.5 and 7.4 here (64 slots 4.5 -> 2.7); summing every eighth slot in a warp of its own takes 4.6 and 5.9 but changes the last bit of the means.
+constexpr int kFinishSlots = 256;                          // slots per round: 32 KiB
 __global__ void __launch_bounds__(256)
 rmsnorm_mean_finish_kernel(const float* __restrict__ partial, int64_t slots, int64_t rows, int64_t cols, float* __restrict__ mean) {
-  __shared__ float s_part[8][32];
+  __shared__ float s_part[kFinishSlots][32];
   grid_dependency_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + lane;
   float sum = 0.0f;
-  if (c < cols) {
-    const float* src = partial + warp * cols + c;
-    const int mine = ((int)slots - warp + 7) >> 3;
-    const int64_t step = 8 * cols;
+  for (int64_t base = 0; base < slots; base += kFinishSlots) {
+    const int n = (int)(slots - base < kFinishSlots ? slots - base : kFinishSlots);
+    if (base > 0) __syncthreads();                         // the previous round's sums have been read
+    if (c < cols) {
 #pragma unroll 8
-    for (int i = 0; i < mine; ++i) sum += src[i * step];
+      for (int i = warp; i < n; i += 8) s_part[i][lane] = partial[(base + i) * cols + c];
+    }
+    __syncthreads();
+    if (warp == 0 && c < cols) {
+#pragma unroll 8
+      for (int i = 0; i < n; ++i) sum += s_part[i][lane];
+    }
   }
-  s_part[warp][lane] = sum;
-  __syncthreads();
-  if (warp == 0 && c < cols) {
-    float total = s_part[0][lane];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) total += s_part[w][lane];
-    mean[c] = __fdiv_rn(total, (float)rows);
-  }
+  if (warp == 0 && c < cols) mean[c] = __fdiv_rn(sum, (float)rows);
 }
 
 struct NormShape { int bx, by, per_thread; };

@@ -15,7 +15,7 @@ from . import cabi
 _DTYPES = {torch.bfloat16: cabi.DTYPE_BF16, torch.float32: cabi.DTYPE_F32}
 
 # Kernels of this library launched since import, by entry point (two per quantizer call: the
-# streaming pass and the scale pass; the memset between them is not a kernel).
+# streaming pass and the scale pass; a memset in front of them is not a kernel).
 LAUNCHES = {"quantize": 0, "rmsnorm_quantize": 0, "dequantize": 0, "col_mean": 0, "gemv": 0, "gemm": 0, "lowrank_bwd": 0, "decoder": 0}
 
 

@@ -145,9 +145,10 @@ int64_t metis_nvfp4_quantize_workspace_bytes(int64_t R, int64_t C);
  * codes are taken.  Two operands rotated alike along their contraction dimension give 16 times the plain
  * product (H s is orthogonal up to that factor), so the weight-gradient GEMM runs with alpha = 1/16.
  *
- * Launches: large tensors take a zero-fill of the workspace header, one streaming pass and a scale
- * pass.  Round-to-nearest, untransposed tensors of at most 16384 blocks (rollout-sized
- * activations) take ONE kernel that runs as a single thread-block cluster and does not touch the
+ * Launches: large tensors take one streaming pass and a scale pass, with a zero-fill of the workspace
+ * header in front unless the workspace has METIS_QUANTIZE_EXTRA_WORKSPACE more bytes and the pass at most
+ * 640 CTAs.  Round-to-nearest, untransposed tensors of at most 16384 blocks (rollout-sized
+ * activations; 4096 where that zero-fill is not needed) take ONE kernel that runs as a single thread-block cluster and does not touch the
  * workspace (it must still be passed and large enough); results are bit-identical.
  */
 int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t rows, int64_t cols, int64_t ld,

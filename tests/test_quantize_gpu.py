@@ -487,11 +487,11 @@ def test_scale_pass_at_the_edges_of_its_walk(rows, cols, layout):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,cols", [(512, 512), (515, 544), (1027, 2080), (1120, 4128), (3584, 7328), (1024, 18944), (129 * 128, 1024), (96, 4096), (31, 2048)])
+@pytest.mark.parametrize("rows,cols", [(512, 512), (515, 544), (1027, 2080), (1120, 4128), (3584, 7328), (1024, 18944), (129 * 128, 1024), (1030, 16 * 2561), (1030, 80016), (2050, 2064), (96, 4096), (31, 2048)])
 def test_vector_product_along_the_tiled_scales(rows, cols):
-    """Rows that end inside a 128-row block, widths that no group of 64 columns and no cluster's slice divides.  Against
-    float64 sums of the same values; fp32 products and sums of `cols` terms: error within 2^-24 times the sum of
-    magnitudes times the depth of the additions (cols / 32 in a lane's two partial sums, then a tree)."""
+    """Rows that end inside a 128-row block, widths that are no multiple of a round of 512 columns, every number of warps that
+    share four rows.  The same bits as the kernels for the row-major scale layout give, and against float64 sums of the same values; fp32 products and sums of `cols` terms: error within 2^-24 times the sum of
+    magnitudes times the depth of the additions (16 in a block, cols / 512 in a lane, then a tree)."""
     x = synthetic(rows, cols, "weights", rows, torch.float32)
     v = torch.randn(cols, generator=torch.Generator().manual_seed(cols))
     q = ops.nvfp4_quantize(x.cuda())
@@ -500,7 +500,8 @@ def test_vector_product_along_the_tiled_scales(rows, cols):
     want = deq @ v.double().cuda()
     bound = 2.0 ** -24 * (cols / 32 + 40) * (deq.abs() @ v.double().abs().cuda())
     assert got.shape == (rows,) and bool(((got - want).abs() <= bound).all())
-    assert torch.equal(got, ops.nvfp4_gemv(q, v.cuda()).double())
+    rowmajor = ops.nvfp4_quantize(x.cuda(), sf_layout=cabi.SF_ROWMAJOR)
+    assert torch.equal(got, ops.nvfp4_gemv(rowmajor, v.cuda()).double())
 
 
 @pytest.mark.gpu
