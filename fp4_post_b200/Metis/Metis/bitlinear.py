@@ -887,7 +887,6 @@ class MetisFusedFunction(torch.autograd.Function):
         act = xa.dtype if xa.dtype in (torch.bfloat16, torch.float32) else torch.float32
         rank1_v, rank1_r = [], []
         join_residual = bias_row = None
-        late = False
 
         def ready(op):
             if op.ready_event is not None:             # quantized on another stream: order this stream after it, once
@@ -913,28 +912,15 @@ class MetisFusedFunction(torch.autograd.Function):
                 # a parameter is complete whatever stream this is (a cast of one is ordered on the current stream only)
                 if isinstance(bias, torch.nn.Parameter):
                     bias_row = bias.float()
-                late = overlap and M <= 128
                 if overlap and rq.ready_event is not None:
                     current_stream(xa.mean.device).wait_event(rq.ready_event)
-                if not late:
-                    row_r = ops.nvfp4_gemv(rq.q, xa.mean)
+                row_r = ops.nvfp4_gemv(rq.q, xa.mean)
             if v_ready is not None:
                 current_stream(xa.mean.device).wait_event(v_ready)
                 row_v.record_stream(current_stream(xa.mean.device))
-                if not late:
-                    join_residual = lambda: join(row_r, bias_row)
+                join_residual = lambda: join(row_r, bias_row)
             rank1_v.append((None, row_v))
-            if late:
-                # At decode sizes the pass over the residual weight fills every SM for longer than the quantization takes;
-                # issued in front of the product with V it would make that one (a few CTAs that need an SM each) wait.
-                quantized = recorded_event(current_stream(xa.mean.device))
-
-                def row_of_residual():
-                    with _beside(quantized, xa.mean.device) as join_late:
-                        row = ops.nvfp4_gemv(rq.q, xa.mean)
-                    return row, lambda: join_late(row, bias_row)
-            else:
-                rank1_r.append((None, row_r))
+            rank1_r.append((None, row_r))
         if bias is not None:
             rank1_r.append((None, bias.float() if bias_row is None else bias_row))
         ready(vq)
@@ -953,9 +939,6 @@ class MetisFusedFunction(torch.autograd.Function):
             ready(rq)
             ts = yv * s.to(act)
             lowrank = _bf16_factors(ts.float() / (xa.q.unit * rq.q.unit), u_weight.detach(), act)
-        if late:
-            row_r, join_residual = row_of_residual()
-            rank1_r.insert(0, (None, row_r))
         if join_residual is not None:
             join_residual()
         ready(rq)

@@ -156,24 +156,25 @@ __device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
 // once more.)  The additions are those of the other kernels, in the same order: 16 products of a block one after the other,
 // a lane's blocks one after the other, then the lanes pairwise, so which kernel runs does not show in the result (a sum that
 // differs in its last bit can flip the rounding of an activation, and a block of decoder layers makes 1 % of that).
-// With too few rows to fill the SMs that way, `split` warps share the four rows: each takes every split-th round of
+// With too few rows to fill the SMs that way, two or four warps (`split`) share the four rows: each takes every split-th round of
 // 32 blocks and parks the block sums in shared memory, and the lanes' sums are then formed from there in order.
 // Two e2m1 codes become two halves with one conversion (exact).  Bound by issue and by the conversions (the bytes alone
 // take 6 us at 18944 x 3584).
 // Measured, gemv_staged_kernel (or, below 2048 columns, gemv_kernel) before and this one after, six weights in turn:
-// 18944 x 3584 20.6 -> 14.1 us, 3584 x 18944 23.8 -> 19.0, 14336 x 4096 21.4 -> 15.3, 4096 x 14336 18.5 -> 16.5,
-// 8960 x 1536 10.4 -> 5.9, 1536 x 8960 7.9 -> 5.9, 4096 x 4096 6.6 -> 6.4.  A form that split the columns over a cluster,
-// with packed multiply-adds and another order of the additions, took 14.6, 16.9, 13.3, 14.7, 5.8, 5.8 and 5.9.
-constexpr int kGemvRowsCtasPerSm = 4;
+// 18944 x 3584 20.5 -> 13.5 us, 3584 x 18944 23.6 -> 17.4, 14336 x 4096 21.5 -> 13.1, 4096 x 14336 18.5 -> 14.6,
+// 8960 x 1536 10.2 -> 4.4, 1536 x 8960 7.7 -> 5.7, 4096 x 4096 6.4 -> 5.5.  Eight warps in a CTA instead of four end less
+// evenly (14.1, 19.0, 15.3, 16.5, 5.9, 5.9, 6.4); a warp per two rows reads v and the scales twice (3584 x 18944: 30 us).
+// A form that split the columns over a cluster, with another order of the additions, took 14.6, 16.9, 13.3, 14.7, 5.8, 5.8, 5.9.
+constexpr int kGemvWarps = 4, kGemvCtasPerSm = 8;
 template <bool kSplit>
-__global__ void __launch_bounds__(256, kGemvRowsCtasPerSm)
+__global__ void __launch_bounds__(32 * kGemvWarps, kGemvCtasPerSm)
 gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, const float* __restrict__ unit_ptr,
                  int64_t R, int64_t C, int trips, int split, const float* __restrict__ v, float* __restrict__ out) {
   extern __shared__ uint32_t s_sums[];                    // kSplit, per four rows: [5][trips][32], the sums of four rows and their scales
   grid_dependency_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int local = kSplit ? warp / split : warp, share = kSplit ? warp - local * split : 0;
-  const int64_t quad = (int64_t)blockIdx.x * (kSplit ? 8 / split : 8) + local;
+  const int64_t quad = (int64_t)blockIdx.x * (kSplit ? kGemvWarps / split : kGemvWarps) + local;
   const int64_t row0 = (quad >> 5) * 128 + (quad & 31);   // this warp's rows: row0 + 32 c
   if (!kSplit && row0 >= R) return;
   const int sf_cols = (int)(C >> 4);
@@ -219,7 +220,7 @@ gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ 
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     if (kSplit) {
-      if (c % split != share) continue;                   // with more than four warps, four of them have a row each
+      if (c % split != share) continue;                   // four warps: a row each
 #pragma unroll 8
       for (int t = 0; t < trips; ++t) {
         if (t * 32 + lane < sf_cols)
@@ -238,7 +239,7 @@ gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ 
 // matrices keep gemv_kernel: with four rows per warp they would not fill the SMs.
 constexpr int kGemvTallRows = 4;          // rows per warp
 constexpr int64_t kGemvTallMinRows = 12288;
-constexpr int64_t kGemvTileMinCols = 512, kGemvTileMinRows = 1024;
+constexpr int64_t kGemvTileMinCols = 512;
 
 __global__ void __launch_bounds__(256)
 gemv_tall_kernel(const uint2* __restrict__ codes, const uint8_t* __restrict__ scales,
@@ -412,22 +413,46 @@ static cudaError_t launch_gemv_staged(const uint2* codes, const uint8_t* scales,
                            codes, scales, unit, sf_layout, R, C, v, out);
 }
 
-// How many warps share four rows: enough to give every scheduler six warps, as long as each has two rounds, and no fewer than
-// keep the block sums of a CTA within 24 KiB (v has to stay in what that leaves of L1).
-constexpr int64_t kGemvSumBytes = 24 << 10, kGemvSumBytesMax = 96 << 10;
+// How many warps share four rows.  24 warps per SM run at full rate, 12 to 15 at 0.88 of it (4096 x 4096: 5.5 us with 28 and 6.2
+// with 14), so the rows are shared further up to there, unless the rounds that the last warps lack cost as much (8960 x 1536 has
+// three rounds: 4.4 us with a warp per four rows, 5.6 with two); below 8 warps always.  Finally the block sums of eight
+// CTAs have to leave room for v in L1.
+constexpr int64_t kGemvWarpsPerSm = 24, kGemvFewWarpsPerSm = 8, kGemvL1Bytes = 208 << 10, kGemvSumBytesMax = 96 << 10;
+static int64_t gemv_sum_bytes(int64_t C, int split) { return kGemvWarps / split * ceil_div(C, 512) * 5 * 32 * (int64_t)sizeof(float); }
+static int gemv_split(int64_t R, int64_t C) {
+  const int64_t sms = device_sm_count(), quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512);
+  auto padded = [&](int k) { return ceil_div(trips, k) * k; };              // rounds, the missing ones of the last included
+  int split = 1;
+  while (split < kGemvWarps && trips >= 2 * split && quads * split < sms * kGemvWarpsPerSm &&
+         (quads * split < sms * kGemvFewWarpsPerSm || padded(2 * split) * 10 <= padded(split) * 11)) split *= 2;
+  while (split > 1 && split < kGemvWarps && kGemvCtasPerSm * gemv_sum_bytes(C, split) + C * (int64_t)sizeof(float) > kGemvL1Bytes) split *= 2;
+  return gemv_sum_bytes(C, split) > kGemvSumBytesMax ? 1 : split;
+}
+
+// Whether gemv_quad_kernel is the faster one for a matrix in the tiled layout (staged -> this one, us).  From 8192 columns on the staged
+// kernel fits two CTAs on an SM at most: always (2048 x 8192 7.0 -> 6.0, 8976 x 8192 22.5 -> 18.0, 12288 x 12288 38.9 -> 32.2).
+// So too where the staged kernel would give four rows to a warp (18944 x 3584 20.5 -> 13.5).  Between, up to 15 warps per SM of
+// four rows each and with less than a quarter of the rounds missing (4608 x 5120 8.6 -> 7.7, 8192 x 4096 10.0 -> 9.6; but
+// 10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8) and of seven rounds or more (3584 x 3584 5.7 -> 5.1; 3072 x 3072 4.4 -> 5.0,
+// 2048 x 2048 2.9 -> 3.15).  Below 2048 columns it replaces gemv_kernel (1536 x 1536 3.55 -> 3.4, 8960 x 1536 10.2 -> 4.4).
+static bool gemv_quad_wins(int64_t R, int64_t C) {
+  if (C < kGemvStagedMinCols) return R >= 512;
+  if (R < 1024) return false;                                               // 512 x 3584: 3.5 -> 4.3
+  const int64_t sms = device_sm_count(), split = gemv_split(R, C);
+  if (C >= 8192 || ceil_div(R, 32) >= 3 * sms) return true;
+  return C >= 3584 && ceil_div(R, 128) * 32 < 15 * sms && ceil_div(ceil_div(C, 512), split) * split * 512 * 4 < 5 * C;
+}
+
 static cudaError_t launch_gemv_quad(const uint8_t* codes, const uint8_t* scales, const float* unit, int64_t R, int64_t C,
                                     const float* v, float* out, cudaStream_t st) {
-  const int64_t quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512), bytes = trips * 5 * 32 * sizeof(float);
-  int split = 1;
-  while (split < 8 && quads * split < (int64_t)device_sm_count() * 24 && trips >= 2 * split) split *= 2;
-  while (split > 1 && split < 8 && 8 / split * bytes > kGemvSumBytes) split *= 2;
-  if (8 / split * bytes > kGemvSumBytesMax) split = 1;
-  const dim3 grid((unsigned)ceil_div(quads * split, 8));
-  if (split == 1) return launch_overlapped(kLaunchShort, gemv_quad_kernel<false>, grid, dim3(256), 0, st, codes, scales, unit, R, C, (int)trips, 1, v, out);
-  const size_t smem = (size_t)(8 / split * bytes);
+  const int64_t quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512);
+  const int split = gemv_split(R, C);
+  const dim3 grid((unsigned)ceil_div(quads * split, kGemvWarps)), block(32 * kGemvWarps);
+  if (split == 1) return launch_overlapped(kLaunchShort, gemv_quad_kernel<false>, grid, block, 0, st, codes, scales, unit, R, C, (int)trips, 1, v, out);
+  const size_t smem = (size_t)gemv_sum_bytes(C, split);
   cudaError_t e = cudaFuncSetAttribute(gemv_quad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSumBytesMax);
   if (e != cudaSuccess) return e;
-  return launch_overlapped(kLaunchShort, gemv_quad_kernel<true>, grid, dim3(256), smem, st, codes, scales, unit, R, C, (int)trips, split, v, out);
+  return launch_overlapped(kLaunchShort, gemv_quad_kernel<true>, grid, block, smem, st, codes, scales, unit, R, C, (int)trips, split, v, out);
 }
 
 // t = bf16( float(bf16(yv * s)) / (unit_a * unit_b) ), 8 elements per thread
@@ -534,12 +559,12 @@ extern "C" int32_t metis_nvfp4_gemv(const uint8_t* codes, const uint8_t* scales,
   if (v && !aligned16(v)) return fail(METIS_ERR_BAD_ALIGNMENT, "v must be 16-byte aligned");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const uint2* c4 = reinterpret_cast<const uint2*>(codes);
-  // The kernel along the tiled scales where that is the layout and there are rows enough for it.
+  // The kernel along the tiled scales where that is the layout and it is the faster one (the bits are the same).
   const bool tiled = sf_layout == METIS_SF_MMA && aligned16(scales) && C >= kGemvTileMinCols && C < ((int64_t)1 << 31);
   // Otherwise, rows of 2048 elements and more: the kernel that stages v in shared memory; too few rows for it: a CTA per
   // row.  Every CTA stages the whole of v, so with very wide rows fewer CTAs of more rows win although they
   // fill the SMs less evenly (3584 x 18944: 16 rows per CTA 19.6 us, 8 rows 28.2).
-  if (v && tiled && R >= (C < kGemvStagedMinCols ? 512 : kGemvTileMinRows)) {
+  if (v && tiled && gemv_quad_wins(R, C)) {
     METIS_CUDA_OK(launch_gemv_quad(codes, scales, unit, R, C, v, out, st));
   } else if (v && C >= kGemvStagedMinCols && C <= kGemvStagedMaxCols) {
     const int64_t sms = device_sm_count();
