@@ -9,6 +9,7 @@
 #include <stdarg.h>
 
 #include "../../include/metis_nvfp4.h"
+#include "rows_shape.cuh"
 
 namespace metis {
 
@@ -45,7 +46,6 @@ int32_t launch_finalize(const WorkspaceView& ws, int64_t R, int64_t C, int32_t s
 // Where a workspace that holds METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than [R, C] needs has its per-CTA records
 // (nullptr: it does not).  Word -1 is their number, three words each: largest maximum (of the row-major, of the
 // transposed output), error.
-constexpr int kMaxRecords = 640;
 unsigned int* workspace_records(void* workspace, int64_t workspace_bytes, int64_t R, int64_t C);
 int32_t check_quant_outputs(int64_t R, int64_t C, int32_t sf_layout, const void* codes,
                             const void* scales, const void* unit, const void* workspace,

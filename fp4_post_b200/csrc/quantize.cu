@@ -19,7 +19,6 @@
 
 namespace metis {
 
-constexpr int kQuantThreads = 256;
 constexpr int kHeaderBytes = kWorkspaceHeaderBytes;
 
 __device__ __forceinline__ void fold_global_max(unsigned int* gmax, float local) {
@@ -907,40 +906,24 @@ unsigned int* workspace_records(void* workspace, int64_t workspace_bytes, int64_
 }
 static int sm_count() { return device_sm_count(); }
 
+// *records: in: where the per-CTA records may go (or nullptr); out: nullptr if the running maximum was used instead
 template <typename T>
-static void launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, const float* mean, bool sr,
-                        uint64_t seed, uint64_t offset, const uint64_t* ctr, uint32_t* codes, const WorkspaceView& ws,
-                        cudaStream_t st, uint32_t sr16 = 0, unsigned int* records = nullptr) {
+static int32_t launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, const float* mean, bool sr,
+                           uint64_t seed, uint64_t offset, const uint64_t* ctr, uint32_t* codes, const WorkspaceView& ws,
+                           cudaStream_t st, uint32_t sr16, unsigned int** records) {
   const int bpr = (int)(cols >> 4);
-  // threads along the row: the power of two that pads the row least (hidden 1536 = 96 blocks runs
-  // as 3 x 32, not as 128 with a quarter of the lanes idle); ties go to the wider shape
-  int bx = 1;
-  while (bx < bpr && bx < kQuantThreads) bx <<= 1;
-  for (int cand = bx >> 1; cand >= 32; cand >>= 1)
-    if ((bpr + cand - 1) / cand * cand < (bpr + bx - 1) / bx * bx) bx = cand;
-  const int by = kQuantThreads / bx;
-  const int gx = (bpr + bx - 1) / bx;
-  int64_t gy = ceil_div(rows, by);
-  // four waves of resident CTAs (grid-stride over the rows): whole waves leave no tail
-  int per_sm = 0;
-#define METIS_OCC_ROWS(MEAN, SR) per_sm = resident_ctas(reinterpret_cast<const void*>(quantize_rows_kernel<T, MEAN, SR>), kQuantThreads, 0)
-  if (mean) { if (sr) METIS_OCC_ROWS(true, true); else METIS_OCC_ROWS(true, false); }
-  else      { if (sr) METIS_OCC_ROWS(false, true); else METIS_OCC_ROWS(false, false); }
-#undef METIS_OCC_ROWS
-  if (per_sm < 1) per_sm = 1;
-  int64_t cap = (int64_t)sm_count() * per_sm * 4 / gx;
-  if (records && cap > kDualMaxCtas / gx) cap = kDualMaxCtas / gx;
-  if (cap < 1) cap = 1;
-  if (gy > cap) gy = cap;
-  if (gy > 65535) gy = 65535;
-  if (gy < 1) gy = 1;
-  const dim3 g((unsigned)gx, (unsigned)gy), b((unsigned)bx, (unsigned)by);
-#define METIS_LAUNCH_ROWS(MEAN, SR)                                                              \
-  launch_overlapped(kLaunchStream, quantize_rows_kernel<T, MEAN, SR>, g, b, 0, st, x, (int)rows, bpr, ld, mean, seed, offset, ctr, \
-                    reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, records, sr16)
-  if (mean) { if (sr) METIS_LAUNCH_ROWS(true, true); else METIS_LAUNCH_ROWS(true, false); }
-  else      { if (sr) METIS_LAUNCH_ROWS(false, true); else METIS_LAUNCH_ROWS(false, false); }
-#undef METIS_LAUNCH_ROWS
+  auto kern = mean ? (sr ? quantize_rows_kernel<T, true, true> : quantize_rows_kernel<T, true, false>)
+                   : (sr ? quantize_rows_kernel<T, false, true> : quantize_rows_kernel<T, false, false>);
+  const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), kQuantThreads, 0);
+  const RowsShape s = rows_shape(rows, bpr, (int64_t)sm_count() * per_sm, *records != nullptr);
+  if (!s.records) {
+    *records = nullptr;
+    METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));       // running maximum and error word
+  }
+  METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)s.gx, (unsigned)s.gy), dim3((unsigned)s.bx, (unsigned)(kQuantThreads / s.bx)),
+                                  0, st, x, (int)rows, bpr, ld, mean, seed, offset, ctr, reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax,
+                                  *records, sr16));
+  return METIS_OK;
 }
 
 template <typename T>
@@ -1086,30 +1069,29 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
         : launch_small(static_cast<const float*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st);
   }
   const WorkspaceView ws = view_workspace(workspace);
-  if (!records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));
   // Large row-major tensors take the tile kernel too (row phase only): its TMA ring keeps two tiles in
   // flight per CTA, where the register-fed kernel waits on its loads.  Same arithmetic, same bytes.
   const bool rows_by_tiles = !transpose && rows * cols >= kTileRowsMinElements && (ld * esz) % 16 == 0;
-  if (rows_by_tiles) {
-    const TileOutputs out = {nullptr, nullptr, nullptr, codes, ws.amax, ws.gmax, ws.gmax + 1, records, 0u, sr16};
-    const int32_t rc = x_dtype == METIS_DTYPE_BF16
+  int32_t rc;
+  if (transpose || rows_by_tiles) {
+    if (!records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));     // running maximum and error word
+    TileOutputs out = {};
+    if (transpose) { out.codes_t = codes; out.amax_t = ws.amax; out.gmax_t = ws.gmax; out.hadamard = rht; }
+    else           { out.codes_r = codes; out.amax_r = ws.amax; out.gmax_r = ws.gmax; }
+    out.error = ws.gmax + 1;
+    out.records = records;
+    out.sr16 = sr16;
+    rc = x_dtype == METIS_DTYPE_BF16
         ? launch_tile(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st)
         : launch_tile(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st);
-    if (rc) return rc;
-  } else if (!transpose) {
-    if (x_dtype == METIS_DTYPE_BF16)
-      launch_rows(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
-                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16, records);
-    else
-      launch_rows(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
-                  reinterpret_cast<uint32_t*>(codes), ws, st, sr16, records);
   } else {
-    const TileOutputs out = {codes, ws.amax, ws.gmax, nullptr, nullptr, nullptr, ws.gmax + 1, records, rht, sr16};
-    const int32_t rc = x_dtype == METIS_DTYPE_BF16
-        ? launch_tile(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st)
-        : launch_tile(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr, out, st);
-    if (rc) return rc;
+    rc = x_dtype == METIS_DTYPE_BF16
+        ? launch_rows(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
+                      reinterpret_cast<uint32_t*>(codes), ws, st, sr16, &records)
+        : launch_rows(static_cast<const float*>(x), rows, cols, ld, col_mean, sr, seed, offset, ctr,
+                      reinterpret_cast<uint32_t*>(codes), ws, st, sr16, &records);
   }
+  if (rc) return rc;
   METIS_CUDA_OK(cudaGetLastError());
   return launch_finalize(ws, R, C, sf_layout, scales, unit, st, ctr, records, transpose ? 1 : 0);
 }
@@ -1301,11 +1283,11 @@ extern "C" int32_t metis_nvfp4_quantize_static(const void* x, int32_t x_dtype, i
   const WorkspaceView ws = view_workspace(scratch);
   // The array keeps whatever the previous call left.  Only the running maximum and the error word
   // have to start at zero; every block maximum this call reads back is written by this call first.
-  METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
-  if (x_dtype == METIS_DTYPE_BF16)
-    launch_rows(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, nullptr, false, 0, 0, nullptr, reinterpret_cast<uint32_t*>(codes), ws, st);
-  else
-    launch_rows(static_cast<const float*>(x), rows, cols, ld, nullptr, false, 0, 0, nullptr, reinterpret_cast<uint32_t*>(codes), ws, st);
+  unsigned int* records = nullptr;                      // the built-in scratch has no room for them
+  const int32_t rc = x_dtype == METIS_DTYPE_BF16
+      ? launch_rows(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, nullptr, false, 0, 0, nullptr, reinterpret_cast<uint32_t*>(codes), ws, st, 0u, &records)
+      : launch_rows(static_cast<const float*>(x), rows, cols, ld, nullptr, false, 0, 0, nullptr, reinterpret_cast<uint32_t*>(codes), ws, st, 0u, &records);
+  if (rc) return rc;
   METIS_CUDA_OK(cudaGetLastError());
   return launch_finalize(ws, rows, cols, sf_layout, scales, unit, st);
 }

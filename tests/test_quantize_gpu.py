@@ -506,10 +506,12 @@ def test_vector_product_along_the_tiled_scales(rows, cols):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols,transpose", [(16, 4096, False), (17, 4112, False), (64, 3584, False), (16, 14336, False), (300, 4096, False),
-                                                 (1, 81920, False), (48, 1040, True), (512, 4096, True)])
+                                                 (1, 81920, False), (48, 1040, True), (512, 4096, True),
+                                                 (1, 327680, False), (1, 327696, False), (2, 349696, False), (1, 1048064, False)])
 @pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
 def test_a_workspace_with_room_for_records_gives_the_same_bytes(rows, cols, transpose, layout):
-    """Both forms of the workspace, on either side of the one-cluster limit, over a workspace full of old bytes."""
+    """Both forms of the workspace, on either side of the one-cluster limit and of the widest row whose CTAs' records it
+    holds, over a workspace full of old bytes; nothing behind it is written."""
     x = synthetic(rows, cols, "normal", rows + cols, torch.bfloat16).to(DEV)
     L = cabi.lib()
     R, C = (cols, rows) if transpose else (rows, cols)
@@ -518,11 +520,13 @@ def test_a_workspace_with_room_for_records_gives_the_same_bytes(rows, cols, tran
         codes = torch.empty(R, C // 2, dtype=torch.uint8, device=DEV)
         scales = torch.full((L.metis_nvfp4_sf_bytes(R, C, layout),), 0xA5, dtype=torch.uint8, device=DEV)
         unit = torch.empty(1, device=DEV)
-        ws = torch.full((L.metis_nvfp4_quantize_workspace_bytes(R, C) + extra,), 0xFF, dtype=torch.uint8, device=DEV)
+        ws_bytes = L.metis_nvfp4_quantize_workspace_bytes(R, C) + extra
+        ws = torch.full((ws_bytes + 65536,), 0xFF, dtype=torch.uint8, device=DEV)
         rc = L.metis_nvfp4_quantize(x.data_ptr(), cabi.DTYPE_BF16, rows, cols, cols, None, cabi.Q_TRANSPOSE if transpose else 0, 0, 0, layout,
-                                    codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), ws.data_ptr(), ws.numel(),
+                                    codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), ws.data_ptr(), ws_bytes,
                                     torch.cuda.current_stream().cuda_stream)
         cabi.check(rc, "metis_nvfp4_quantize")
+        assert bool((ws[ws_bytes:] == 0xFF).all())
         got.append((codes, scales, unit))
     for a, b in zip(*got):
         assert torch.equal(a, b)
