@@ -902,6 +902,11 @@ class MetisFusedFunction(torch.autograd.Function):
             if not overlap:
                 ready(vq)
                 ready(rq)
+            # The bias is cast beside the product too, but `mean_event` says nothing about it: a grouped activation's
+            # event is that of the call that quantized it, and the bias may have been written since.  An event of this
+            # call orders the cast behind whatever the current stream has queued.
+            cast_bias = overlap and bias is not None and bias.dtype != torch.float32
+            entered = recorded_event(current_stream(xa.mean.device)) if cast_bias else None
             with _beside(xa.mean_event if overlap else None, xa.mean.device) as join:
                 if overlap and vq.ready_event is not None:      # quantized on a stream of their own: order this one after each
                     current_stream(xa.mean.device).wait_event(vq.ready_event)
@@ -909,12 +914,12 @@ class MetisFusedFunction(torch.autograd.Function):
                 # the product with V needs only this one: the pass over the (much larger) residual
                 # weight stays off the critical path until the residual product
                 v_ready = recorded_event(current_stream(xa.mean.device)) if overlap else None
-                # a parameter is complete whatever stream this is (a cast of one is ordered on the current stream only)
-                if isinstance(bias, torch.nn.Parameter):
-                    bias_row = bias.float()
                 if overlap and rq.ready_event is not None:
                     current_stream(xa.mean.device).wait_event(rq.ready_event)
                 row_r = ops.nvfp4_gemv(rq.q, xa.mean)
+                if cast_bias:
+                    current_stream(xa.mean.device).wait_event(entered)
+                    bias_row = bias.float()
             if v_ready is not None:
                 current_stream(xa.mean.device).wait_event(v_ready)
                 row_v.record_stream(current_stream(xa.mean.device))

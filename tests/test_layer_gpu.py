@@ -283,6 +283,38 @@ def test_second_stream_gives_the_gradients_of_the_single_stream_order_bit_for_bi
             MetisFusedFunction.concurrent_branches = True
 
 
+def test_a_bias_written_between_two_calls_on_one_activation_is_read_after_the_write():
+    """Cached weights and a grouped activation that is found again: nothing but the order on the current stream says when
+    the bias may be read."""
+    torch.manual_seed(3)
+    block = torch.nn.Module()
+    block.q_proj, block.k_proj = torch.nn.Linear(512, 512, bias=True), torch.nn.Linear(512, 128, bias=True)
+    model = torch.nn.Sequential(block).to(DEV).to(torch.bfloat16)
+    args = MetisArgs(forward_svd_rank=64, cache_quantized_weight=True)
+    args.device = DEV
+    replace_linear_with_metis(model, dtype=torch.bfloat16, metis_args=args, compute_dtype=torch.bfloat16)
+    layer = model[0].q_proj
+    assert layer.activation_group is not None
+    bias = layer.warmup_linear.bias
+    x = torch.randn(1, 64, 512, device=DEV, dtype=torch.bfloat16)
+    busy = torch.randn(8192, 8192, device=DEV, dtype=torch.bfloat16)
+    values = [torch.full_like(bias, 7.0 * i) for i in range(3)]
+    with torch.no_grad():
+        want = []
+        for v in values:
+            bias.copy_(v)
+            torch.cuda.synchronize()
+            want.append(layer(x).clone())
+            torch.cuda.synchronize()
+        for rep in range(2):
+            for v, w in zip(values, want):
+                for _ in range(4):                      # milliseconds of work in front of the write
+                    torch.mm(busy, busy)
+                bias.copy_(v)
+                assert torch.equal(layer(x), w)
+    assert not torch.equal(want[0], want[1])
+
+
 def test_grpo_defaults_bf16_stochastic_backward_and_shared_activation():
     torch.manual_seed(1)
     block = torch.nn.Module()
