@@ -507,6 +507,32 @@ __device__ __forceinline__ void e4m3x4_to_float(uint32_t packed, float (&f)[4]) 
   f[0] = l.x; f[1] = l.y; f[2] = h.x; f[3] = h.y;
 }
 
+// Scale pass of one row: every `step`-th group of four blocks from k on, up to k_live; its bytes go to `to` + k * pitch
+// (from there to k_end: zeros, the padding of the tiled layout).  Returns the sum of code x scale.  Not inlined either: the
+// loop has four groups in flight and the kernel around it other paths.
+__device__ __noinline__ float finish_row(const float* from, const uint2* codes, uint8_t* to, int pitch, int k, int k_live, int k_end,
+                                         int step, float unit, float inv_unit) {
+  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+  float sum = 0.0f;
+#pragma unroll 4
+  for (; k < k_live; k += step) {
+    const float4 a = *reinterpret_cast<const float4*>(from + 4 * (int64_t)k);
+    const uint4* w = reinterpret_cast<const uint4*>(codes + 4 * (int64_t)k);
+    const uint4 w0 = w[0], w1 = w[1];
+    uint32_t bytes;
+    if (!scale_bytes4(a, inv_unit2, bytes)) bytes = scale_bytes4_exact(a, unit);
+    float f[4];
+    e4m3x4_to_float(bytes, f);
+    sum = fmaf((float)block_code_sum(make_uint2(w0.x, w0.y)), f[0], sum);
+    sum = fmaf((float)block_code_sum(make_uint2(w0.z, w0.w)), f[1], sum);
+    sum = fmaf((float)block_code_sum(make_uint2(w1.x, w1.y)), f[2], sum);
+    sum = fmaf((float)block_code_sum(make_uint2(w1.z, w1.w)), f[3], sum);
+    *reinterpret_cast<uint32_t*>(to + (int64_t)k * pitch) = bytes;
+  }
+  for (; k < k_end; k += step) *reinterpret_cast<uint32_t*>(to + (int64_t)k * pitch) = 0u;
+  return sum;
+}
+
 // A thread finishes one 16-byte piece of the tiled layout at a time: the scales of the rows l, l + 32, l + 64, l + 96 of
 // a 128-row block for 4 scale columns, i.e. four 16-byte reads of maxima and one 16-byte store (row-major scales: four
 // words of four rows).  Two neighbouring lanes take two neighbouring l, the next ones the tiles to the right, so a warp
@@ -517,9 +543,13 @@ __device__ __forceinline__ void e4m3x4_to_float(uint32_t packed, float (&f)[4]) 
 // waits for instruction fetch).  Measured at 16384 x 4096, one output / both / both with token sums: 11.2 / 21.0 / 28.2
 // us then, 5.8 / 10.4 / 21.2 now; at 65536 x 4096 32 / 62 / 79 -> 16 / 30 / 67 (the bytes alone take 13 / 26 / 46); 64 x 18944, fewer rows than a block has: 4.0 -> 2.8.
 constexpr int kFinThreads = 128;
-template <bool kSums>                                            // some job of the launch wants row sums (twice the registers)
+// What the jobs of a launch want: no row sums; sums, four rows to a thread; sums, a row to a thread (finalize_form has the
+// rule).  Kernels of their own: what stands beside the unrolled path of the second one costs it 3 to 15 %.
+enum FinalizeForm { kFinPlain, kFinSums, kFinSumsByRow };
+template <FinalizeForm kForm>
 __global__ void __launch_bounds__(kFinThreads)
 finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t* __restrict__ offset_ctr) {
+  constexpr bool kSums = kForm != kFinPlain, kQuadSums = kForm == kFinSums;
   __shared__ unsigned int s_top[kFinThreads / 32], s_bad[kFinThreads / 32];
   __shared__ float s_sum[kFinThreads / 32][2][4];
   grid_dependency_wait();
@@ -563,12 +593,13 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
   const int64_t items = ((R + 127) / 128) * 16;
   // without row sums a row is cut into segments of tx tiles, so that a few wide rows still fill the SMs
   const int segments = sums ? 1 : (groups + tx - 1) >> J.log_tx;
-  const int64_t work = items * segments;
+  const bool by_row = kForm == kFinSumsByRow && sums;            // row0 + 32 (index & 3) of a thread's four rows: four times the items
+  const int64_t work = items * segments << (by_row ? 2 : 0);
   const int64_t row_pitch = 32 * sf_cols;                        // between a thread's four rows
   // the item loop is uniform over the CTA (the sums of a row meet at a barrier)
   for (int64_t first = (int64_t)blockIdx.x * per_cta; first < work; first += (int64_t)gridDim.x * per_cta) {
     const bool live = first + sub < work;
-    const int64_t item = segments == 1 ? first + sub : (first + sub) / segments;
+    const int64_t item = by_row ? (first + sub) >> 2 : segments == 1 ? first + sub : (first + sub) / segments;
     const int k_first = segments == 1 ? 0 : (int)((first + sub) - item * segments) << J.log_tx;
     const int k_end = segments == 1 ? groups : min(groups, k_first + tx);
     const int64_t row0 = (item >> 4) * 128 + (item & 15) * 2 + (tid & 1);       // this thread's rows: row0 + 32 c
@@ -592,7 +623,7 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
           else     a[c] = make_float4(from[0], from[1], from[2], from[3]);
         }
       }
-      if (sums) {
+      if (kQuadSums && sums) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           cd[c][0] = cd[c][1] = make_uint4(0u, 0u, 0u, 0u);
@@ -614,7 +645,7 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) if (!kWhole && c >= rows) out[c] = 0u;            // padding
-      if (sums) {
+      if (kQuadSums && sums) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           float f[4];
@@ -632,11 +663,16 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
         for (int c = 0; c < 4; ++c) if (kWhole || c < rows) *reinterpret_cast<uint32_t*>(dst + c * row_pitch + 4 * k) = out[c];
       }
     };
-    for (int k = k_first + k_lane; live && k < k_end; k += tx) {
+    const int only = (int)(first + sub) & 3;                      // by_row: which of the four
+    if (by_row && live) {
+      acc[0] = finish_row(src + only * row_pitch, codes + only * row_pitch, dst + (tiled ? 4 * only : only * row_pitch), tiled ? 512 : 4,
+                          k_lane, only < rows ? (int)(sf_cols >> 2) : 0, tiled ? groups : 0, tx, unit, inv_unit);
+    }
+    for (int k = k_first + k_lane; live && !by_row && k < k_end; k += tx) {
       const bool full = (vec || tiled) && 4 * k + 4 <= sf_cols;
       if (full && rows == 4) {
         piece(std::true_type{}, k);
-      } else if (!kSums && full) {                                  // decode: fewer than 128 rows (a second copy beside the sums costs a third more registers)
+      } else if (!kQuadSums && full) {                              // decode: fewer than 128 rows
         piece(std::false_type{}, k);
       } else {                                                      // an edge of the tensor, or padding: kept short
 #pragma unroll 1
@@ -684,7 +720,10 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
       if (live && k_lane == 0) {
         const float half_unit = 0.5f * unit;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) if (row0 + 32 * c < R) J.row_sums[row0 + 32 * c] = acc[c] * half_unit;
+        for (int c = 0; c < 4; ++c) {
+          const int64_t r = row0 + 32 * (by_row ? only : c);
+          if (r < R && (!by_row || c == 0)) J.row_sums[r] = acc[c] * half_unit;
+        }
       }
     }
   }
@@ -961,7 +1000,22 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
   return METIS_OK;
 }
 
+// Which kernel forms the row sums.  Four rows to a thread move the fewest bytes per instruction, but leave few CTAs where the
+// tensor has few rows (16 per 128-row block), and where its last row block is not full the missing rows send that block
+// down the edge path, a chain of loads per block.  Measured, dual quantizer with sums, four rows / one row to a thread (us):
+// 16384 tokens x 128 columns 12.0 / 10.2, x 1024 28.2 / 27.4, 65536 x 1024 106.7 / 94.7, but 16384 x 1536 38.4 / 39.9,
+// 16384 x 4096 90.4 / 95.7; last row block not full: 16384 x 1104 42.0 / 31.5, x 2032 66.8 / 50.4, x 4208 114 / 106,
+// 4096 x 8304 51.5 / 54.8.
+static FinalizeForm finalize_form(const FinalizeJobs& jobs, int njobs) {
+  for (int j = 0; j < njobs; ++j) {
+    const FinalizeJob& J = jobs.job[j];
+    if (J.row_sums) return J.R <= 1280 || (J.R % 128 != 0 && J.R <= 6144) ? kFinSumsByRow : kFinSums;          // one job at most wants them
+  }
+  return kFinPlain;
+}
+
 static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t st, uint64_t* offset_ctr) {
+  const FinalizeForm form = finalize_form(jobs, njobs);
   int64_t blocks = 1;
   for (int j = 0; j < njobs; ++j) {
     FinalizeJob& J = jobs.job[j];
@@ -969,12 +1023,12 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
     J.log_tx = 2;                                             // a warp holds at most 8 rows' lanes of 4 tiles
     while (J.log_tx < 6 && (1 << J.log_tx) < groups) ++J.log_tx;
     const int64_t segments = J.row_sums ? 1 : ceil_div(groups, (int64_t)1 << J.log_tx);
-    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16 * segments, 64 >> J.log_tx);
+    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16 * segments << (form == kFinSumsByRow && J.row_sums ? 2 : 0), 64 >> J.log_tx);
     if (need > blocks) blocks = need;
   }
   if (njobs == 1) jobs.job[1] = jobs.job[0];
-  const bool sums = jobs.job[0].row_sums || jobs.job[1].row_sums;
-  auto kern = sums ? finalize_scales_kernel<true> : finalize_scales_kernel<false>;
+  const bool sums = form != kFinPlain;
+  auto kern = form == kFinPlain ? finalize_scales_kernel<kFinPlain> : form == kFinSums ? finalize_scales_kernel<kFinSums> : finalize_scales_kernel<kFinSumsByRow>;
   const int64_t cap = (int64_t)sm_count() * (sums ? 10 : 8) / njobs;     // resident at once: 5 (sums) and 8 per SM
   if (blocks > cap) blocks = ceil_div(blocks, ceil_div(blocks, cap));    // the fewest CTAs that need no more rounds than `cap` would
   METIS_CUDA_OK(launch_overlapped(kLaunchShort, kern, dim3((unsigned)blocks, (unsigned)njobs), dim3(kFinThreads), 0, st,

@@ -399,7 +399,8 @@ def test_two_operands_rotated_alike_give_sixteen_times_the_plain_product():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,cols", [(64, 32), (128, 4096), (1024, 528), (16384, 128), (4096, 4096)])
+@pytest.mark.parametrize("rows,cols", [(64, 32), (128, 4096), (1024, 528), (16384, 128), (4096, 4096),
+                                       (64, 16), (192, 48), (4160, 80), (576, 1104), (2048, 1136)])      # the last row block partly there
 @pytest.mark.parametrize("stochastic", [False, True])
 def test_dual_quantizer_forms_the_token_sums_of_the_transposed_output(rows, cols, stochastic):
     """token_sums_t[k] = sum over the tokens of the quantized values of column k: equal to the row sums the
