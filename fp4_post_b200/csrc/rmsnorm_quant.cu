@@ -225,7 +225,10 @@ __device__ __forceinline__ float norm_block(const float (&v)[16], float rs, cons
 // the block maxima there for the scale pass) change nothing here and cost the tile kernels of quantize.cu 20 %; a prefetch
 // of the next row into L2 changes nothing either.
 constexpr int kNormRowThreads = 256;
-constexpr int64_t kNormRowsMinRows = 1024;                  // fewer rows do not fill the SMs: 512 x 4096 6.8 us against 3.8
+// Fewer rows do not fill the SMs with a warp each (both launches, a CTA / a warp per row, us): 896 x 4096 7.6 / 9.2, 640 x 3584
+// 6.5 / 8.3, 640 x 2048 7.0 / 7.5, 800 x 2048 6.0 / 6.1; equal from 1024 x 3584 (9.5 / 9.6) on, and rows of 512 elements do not
+// care (896: 4.9 / 4.5).
+constexpr int64_t kNormRowsMinRows = 1024;
 template <typename TG, int kM, bool kWriteNorm>
 __global__ void __launch_bounds__(kNormRowThreads, kM <= 3 ? 3 : 2)
 rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
@@ -499,17 +502,22 @@ static int32_t try_small(const TX* x, int64_t rows, int64_t cols, int64_t ld, co
   return METIS_OK;
 }
 
+// CTAs of the CTA-per-row kernel: persistent, as many as are resident at once, so that all of them finish together
+template <typename TX, typename TG, int kBlocks>
+static int64_t norm_ctas(int64_t rows, int bx, bool with_norm, int sms) {
+  const int by = kNormThreads / bx;
+  const void* kern = with_norm ? reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, true>)
+                               : reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, false>);
+  const int64_t blocks = (int64_t)sms * resident_ctas(kern, bx * by, 0), need = ceil_div(rows, by);
+  return blocks < need ? blocks : need;
+}
+
 // *records: in: where the per-CTA records may go (or nullptr); out: nullptr if the running maximum was used instead
 template <typename TX, typename TG, int kBlocks>
 static int32_t launch_norm(const TX* x, int64_t rows, int bpr, int bx, int64_t ld, const TG* gamma, float eps,
                            uint32_t* codes, const WorkspaceView& ws, unsigned int** records, void* norm_out, int sms, cudaStream_t st) {
   const int by = kNormThreads / bx;
-  // persistent CTAs: exactly as many as are resident at once, so that all of them finish together
-  const void* kern = norm_out ? reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, true>)
-                              : reinterpret_cast<const void*>(rmsnorm_quantize_kernel<TX, TG, kBlocks, false>);
-  int64_t blocks = (int64_t)sms * resident_ctas(kern, bx * by, 0);
-  const int64_t need = ceil_div(rows, by);
-  if (blocks > need) blocks = need;
+  const int64_t blocks = norm_ctas<TX, TG, kBlocks>(rows, bx, norm_out != nullptr, sms);
   if (blocks > kMaxRecords) *records = nullptr;
   if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
   const dim3 b((unsigned)bx, (unsigned)by);
@@ -543,16 +551,6 @@ static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t 
                                float eps, uint32_t* codes, const WorkspaceView& ws, unsigned int** records, void* norm_out,
                                int sms, cudaStream_t st) {
   const int bpr = (int)(cols >> 4);
-  if constexpr (sizeof(TX) == 2) {
-    if (bpr >= 32 && bpr <= 256 && rows >= kNormRowsMinRows) {
-      switch ((bpr + 31) / 32) {
-#define METIS_NORM_ROWS(M) case M: return launch_norm_rows<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
-        METIS_NORM_ROWS(1); METIS_NORM_ROWS(2); METIS_NORM_ROWS(3); METIS_NORM_ROWS(4);
-        METIS_NORM_ROWS(5); METIS_NORM_ROWS(6); METIS_NORM_ROWS(7); METIS_NORM_ROWS(8);
-#undef METIS_NORM_ROWS
-      }
-    }
-  }
   // threads along the row: whole warps, as many as the row has 32-block groups (hidden 1536 runs
   // with 96 threads per row and two rows per CTA instead of 128 with a quarter of them idle);
   // rows shorter than a warp take the next power of two
@@ -562,6 +560,18 @@ static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t 
     if (bx > kNormThreads) bx = kNormThreads;
   } else {
     while (bx < bpr) bx <<= 1;
+  }
+  if constexpr (sizeof(TX) == 2) {
+    // a warp per row from kNormRowsMinRows on, and where a CTA per row has more CTAs than there are records
+    if (bpr >= 32 && bpr <= 256 &&
+        (rows >= kNormRowsMinRows || (*records && norm_ctas<TX, TG, 1>(rows, bx, norm_out != nullptr, sms) > kMaxRecords))) {
+      switch ((bpr + 31) / 32) {
+#define METIS_NORM_ROWS(M) case M: return launch_norm_rows<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
+        METIS_NORM_ROWS(1); METIS_NORM_ROWS(2); METIS_NORM_ROWS(3); METIS_NORM_ROWS(4);
+        METIS_NORM_ROWS(5); METIS_NORM_ROWS(6); METIS_NORM_ROWS(7); METIS_NORM_ROWS(8);
+#undef METIS_NORM_ROWS
+      }
+    }
   }
   const int per_thread = (bpr + bx - 1) / bx;
   if (per_thread <= 1) return launch_norm<TX, TG, 1>(x, rows, bpr, bx, ld, gamma, eps, codes, ws, records, norm_out, sms, st);

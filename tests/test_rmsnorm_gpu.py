@@ -65,6 +65,31 @@ def test_bf16_rows(rows, cols, gdtype):
     assert mism < 2e-3
 
 
+# The warp-per-row kernel: every number of blocks per lane, rows that end inside a round of 32 blocks and inside a CTA's
+# eight rows, and fewer than 1024 rows where a CTA per row would leave more records than there is room for (whether it
+# would depends on the type of gamma; both kernels have to pass).
+@pytest.mark.parametrize("rows,cols", [(1024, 512), (1025, 528), (1031, 1040), (1024, 1536), (1100, 2064), (1024, 2560), (1024, 3072),
+                                       (1024, 3600), (1027, 4096), (641, 2576), (700, 3072), (1023, 3584), (640, 3584)])
+@pytest.mark.parametrize("gdtype", [torch.bfloat16, torch.float32])
+def test_a_warp_per_row_for_long_inputs(rows, cols, gdtype):
+    x = synthetic(rows, cols, "student", seed=rows + cols, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(cols)
+    gamma = (1.0 + 0.1 * torch.randn(cols, generator=g)).to(gdtype)
+    q, y = ops.rmsnorm_nvfp4_quantize(x.to(DEV), gamma.to(DEV), 1e-6, return_norm=True)
+    assert_packed_equal(q, y.float().cpu().numpy(), cabi.SF_MMA, what="a warp per row")
+    # a row's norm does not depend on the others: bit for bit what the CTA-per-row kernel makes of 500 of them
+    for first in (0, rows - 500):
+        _, part = ops.rmsnorm_nvfp4_quantize(x[first:first + 500].to(DEV), gamma.to(DEV), 1e-6, return_norm=True)
+        assert torch.equal(y[first:first + 500], part)
+    # against torch: a bf16 rounding of the normalised value that falls the other way is at most 2^-7 of it, and with a
+    # bf16 gamma the rounding of the product can add as much
+    want = reference_norm(x, gamma, 1e-6).float()
+    assert bool(((y.float().cpu() - want).abs() <= want.abs() * 2.0 ** (-6 if gdtype == torch.bfloat16 else -7) + 1e-30).all())
+    assert float((y.float().cpu() == want).float().mean()) > 0.995
+    q1 = ops.rmsnorm_nvfp4_quantize(x.to(DEV), gamma.to(DEV), 1e-6)
+    assert torch.equal(q1.codes, q.codes) and torch.equal(q1.scales, q.scales) and torch.equal(q1.unit, q.unit)
+
+
 # Decode-sized inputs (a handful of rows of up to 8192 elements) take the one-launch cluster kernel:
 # one row, rows that fill one pass / all four passes of the 8 CTAs, two blocks per thread, a hidden
 # size that is not a power of two, and the first row count past the limit (the streaming kernels).
