@@ -740,7 +740,15 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
 // 8.0, 32 x 4096 5.2, 64 x 4096 6.8 against 8.1.
 constexpr int kSmallThreads = 512;
 constexpr int kSmallBlocks = 4;                    // blocks per thread
-constexpr int64_t kClusterMaxBlocksWithRecords = 4096;
+// Blocks per thread up to which the cluster is taken although the streaming path needs no zero-fill either.  8 CTAs of 512
+// threads: a round is 4096 blocks and costs 0.75 us for bf16, 1.1 for fp32, where the two launches stay at 3.9 to 5.5.  So one
+// round, one more for bf16, one more where no padding has to be cleared, one more where the scale pass would go down its edge
+// path.  Cluster / two launches, us: bf16 tiled 17 x 4096 3.9 / 4.3, 64 x 2048 4.3 / 5.0, 40 x 4096 5.0 / 4.8, row-major
+// 64 x 1040 3.3 / 5.3, 48 x 4096 4.3 / 4.6, 56 x 4096 4.9 / 4.2, 63 x 4112 5.0 / 5.5; fp32 tiled 32 x 4096 5.1 / 4.3, 2100 x 32
+// 4.3 / 5.5, row-major 64 x 2048 4.4 / 4.5, 48 x 4096 5.3 / 4.2, 120 x 1552 5.3 / 6.6.
+static int cluster_rounds(int64_t C, int32_t sf_layout, int64_t element_bytes) {
+  return 1 + (element_bytes == 2) + (sf_layout == METIS_SF_ROWMAJOR) + (C % 64 != 0);
+}
 constexpr int64_t kSmallMaxBlocks = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks;
 
 template <typename T, bool kMean>
@@ -1120,11 +1128,10 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
   // pass, as in the dual quantizer; without them the running maximum and the error word are zeroed in front of it, and
   // that memset node costs 3-4 us (16 x 14336: 8.2 us with it, 4.9 without; 1120 x 3584: 12.4, 8.1).
   unsigned int* records = workspace_records(workspace, workspace_bytes, R, C);
-  // One cluster for the whole tensor: with records, only where two launches over many SMs are not faster (16 x 4096:
-  // 4.3 us against 4.5; 64 x 3584 on the cluster's 8 SMs: 7.1 against 5.0).
+  // One cluster for the whole tensor; with records, only where two launches over many SMs are not faster.
   int64_t tiles = 0, padded_words = 0;
   if (!transpose && !sr && aligned16(scales) && small_path(R, C, sf_layout, &tiles, &padded_words) &&
-      (!records || R * (C / 16) <= kClusterMaxBlocksWithRecords)) {
+      (!records || R * (C / 16) <= (int64_t)kSmallCtas * kSmallThreads * cluster_rounds(C, sf_layout, esz))) {
     return x_dtype == METIS_DTYPE_BF16
         ? launch_small(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st)
         : launch_small(static_cast<const float*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st);

@@ -147,9 +147,10 @@ int64_t metis_nvfp4_quantize_workspace_bytes(int64_t R, int64_t C);
  *
  * Launches: large tensors take one streaming pass and a scale pass, with a zero-fill of the workspace
  * header in front unless the workspace has METIS_QUANTIZE_EXTRA_WORKSPACE more bytes and the pass at most
- * 640 CTAs.  Round-to-nearest, untransposed tensors of at most 16384 blocks (rollout-sized
- * activations; 4096 where that zero-fill is not needed) take ONE kernel that runs as a single thread-block cluster and does not touch the
- * workspace (it must still be passed and large enough); results are bit-identical.
+ * 640 CTAs.  Round-to-nearest, untransposed tensors of at most 16384 blocks (rollout-sized activations; where
+ * that zero-fill is not needed 4096 to 16384, by type, layout and width) take ONE kernel that runs as a single
+ * thread-block cluster and does not touch the workspace (it must still be passed and large enough); results are
+ * bit-identical.
  */
 int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t rows, int64_t cols, int64_t ld,
                              const float* col_mean, uint32_t flags, uint64_t seed, uint64_t offset,
