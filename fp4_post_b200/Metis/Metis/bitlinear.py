@@ -1047,6 +1047,10 @@ class MetisFusedFunction(torch.autograd.Function):
             x_t = xa.transposed()
             if centred and getattr(x_t, "_row_sums", None) is None:
                 _row_sums(x_t, xa.rotate)   # cached on x_t and read by both branches
+            if centred and x_t.col_vec is not None and getattr(x_t, "_tail", None) is None:
+                # read by both branches too: formed on the second stream, it would make this one wait for the
+                # low-rank chain in front of it
+                _token_tail(x_t, xa.rotate, M)
             main, aux = current_stream(g.device), _aux_stream(g.device)
             aux.wait_stream(main)
             # the weight-gradient product comes first and reads the transposed output only

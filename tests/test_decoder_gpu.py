@@ -69,6 +69,27 @@ def test_fused_norms_feed_the_projection_groups_and_match_plain_norms():
     assert torch.nn.functional.cosine_similarity(a.flatten(), b.flatten(), dim=0) > 0.9
 
 
+def test_the_backward_forms_no_shared_row_vector_behind_the_low_rank_chain():
+    """Qx^T 1 + M mu_x is read by both weight-gradient products.  Behind a fused norm it does not exist when the backward
+    starts; formed on the second stream it would hold the big product back until the low-rank chain gets there."""
+    model = _metis_decoder(True)
+    ids = torch.randint(0, SMALL.vocab, (2, 64), device=DEV, generator=torch.Generator(device=DEV).manual_seed(4))
+    second = bitlinear._aux_stream(torch.device(DEV, 0)).cuda_stream
+    seen, real = [], bitlinear._add_mean
+
+    def recording(*args):
+        seen.append(torch.cuda.current_stream().cuda_stream)
+        return real(*args)
+    loss = model.loss(ids)
+    bitlinear._add_mean = recording
+    try:
+        loss.backward()
+    finally:
+        bitlinear._add_mean = real
+    assert len(seen) == 2 * SMALL.layers                    # once per norm: the groups behind them share it
+    assert second not in seen
+
+
 def test_a_whole_decoder_step_replays_from_one_graph():
     model = _metis_decoder(True, backward_q="nvfp4e2m1b")
     params = list(model.parameters())
