@@ -35,7 +35,10 @@ def _need_cuda(t: torch.Tensor, what: str) -> None:
         raise RuntimeError(f"{what} must be a CUDA tensor: the NVFP4 path has no CPU fallback")
 
 
-_current_device = torch._C._cuda_getDevice            # torch.cuda.current_device() without its checks: a CUDA tensor exists
+def _current_device() -> int:
+    """torch.cuda.current_device() without its checks: a CUDA tensor exists.  (Looked up when called: a torch without CUDA
+    does not have it, and imports this module all the same.)"""
+    return torch._C._cuda_getDevice()
 
 
 def _stream() -> int:

@@ -139,3 +139,13 @@ def test_gemm_rejects_reserved_bits_other_than_the_two_test_hooks(L):
         a.ldd, a.d_dtype, a.alpha, a.reserved = 256, cabi.DTYPE_BF16, 1.0, bits
         rc = L.metis_nvfp4_gemm(C.byref(a))
         assert rc == -1 and b"reserved" in L.metis_last_error_string(), bits
+
+
+def test_the_package_imports_on_a_torch_without_cuda():
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda')]:\n"
+            "    delattr(torch._C, name)\n"
+            "import fp4_post_b200.ops, fp4_post_b200.decoder, fp4_post_b200.checkpoint, fp4_post_b200.Metis.Metis.bitlinear\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
