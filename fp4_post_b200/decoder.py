@@ -20,6 +20,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as Fn
 from torch import nn
+from torch.autograd import forward_ad
 
 from fp4_post_b200 import ops
 from fp4_post_b200.Metis.Metis.bitlinear import forward_group
@@ -58,8 +59,20 @@ def _rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor
 
 
 def _native(*tensors) -> bool:
-    """Inference on bf16 CUDA tensors: the elementwise pieces run as one launch each, with the same roundings."""
-    return not torch.is_grad_enabled() and all(t.is_cuda and t.dtype == torch.bfloat16 and t.device == tensors[0].device for t in tensors)
+    """Inference on plain bf16 CUDA tensors: the elementwise pieces run as one launch each, with the same roundings.  Whatever
+    has to see the torch operations gets them: autograd, forward-mode derivatives (which no_grad leaves on), vmap and the
+    other function transforms, tensor subclasses, dispatch modes, tracing."""
+    first = tensors[0]
+    return (not torch.is_grad_enabled()
+            and all(type(t) in (torch.Tensor, nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.device == first.device
+                    and t.numel() > 0 and forward_ad.unpack_dual(t).tangent is None for t in tensors)
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._len_torch_dispatch_stack() == 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
+
+
+def _table_of(t: torch.Tensor, T: int, D: int) -> bool:
+    """T rows of D elements, the same for every batch entry and head."""
+    return t.dim() >= 2 and t.shape[-2:] == (T, D) and t.numel() == T * D
 
 
 class Attention(nn.Module):
@@ -78,7 +91,7 @@ class Attention(nn.Module):
         q = q.view(B, T, c.heads, c.head_dim)
         k = k.view(B, T, c.kv_heads, c.head_dim)
         v = v.view(B, T, c.kv_heads, c.head_dim).transpose(1, 2)
-        if _native(q, k, cos, sin) and c.head_dim % 8 == 0 and cos.numel() == sin.numel() == T * c.head_dim:
+        if c.head_dim % 8 == 0 and _table_of(cos, T, c.head_dim) and _table_of(sin, T, c.head_dim) and _native(q, k, cos, sin):
             q, k = (t.transpose(1, 2) for t in ops.rope_pair(q, k, cos, sin))
         else:
             q, k = _rope(q.transpose(1, 2), cos, sin), _rope(k.transpose(1, 2), cos, sin)
@@ -95,7 +108,7 @@ class MLP(nn.Module):
 
     def forward(self, h):
         gate, up = forward_group((self.gate_proj, self.up_proj), h)
-        if _native(gate, up) and gate.numel() % 8 == 0:
+        if gate.shape == up.shape and gate.numel() % 8 == 0 and _native(gate, up):
             return self.down_proj(ops.silu_mul(gate, up))
         return self.down_proj(Fn.silu(gate) * up)
 

@@ -603,6 +603,18 @@ def lowrank_du(g: torch.Tensor, ts: torch.Tensor, out_dtype: torch.dtype = torch
     return out
 
 
+def _same_device(first: torch.Tensor, **others) -> None:
+    for name, t in others.items():
+        if t.device != first.device:
+            raise ValueError(f"{name} is on {t.device}, not on {first.device}")
+
+
+def _dense(t: torch.Tensor, alignment: int) -> torch.Tensor:
+    """t with contiguous elements on an aligned address (copied only if it has to be)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % alignment == 0 else t.clone()
+
+
 def rope_pair(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
     """Rotary embedding (rotate-half convention) of q [B, T, Hq, D] and k [B, T, Hk, D], bf16 and contiguous, in one
     launch, with every rounding of `x * cos + cat(-x2, x1) * sin` on bf16 tensors.  cos, sin: bf16, T rows of D elements
@@ -615,7 +627,8 @@ def rope_pair(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.Te
     Hk = k.shape[2]
     if k.shape != (B, T, Hk, D) or cos.numel() != T * D or sin.numel() != T * D:
         raise ValueError(f"shapes do not fit: q {tuple(q.shape)}, k {tuple(k.shape)}, cos {tuple(cos.shape)}, sin {tuple(sin.shape)}")
-    q, k, cos, sin = q.contiguous(), k.contiguous(), cos.contiguous(), sin.contiguous()
+    _same_device(q, k=k, cos=cos, sin=sin)
+    q, k, cos, sin = (_dense(t, 8) for t in (q, k, cos, sin))
     with _on_device(q.device):
         qo, ko = torch.empty_like(q), torch.empty_like(k)
         rc = cabi.lib().metis_rope_pair(q.data_ptr(), k.data_ptr(), cos.data_ptr(), sin.data_ptr(), qo.data_ptr(), ko.data_ptr(),
@@ -631,7 +644,8 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     _need_cuda(up, "up")
     if gate.dtype != torch.bfloat16 or up.dtype != torch.bfloat16 or gate.shape != up.shape:
         raise TypeError("gate and up must be bfloat16 tensors of one shape")
-    gate, up = gate.contiguous(), up.contiguous()
+    _same_device(gate, up=up)
+    gate, up = _dense(gate, 16), _dense(up, 16)
     with _on_device(gate.device):
         out = torch.empty_like(gate)
         rc = cabi.lib().metis_silu_mul(gate.data_ptr(), up.data_ptr(), out.data_ptr(), gate.numel(), _stream())

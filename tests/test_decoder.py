@@ -49,3 +49,16 @@ def test_metis_layers_install_by_name_and_reproduce_the_plain_model_with_identit
     assert torch.isfinite(loss)
     for n, p in metis.named_parameters():
         assert p.grad is not None and torch.isfinite(p.grad).all(), n
+
+
+def test_fake_tensors_go_through_the_torch_expressions():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from fp4_post_b200.decoder import Block
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        with FakeTensorMode(), torch.no_grad(), torch.device("cuda"):
+            block = Block(TINY, fuse_norms=False)
+            x, table = torch.empty(2, 12, TINY.hidden), torch.empty(1, 1, 12, TINY.head_dim)
+            assert x.is_cuda and block(x, table, table).shape == x.shape
+    finally:
+        torch.set_default_dtype(torch.float32)

@@ -173,3 +173,51 @@ def test_silu_times_up_in_one_launch_is_the_torch_expression(shape):
     ok = (got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7
     assert bool((ok | (got.isnan() & want.isnan())).all())
     assert float(((got == want) | want.isnan()).float().mean()) > 0.99
+
+
+def _dense_block():
+    from fp4_post_b200.decoder import Block
+    torch.manual_seed(5)
+    return Block(SMALL, fuse_norms=False).to(DEV, torch.bfloat16)
+
+
+def test_forward_mode_derivatives_without_grad_pass_through_the_elementwise_pieces():
+    import torch.autograd.forward_ad as fwad
+    block = _dense_block()
+    h, dh = (torch.randn(2, 24, SMALL.hidden, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    with torch.no_grad(), fwad.dual_level():
+        got = fwad.unpack_dual(block.mlp(fwad.make_dual(h, dh)))
+        assert got.tangent is not None
+    with torch.enable_grad(), fwad.dual_level():
+        want = fwad.unpack_dual(block.mlp(fwad.make_dual(h, dh)))
+    assert torch.equal(got.primal, want.primal)
+    # the two modes take the derivative of silu apart differently: five or six bf16 roundings (2^-9 each) on either side
+    a, b = got.tangent.float(), want.tangent.float()
+    assert float((a - b).norm()) <= 12 * 2.0 ** -9 * float(b.norm())
+
+
+def test_vmap_and_empty_batches_go_through_the_torch_expressions():
+    block = _dense_block()
+    with torch.no_grad():
+        x = torch.randn(3, 2, 24, SMALL.hidden, device=DEV, dtype=torch.bfloat16)
+        mapped = torch.vmap(block.mlp)(x)
+        each = torch.stack([block.mlp(t) for t in x])
+        assert torch.allclose(mapped.float(), each.float(), rtol=2.0 ** -6, atol=1e-3 * float(each.abs().max()))    # other GEMM shapes
+        assert block.mlp(x[0, :0]).shape == (0, 24, SMALL.hidden)
+
+
+def test_tables_on_odd_addresses_and_tensors_of_two_devices():
+    from fp4_post_b200 import decoder, ops
+    q = torch.randn(2, 24, 4, 64, device=DEV, dtype=torch.bfloat16)
+    k = torch.randn(2, 24, 2, 64, device=DEV, dtype=torch.bfloat16)
+    table = torch.randn(24 * 64 + 1, device=DEV, dtype=torch.bfloat16)
+    cos = sin = table[1:].view(24, 64)                              # two bytes past an aligned address
+    for x, y in zip((q, k), ops.rope_pair(q, k, cos, sin)):
+        assert torch.equal(y, decoder._rope(x.transpose(1, 2), cos, sin).transpose(1, 2))
+    flat = torch.randn(65, device=DEV, dtype=torch.bfloat16)
+    want = ops.silu_mul(flat[1:].clone(), flat[1:].clone())
+    assert torch.equal(ops.silu_mul(flat[1:], flat[1:]), want)
+    with pytest.raises(RuntimeError):
+        ops.silu_mul(flat, flat.cpu())
+    with pytest.raises(RuntimeError):
+        ops.rope_pair(q, k, cos, sin.cpu())
