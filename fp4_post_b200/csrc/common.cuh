@@ -286,10 +286,11 @@ __device__ __forceinline__ uint32_t quantize8_rn(const float (&x)[8], float s) {
 struct Philox {
   uint32_t k0, k1;
   __device__ __forceinline__ Philox(uint64_t seed) : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)) {}
-  // Counter words {block, 0, offset}: block indexes stay below 2^32 (a tensor of 2^36 elements does not fit this GPU's
-  // memory with its codes), and with the second word known to be zero the first round's product with c2 and the
-  // second round's with c0 are the same for the whole launch: the compiler takes them out of the loop.  (One wide
-  // multiplication in place of each pair of high and low products was measured slower: 80 -> 89 us, 16384 x 4096 both.)
+  // Counter words {block, 0, offset}: block indexes stay below 2^32 (the entry points refuse more, kMaxStochasticElements;
+  // this GPU's memory does not hold such a tensor and its codes), and with the second word known to be zero the first
+  // round's product with c2 and the second round's with c0 are the same for the whole launch: the compiler takes them
+  // out of the loop.  (One wide multiplication in place of each pair of high and low products was measured slower:
+  // 80 -> 89 us, 16384 x 4096 both.)
   __device__ __forceinline__ uint4 operator()(uint32_t block, uint64_t ctr_hi) const {
     uint32_t c0 = block, c1 = 0u;
     uint32_t c2 = (uint32_t)ctr_hi, c3 = (uint32_t)(ctr_hi >> 32);

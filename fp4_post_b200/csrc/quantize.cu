@@ -137,6 +137,7 @@ template <typename T> struct TileCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 2 * kCols * 4 + 64 + 1024;
 };
 constexpr int64_t kTileRowsMinElements = 1 << 20;          // row-major tensors from this size on go through the tile kernel
+constexpr int64_t kMaxStochasticElements = (int64_t)1 << 36;   // blocks are counted in 32 bits (struct Philox)
 constexpr uint64_t kColumnStream = 1ull << 63;             // Philox counter space of the transposed output in dual mode
 
 // Workspace of the dual quantizer: word 63 = number of CTA records, records from word 64 on (3 words per CTA),
@@ -1122,6 +1123,7 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
     return fail(METIS_ERR_BAD_ALIGNMENT, "x must be 16-byte aligned with cols and ld multiples of %lld", (long long)need);
   if (col_mean && !aligned16(col_mean)) return fail(METIS_ERR_BAD_ALIGNMENT, "col_mean must be 16-byte aligned");
   if (rows >= ((int64_t)1 << 31) || cols >= ((int64_t)1 << 31)) return fail(METIS_ERR_TOO_LARGE, "tensor too large");
+  if (sr && rows * cols >= kMaxStochasticElements) return fail(METIS_ERR_TOO_LARGE, "stochastic rounding of 2^36 elements or more");
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // With METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than it needs the workspace also holds a record per CTA of the first
@@ -1219,6 +1221,7 @@ extern "C" int32_t metis_nvfp4_quantize_dual(const void* x, int32_t x_dtype, int
     return fail(METIS_ERR_WORKSPACE, "workspace of %lld bytes, need %lld", (long long)workspace_bytes,
                 (long long)metis_nvfp4_quantize_dual_workspace_bytes(rows, cols));
   if (rows >= ((int64_t)1 << 31) || cols >= ((int64_t)1 << 31)) return fail(METIS_ERR_TOO_LARGE, "tensor too large");
+  if (sr && rows * cols >= kMaxStochasticElements) return fail(METIS_ERR_TOO_LARGE, "stochastic rounding of 2^36 elements or more");
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // every CTA of the first pass leaves its maxima and its error word in a record of its own: nothing to zero first
