@@ -523,25 +523,22 @@ static int32_t run_gemm(const metis_gemm_args* a, const ScaledOutput* scaled) {
     p.partial = static_cast<float*>(a->workspace);
     p.ldp = ceil_div(a->N, 32) * 32;
   }
-  if (scaled) {
-    // Only the split-K finish of a decode-sized product writes the scaled copy itself (one launch of 4 us less in the
-    // chain).  In the epilogue of the unsplit kernel it was measured slower than the launch it saves: 15.5 + 7.0 us ->
-    // 24.4 at 16384 x 128 x 4096, where four warps per SM do all the divisions.
-    if (p.splits == 1) {
-      if (int32_t rc = run_gemm(a, nullptr)) return rc;
-      return metis_lowrank_scale(a->d, a->M, a->N, a->ldd, scaled->s, scaled->s_dtype, scaled->unit_a, scaled->unit_b, scaled->t, a->stream);
-    }
+  // Only the split-K finish of a decode-sized product writes the scaled copy itself (one launch of 4 us less in the
+  // chain).  In the epilogue of the unsplit kernel it was measured slower than the launch it saves: 15.5 + 7.0 us ->
+  // 24.4 at 16384 x 128 x 4096, where four warps per SM do all the divisions.
+  const bool scale_behind = scaled && p.splits == 1;
+  if (scaled && !scale_behind) {
     p.s = scaled->s; p.s_is_f32 = scaled->s_dtype == METIS_DTYPE_F32;
     p.s_unit_a = scaled->unit_a; p.s_unit_b = scaled->unit_b;
     p.scaled = static_cast<__nv_bfloat16*>(scaled->t);
   }
-  if (pair) return launch_gemm_pair(a, ma, mb, mt, mu, p);
-  if (bn == 256) {
-    if (a->d_dtype == METIS_DTYPE_BF16) return launch_gemm<256, __nv_bfloat16>(a, ma, mb, mt, mu, p);
-    return launch_gemm<256, float>(a, ma, mb, mt, mu, p);
-  }
-  if (a->d_dtype == METIS_DTYPE_BF16) return launch_gemm<128, __nv_bfloat16>(a, ma, mb, mt, mu, p);
-  return launch_gemm<128, float>(a, ma, mb, mt, mu, p);
+  const bool bf16 = a->d_dtype == METIS_DTYPE_BF16;
+  int32_t rc;
+  if (pair) rc = launch_gemm_pair(a, ma, mb, mt, mu, p);
+  else if (bn == 256) rc = bf16 ? launch_gemm<256, __nv_bfloat16>(a, ma, mb, mt, mu, p) : launch_gemm<256, float>(a, ma, mb, mt, mu, p);
+  else rc = bf16 ? launch_gemm<128, __nv_bfloat16>(a, ma, mb, mt, mu, p) : launch_gemm<128, float>(a, ma, mb, mt, mu, p);
+  if (rc || !scale_behind) return rc;
+  return metis_lowrank_scale(a->d, a->M, a->N, a->ldd, scaled->s, scaled->s_dtype, scaled->unit_a, scaled->unit_b, scaled->t, a->stream);
 }
 
 extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) { return run_gemm(a, nullptr); }

@@ -456,7 +456,8 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
     accumulator units.  rank1 = up to two (cvec or None, rvec) pairs of fp32 vectors.
     Only the packed parts of a and b enter the product; their mean vectors do not.
     sm_limit > 0 caps the SMs this launch occupies (room for a collective's kernel beside it).
-    scaled = (s, unit_a, unit_b), for a bf16 D: returns (D, lowrank_scale(D, s, unit_a, unit_b)) from the same launch."""
+    scaled = (s, unit_a, unit_b), for a bf16 D: returns (D, lowrank_scale(D, s, unit_a, unit_b)); the second value costs
+    no launch of its own where the product is split along K."""
     M, K = a.shape
     N, K2 = b.shape
     if K != K2:

@@ -350,9 +350,10 @@ typedef struct metis_gemm_args {
 int32_t metis_nvfp4_gemm(const metis_gemm_args* args);
 
 /*
- * metis_nvfp4_gemm with a bf16 D [M, N] (N a multiple of 8), and metis_lowrank_scale of it in the same launch:
+ * metis_nvfp4_gemm with a bf16 D [M, N] (N a multiple of 8), and metis_lowrank_scale of it:
  * t[m][n] = bf16( float(bf16(D[m][n] * s[n])) / (unit_a * unit_b) ), row pitch N: the product with V and the
- * scaling behind it (bitlinear.py:752-756).
+ * scaling behind it (bitlinear.py:752-756).  A product split along K (see the workspace below) writes t in the
+ * launch that adds its partial sums; any other takes a second launch.
  */
 int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* args, const void* s, int32_t s_dtype, const float* unit_a,
                                 const float* unit_b, void* t);
