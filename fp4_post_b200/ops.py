@@ -15,7 +15,8 @@ from . import cabi
 _DTYPES = {torch.bfloat16: cabi.DTYPE_BF16, torch.float32: cabi.DTYPE_F32}
 
 # Kernels of this library launched since import, by entry point (two per quantizer call: the
-# streaming pass and the scale pass; a memset in front of them is not a kernel).
+# streaming pass and the scale pass; a memset in front of them is not a kernel).  The quantizers and the column
+# mean have one-launch forms for small inputs; those calls are counted as two all the same.
 LAUNCHES = {"quantize": 0, "rmsnorm_quantize": 0, "dequantize": 0, "col_mean": 0, "gemv": 0, "gemm": 0, "lowrank_bwd": 0, "decoder": 0}
 
 
@@ -525,7 +526,7 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
             rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), s.data_ptr(), _dtype_code(s, "s"), unit_a.data_ptr(),
                                                     unit_b.data_ptr(), t.data_ptr())
     cabi.check(rc, "metis_nvfp4_gemm")
-    LAUNCHES["gemm"] += 2 if ws_bytes > 0 else 1
+    LAUNCHES["gemm"] += 2 if ws_bytes > 0 or scaled is not None else 1       # the sum of the splits, or the scaling
     return out if scaled is None else (out, t)
 
 
@@ -581,7 +582,9 @@ def lowrank_dts(g: torch.Tensor, u: torch.Tensor, yv: torch.Tensor, s: torch.Ten
                                       s.data_ptr(), _dtype_code(s, "s"), d_yv.data_ptr(), d_yv.stride(0), ds.data_ptr(),
                                       _DTYPES[ds_dtype], _ptr(mean), ws.data_ptr(), ws.numel(), _ptr(status), _stream())
     cabi.check(rc, "metis_lowrank_dts_mean")
-    LAUNCHES["lowrank_bwd"] += 2
+    # the product, the sum of its splits where it has more than one, the sums over the CTAs
+    one_split = M * ((r + 63) // 64 * 64) * 4
+    LAUNCHES["lowrank_bwd"] += 2 if L.metis_bf16_panel_gemm_workspace_bytes(M, r, N) == one_split else 3
     return (d_yv, ds, mean) if want_mean else (d_yv, ds)
 
 

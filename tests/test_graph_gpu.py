@@ -105,3 +105,41 @@ def test_light_stream_helpers_agree_with_torch():
             assert ops.current_stream(dev) == st
             raise KeyError
     assert torch.cuda.current_stream(dev) == before
+
+
+def _kernel_nodes(fn):
+    """Kernel nodes of a captured call of fn."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        keep = fn()                                                    # noqa: F841
+    handle = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, count = runtime.cudaGraphGetNodes(handle)
+    assert int(err) == 0
+    err, nodes, _ = runtime.cudaGraphGetNodes(handle, count)
+    assert int(err) == 0
+    kinds = [runtime.cudaGraphNodeGetType(n)[1] for n in nodes[:count]]
+    graph.reset()
+    return sum(k == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)
+
+
+@pytest.mark.parametrize("M,N,r", [(1120, 4096, 128), (19000, 512, 64), (64, 1024, 32)])       # several splits, one, several
+def test_the_launch_counter_counts_the_kernels_of_the_low_rank_backward(M, N, r):
+    g, u = torch.randn(M, N, device=DEV).to(torch.bfloat16), torch.randn(N, r, device=DEV).to(torch.bfloat16)
+    yv, s = torch.randn(M, r, device=DEV).to(torch.bfloat16), torch.ones(r, device=DEV)
+    for fn in (lambda: ops.lowrank_dts(g, u, yv, s), lambda: ops.lowrank_dts(g, u, yv, s, want_mean=True), lambda: ops.lowrank_du(g, yv)):
+        before = ops.launch_count()
+        nodes = _kernel_nodes(fn)
+        assert ops.launch_count() - before == 2 * nodes                # an eager call and the captured one
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 128, 4096), (16, 4096, 14336), (5, 256, 256), (300, 128, 512)])        # split twice, not split twice
+def test_the_launch_counter_counts_the_kernels_of_a_product(M, N, K):
+    a, b = ops.nvfp4_quantize(torch.randn(M, K, device=DEV)), ops.nvfp4_quantize(torch.randn(N, K, device=DEV))
+    s, one = torch.ones(N, device=DEV), torch.ones(1, device=DEV)
+    for fn in (lambda: ops.nvfp4_gemm(a, b), lambda: ops.nvfp4_gemm(a, b, scaled=(s, one, one))):
+        before = ops.launch_count()
+        nodes = _kernel_nodes(fn)
+        assert ops.launch_count() - before == 2 * nodes
