@@ -397,15 +397,21 @@ def nvfp4_dequantize(q: NVFP4Tensor, dtype: torch.dtype = torch.float32, add_mea
     return out
 
 
+def _unit_ptr(unit: torch.Tensor, dev: torch.device) -> int:
+    if unit.dtype != torch.float32 or unit.numel() != 1 or unit.device != dev:
+        raise ValueError(f"a unit is one fp32 value on {dev}, not {unit.numel()} of {unit.dtype} on {unit.device}")
+    return unit.data_ptr()
+
+
 def nvfp4_dequantize_ratio(q: NVFP4Tensor, dtype: torch.dtype, unit0, unit1, over0, over1) -> torch.Tensor:
     """Dense [R, C] tensor of q with (unit0 * unit1) / (over0 * over1) in place of its unit (device fp32 [1] each); the
     mean vectors of q are left out."""
     R, Cc = q.shape
+    units = [_unit_ptr(t, q.device) for t in (unit0, unit1, over0, over1)]
     with _on_device(q.device):
         out = torch.empty((R, Cc), dtype=dtype, device=q.device)
-        rc = cabi.lib().metis_nvfp4_dequantize_ratio(q.codes.data_ptr(), q.scales.data_ptr(), unit0.data_ptr(), unit1.data_ptr(),
-                                                     over0.data_ptr(), over1.data_ptr(), q.sf_layout, R, Cc, out.data_ptr(),
-                                                     _DTYPES[dtype], out.stride(0), _stream())
+        rc = cabi.lib().metis_nvfp4_dequantize_ratio(q.codes.data_ptr(), q.scales.data_ptr(), *units, q.sf_layout, R, Cc,
+                                                     out.data_ptr(), _DTYPES[dtype], out.stride(0), _stream())
     cabi.check(rc, "metis_nvfp4_dequantize_ratio")
     LAUNCHES["dequantize"] += 1
     return out
@@ -523,8 +529,8 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
             s = s.reshape(-1).contiguous()
             assert s.numel() == N and s.device == dev
             t = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), s.data_ptr(), _dtype_code(s, "s"), unit_a.data_ptr(),
-                                                    unit_b.data_ptr(), t.data_ptr())
+            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), s.data_ptr(), _dtype_code(s, "s"), _unit_ptr(unit_a, dev),
+                                                    _unit_ptr(unit_b, dev), t.data_ptr())
     cabi.check(rc, "metis_nvfp4_gemm")
     LAUNCHES["gemm"] += 2 if ws_bytes > 0 or scaled is not None else 1       # the sum of the splits, or the scaling
     return out if scaled is None else (out, t)

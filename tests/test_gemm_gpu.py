@@ -248,3 +248,14 @@ def test_scaled_copy_of_the_output_is_lowrank_scale_of_it(M, N, K, s_dtype):
     out, t = ops.nvfp4_gemm(a, b, rank1=[(None, row)], scaled=(s, ua, ub))
     assert torch.equal(out, plain)
     assert torch.equal(t, ops.lowrank_scale(plain, s, ua, ub))
+
+
+def test_units_of_another_type_size_or_device_are_refused():
+    a, b = ops.nvfp4_quantize(torch.randn(16, 256, device=DEV)), ops.nvfp4_quantize(torch.randn(32, 256, device=DEV))
+    s, one = torch.ones(32, device=DEV), torch.ones(1, device=DEV)
+    for bad in (one.double(), torch.ones(2, device=DEV), one.cpu(), one.to(torch.bfloat16)):
+        for units in ((bad, one), (one, bad)):
+            with pytest.raises(ValueError):
+                ops.nvfp4_gemm(a, b, scaled=(s, *units))
+            with pytest.raises(ValueError):
+                ops.nvfp4_dequantize_ratio(a, torch.bfloat16, one, *units, one)
