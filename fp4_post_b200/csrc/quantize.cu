@@ -12,6 +12,7 @@
 #include "tma.cuh"
 
 #include <atomic>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -940,13 +941,15 @@ int resident_ctas(const void* kernel, int threads, size_t smem) {
   static std::map<std::tuple<const void*, int, size_t, int>, int> known;
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 1;
-  std::lock_guard<std::mutex> lock(mutex);
-  const auto key = std::make_tuple(kernel, threads, smem, dev);
-  const auto hit = known.find(key);
-  if (hit != known.end()) return hit->second;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1) return 1;
-  known[key] = n;
-  return n;
+  // nothing may be thrown through the C entry points: without a lock or memory for it the answer is not kept
+  try {
+    std::lock_guard<std::mutex> lock(mutex);
+    int& kept = known[std::make_tuple(kernel, threads, smem, dev)];            // 0: not asked yet
+    if (kept == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) == cudaSuccess && n > 0) kept = n;
+    return kept > 0 ? kept : 1;
+  } catch (const std::exception&) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) == cudaSuccess && n > 0 ? n : 1;
+  }
 }
 unsigned int* workspace_records(void* workspace, int64_t workspace_bytes, int64_t R, int64_t C) {
   const int64_t at = (metis_nvfp4_quantize_workspace_bytes(R, C) + 15) / 16 * 16;
