@@ -254,8 +254,8 @@ __device__ __forceinline__ f32x2 round_like_folded2(f32x2 v) {
 // the low nibble.  Every element goes through the reference's own arithmetic: the correctly
 // rounded quotient x/s (half the reference's |x|/(s/2), exactly), its second rounding, and round
 // half to even onto the e2m1 grid by the hardware conversion, which packs two codes with their
-// sign bits per instruction (4 cycles per warp instruction and scheduler, i.e. 2 per element; packing the codes by
-// integer arithmetic instead was measured slower).  Division and second rounding run on the packed fp32
+// sign bits per instruction (four of them into one word take 8.0 cycles per warp and scheduler, 1 per element; packing
+// the codes by integer arithmetic instead was measured slower).  Division and second rounding run on the packed fp32
 // instructions, two elements per issue slot: these kernels are bound by issue, not by a pipe.
 // There is no approximate fast path because with bf16
 // inputs exact ties (an element equal to amax/8, 5/24 amax, ...) are common.  The division is

@@ -151,20 +151,17 @@ __device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
 
 // The same product along the tiled scale layout.  A 16-byte piece of that layout holds the scales of the rows l, l + 32,
 // l + 64, l + 96 of a 128-row block for 4 blocks of 16 columns: a warp takes these four rows, lane k of it every 32nd block
-// from k on, so that one 16-byte read of scales (shared by four lanes) and the 16 floats of v (which stay in L1) serve four
-// rows.  (Reading one scale byte per block and row instead costs a 32-byte sector per 4 blocks, i.e. the bytes of the codes
-// once more.)  The additions are those of the other kernels, in the same order: 16 products of a block one after the other,
-// a lane's blocks one after the other, then the lanes pairwise, so which kernel runs does not show in the result (a sum that
+// from k on, so that one 16-byte read of scales (shared by four lanes) and the 16 floats of v (which stay in L1) serve
+// four rows.  With too few rows to fill the SMs that way, two or four warps (`split`) share the four rows: each takes every
+// split-th round of 32 blocks and parks the block sums in shared memory; the lanes' sums are formed from there in order.
+// The additions are those of the other kernels, in the same order: 16 products of a block one after the other, a lane's
+// blocks one after the other, then the lanes pairwise, so which kernel runs does not show in the result (a sum that
 // differs in its last bit can flip the rounding of an activation, and a block of decoder layers makes 1 % of that).
-// With too few rows to fill the SMs that way, two or four warps (`split`) share the four rows: each takes every split-th round of
-// 32 blocks and parks the block sums in shared memory, and the lanes' sums are then formed from there in order.
-// Two e2m1 codes become two halves with one conversion (exact).  Bound by issue and by the conversions (the bytes alone
-// take 6 us at 18944 x 3584).
-// Measured, gemv_staged_kernel (or, below 2048 columns, gemv_kernel) before and this one after, six weights in turn:
-// 18944 x 3584 20.5 -> 13.5 us, 3584 x 18944 23.6 -> 17.4, 14336 x 4096 21.5 -> 13.1, 4096 x 14336 18.5 -> 14.6,
-// 8960 x 1536 10.2 -> 4.4, 1536 x 8960 7.7 -> 5.7, 4096 x 4096 6.4 -> 5.5.  Eight warps in a CTA instead of four end less
-// evenly (14.1, 19.0, 15.3, 16.5, 5.9, 5.9, 6.4); a warp per two rows reads v and the scales twice (3584 x 18944: 30 us).
-// A form that split the columns over a cluster, with another order of the additions, took 14.6, 16.9, 13.3, 14.7, 5.8, 5.8, 5.9.
+// Bound by issue and by the conversions (two codes become two halves with one, exactly): 18944 x 3584 takes 13.5 us, its
+// bytes 6.  Against the kernel it replaced there, six weights in turn, us: 18944 x 3584 20.5 -> 13.5, 3584 x 18944
+// 23.6 -> 17.4, 14336 x 4096 21.5 -> 13.1, 4096 x 14336 18.5 -> 14.6, 8960 x 1536 10.2 -> 4.4, 1536 x 8960 7.7 -> 5.7,
+// 4096 x 4096 6.4 -> 5.5.  Four warps in a CTA: with eight the last ones end less evenly (3584 x 18944 19.0); a warp per
+// two rows reads v and the scales twice (30).
 constexpr int kGemvWarps = 4, kGemvCtasPerSm = 8;
 template <bool kSplit>
 __global__ void __launch_bounds__(32 * kGemvWarps, kGemvCtasPerSm)
@@ -233,10 +230,11 @@ gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ 
   }
 }
 
-// The same product for a tall matrix (12288 rows and more) that gemv_quad_kernel does not take (row-major scales).  Two e2m1 codes become two
-// halves with one cvt (exact), and the 16 floats of v for a lane's block stay in registers across the
-// 4 rows of the warp (v otherwise costs 8 times the bytes of the codes in L1 traffic).  Shorter
-// matrices keep gemv_kernel: with four rows per warp they would not fill the SMs.
+// The same product for a tall matrix (12288 rows and more) that neither gemv_quad_kernel nor gemv_staged_kernel takes: mostly
+// narrow ones, of either layout (gemv_kernel / this, us: 152064 x 128 47 / 25, 12288 x 64 4.8 / 2.9, 18944 x 496 7.5 / 5.4).  Two
+// e2m1 codes become two halves with one cvt (exact), and the 16 floats of v for a lane's block stay in registers across the
+// 4 rows of the warp (v otherwise costs 8 times the bytes of the codes in L1 traffic).  Shorter matrices keep gemv_kernel:
+// with four rows per warp they would not fill the SMs.
 constexpr int kGemvTallRows = 4;          // rows per warp
 constexpr int64_t kGemvTallMinRows = 12288;
 constexpr int64_t kGemvTileMinCols = 512;
@@ -413,10 +411,9 @@ static cudaError_t launch_gemv_staged(const uint2* codes, const uint8_t* scales,
                            codes, scales, unit, sf_layout, R, C, v, out);
 }
 
-// How many warps share four rows.  24 warps per SM run at full rate, 12 to 15 at 0.88 of it (4096 x 4096: 5.5 us with 28 and 6.2
-// with 14), so the rows are shared further up to there, unless the rounds that the last warps lack cost as much (8960 x 1536 has
-// three rounds: 4.4 us with a warp per four rows, 5.6 with two); below 8 warps always.  Finally the block sums of eight
-// CTAs have to leave room for v in L1.
+// How many warps share four rows: as many as bring an SM to 24 warps (12 to 15 run at 0.88 of the rate: 4096 x 4096 5.5 us
+// with 28, 6.2 with 14), unless the rounds that the last warps lack cost as much (8960 x 1536 has three rounds: 4.4 us with
+// a warp per four rows, 5.6 with two); below 8 warps always.  The block sums of eight CTAs have to leave room for v in L1.
 constexpr int64_t kGemvWarpsPerSm = 24, kGemvFewWarpsPerSm = 8, kGemvL1Bytes = 208 << 10, kGemvSumBytesMax = 96 << 10;
 static int64_t gemv_sum_bytes(int64_t C, int split) { return kGemvWarps / split * ceil_div(C, 512) * 5 * 32 * (int64_t)sizeof(float); }
 static int gemv_split(int64_t R, int64_t C) {
@@ -429,12 +426,14 @@ static int gemv_split(int64_t R, int64_t C) {
   return gemv_sum_bytes(C, split) > kGemvSumBytesMax ? 1 : split;
 }
 
-// Whether gemv_quad_kernel is the faster one for a matrix in the tiled layout (staged -> this one, us).  From 8192 columns on the staged
-// kernel fits two CTAs on an SM at most: always (2048 x 8192 7.0 -> 6.0, 8976 x 8192 22.5 -> 18.0, 12288 x 12288 38.9 -> 32.2).
-// So too where the staged kernel would give four rows to a warp (18944 x 3584 20.5 -> 13.5).  Between, up to 15 warps per SM of
-// four rows each and with less than a quarter of the rounds missing (4608 x 5120 8.6 -> 7.7, 8192 x 4096 10.0 -> 9.6; but
-// 10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8) and of seven rounds or more (3584 x 3584 5.7 -> 5.1; 3072 x 3072 4.4 -> 5.0,
-// 2048 x 2048 2.9 -> 3.15).  Below 2048 columns it replaces gemv_kernel (1536 x 1536 3.55 -> 3.4, 8960 x 1536 10.2 -> 4.4).
+// Whether gemv_quad_kernel is the faster one for a matrix in the tiled layout.  Against gemv_staged_kernel (staged -> quad, us):
+// - from 8192 columns on, where that one fits two CTAs on an SM at most: always (2048 x 8192 7.0 -> 6.0, 8976 x 8192
+//   22.5 -> 18.0, 12288 x 12288 38.9 -> 32.2);
+// - where that one would give four rows to a warp: always (18944 x 3584 20.5 -> 13.5);
+// - between: seven rounds or more (3584 x 3584 5.7 -> 5.1; 3072 x 3072 4.4 -> 5.0, 2048 x 2048 2.9 -> 3.15), up to 15 warps per
+//   SM of four rows each, less than a quarter of the rounds missing (4608 x 5120 8.6 -> 7.7, 8192 x 4096 10.0 -> 9.6; but
+//   10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8).
+// Below 2048 columns it replaces gemv_kernel (1536 x 1536 3.55 -> 3.4, 8960 x 1536 10.2 -> 4.4).
 static bool gemv_quad_wins(int64_t R, int64_t C) {
   if (C < kGemvStagedMinCols) return R >= 512;
   if (R < 1024) return false;                                               // 512 x 3584: 3.5 -> 4.3

@@ -90,7 +90,6 @@ struct GemmParams {
   __nv_bfloat16* scaled = nullptr;
 };
 
-
 // Tile order: bands of `group` row tiles; inside a band the row tile runs fastest, then the column
 // tile.  The CTAs that run at the same time then share a few A row panels and walk the B column
 // panels together, so both stay in L2 whatever M, N and K are (row tile fastest over the whole of M

@@ -286,10 +286,9 @@ bf16_panel_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // go to block_sums [gridDim.x, 2, r], which lowrank_ds_kernel adds into ds and the column mean of d_yv.
 // A thread takes four columns of a row and has the partial sums of all splits in flight before it adds them; a CTA
 // takes 512 / r rows at a time and the grid as many CTAs as there are such groups (up to kDtsFinishCtas).  Bound by
-// the read of the partial sums.  The CTAs are small (128 threads of up to 64 registers) because they run beside a
-// weight-gradient product, whose CTA leaves 22 K registers of an SM: CTAs of 256 threads and 128 registers waited
-// for that product to end (58 us in a step of 8192 x 1536 x 8960), and a CTA per 64 rows with one column per thread
-// and one load in flight took 52 us by itself (1120 x 128, 7 splits).
+// the read of the partial sums (1120 x 128, 7 splits, with the product and the sums behind it: 13 us; 58 with a column
+// per thread and one load in flight).  128 threads of up to 64 registers, because the CTAs run beside a weight-gradient
+// product whose own CTA leaves 22 K registers of an SM: larger ones wait for that product to end.
 constexpr int kFinishThreads = 128;
 constexpr int kPanelMaxSplits = 16;
 // v += the partial sums at src of all splits, in split order, eight loads in flight

@@ -539,11 +539,11 @@ __device__ __noinline__ float finish_row(const float* from, const uint2* codes, 
 // a 128-row block for 4 scale columns, i.e. four 16-byte reads of maxima and one 16-byte store (row-major scales: four
 // words of four rows).  Two neighbouring lanes take two neighbouring l, the next ones the tiles to the right, so a warp
 // reads runs of up to 256 bytes and stores whole 32-byte sectors.  An item is such a pair of l (8 rows) over a segment of
-// the row (the whole of it where its sum is wanted); a CTA takes 64 / tx items at once.  With one 4-column group of two rows per thread, scalar arithmetic and 64-bit
-// index arithmetic this pass took 62 instructions per block and was bound by issue; what counts beside the arithmetic is
-// that edges, padding and divisions stay out of the unrolled path (with them inside it 27 instructions per block and
-// waits for instruction fetch).  Measured at 16384 x 4096, one output / both / both with token sums: 11.2 / 21.0 / 28.2
-// us then, 5.8 / 10.4 / 21.2 now; at 65536 x 4096 32 / 62 / 79 -> 16 / 30 / 67 (the bytes alone take 13 / 26 / 46); 64 x 18944, fewer rows than a block has: 4.0 -> 2.8.
+// the row (the whole of it where its sum is wanted); a CTA takes 64 / tx items at once.
+// Bound by issue: edges, padding and divisions stay out of the unrolled path (62 instructions per block with them and with
+// scalar arithmetic, 27 with packed arithmetic alone).  One output / both / both with token sums, us: 16384 x 4096
+// 11.2 / 21.0 / 28.2 before that, 5.8 / 10.4 / 21.2 now; 65536 x 4096 32 / 62 / 79 and 16 / 30 / 67 (the bytes alone take
+// 13 / 26 / 46); 64 x 18944, one output, 4.0 and 2.8.
 constexpr int kFinThreads = 128;
 // What the jobs of a launch want: no row sums; sums, four rows to a thread; sums, a row to a thread (finalize_form has the
 // rule).  Kernels of their own: what stands beside the unrolled path of the second one costs it 3 to 15 %.
