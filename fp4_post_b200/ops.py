@@ -36,10 +36,8 @@ def _need_cuda(t: torch.Tensor, what: str) -> None:
         raise RuntimeError(f"{what} must be a CUDA tensor: the NVFP4 path has no CPU fallback")
 
 
-def _current_device() -> int:
-    """torch.cuda.current_device() without its checks: a CUDA tensor exists.  (Looked up when called: a torch without CUDA
-    does not have it, and imports this module all the same.)"""
-    return torch._C._cuda_getDevice()
+# torch.cuda.current_device() without its checks: a CUDA tensor exists.  (A torch without CUDA has the checked one only.)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
