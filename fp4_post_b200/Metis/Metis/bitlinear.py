@@ -902,11 +902,15 @@ class MetisFusedFunction(torch.autograd.Function):
             if not overlap:
                 ready(vq)
                 ready(rq)
-            # The bias is cast beside the product too, but `mean_event` says nothing about it: a grouped activation's
-            # event is that of the call that quantized it, and the bias may have been written since.  An event of this
-            # call orders the cast behind whatever the current stream has queued.
-            cast_bias = overlap and bias is not None and bias.dtype != torch.float32
-            entered = recorded_event(current_stream(xa.mean.device)) if cast_bias else None
+            if overlap and bias is not None and bias.dtype != torch.float32:
+                # The bias is cast beside the product too, on a stream of its own: `mean_event` says nothing about it (a
+                # grouped activation's event is that of the call that quantized it, and the bias may have been written
+                # since), so an event of this call orders the cast behind whatever the current stream has queued.
+                here, side = current_stream(xa.mean.device), _aux_stream(xa.mean.device, 1)
+                side.wait_event(recorded_event(here))
+                with on_stream(side):
+                    bias_row = bias.float()
+                    bias_done = recorded_event(side)
             with _beside(xa.mean_event if overlap else None, xa.mean.device) as join:
                 if overlap and vq.ready_event is not None:      # quantized on a stream of their own: order this one after each
                     current_stream(xa.mean.device).wait_event(vq.ready_event)
@@ -917,13 +921,10 @@ class MetisFusedFunction(torch.autograd.Function):
                 if overlap and rq.ready_event is not None:
                     current_stream(xa.mean.device).wait_event(rq.ready_event)
                 row_r = ops.nvfp4_gemv(rq.q, xa.mean)
-                if cast_bias:
-                    current_stream(xa.mean.device).wait_event(entered)
-                    bias_row = bias.float()
             if v_ready is not None:
                 current_stream(xa.mean.device).wait_event(v_ready)
                 row_v.record_stream(current_stream(xa.mean.device))
-                join_residual = lambda: join(row_r, bias_row)
+                join_residual = lambda: join(row_r)
             rank1_v.append((None, row_v))
             rank1_r.append((None, row_r))
         if bias is not None:
@@ -946,6 +947,9 @@ class MetisFusedFunction(torch.autograd.Function):
             lowrank = _bf16_factors(ts.float() / (xa.q.unit * rq.q.unit), u_weight.detach(), act)
         if join_residual is not None:
             join_residual()
+        if bias_row is not None:
+            here.wait_event(bias_done)
+            bias_row.record_stream(here)
         ready(rq)
         y = _packed_matmul(xa.q, rq.q, rank1=rank1_r, lowrank=lowrank, out_dtype=act)
         if (MetisFusedFunction.concurrent_branches and xa.q.codes.is_cuda and any(ctx.needs_input_grad)
