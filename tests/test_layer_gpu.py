@@ -283,6 +283,38 @@ def test_second_stream_gives_the_gradients_of_the_single_stream_order_bit_for_bi
             MetisFusedFunction.concurrent_branches = True
 
 
+@pytest.mark.parametrize("tokens", [64, 512])
+def test_the_forward_waits_for_a_residual_weight_that_is_quantized_late(tokens):
+    """Both weights are quantized on a stream of their own; the scaling of the rank-r factor reads the residual weight's unit
+    before the residual product does.  Other weights every time: what an earlier call left in memory does not help."""
+    from Metis.Metis.bitlinear import MetisFusedFunction
+    torch.manual_seed(4)
+    layer = BitLinear(512, 384, args=metis_args(64), bias=True, dtype=torch.bfloat16, compute_dtype=torch.bfloat16)
+    layer.layer_name = "late"
+    layer.split()
+    layer = layer.to(DEV)
+    x = torch.randn(1, tokens, 512, device=DEV, dtype=torch.bfloat16)
+    busy = torch.randn(8192, 8192, device=DEV, dtype=torch.bfloat16)
+    quantize = layer.warmup_linear._get_quantized_weight
+
+    def late(weight):
+        for _ in range(4):
+            torch.mm(busy, busy)
+        return quantize(weight)
+    for rep in range(4):
+        with torch.no_grad():
+            layer.warmup_linear.weight.mul_(3.0)
+        layer.warmup_linear._get_quantized_weight = late
+        y = layer(x).detach().clone()
+        layer.warmup_linear._get_quantized_weight = quantize
+        MetisFusedFunction.concurrent_branches = False
+        try:
+            want = layer(x).detach()
+        finally:
+            MetisFusedFunction.concurrent_branches = True
+        assert torch.equal(y, want), rep
+
+
 def test_a_bias_written_between_two_calls_on_one_activation_is_read_after_the_write():
     """Cached weights and a grouped activation that is found again: nothing but the order on the current stream says when
     the bias may be read."""
