@@ -535,6 +535,36 @@ __device__ __noinline__ float finish_row(const float* from, const uint2* codes, 
   return sum;
 }
 
+// Scale pass of four blocks of each of four rows (row_pitch floats apart) of which only the first `rows` and `blocks` exist, or
+// which no vector load reaches: `dst` gets a 16-byte piece of the tiled layout, or single bytes of the rows.  All maxima are
+// in flight at once: one after the other they make a chain of sixteen loads at the end of a small tensor.
+__device__ __noinline__ void finish_edge(const float* from, int64_t row_pitch, int rows, int blocks, uint8_t* dst, bool tiled, float unit,
+                                         float inv_unit) {
+  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+  float a[4][4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[c][j] = c < rows && j < blocks ? from[c * row_pitch + j] : 0.0f;
+  }
+  uint32_t out[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    out[c] = 0u;
+    if (c >= rows || blocks <= 0) continue;
+#pragma unroll
+    for (int j = 1; j < 4; ++j) if (j >= blocks) a[c][j] = a[c][0];          // what is not there does not ask for divisions
+    const float4 v = make_float4(a[c][0], a[c][1], a[c][2], a[c][3]);
+    if (!scale_bytes4(v, inv_unit2, out[c])) out[c] = scale_bytes4_exact(v, unit);
+    if (blocks < 4) out[c] &= (1u << (8 * blocks)) - 1u;
+    if (!tiled) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if (j < blocks) dst[c * row_pitch + j] = (uint8_t)(out[c] >> (8 * j));
+    }
+  }
+  if (tiled) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+}
+
 // A thread finishes one 16-byte piece of the tiled layout at a time: the scales of the rows l, l + 32, l + 64, l + 96 of
 // a 128-row block for 4 scale columns, i.e. four 16-byte reads of maxima and one 16-byte store (row-major scales: four
 // words of four rows).  Two neighbouring lanes take two neighbouring l, the next ones the tiles to the right, so a warp
@@ -545,13 +575,40 @@ __device__ __noinline__ float finish_row(const float* from, const uint2* codes, 
 // 11.2 / 21.0 / 28.2 before that, 5.8 / 10.4 / 21.2 now; 65536 x 4096 32 / 62 / 79 and 16 / 30 / 67 (the bytes alone take
 // 13 / 26 / 46); 64 x 18944, one output, 4.0 and 2.8.
 constexpr int kFinThreads = 128;
-// What the jobs of a launch want: no row sums; sums, four rows to a thread; sums, a row to a thread (finalize_form has the
-// rule).  Kernels of their own: what stands beside the unrolled path of the second one costs it 3 to 15 %.
-enum FinalizeForm { kFinPlain, kFinSums, kFinSumsByRow };
+// What the jobs of a launch want: no row sums, every row made of whole groups of four blocks; no row sums; sums, four rows to
+// a thread; sums, up to a CTA to a row (finalize_form has the rule).  Kernels of their own: what stands beside the unrolled
+// path costs it 1 % (a call for the edges) to 15 %.
+enum FinalizeForm { kFinPlain, kFinEdges, kFinSums, kFinSumsByRow };
+// The rows of a job with sums, 2^log_tx threads (up to the whole CTA) to each.
+__device__ __forceinline__ void finish_rows(const FinalizeJob& J, bool tiled, int tiles, int groups, float unit, float inv_unit,
+                                            float (&s_sum)[kFinThreads / 32][2][4]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = 1 << J.log_tx, per_cta = kFinThreads >> J.log_tx;
+  const int k_lane = tid & (tx - 1), sub = tid >> J.log_tx;
+  const int64_t out_rows = tiled ? (J.R + 127) / 128 * 128 : J.R;                   // whole tiles: zeros behind the last row
+  for (int64_t first = (int64_t)blockIdx.x * per_cta; first < out_rows; first += (int64_t)gridDim.x * per_cta) {
+    const int64_t r = first + sub;
+    float sum = 0.0f;
+    if (r < out_rows) {
+      uint8_t* to = tiled ? J.scales + (r >> 7) * tiles * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4 : J.scales + r * J.sf_cols;
+      sum = finish_row(J.amax + r * J.sf_cols, J.codes + r * J.sf_cols, to, tiled ? 512 : 4, k_lane, r < J.R ? (int)(J.sf_cols >> 2) : 0,
+                       tiled ? groups : 0, tx, unit, inv_unit);
+    }
+    // fixed order: lanes of a row by butterfly, then its warps one after the other
+    for (int o = (tx < 32 ? tx : 32) >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (tx > 32) {
+      __syncthreads();                                         // the previous round's sums have been read
+      if (lane == 0) s_sum[warp][0][0] = sum;
+      __syncthreads();
+      if (k_lane == 0) for (int w = 1; w < tx >> 5; ++w) sum += s_sum[warp + w][0][0];
+    }
+    if (k_lane == 0 && r < J.R) J.row_sums[r] = sum * (0.5f * unit);
+  }
+}
+
 template <FinalizeForm kForm>
-__global__ void __launch_bounds__(kFinThreads)
-finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t* __restrict__ offset_ctr) {
-  constexpr bool kSums = kForm != kFinPlain, kQuadSums = kForm == kFinSums;
+__device__ __forceinline__ void finalize_scales(const FinalizeJob& job0, const FinalizeJob& job1, uint64_t* __restrict__ offset_ctr) {
+  constexpr bool kSums = kForm == kFinSums || kForm == kFinSumsByRow, kQuadSums = kForm == kFinSums;
   __shared__ unsigned int s_top[kFinThreads / 32], s_bad[kFinThreads / 32];
   __shared__ float s_sum[kFinThreads / 32][2][4];
   grid_dependency_wait();
@@ -590,18 +647,23 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
   const int groups = tiled ? tiles : (int)((sf_cols + 3) >> 2);
   const bool vec = (sf_cols & 3) == 0;
   const bool sums = kSums && J.row_sums != nullptr;              // the host asks for them only when vec holds
+  if constexpr (kForm == kFinSumsByRow) {
+    if (sums) {
+      finish_rows(J, tiled, tiles, groups, unit, inv_unit, s_sum);
+      return;
+    }
+  }
   const int tx = 1 << J.log_tx, per_cta = 64 >> J.log_tx;        // threads along a row, items per CTA
   const int k_lane = (tid >> 1) & (tx - 1), sub = tid >> (1 + J.log_tx);
   const int64_t items = ((R + 127) / 128) * 16;
   // without row sums a row is cut into segments of tx tiles, so that a few wide rows still fill the SMs
   const int segments = sums ? 1 : (groups + tx - 1) >> J.log_tx;
-  const bool by_row = kForm == kFinSumsByRow && sums;            // row0 + 32 (index & 3) of a thread's four rows: four times the items
-  const int64_t work = items * segments << (by_row ? 2 : 0);
+  const int64_t work = items * segments;
   const int64_t row_pitch = 32 * sf_cols;                        // between a thread's four rows
   // the item loop is uniform over the CTA (the sums of a row meet at a barrier)
   for (int64_t first = (int64_t)blockIdx.x * per_cta; first < work; first += (int64_t)gridDim.x * per_cta) {
     const bool live = first + sub < work;
-    const int64_t item = by_row ? (first + sub) >> 2 : segments == 1 ? first + sub : (first + sub) / segments;
+    const int64_t item = segments == 1 ? first + sub : (first + sub) / segments;
     const int k_first = segments == 1 ? 0 : (int)((first + sub) - item * segments) << J.log_tx;
     const int k_end = segments == 1 ? groups : min(groups, k_first + tx);
     const int64_t row0 = (item >> 4) * 128 + (item & 15) * 2 + (tid & 1);       // this thread's rows: row0 + 32 c
@@ -665,18 +727,18 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
         for (int c = 0; c < 4; ++c) if (kWhole || c < rows) *reinterpret_cast<uint32_t*>(dst + c * row_pitch + 4 * k) = out[c];
       }
     };
-    const int only = (int)(first + sub) & 3;                      // by_row: which of the four
-    if (by_row && live) {
-      acc[0] = finish_row(src + only * row_pitch, codes + only * row_pitch, dst + (tiled ? 4 * only : only * row_pitch), tiled ? 512 : 4,
-                          k_lane, only < rows ? (int)(sf_cols >> 2) : 0, tiled ? groups : 0, tx, unit, inv_unit);
-    }
-    for (int k = k_first + k_lane; live && !by_row && k < k_end; k += tx) {
+    for (int k = k_first + k_lane; live && k < k_end; k += tx) {
       const bool full = (vec || tiled) && 4 * k + 4 <= sf_cols;
       if (full && rows == 4) {
         piece(std::true_type{}, k);
       } else if (!kQuadSums && full) {                              // decode: fewer than 128 rows
         piece(std::false_type{}, k);
-      } else {                                                      // an edge of the tensor, or padding: kept short
+      } else if constexpr (kForm == kFinPlain) {                    // what is left then is padding
+        if (tiled) *reinterpret_cast<uint4*>(dst + (int64_t)k * 512) = make_uint4(0u, 0u, 0u, 0u);
+      } else if constexpr (!kQuadSums) {                            // an edge of the tensor, or padding
+        const int blocks = (int)(sf_cols - 4 * k < 4 ? sf_cols - 4 * k : 4);
+        finish_edge(src + 4 * k, row_pitch, rows, blocks, dst + (tiled ? (int64_t)k * 512 : (int64_t)4 * k), tiled, unit, inv_unit);
+      } else {                                                      // the same with sums: kept short
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           const int64_t r = row0 + 32 * c;
@@ -722,13 +784,21 @@ finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t*
       if (live && k_lane == 0) {
         const float half_unit = 0.5f * unit;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int64_t r = row0 + 32 * (by_row ? only : c);
-          if (r < R && (!by_row || c == 0)) J.row_sums[r] = acc[c] * half_unit;
-        }
+        for (int c = 0; c < 4; ++c) if (row0 + 32 * c < R) J.row_sums[row0 + 32 * c] = acc[c] * half_unit;
       }
     }
   }
+}
+// Resident at once: 8 CTAs per SM, 5 and 7 with sums.  The kernel with sums by four rows is left to the compiler (96 registers): asked for its five
+// CTAs it is scheduled worse (16384 x 4096, dual quantizer with sums: 92.4 us against 89.9).
+template <FinalizeForm kForm>
+__global__ void __launch_bounds__(kFinThreads, kForm == kFinSumsByRow ? 7 : 8)
+finalize_scales_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t* __restrict__ offset_ctr) {
+  finalize_scales<kForm>(job0, job1, offset_ctr);
+}
+__global__ void __launch_bounds__(kFinThreads)
+finalize_scales_sums_kernel(const FinalizeJob job0, const FinalizeJob job1, uint64_t* __restrict__ offset_ctr) {
+  finalize_scales<kFinSums>(job0, job1, offset_ctr);
 }
 
 // ---- small tensors (decode-sized activations): one launch --------------------------------------------------
@@ -1021,16 +1091,18 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
 
 // Which kernel forms the row sums.  Four rows to a thread move the fewest bytes per instruction, but leave few CTAs where the
 // tensor has few rows (16 per 128-row block), and where its last row block is not full the missing rows send that block
-// down the edge path, a chain of loads per block.  Measured, dual quantizer with sums, four rows / one row to a thread (us):
-// 16384 tokens x 128 columns 12.0 / 10.2, x 1024 28.2 / 27.4, 65536 x 1024 106.7 / 94.7, but 16384 x 1536 38.4 / 39.9,
-// 16384 x 4096 90.4 / 95.7; last row block not full: 16384 x 1104 42.0 / 31.5, x 2032 66.8 / 50.4, x 4208 114 / 106,
-// 4096 x 8304 51.5 / 54.8.
+// down the edge path, a chain of loads per block.  Measured, dual quantizer with sums, four rows to a thread / a CTA to a row (us):
+// 16384 tokens x 128 columns 12.0 / 8.7, 65536 x 256 42.0 / 27.9, 65536 x 1024 106 / 90, 8192 x 1024 16.9 / 16.9, but
+// 8192 x 1536 21.3 / 22.0, 16384 x 4096 89.9 / 94.7; last row block not full: 65536 x 1136 189 / 109, 16384 x 2032 66.6 / 51.2,
+// x 4208 114 / 101, 4096 x 8304 52.2 / 53.8 (16384 tokens 197 / 189), 8192 x 14352 154 / 170.
 static FinalizeForm finalize_form(const FinalizeJobs& jobs, int njobs) {
+  FinalizeForm form = kFinPlain;
   for (int j = 0; j < njobs; ++j) {
     const FinalizeJob& J = jobs.job[j];
-    if (J.row_sums) return J.R <= 1280 || (J.R % 128 != 0 && J.R <= 6144) ? kFinSumsByRow : kFinSums;          // one job at most wants them
+    if (J.row_sums) return J.R <= 1280 || (J.R % 128 != 0 && J.R <= 8448) ? kFinSumsByRow : kFinSums;          // one job at most wants them
+    if (J.sf_cols % 4 != 0) form = kFinEdges;
   }
-  return kFinPlain;
+  return form;
 }
 
 static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t st, uint64_t* offset_ctr) {
@@ -1039,15 +1111,18 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
   for (int j = 0; j < njobs; ++j) {
     FinalizeJob& J = jobs.job[j];
     const int64_t groups = J.sf_layout == METIS_SF_MMA ? sf_tiles_per_row(J.sf_cols * 16) : ceil_div(J.sf_cols, 4);
+    const bool by_row = form == kFinSumsByRow && J.row_sums;
     J.log_tx = 2;                                             // a warp holds at most 8 rows' lanes of 4 tiles
-    while (J.log_tx < 6 && (1 << J.log_tx) < groups) ++J.log_tx;
+    while (J.log_tx < (by_row ? 7 : 6) && (1 << J.log_tx) < groups) ++J.log_tx;
     const int64_t segments = J.row_sums ? 1 : ceil_div(groups, (int64_t)1 << J.log_tx);
-    const int64_t need = ceil_div(ceil_div(J.R, 128) * 16 * segments << (form == kFinSumsByRow && J.row_sums ? 2 : 0), 64 >> J.log_tx);
+    const int64_t need = by_row ? ceil_div(ceil_div(J.R, 128) * 128, kFinThreads >> J.log_tx)
+                                : ceil_div(ceil_div(J.R, 128) * 16 * segments, 64 >> J.log_tx);
     if (need > blocks) blocks = need;
   }
   if (njobs == 1) jobs.job[1] = jobs.job[0];
-  const bool sums = form != kFinPlain;
-  auto kern = form == kFinPlain ? finalize_scales_kernel<kFinPlain> : form == kFinSums ? finalize_scales_kernel<kFinSums> : finalize_scales_kernel<kFinSumsByRow>;
+  const bool sums = form == kFinSums || form == kFinSumsByRow;
+  auto kern = form == kFinPlain ? finalize_scales_kernel<kFinPlain> : form == kFinEdges ? finalize_scales_kernel<kFinEdges>
+            : form == kFinSums ? finalize_scales_sums_kernel : finalize_scales_kernel<kFinSumsByRow>;
   const int64_t cap = (int64_t)sm_count() * (sums ? 10 : 8) / njobs;     // resident at once: 5 (sums) and 8 per SM
   if (blocks > cap) blocks = ceil_div(blocks, ceil_div(blocks, cap));    // the fewest CTAs that need no more rounds than `cap` would
   METIS_CUDA_OK(launch_overlapped(kLaunchShort, kern, dim3((unsigned)blocks, (unsigned)njobs), dim3(kFinThreads), 0, st,

@@ -468,7 +468,8 @@ def test_deferred_scale_pass_writes_what_the_undeferred_call_writes(defer, stoch
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
-@pytest.mark.parametrize("rows,cols", [(16, 16), (1120, 208), (144, 2064), (320, 4112), (2112, 1040)])
+@pytest.mark.parametrize("rows,cols", [(16, 16), (1120, 208), (144, 2064), (320, 4112), (2112, 1040),
+                                       (64, 48), (192, 112), (4160, 80), (64, 1536), (64, 6864), (64, 8464)])
 def test_scale_pass_at_the_edges_of_its_walk(rows, cols, layout):
     """Rows that end inside a 128-row block, scale columns that no group of four and no stage of the GEMM divides
     (1120 / 16 = 70, 2064 / 16 = 129), several trips along a row (4112 / 64 > 64 tiles), both layouts; the token sums
