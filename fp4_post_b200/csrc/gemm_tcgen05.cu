@@ -351,7 +351,9 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 // ---- split-K: sum of the partial products + the epilogue terms -----------------------------------------
 
 constexpr int kMaxSplits = 8;
-template <typename TD>
+// kInFlight: at least as many as there are splits (its registers decide how many CTAs are resident).  kScaled: may write the
+// scaled copy of D; without it the divisions stand in nobody's way.
+template <typename TD, int kInFlight, bool kScaled>
 __global__ void __launch_bounds__(256)
 splitk_finish_kernel(const GemmParams p) {
   grid_dependency_wait();
@@ -359,24 +361,25 @@ splitk_finish_kernel(const GemmParams p) {
   const int64_t groups_per_row = (p.N + 3) / 4;
   const bool small = p.M * groups_per_row < ((int64_t)1 << 31);
   const float g = p.alpha * __ldg(p.a_unit) * __ldg(p.b_unit);
-  const float units = p.scaled ? __fmul_rn(__ldg(p.s_unit_a), __ldg(p.s_unit_b)) : 1.0f;
+  const bool scaled = kScaled && p.scaled;
+  const float units = scaled ? __fmul_rn(__ldg(p.s_unit_a), __ldg(p.s_unit_b)) : 1.0f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.M * groups_per_row; i += (int64_t)gridDim.x * blockDim.x) {
     // 32-bit index arithmetic where it fits (a 64-bit division is a subroutine of ~100 instructions)
     const int64_t row = small ? (int64_t)((uint32_t)i / (uint32_t)groups_per_row) : i / groups_per_row, col = (i - row * groups_per_row) * 4;
     const float* src = p.partial + row * p.ldp + col;
-    float4 v[kMaxSplits];
+    float4 v[kInFlight];
 #pragma unroll
-    for (int s = 0; s < kMaxSplits; ++s)            // every load in flight before the first addition
+    for (int s = 0; s < kInFlight; ++s)            // every load in flight before the first addition
       if (s < p.splits) v[s] = *reinterpret_cast<const float4*>(src + (int64_t)s * p.M * p.ldp);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int s = 0; s < kMaxSplits; ++s)            // fixed order: the result does not depend on timing
+    for (int s = 0; s < kInFlight; ++s)            // fixed order: the result does not depend on timing
       if (s < p.splits) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
     float o[4] = {acc.x * g, acc.y * g, acc.z * g, acc.w * g};
     const float c0 = p.rvec0 ? (p.cvec0 ? __ldg(p.cvec0 + row) : 1.0f) : 0.0f;
     const float c1 = p.rvec1 ? (p.cvec1 ? __ldg(p.cvec1 + row) : 1.0f) : 0.0f;
     __nv_bfloat16 sv[4];
-    if (p.scaled) {                                 // N is a multiple of 8 then
+    if (scaled) {                                   // N is a multiple of 8 then
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         sv[j] = p.s_is_f32 ? __float2bfloat16_rn(__ldg(static_cast<const float*>(p.s) + col + j))
@@ -395,7 +398,7 @@ splitk_finish_kernel(const GemmParams p) {
         const __nv_bfloat16 y = __float2bfloat16_rn(o[j]);
         static_cast<__nv_bfloat16*>(p.d)[row * p.ldd + col + j] = y;
         // torch.mul(s, y) in bf16 (the product is exact in fp32: one rounding), in the side product's accumulator units
-        if (p.scaled) p.scaled[row * p.N + col + j] = __float2bfloat16_rn(__fdiv_rn(__bfloat162float(__hmul(y, sv[j])), units));
+        if (scaled) p.scaled[row * p.N + col + j] = __float2bfloat16_rn(__fdiv_rn(__bfloat162float(__hmul(y, sv[j])), units));
       } else {
         static_cast<float*>(p.d)[row * p.ldd + col + j] = o[j];
       }
@@ -441,7 +444,10 @@ static int32_t launch_gemm(const metis_gemm_args* a, const CUtensorMap& ma, cons
     const int64_t threads = a->M * ceil_div(a->N, 4);
     int64_t blocks = ceil_div(threads, 256);
     if (blocks > (int64_t)device_sm_count() * 8) blocks = (int64_t)device_sm_count() * 8;
-    METIS_CUDA_OK(launch_overlapped(kLaunchGemm, splitk_finish_kernel<TD>, dim3((unsigned)blocks), dim3(256), 0, st, p));
+    auto finish = p.splits > 4 ? splitk_finish_kernel<TD, kMaxSplits, true>
+                : p.splits > 2 ? (p.scaled ? splitk_finish_kernel<TD, 4, true> : splitk_finish_kernel<TD, 4, false>)
+                               : (p.scaled ? splitk_finish_kernel<TD, 2, true> : splitk_finish_kernel<TD, 2, false>);
+    METIS_CUDA_OK(launch_overlapped(kLaunchGemm, finish, dim3((unsigned)blocks), dim3(256), 0, st, p));
   }
   return METIS_OK;
 }
