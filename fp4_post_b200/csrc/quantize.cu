@@ -812,14 +812,18 @@ finalize_scales_sums_kernel(const FinalizeJob job0, const FinalizeJob job1, uint
 // 8.0, 32 x 4096 5.2, 64 x 4096 6.8 against 8.1.
 constexpr int kSmallThreads = 512;
 constexpr int kSmallBlocks = 4;                    // blocks per thread
-// Blocks per thread up to which the cluster is taken although the streaming path needs no zero-fill either.  8 CTAs of 512
-// threads: a round is 4096 blocks and costs 0.75 us for bf16, 1.1 for fp32, where the two launches stay at 3.9 to 5.5.  So one
-// round, one more for bf16, one more where no padding has to be cleared, one more where the scale pass would go down its edge
-// path.  Cluster / two launches, us: bf16 tiled 17 x 4096 3.9 / 4.3, 64 x 2048 4.3 / 5.0, 40 x 4096 5.0 / 4.8, row-major
-// 64 x 1040 3.3 / 5.3, 48 x 4096 4.3 / 4.6, 56 x 4096 4.9 / 4.2, 63 x 4112 5.0 / 5.5; fp32 tiled 32 x 4096 5.1 / 4.3, 2100 x 32
-// 4.3 / 5.5, row-major 64 x 2048 4.4 / 4.5, 48 x 4096 5.3 / 4.2, 120 x 1552 5.3 / 6.6.
-static int cluster_rounds(int64_t C, int32_t sf_layout, int64_t element_bytes) {
-  return 1 + (element_bytes == 2) + (sf_layout == METIS_SF_ROWMAJOR) + (C % 64 != 0);
+// Blocks up to which the cluster is taken although the streaming path needs no zero-fill either.  8 CTAs of 512 threads: a
+// round is 4096 blocks and costs 0.75 us for bf16, 1.1 for fp32, where the two launches stay at 3.7 to 5.5 (a few blocks more
+// than whole rounds cost nothing).  Row-major scales, without padding to clear: three rounds for bf16, two for fp32.  Tiled ones:
+// one, and a second for bf16 rows of up to 1024 elements.  Cluster / two launches back to back, us: bf16 row-major 64 x 1040
+// 3.2 / 4.4, 48 x 4096 4.2 / 4.5, 56 x 4096 4.7 / 4.1, tiled 16 x 4112 3.7 / 4.6, 200 x 528 4.2 / 6.5, 64 x 1536 4.2 / 3.7, 40 x 4096
+// 4.9 / 4.5; fp32 row-major 32 x 4112 4.4 / 4.7, 100 x 1536 5.1 / 4.0, tiled 16 x 4112 4.0 / 4.6, 24 x 4096 4.9 / 4.2.  In a chain of
+// decode layers, where eight free SMs next to each other have to be found beside the vector products, 20 x 4096 takes
+// 21.3 / 20.9 per layer and 24 x 4096 22.2 / 21.7; a single layer of 16 x 8192 35 / 29.
+static int64_t cluster_blocks(int64_t C, int32_t sf_layout, int64_t element_bytes) {
+  const bool bf16 = element_bytes == 2, narrow = C <= 1024;
+  const int rounds = sf_layout == METIS_SF_ROWMAJOR ? (bf16 ? 3 : 2) : (bf16 && narrow ? 2 : 1);
+  return (int64_t)rounds * kSmallCtas * kSmallThreads + 64;
 }
 constexpr int64_t kSmallMaxBlocks = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks;
 
@@ -1211,7 +1215,7 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
   // One cluster for the whole tensor; with records, only where two launches over many SMs are not faster.
   int64_t tiles = 0, padded_words = 0;
   if (!transpose && !sr && aligned16(scales) && small_path(R, C, sf_layout, &tiles, &padded_words) &&
-      (!records || R * (C / 16) <= (int64_t)kSmallCtas * kSmallThreads * cluster_rounds(C, sf_layout, esz))) {
+      (!records || R * (C / 16) <= cluster_blocks(C, sf_layout, esz))) {
     return x_dtype == METIS_DTYPE_BF16
         ? launch_small(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st)
         : launch_small(static_cast<const float*>(x), rows, cols, ld, col_mean, codes, sf_layout, tiles, padded_words, scales, unit, st);

@@ -149,7 +149,7 @@ int64_t metis_nvfp4_quantize_workspace_bytes(int64_t R, int64_t C);
  * Launches: large tensors take one streaming pass and a scale pass, with a zero-fill of the workspace
  * header in front unless the workspace has METIS_QUANTIZE_EXTRA_WORKSPACE more bytes and the pass at most
  * 640 CTAs.  Round-to-nearest, untransposed tensors of at most 16384 blocks (rollout-sized activations; where
- * that zero-fill is not needed 4096 to 16384, by type, layout and width) take ONE kernel that runs as a single
+ * that zero-fill is not needed 4160 to 12352, by type, layout and width) take ONE kernel that runs as a single
  * thread-block cluster and does not touch the workspace (it must still be passed and large enough); results are
  * bit-identical.
  */
