@@ -413,15 +413,20 @@ static cudaError_t launch_gemv_staged(const uint2* codes, const uint8_t* scales,
 
 // How many warps share four rows: as many as bring an SM to 24 warps (12 to 15 run at 0.88 of the rate: 4096 x 4096 5.5 us
 // with 28, 6.2 with 14), unless the rounds that the last warps lack cost as much (8960 x 1536 has three rounds: 4.4 us with
-// a warp per four rows, 5.6 with two); below 8 warps always.  The block sums of eight CTAs have to leave room for v in L1.
+// a warp per four rows, 5.6 with two) or there are two rounds only, of which each warp would then have one (8960 x 768
+// 3.2 us with a warp per four rows, 4.2 with two; 13038 x 560 3.9 / 5.8); below 8 warps always.  The block sums of eight CTAs
+// have to leave room for v in L1.
 constexpr int64_t kGemvWarpsPerSm = 24, kGemvFewWarpsPerSm = 8, kGemvL1Bytes = 208 << 10, kGemvSumBytesMax = 96 << 10;
 static int64_t gemv_sum_bytes(int64_t C, int split) { return kGemvWarps / split * ceil_div(C, 512) * 5 * 32 * (int64_t)sizeof(float); }
 static int gemv_split(int64_t R, int64_t C) {
   const int64_t sms = device_sm_count(), quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512);
   auto padded = [&](int k) { return ceil_div(trips, k) * k; };              // rounds, the missing ones of the last included
   int split = 1;
-  while (split < kGemvWarps && trips >= 2 * split && quads * split < sms * kGemvWarpsPerSm &&
-         (quads * split < sms * kGemvFewWarpsPerSm || padded(2 * split) * 10 <= padded(split) * 11)) split *= 2;
+  auto sharing_pays = [&] {
+    if (quads * split < sms * kGemvFewWarpsPerSm) return true;
+    return trips > 2 && quads * split < sms * kGemvWarpsPerSm && padded(2 * split) * 10 <= padded(split) * 11;
+  };
+  while (split < kGemvWarps && trips >= 2 * split && sharing_pays()) split *= 2;
   while (split > 1 && split < kGemvWarps && kGemvCtasPerSm * gemv_sum_bytes(C, split) + C * (int64_t)sizeof(float) > kGemvL1Bytes) split *= 2;
   return gemv_sum_bytes(C, split) > kGemvSumBytesMax ? 1 : split;
 }
@@ -433,9 +438,10 @@ static int gemv_split(int64_t R, int64_t C) {
 // - between: seven rounds or more (3584 x 3584 5.7 -> 5.1; 3072 x 3072 4.4 -> 5.0, 2048 x 2048 2.9 -> 3.15), up to 15 warps per
 //   SM of four rows each, less than a quarter of the rounds missing (4608 x 5120 8.6 -> 7.7, 8192 x 4096 10.0 -> 9.6; but
 //   10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8).
-// Below 2048 columns it replaces gemv_kernel (1536 x 1536 3.55 -> 3.4, 8960 x 1536 10.2 -> 4.4).
+// Below 2048 columns it replaces gemv_kernel (8960 x 1536 10.2 -> 4.3, 4096 x 768 4.0 -> 3.2, 1024 x 1792 4.3 -> 2.7), except for
+// few rows of two or three rounds (1024 x 768 2.1 -> 2.6, 2048 x 1024 2.7 -> 2.9, 3072 x 1024 3.4 -> 3.1).
 static bool gemv_quad_wins(int64_t R, int64_t C) {
-  if (C < kGemvStagedMinCols) return R >= 512;
+  if (C < kGemvStagedMinCols) return R >= (C > 512 && C <= 1536 ? 2560 : 512);
   if (R < 1024) return false;                                               // 512 x 3584: 3.5 -> 4.3
   const int64_t sms = device_sm_count(), split = gemv_split(R, C);
   if (C >= 8192 || ceil_div(R, 32) >= 3 * sms) return true;
