@@ -687,11 +687,27 @@ rmsnorm_colsum_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, in
   }
 }
 
-// A CTA takes 32 columns: its eight warps fetch the row slots' sums into shared memory (coalesced, eight loads of a
-// warp in flight), the first warp adds them up slot by slot: a fixed order.  One thread per column that walks all slots in global memory
-// is a chain of loads: 13.4 us for 256 slots, 15.5 for 296 (hidden 4096),
-// 5.5 and 7.4 here (64 slots 4.5 -> 2.7); summing every eighth slot in a warp of its own takes 4.6 and 5.9 but changes the last bit of the means.
+// A CTA takes 32 columns: its eight warps fetch the row slots' sums into shared memory (coalesced, eight loads of a warp in
+// flight), the first warp adds them up slot by slot: a fixed order.  Up to 32 slots it reads them itself, all at once.  A thread
+// per column that walks all slots in global memory is a chain of loads: 13.4 us for 256 slots, 15.5 for 296 (hidden 4096), 5.5
+// and 7.4 here (64 slots 4.5 -> 2.7); summing every eighth slot in a warp of its own takes 4.6 and 5.9 but changes the last bit
+// of the means.
 constexpr int kFinishSlots = 256;                          // slots per round: 32 KiB
+constexpr int kFinishDirectSlots = 32, kFinishFewSlots = 16;
+// A handful of slots (decode): a thread per column.  Norm and mean, this / the kernel below, us: 1 x 4096 3.6 / 3.7, 8 x 3584
+// 3.6 / 4.1, 16 x 1536 3.8 / 3.9, but 20 x 4096 4.7 / 4.3.
+__global__ void __launch_bounds__(256)
+rmsnorm_mean_finish_few_kernel(const float* __restrict__ partial, int slots, int64_t rows, int64_t cols, float* __restrict__ mean) {
+  grid_dependency_wait();
+  const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (c >= cols) return;
+  float v[kFinishFewSlots], sum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kFinishFewSlots; ++i) v[i] = i < slots ? partial[i * cols + c] : 0.0f;
+#pragma unroll
+  for (int i = 0; i < kFinishFewSlots; ++i) if (i < slots) sum += v[i];
+  mean[c] = __fdiv_rn(sum, (float)rows);
+}
 __global__ void __launch_bounds__(256)
 rmsnorm_mean_finish_kernel(const float* __restrict__ partial, int64_t slots, int64_t rows, int64_t cols, float* __restrict__ mean) {
   __shared__ float s_part[kFinishSlots][32];
@@ -699,12 +715,28 @@ rmsnorm_mean_finish_kernel(const float* __restrict__ partial, int64_t slots, int
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + lane;
   float sum = 0.0f;
+  if (slots <= kFinishDirectSlots) {
+    if (warp != 0 || c >= cols) return;
+    float v[kFinishDirectSlots];
+#pragma unroll
+    for (int i = 0; i < kFinishDirectSlots; ++i) v[i] = i < slots ? partial[i * cols + c] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < kFinishDirectSlots; ++i) if (i < slots) sum += v[i];
+    mean[c] = __fdiv_rn(sum, (float)rows);
+    return;
+  }
   for (int64_t base = 0; base < slots; base += kFinishSlots) {
     const int n = (int)(slots - base < kFinishSlots ? slots - base : kFinishSlots);
     if (base > 0) __syncthreads();                         // the previous round's sums have been read
     if (c < cols) {
+      int i = warp;
 #pragma unroll 8
-      for (int i = warp; i < n; i += 8) s_part[i][lane] = partial[(base + i) * cols + c];
+      for (const int whole = warp + ((n - warp + 7) / 64) * 64; i < whole; i += 8) s_part[i][lane] = partial[(base + i) * cols + c];
+      float v[8];                                          // the last ones not one by one
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = i + 8 * j < n ? partial[(base + i + 8 * j) * cols + c] : 0.0f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) if (i + 8 * j < n) s_part[i + 8 * j][lane] = v[j];
     }
     __syncthreads();
     if (warp == 0 && c < cols) {
@@ -829,7 +861,11 @@ extern "C" int32_t metis_rmsnorm_mean(const void* x, int32_t x_dtype, int64_t ro
   if (rc) return rc;
   const NormShape sh = norm_shape((int)(cols >> 4));
   const int64_t slots = colsum_ctas(rows, sh.by) * sh.by;
-  METIS_CUDA_OK(launch_overlapped(kLaunchShort, rmsnorm_mean_finish_kernel, dim3((unsigned)ceil_div(cols, 32)), dim3(256), 0, st,
-                                  (const float*)partial, slots, rows, cols, mean));
+  if (slots <= kFinishFewSlots)
+    METIS_CUDA_OK(launch_overlapped(kLaunchShort, rmsnorm_mean_finish_few_kernel, dim3((unsigned)ceil_div(cols, 256)), dim3(256), 0, st,
+                                    (const float*)partial, (int)slots, rows, cols, mean));
+  else
+    METIS_CUDA_OK(launch_overlapped(kLaunchShort, rmsnorm_mean_finish_kernel, dim3((unsigned)ceil_div(cols, 32)), dim3(256), 0, st,
+                                    (const float*)partial, slots, rows, cols, mean));
   return METIS_OK;
 }
