@@ -694,8 +694,8 @@ rmsnorm_colsum_kernel(const TX* __restrict__ x, int rows, int blocks_per_row, in
 // of the means.
 constexpr int kFinishSlots = 256;                          // slots per round: 32 KiB
 constexpr int kFinishDirectSlots = 32, kFinishFewSlots = 16;
-// A handful of slots (decode): a thread per column.  Norm and mean, this / the kernel below, us: 1 x 4096 3.6 / 3.7, 8 x 3584
-// 3.6 / 4.1, 16 x 1536 3.8 / 3.9, but 20 x 4096 4.7 / 4.3.
+// A handful of slots (decode): a thread per column, all loads in flight.  Norm and mean, this / the kernel below, us: 1 x 4096
+// 3.6 / 3.9, 8 x 3584 3.7 / 4.1, 16 x 1536 3.5 / 3.9, but 20 x 4096 4.7 / 4.3.
 __global__ void __launch_bounds__(256)
 rmsnorm_mean_finish_few_kernel(const float* __restrict__ partial, int slots, int64_t rows, int64_t cols, float* __restrict__ mean) {
   grid_dependency_wait();
