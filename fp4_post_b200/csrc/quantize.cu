@@ -1095,15 +1095,22 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
 
 // Which kernel forms the row sums.  Four rows to a thread move the fewest bytes per instruction, but leave few CTAs where the
 // tensor has few rows (16 per 128-row block), and where its last row block is not full the missing rows send that block
-// down the edge path, a chain of loads per block.  Measured, dual quantizer with sums, four rows to a thread / a CTA to a row (us):
-// 16384 tokens x 128 columns 12.0 / 8.7, 65536 x 256 42.0 / 27.9, 65536 x 1024 106 / 90, 8192 x 1024 16.9 / 16.9, but
-// 8192 x 1536 21.3 / 22.0, 16384 x 4096 89.9 / 94.7; last row block not full: 65536 x 1136 189 / 109, 16384 x 2032 66.6 / 51.2,
-// x 4208 114 / 101, 4096 x 8304 52.2 / 53.8 (16384 tokens 197 / 189), 8192 x 14352 154 / 170.
+// down the edge path, a chain of loads per block; with 32 rows or fewer in it the tiled layout loses less there than the rows one
+// by one lose to scattered words, and with many rows that chain is a small part.  Measured, dual quantizer with sums,
+// four rows to a thread / threads of its own for each row (us): 16384 tokens x 128 columns 12.0 / 8.7, 65536 x 256 42.0 / 27.9,
+// 65536 x 1024 106 / 90, 8192 x 1024 16.9 / 16.9, but 8192 x 1536 21.3 / 22.0, 16384 x 4096 89.9 / 94.7; last row block not
+// full, tiled: 16384 x 2032 69.9 / 53.6, x 4144 113 / 105, 8192 x 7056 86.0 / 91.6, 10032 64.3 / 69.2; row-major: 9856 x 3744
+// 62.7 / 56.8, 2176 x 8304 36.1 / 31.2, 256 x 14352 14.5 / 11.4, 4096 x 5056 34.8 / 36.7.
+static bool rows_one_by_one(const FinalizeJob& J) {
+  const int64_t last = J.R % 128;
+  return J.R <= 1280 || (last != 0 && (J.sf_layout != METIS_SF_MMA || (last > 32 && J.R <= 8448)));
+}
+
 static FinalizeForm finalize_form(const FinalizeJobs& jobs, int njobs) {
   FinalizeForm form = kFinPlain;
   for (int j = 0; j < njobs; ++j) {
     const FinalizeJob& J = jobs.job[j];
-    if (J.row_sums) return J.R <= 1280 || (J.R % 128 != 0 && J.R <= 8448) ? kFinSumsByRow : kFinSums;          // one job at most wants them
+    if (J.row_sums) return rows_one_by_one(J) ? kFinSumsByRow : kFinSums;          // one job at most wants them
     if (J.sf_cols % 4 != 0) form = kFinEdges;
   }
   return form;
@@ -1118,6 +1125,13 @@ static int32_t launch_finalize_jobs(FinalizeJobs jobs, int njobs, cudaStream_t s
     const bool by_row = form == kFinSumsByRow && J.row_sums;
     J.log_tx = 2;                                             // a warp holds at most 8 rows' lanes of 4 tiles
     while (J.log_tx < (by_row ? 7 : 6) && (1 << J.log_tx) < groups) ++J.log_tx;
+    // Rows one by one: fewer threads to a row where that leaves fewer of them idle in its last round and the rows still give
+    // every SM 256 of them.  2176 tokens (34 groups of blocks, 16 threads for 64) x 5056 columns 25.8 -> 21.2 us (tiled), 9856
+    // (154, 32 for 128) x 3744 63.0 -> 56.8 (row-major).
+    if (by_row) {
+      auto lanes = [&](int log_tx) { return (((groups - 1) >> log_tx) + 1) << log_tx; };
+      for (int l = J.log_tx - 1; l >= 3 && (J.R << l) >= (int64_t)sm_count() * 256; --l) if (lanes(l) < lanes(J.log_tx)) J.log_tx = l;
+    }
     const int64_t segments = J.row_sums ? 1 : ceil_div(groups, (int64_t)1 << J.log_tx);
     const int64_t need = by_row ? ceil_div(ceil_div(J.R, 128) * 128, kFinThreads >> J.log_tx)
                                 : ceil_div(ceil_div(J.R, 128) * 16 * segments, 64 >> J.log_tx);

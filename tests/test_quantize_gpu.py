@@ -489,6 +489,25 @@ def test_scale_pass_at_the_edges_of_its_walk(rows, cols, layout):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
+@pytest.mark.parametrize("rows,cols", [(2176, 5056), (2176, 2352), (576, 5072), (9856, 1504), (1088, 8496), (64, 8240)])
+def test_token_sums_with_few_threads_to_a_row(rows, cols, layout):
+    """Rows of the scale pass one by one where 128 or 64 threads would stand idle in its last trip along a row (34 and 154 groups
+    of blocks: 16 and 32 threads), on both sides of the number of rows that still fill the chip, and a last row block with 16, 48, 64
+    and 96 rows: the same bytes as the quantizer without sums, the sums against float64."""
+    torch.manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device=DEV, dtype=torch.bfloat16)
+    x[:, 5] = 0.0
+    _, qt = ops.nvfp4_quantize_dual(x, sf_layout=layout, token_sums=True)
+    alone = ops.nvfp4_quantize(x, transpose=True, sf_layout=layout)
+    assert torch.equal(qt.codes, alone.codes) and torch.equal(qt.scales, alone.scales) and torch.equal(qt.unit, alone.unit)
+    values = qt.dequantize(torch.float32).double()
+    # fp32 sum of `rows` terms, each exact up to its scale product
+    bound = 2.0 ** -23 * (rows / 16 + 8) * values.abs().sum(1) + 1e-30
+    assert bool(((qt.token_sums.double() - values.sum(1)).abs() <= bound).all())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols", [(512, 512), (515, 544), (1027, 2080), (1120, 4128), (3584, 7328), (1024, 18944), (129 * 128, 1024), (1030, 16 * 2561), (1030, 80016), (2050, 5136), (8960, 3600), (96, 4096), (31, 2048)])
 def test_vector_product_along_the_tiled_scales(rows, cols):
     """Rows that end inside a 128-row block, widths that are no multiple of a round of 512 columns, every number of warps that
