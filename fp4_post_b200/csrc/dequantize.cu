@@ -437,7 +437,8 @@ static int gemv_split(int64_t R, int64_t C) {
 // - where that one would give four rows to a warp: always (18944 x 3584 20.5 -> 13.5);
 // - between: seven rounds or more (3584 x 3584 5.7 -> 5.1; 3072 x 3072 4.4 -> 5.0, 2048 x 2048 2.9 -> 3.15), up to 15 warps per
 //   SM of four rows each, less than a quarter of the rounds missing (4608 x 5120 8.6 -> 7.7, 8192 x 4096 10.0 -> 9.6; but
-//   10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8).
+//   10240 x 6432 18.5 -> 19.8, 3072 x 6432 7.1 -> 7.8); where warps share rows only to bring an SM to 24 of them, up to 14 and a
+//   twentieth (6144 x 6144 12.3 -> 10.6; but 5816 x 5600 9.0 -> 10.0, 8357 x 5600 11.2 -> 12.2, 8357 x 4096 9.0 -> 9.4).
 // Below 2048 columns it replaces gemv_kernel (8960 x 1536 10.2 -> 4.3, 4096 x 768 4.0 -> 3.2, 1024 x 1792 4.3 -> 2.7), except for
 // few rows of two or three rounds (1024 x 768 2.1 -> 2.6, 2048 x 1024 2.7 -> 2.9, 3072 x 1024 3.4 -> 3.1).
 static bool gemv_quad_wins(int64_t R, int64_t C) {
@@ -445,7 +446,9 @@ static bool gemv_quad_wins(int64_t R, int64_t C) {
   if (R < 1024) return false;                                               // 512 x 3584: 3.5 -> 4.3
   const int64_t sms = device_sm_count(), split = gemv_split(R, C);
   if (C >= 8192 || ceil_div(R, 32) >= 3 * sms) return true;
-  return C >= 3584 && ceil_div(R, 128) * 32 < 15 * sms && ceil_div(ceil_div(C, 512), split) * split * 512 * 4 < 5 * C;
+  const int64_t quads = ceil_div(R, 128) * 32, columns = ceil_div(ceil_div(C, 512), split) * split * 512;   // missing ones included
+  if (split > 1 && quads >= kGemvFewWarpsPerSm * sms && (quads >= 14 * sms || columns * 20 > 21 * C)) return false;
+  return C >= 3584 && quads < 15 * sms && columns * 4 < 5 * C;
 }
 
 static cudaError_t launch_gemv_quad(const uint8_t* codes, const uint8_t* scales, const float* unit, int64_t R, int64_t C,

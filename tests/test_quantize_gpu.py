@@ -508,7 +508,7 @@ def test_token_sums_with_few_threads_to_a_row(rows, cols, layout):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,cols", [(512, 512), (515, 544), (1027, 2080), (1120, 4128), (3584, 7328), (1024, 18944), (129 * 128, 1024), (1030, 16 * 2561), (1030, 80016), (2050, 5136), (8960, 3600), (96, 4096), (31, 2048)])
+@pytest.mark.parametrize("rows,cols", [(512, 512), (515, 544), (1027, 2080), (1120, 4128), (3584, 7328), (1024, 18944), (129 * 128, 1024), (1030, 16 * 2561), (1030, 80016), (2050, 5136), (8960, 3600), (96, 4096), (31, 2048), (5816, 5600), (8357, 4096), (5120, 6144)])
 def test_vector_product_along_the_tiled_scales(rows, cols):
     """Rows that end inside a 128-row block, widths that are no multiple of a round of 512 columns, every number of warps that
     share four rows.  The same bits as the kernels for the row-major scale layout give, and against float64 sums of the same values; fp32 products and sums of `cols` terms: error within 2^-24 times the sum of
