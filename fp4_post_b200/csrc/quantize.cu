@@ -468,37 +468,33 @@ struct FinalizeJob {
 };
 struct FinalizeJobs { FinalizeJob job[2]; };
 
-// E4M3 bytes of 4 neighbouring blocks from their maxima (quant.py:23): RN_e4m3(RN_fp32(s / unit)), two packed
-// conversions.  The division is replaced by a product with RN(1 / unit), which lies within 3 fp32 steps of the
-// correctly rounded quotient; the E4M3 byte of a normal value changes only where the 20 dropped mantissa bits
-// pass 0x80000 (the tie), so a product further than that from a tie converts to the same byte.  The others and
-// everything in E4M3's subnormal range (other tie positions) take the division itself; a NaN (of s or of the unit) is
-// a NaN either way.  Whether any of the four needs it is one test: the smallest distance and the smallest product.
-// Returns whether the bytes stand (else: scale_bytes4_exact).
-__device__ __forceinline__ bool scale_bytes4(const float4 a, f32x2 inv_unit2, uint32_t& bytes) {
+// E4M3 bytes of 4 neighbouring blocks from their maxima (quant.py:23): RN_e4m3(RN_fp32(s / unit)), packed conversions.
+// The quotient is the correctly rounded one without a division: s times the reciprocal of the unit in two parts (y, the
+// correctly rounded one, and what is left of it) lies within one fp32 step of it, and from there one correction by the
+// exact remainder rounds correctly (Markstein: y correctly rounded, the quotient within one step).  Four packed
+// instructions for two blocks, no branch.  (The product s y alone, with the division itself next to E4M3 ties, was slower
+// wherever the largest maximum of a bf16 tensor puts one of its 128 mantissas on a tie, as 19968 does with 117: a warp in
+// 512 blocks then meets some, and the scale pass of one output of 65536 x 3584 took 16 or 29 us from tensor to tensor, 16
+// now.)  No quotient overflows: unit comes from the largest s.  A NaN (of s or of the unit) is a NaN either way.
+struct UnitDivisor { f32x2 minus_unit, y, y_rest; };
+__device__ __forceinline__ UnitDivisor unit_divisor(float unit) {
+  const float y = __fdiv_rn(1.0f, unit), rest = __fmul_rn(__fmaf_rn(-unit, y, 1.0f), y);
+  return {pack2(-unit, -unit), pack2(y, y), pack2(rest, rest)};
+}
+__device__ __forceinline__ uint32_t scale_bytes4(const float4 a, const UnitDivisor& by) {
   const f32x2 r6 = pack2(0x1.555556p-3f, 0x1.555556p-3f), minus6 = pack2(-6.0f, -6.0f), tiny = pack2(1e-9f, 1e-9f);
   const f32x2 a2[2] = {pack2(a.x, a.y), pack2(a.z, a.w)};
   float q[4];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {                            // block_scale_from_amax, two at a time
-    const f32x2 q0 = mul2(a2[h], r6);
-    split2(mul2(add2(fma2(fma2(minus6, q0, a2[h]), r6, q0), tiny), inv_unit2), q[2 * h], q[2 * h + 1]);
+    const f32x2 sixth = mul2(a2[h], r6);
+    const f32x2 s = add2(fma2(fma2(minus6, sixth, a2[h]), r6, sixth), tiny);
+    const f32x2 quot = fma2(s, by.y, mul2(s, by.y_rest));
+    split2(fma2(fma2(by.minus_unit, quot, s), by.y, quot), q[2 * h], q[2 * h + 1]);
   }
-  uint32_t nearest = 0xFFFFFFFFu;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) nearest = min(nearest, (__float_as_uint(q[j]) & 0xFFFFFu) - 0x7FFF8u);
   const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), __NV_SATFINITE, __NV_E4M3);
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), __NV_SATFINITE, __NV_E4M3);
-  bytes = lo | (hi << 16);
-  return nearest > 16u && fminf(fminf(q[0], q[1]), fminf(q[2], q[3])) >= 0.0157f;
-}
-// Not inlined: four divisions at each of its uses would push the loop out of the instruction cache.
-__device__ __noinline__ uint32_t scale_bytes4_exact(float4 a, float unit) {
-  const float v[4] = {a.x, a.y, a.z, a.w};
-  uint32_t bytes = 0;
-#pragma unroll 1
-  for (int j = 0; j < 4; ++j) bytes |= (uint32_t)float_to_e4m3(__fdiv_rn(block_scale_from_amax(v[j]), unit)) << (8 * j);
-  return bytes;
+  return lo | (hi << 16);
 }
 
 // the four E4M3 bytes of a word as floats (exact)
@@ -513,16 +509,14 @@ __device__ __forceinline__ void e4m3x4_to_float(uint32_t packed, float (&f)[4]) 
 // (from there to k_end: zeros, the padding of the tiled layout).  Returns the sum of code x scale.  Not inlined either: the
 // loop has four groups in flight and the kernel around it other paths.
 __device__ __noinline__ float finish_row(const float* from, const uint2* codes, uint8_t* to, int pitch, int k, int k_live, int k_end,
-                                         int step, float unit, float inv_unit) {
-  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+                                         int step, const UnitDivisor by) {
   float sum = 0.0f;
 #pragma unroll 4
   for (; k < k_live; k += step) {
     const float4 a = *reinterpret_cast<const float4*>(from + 4 * (int64_t)k);
     const uint4* w = reinterpret_cast<const uint4*>(codes + 4 * (int64_t)k);
     const uint4 w0 = w[0], w1 = w[1];
-    uint32_t bytes;
-    if (!scale_bytes4(a, inv_unit2, bytes)) bytes = scale_bytes4_exact(a, unit);
+    const uint32_t bytes = scale_bytes4(a, by);
     float f[4];
     e4m3x4_to_float(bytes, f);
     sum = fmaf((float)block_code_sum(make_uint2(w0.x, w0.y)), f[0], sum);
@@ -538,9 +532,7 @@ __device__ __noinline__ float finish_row(const float* from, const uint2* codes, 
 // Scale pass of four blocks of each of four rows (row_pitch floats apart) of which only the first `rows` and `blocks` exist, or
 // which no vector load reaches: `dst` gets a 16-byte piece of the tiled layout, or single bytes of the rows.  All maxima are
 // in flight at once: one after the other they make a chain of sixteen loads at the end of a small tensor.
-__device__ __noinline__ void finish_edge(const float* from, int64_t row_pitch, int rows, int blocks, uint8_t* dst, bool tiled, float unit,
-                                         float inv_unit) {
-  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+__device__ __noinline__ void finish_edge(const float* from, int64_t row_pitch, int rows, int blocks, uint8_t* dst, bool tiled, const UnitDivisor by) {
   float a[4][4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -552,10 +544,7 @@ __device__ __noinline__ void finish_edge(const float* from, int64_t row_pitch, i
   for (int c = 0; c < 4; ++c) {
     out[c] = 0u;
     if (c >= rows || blocks <= 0) continue;
-#pragma unroll
-    for (int j = 1; j < 4; ++j) if (j >= blocks) a[c][j] = a[c][0];          // what is not there does not ask for divisions
-    const float4 v = make_float4(a[c][0], a[c][1], a[c][2], a[c][3]);
-    if (!scale_bytes4(v, inv_unit2, out[c])) out[c] = scale_bytes4_exact(v, unit);
+    out[c] = scale_bytes4(make_float4(a[c][0], a[c][1], a[c][2], a[c][3]), by);
     if (blocks < 4) out[c] &= (1u << (8 * blocks)) - 1u;
     if (!tiled) {
 #pragma unroll
@@ -580,7 +569,7 @@ constexpr int kFinThreads = 128;
 // path costs it 1 % (a call for the edges) to 15 %.
 enum FinalizeForm { kFinPlain, kFinEdges, kFinSums, kFinSumsByRow };
 // The rows of a job with sums, 2^log_tx threads (up to the whole CTA) to each.
-__device__ __forceinline__ void finish_rows(const FinalizeJob& J, bool tiled, int tiles, int groups, float unit, float inv_unit,
+__device__ __forceinline__ void finish_rows(const FinalizeJob& J, bool tiled, int tiles, int groups, float unit, const UnitDivisor& by,
                                             float (&s_sum)[kFinThreads / 32][2][4]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = 1 << J.log_tx, per_cta = kFinThreads >> J.log_tx;
@@ -592,7 +581,7 @@ __device__ __forceinline__ void finish_rows(const FinalizeJob& J, bool tiled, in
     if (r < out_rows) {
       uint8_t* to = tiled ? J.scales + (r >> 7) * tiles * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4 : J.scales + r * J.sf_cols;
       sum = finish_row(J.amax + r * J.sf_cols, J.codes + r * J.sf_cols, to, tiled ? 512 : 4, k_lane, r < J.R ? (int)(J.sf_cols >> 2) : 0,
-                       tiled ? groups : 0, tx, unit, inv_unit);
+                       tiled ? groups : 0, tx, by);
     }
     // fixed order: lanes of a row by butterfly, then its warps one after the other
     for (int o = (tx < 32 ? tx : 32) >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -638,8 +627,7 @@ __device__ __forceinline__ void finalize_scales(const FinalizeJob& job0, const F
     *J.unit = unit;
     if (offset_ctr && blockIdx.y == 0) *offset_ctr += 1;       // pass 1 of this call has finished: the next call draws fresh bits
   }
-  const float inv_unit = __fdiv_rn(1.0f, unit);
-  const f32x2 inv_unit2 = pack2(inv_unit, inv_unit);
+  const UnitDivisor by = unit_divisor(unit);
 
   const bool tiled = J.sf_layout == METIS_SF_MMA;
   const int64_t R = J.R, sf_cols = J.sf_cols;
@@ -649,7 +637,7 @@ __device__ __forceinline__ void finalize_scales(const FinalizeJob& job0, const F
   const bool sums = kSums && J.row_sums != nullptr;              // the host asks for them only when vec holds
   if constexpr (kForm == kFinSumsByRow) {
     if (sums) {
-      finish_rows(J, tiled, tiles, groups, unit, inv_unit, s_sum);
+      finish_rows(J, tiled, tiles, groups, unit, by, s_sum);
       return;
     }
   }
@@ -697,18 +685,8 @@ __device__ __forceinline__ void finalize_scales(const FinalizeJob& job0, const F
           cd[c][1] = w[1];
         }
       }
-      bool stands[4], all = true;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        stands[c] = scale_bytes4(a[c], inv_unit2, out[c]) || (!kWhole && c >= rows);
-        all &= stands[c];
-      }
-      if (!all) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) if (!stands[c]) out[c] = scale_bytes4_exact(a[c], unit);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) if (!kWhole && c >= rows) out[c] = 0u;            // padding
+      for (int c = 0; c < 4; ++c) out[c] = kWhole || c < rows ? scale_bytes4(a[c], by) : 0u;      // 0: padding
       if (kQuadSums && sums) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -737,7 +715,7 @@ __device__ __forceinline__ void finalize_scales(const FinalizeJob& job0, const F
         if (tiled) *reinterpret_cast<uint4*>(dst + (int64_t)k * 512) = make_uint4(0u, 0u, 0u, 0u);
       } else if constexpr (!kQuadSums) {                            // an edge of the tensor, or padding
         const int blocks = (int)(sf_cols - 4 * k < 4 ? sf_cols - 4 * k : 4);
-        finish_edge(src + 4 * k, row_pitch, rows, blocks, dst + (tiled ? (int64_t)k * 512 : (int64_t)4 * k), tiled, unit, inv_unit);
+        finish_edge(src + 4 * k, row_pitch, rows, blocks, dst + (tiled ? (int64_t)k * 512 : (int64_t)4 * k), tiled, by);
       } else {                                                      // the same with sums: kept short
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
@@ -1271,10 +1249,12 @@ static int32_t finish_dual(int64_t rows, int64_t cols, int32_t sf_layout, uint8_
   float* amax_t = amax_r + rows * (cols / 16);
   FinalizeJobs jobs = {};
   int n = 0;
-  if (rowmajor) jobs.job[n++] = {amax_r, nullptr, nullptr, rows, cols / 16, sf_layout, scales, unit, 0, nullptr, nullptr, records, 0};
+  // The job with sums first: its CTAs run longer, and the others fill the SMs that they leave (16384 x 4096, stochastic, both with
+  // sums 97.1 -> 94.6 us; 16384 x 2032 50.5 -> 48.8; row-major 4096 x 5056 36.6 -> 33.9).
   if (transposed)
     jobs.job[n++] = {amax_t, nullptr, nullptr, cols, rows / 16, sf_layout, scales_t, unit_t, 0,
                      token_sums_t ? reinterpret_cast<const uint2*>(codes_t) : nullptr, token_sums_t, records, 1};
+  if (rowmajor) jobs.job[n++] = {amax_r, nullptr, nullptr, rows, cols / 16, sf_layout, scales, unit, 0, nullptr, nullptr, records, 0};
   if (n == 0) return METIS_OK;
   return launch_finalize_jobs(jobs, n, st, ctr);      // job 0 of the launch bumps the Philox offset counter, if there is one
 }

@@ -107,6 +107,17 @@ def test_one_launch_path_for_small_tensors(rows, cols, dtype, layout):
         assert_packed_equal(q, x.float().numpy(), layout, mean=mean.numpy(), what=f"small centred {rows}x{cols}")
 
 
+# Largest maxima that put other maxima of a bf16 tensor exactly on an E4M3 tie of the scale pass (19968 does with 117), and
+# one so large that most scales are E4M3 subnormals or zero; whole pieces of the tiled layout and edges of it.
+@pytest.mark.parametrize("rows,cols", [(256, 4096), (300, 4112)])
+@pytest.mark.parametrize("top", [19968.0, 1.5, 3.0e6])
+@pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
+def test_scales_on_ties_of_the_largest_maximum(rows, cols, top, layout):
+    x = synthetic(rows, cols, "normal", seed=int(top), dtype=torch.bfloat16)
+    x[0, 0] = top
+    assert_packed_equal(ops.nvfp4_quantize(x.to(DEV), sf_layout=layout), x.float().numpy(), layout, what=f"largest {top}")
+
+
 def test_bf16_inputs_sitting_exactly_on_rounding_ties():
     # With bf16 data an element is often an exact fraction of the block maximum that lands on a
     # rounding boundary of the reference (x = amax/8 gives |x|/(s/2) = 1.5 up to the rounding of
