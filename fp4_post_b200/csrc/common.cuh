@@ -138,9 +138,11 @@ __device__ __forceinline__ float block_scale_from_amax(float amax) {
   return __fadd_rn(q, 1e-9f);
 }
 
+// 1 / s for a block scale.  Neither side is ever subnormal (s >= 1e-9, and the largest finite s is 2^127.99 / 6), so the form
+// that flushes subnormals returns the same bits; the other one spends four more instructions per block on them.
 __device__ __forceinline__ float rcp_approx(float v) {
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
 __device__ __forceinline__ float min3(float a, float b, float c) {
@@ -283,28 +285,33 @@ __device__ __forceinline__ uint32_t quantize8_rn(const float (&x)[8], float s) {
 
 // ---- Philox4x32-10 ---------------------------------------------------------------------------------
 
-struct Philox {
-  uint32_t k0, k1;
-  __device__ __forceinline__ Philox(uint64_t seed) : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)) {}
-  // Counter words {block, 0, offset}: block indexes stay below 2^32 (the entry points refuse more, kMaxStochasticElements;
-  // this GPU's memory does not hold such a tensor and its codes), and with the second word known to be zero the first
-  // round's product with c2 and the second round's with c0 are the same for the whole launch: the compiler takes them
-  // out of the loop.  (One wide multiplication in place of each pair of high and low products was measured slower:
-  // 80 -> 89 us, 16384 x 4096 both.)
-  __device__ __forceinline__ uint4 operator()(uint32_t block, uint64_t ctr_hi) const {
-    uint32_t c0 = block, c1 = 0u;
-    uint32_t c2 = (uint32_t)ctr_hi, c3 = (uint32_t)(ctr_hi >> 32);
-    uint32_t a = k0, b = k1;
-#pragma unroll
+// The keys of the ten rounds, made on the host and passed as a kernel parameter: formed on the device they are added up anew for
+// every block, and a kernel that is bound by issue pays for uniform instructions as for any other.
+struct PhiloxKeys {
+  uint32_t k[20];
+  explicit PhiloxKeys(uint64_t seed) {
     for (int i = 0; i < 10; ++i) {
-      const uint32_t h0 = __umulhi(0xD2511F53u, c0), l0 = 0xD2511F53u * c0;
-      const uint32_t h1 = __umulhi(0xCD9E8D57u, c2), l1 = 0xCD9E8D57u * c2;
-      c0 = h1 ^ c1 ^ a;  c1 = l1;  c2 = h0 ^ c3 ^ b;  c3 = l0;
-      a += 0x9E3779B9u;  b += 0xBB67AE85u;
+      k[2 * i] = (uint32_t)seed + (uint32_t)i * 0x9E3779B9u;
+      k[2 * i + 1] = (uint32_t)(seed >> 32) + (uint32_t)i * 0xBB67AE85u;
     }
-    return make_uint4(c0, c1, c2, c3);
   }
 };
+// Counter words {block, 0, offset}: block indexes stay below 2^32 (the entry points refuse more, kMaxStochasticElements;
+// this GPU's memory does not hold such a tensor and its codes), and with the second word known to be zero the first
+// round's product with c2 and the second round's with c0 are the same for the whole launch: the compiler takes them
+// out of the loop.  (One wide multiplication in place of each pair of high and low products was measured slower:
+// 80 -> 89 us, 16384 x 4096 both.)
+__device__ __forceinline__ uint4 philox4x32(const PhiloxKeys& keys, uint32_t block, uint64_t ctr_hi) {
+  uint32_t c0 = block, c1 = 0u;
+  uint32_t c2 = (uint32_t)ctr_hi, c3 = (uint32_t)(ctr_hi >> 32);
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+    const uint32_t h0 = __umulhi(0xD2511F53u, c0), l0 = 0xD2511F53u * c0;
+    const uint32_t h1 = __umulhi(0xCD9E8D57u, c2), l1 = 0xCD9E8D57u * c2;
+    c0 = h1 ^ c1 ^ keys.k[2 * i];  c1 = l1;  c2 = h0 ^ c3 ^ keys.k[2 * i + 1];  c3 = l0;
+  }
+  return make_uint4(c0, c1, c2, c3);
+}
 
 // Stochastic-rounding codes of one block (16 values sharing scale s): floor(folded index + U) with
 // U uniform on [0, 1) in steps of 2^-16, which rounds up with probability frac(index) (quant.py:139-147:
@@ -369,6 +376,10 @@ __device__ __forceinline__ void quantize16_sr_hw(const float (&x)[16], float s, 
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+// The two bf16 of a word plus c0 and c1, in fp32 (mixed-precision additions: the operands are not converted first).
+__device__ __forceinline__ void add_bf16x2(uint32_t w, float c0, float c1, float& lo, float& hi) {
+  asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; add.rn.f32.bf16 %0, l, %3; add.rn.f32.bf16 %1, h, %4; }" : "=f"(lo), "=f"(hi) : "r"(w), "f"(c0), "f"(c1));
+}
 
 // 8 consecutive elements starting at p (16-byte aligned for bf16, 32-byte for fp32).
 template <typename T> struct Load8;
@@ -430,6 +441,11 @@ template <> struct RawBlock<__nv_bfloat16> {
 #pragma unroll
     for (int i = 0; i < 8; ++i) { v[2 * i] = bf16_lo(w[i]); v[2 * i + 1] = bf16_hi(w[i]); }
   }
+  __device__ __forceinline__ void unpack_plus(const float (&c)[16], float (&v)[16]) const {
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) add_bf16x2(w[i], c[2 * i], c[2 * i + 1], v[2 * i], v[2 * i + 1]);
+  }
 };
 template <> struct RawBlock<float> {
   float4 q[4];
@@ -440,6 +456,11 @@ template <> struct RawBlock<float> {
   __device__ __forceinline__ void unpack(float (&v)[16]) const {
 #pragma unroll
     for (int i = 0; i < 4; ++i) { v[4 * i] = q[i].x; v[4 * i + 1] = q[i].y; v[4 * i + 2] = q[i].z; v[4 * i + 3] = q[i].w; }
+  }
+  __device__ __forceinline__ void unpack_plus(const float (&c)[16], float (&v)[16]) const {
+    unpack(v);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) split2(add2(pack2(v[i], v[i + 1]), pack2(c[i], c[i + 1])), v[i], v[i + 1]);
   }
 };
 

@@ -38,7 +38,7 @@ __device__ __forceinline__ void fold_global_max(unsigned int* gmax, float local)
 template <typename T, bool kMean, bool kSR>
 __global__ void __launch_bounds__(kQuantThreads)
 quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
-                     const float* __restrict__ col_mean, uint64_t seed, uint64_t offset,
+                     const float* __restrict__ col_mean, const __grid_constant__ PhiloxKeys keys, uint64_t offset,
                      const uint64_t* __restrict__ offset_ctr, uint2* __restrict__ codes, float* __restrict__ amax_out,
                      unsigned int* __restrict__ gmax, unsigned int* __restrict__ records, uint32_t sr16) {
   grid_dependency_wait();
@@ -49,7 +49,6 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
   if (bc < blocks_per_row) {
     float m[16];
     if (kMean) Load16<float>::load(col_mean + (int64_t)bc * 16, m);
-    const Philox rng(seed);
     auto quantize_block = [&](float (&v)[16], int r) {
       if (kMean) subtract16(v, m);
       const float a = abs_max16(v);
@@ -57,8 +56,8 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
       const int64_t b = (int64_t)r * blocks_per_row + bc;
       uint32_t packed[2];
       if (kSR) {
-        if (sr16) quantize16_sr(v, s, rng((uint32_t)b, offset), packed);      // one counter per block
-        else quantize16_sr_hw(v, s, rng((uint32_t)b, offset), packed);
+        if (sr16) quantize16_sr(v, s, philox4x32(keys, (uint32_t)b, offset), packed);      // one counter per block
+        else quantize16_sr_hw(v, s, philox4x32(keys, (uint32_t)b, offset), packed);
       } else {
         quantize_rn<2>(v, s, packed);
       }
@@ -116,11 +115,13 @@ quantize_rows_kernel(const T* __restrict__ x, int rows, int blocks_per_row, int6
 // r sits at chunk c ^ (r & 7)).  One __syncthreads per tile: staging and the column means are double
 // buffered.  A tile load that does not arrive within the wait limit raises the error word of the
 // workspace header (the scale pass then publishes NaN as the unit) instead of hanging.
-// What bounds it: instruction issue (24 warps per SM; the rows-only form runs at 85 % of the copy bandwidth).
-// Measured at 16384 x 4096 bf16, this pass alone, rows / transposed / both / both centred and stochastic: 37.1 / 48.2 /
-// 76.9 / 91.5 us with scalar fp32 arithmetic and 64-bit divisions in the tile walk, 32.9 / 39.6 / 63.8 / 80.2 us with
-// packed fp32 (3-6 us of it) and the walk by additions with every thread's offsets inside a tile kept (the rest); the last
-// figure is 78.6 with 32-bit block counters in the random number generator.
+// What bounds it: instruction issue (24 warps per SM, 63 % of the slots; the rows-only form runs at 86 % of the copy
+// bandwidth).  So what stands beside the arithmetic is kept short: a tile that lies inside the tensor has no tests of edges,
+// the walk and the block indexes advance by 32-bit additions, the round keys of the random numbers come as parameters, the
+// mean is added by the instruction that takes a bf16 operand, shared memory is addressed as such, and the rotation and the
+// 16-bit rounding, which training does not ask for, have kernels of their own (kPlain: neither).  Measured at 16384 x 4096
+// bf16, this pass alone, rows / transposed / both / both centred and stochastic: 32.9 / 39.6 / 63.8 / 78.6 us before that
+// (199 instructions per block in the last one), 30.4 / 33.2 / 55.5 / 60.2 now (150).
 template <typename T> struct TileCfg {
   static constexpr int kRows = 128;
   static constexpr int kCols = 128 / sizeof(T);            // 64 (bf16) or 32 (fp32): 128 bytes per row
@@ -147,9 +148,12 @@ constexpr int kDualMaxCtas = kMaxRecords;
 constexpr int kDualHeaderBytes = 256 + ((kDualMaxCtas * 3 * 4 + 255) / 256) * 256;
 
 // How a CTA walks the tiles: their number, those along a row of x, and gridDim.x split into whole rows of tiles
-// and a remainder.
+// and a remainder; blocks per row of Q (bpr) and of Qt (bpc), and what a step and the wrap to the next row of tiles add to the index
+// of a tile's first block in Q (_r) and in Qt (_t).  Block indexes are counted modulo 2^32 and a tensor has fewer blocks
+// (launch_tile), so the additions end in the right place whichever way they wrap.
 struct TileWalk {
   uint32_t tiles, col_tiles, step_rows, step_cols;
+  uint32_t bpr, bpc, step_r, wrap_r, step_t, wrap_t;
 };
 
 struct TileOutputs {
@@ -192,17 +196,26 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
+}
 
-template <typename T, bool kMean, bool kSR, bool kRowsOut, bool kColsOut>
+template <typename T, bool kMean, bool kSR, bool kRowsOut, bool kColsOut, bool kPlain>
 __global__ void __launch_bounds__(kQuantThreads, 3)
-quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk walk, int64_t rows, int64_t cols,
-                     const float* __restrict__ col_mean, uint64_t seed, uint64_t offset,
-                     const uint64_t* __restrict__ offset_ctr, const TileOutputs out) {
+quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ TileWalk walk, int64_t rows, int64_t cols,
+                     const float* __restrict__ col_mean, const __grid_constant__ PhiloxKeys keys, uint64_t offset,
+                     const uint64_t* __restrict__ offset_ctr, const __grid_constant__ TileOutputs out) {
   using TC = TileCfg<T>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* s_staging = smem + TC::kStages * TC::kStageBytes;                    // [2][kStagingBytes]
-  float* s_mean = reinterpret_cast<float*>(s_staging + 2 * TC::kStagingBytes);  // [2][kCols]
+  float* s_mean = reinterpret_cast<float*>(s_staging + 2 * TC::kStagingBytes);  // [2][kCols], negated
   uint64_t* full = reinterpret_cast<uint64_t*>(s_mean + 2 * TC::kCols);         // [kStages]
   __shared__ int s_failed;
 
@@ -210,17 +223,11 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
   if (kSR && offset_ctr) offset += *offset_ctr;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int64_t bpr = cols >> 4;                     // blocks per row of Q
-  const int64_t bpc = rows >> 4;                     // blocks per row of Qt
-  // Tile id = row tile * col_tiles + column tile; the CTA takes the ids blockIdx.x + i * gridDim.x.  The two
-  // coordinates advance by additions (walk.step_* = gridDim.x in mixed radix): a 64-bit division per thread and tile
-  // costs as much as three elements' arithmetic.
+  const uint32_t bpr = walk.bpr, bpc = walk.bpc;
+  // Tile id = row tile * col_tiles + column tile; the CTA takes the ids blockIdx.x + i * gridDim.x.  Its coordinates and
+  // its first blocks in Q and Qt advance by additions (walk.step_* = gridDim.x in mixed radix): multiplications and 64-bit
+  // arithmetic there cost as much as three elements of every tile.
   const uint32_t tiles = walk.tiles, col_tiles = walk.col_tiles;
-  auto advance = [&](uint32_t& rt, uint32_t& ct) {
-    ct += walk.step_cols;
-    rt += walk.step_rows;
-    if (ct >= col_tiles) { ct -= col_tiles; ++rt; }
-  };
 
   if (tid == 0) {
     for (int s = 0; s < TC::kStages; ++s) mbar_init(&full[s], 1);
@@ -228,14 +235,14 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  auto fill_mean = [&](uint32_t ct, int buf) {
-    if (kMean && tid < TC::kCols) {
-      const int64_t c = (int64_t)ct * TC::kCols + tid;
-      s_mean[buf * TC::kCols + tid] = c < cols ? __ldg(col_mean + c) : 0.0f;
-    }
+  // -mean of column tile ct's columns, one per thread (added, it rounds as the mean subtracted)
+  auto minus_mean = [&](uint32_t ct) {
+    const uint32_t c = ct * TC::kCols + tid;
+    return kMean && tid < TC::kCols && c < (uint32_t)cols ? -__ldg(col_mean + c) : 0.0f;
   };
   uint32_t rt = blockIdx.x / col_tiles, ct = blockIdx.x - rt * col_tiles;
-  if (blockIdx.x < tiles) fill_mean(ct, 0);
+  uint32_t blk_r = rt * TC::kRows * bpr + ct * TC::kBlocksPerRow, blk_t = ct * TC::kCols * bpc + rt * TC::kRowBlocks;
+  if (kMean && tid < TC::kCols) s_mean[tid] = minus_mean(ct);
   __syncthreads();
 
   uint32_t ahead_rt = rt, ahead_ct = ct, ahead = blockIdx.x;       // the next tile to be requested
@@ -244,173 +251,191 @@ quantize_tile_kernel(const __grid_constant__ CUtensorMap map_x, const TileWalk w
       mbar_expect_tx(&full[stage], TC::kStageBytes);
       tma_load_2d(smem + stage * TC::kStageBytes, &map_x, (int32_t)(ahead_ct * TC::kCols), (int32_t)(ahead_rt * TC::kRows), &full[stage]);
       ahead += gridDim.x;
-      advance(ahead_rt, ahead_ct);
+      ahead_ct += walk.step_cols;
+      ahead_rt += walk.step_rows;
+      if (ahead_ct >= col_tiles) { ahead_ct -= col_tiles; ++ahead_rt; }
     }
   };
   if (tid == 0) {
     for (int s = 0; s < TC::kStages; ++s) issue(s);
   }
 
-  const Philox rng(seed);
   float running_t = 0.0f, running_r = 0.0f;
-  const uint32_t smem_base = smem_u32(smem);
+  const uint32_t smem_base = smem_u32(smem), staging_base = smem_u32(s_staging), mean_base = smem_u32(s_mean), failed_addr = smem_u32(&s_failed);
   // Where this thread's work lies inside a tile does not change from tile to tile: per tile only the tile's own
   // position is added.
-  // column phase: this lane's word of a row, as chunk and offset inside the chunk
-  const uint32_t word_chunk = (uint32_t)lane >> 2, word_in_chunk = ((uint32_t)lane & 3u) * 4u;
-  const uint32_t col_smem = (uint32_t)(warp * 16) * 128u + word_in_chunk;
-  const int64_t col_ctr = (int64_t)(lane * TC::kColsPerWord) * bpc + warp;      // Philox counter of its first block
+  // column phase: this lane's word of row r of its row block, r = 0..7 (the swizzle repeats from there)
+  uint32_t word_at[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) word_at[r] = (uint32_t)(warp * 16 + r) * 128u + ((((uint32_t)lane >> 2) ^ (uint32_t)r) << 4) + ((uint32_t)lane & 3u) * 4u;
+  const uint32_t col_blk = (uint32_t)(lane * TC::kColsPerWord) * bpc + warp;    // its first block in Qt
+  const uint32_t col_staged = (uint32_t)(lane * TC::kCodePitch + warp * 8);
   // row phase: block (row_r + u * kRowStep, row_b)
-  constexpr int kRowStep = kQuantThreads / TC::kBlocksPerRow;
-  const int row_b = tid & (TC::kBlocksPerRow - 1), row_r = tid / TC::kBlocksPerRow;
-  const int64_t row_blk = (int64_t)row_r * bpr + row_b;
+  constexpr uint32_t kRowStep = kQuantThreads / TC::kBlocksPerRow;
+  const uint32_t row_b = tid & (TC::kBlocksPerRow - 1), row_r = tid / TC::kBlocksPerRow;
+  const uint32_t row_blk = row_r * bpr + row_b;
   // write-out of Qt: 8-byte piece out_piece of the out rows out_j, out_j + 32, ...
-  const int out_j = tid >> 3, out_piece = tid & 7;
-  const int64_t pitch_t = rows >> 1;
-  const int64_t out_off = out_j * pitch_t + out_piece * 8;
-  const uint32_t out_staged = (uint32_t)((out_j % TC::kColsPerWord) * TC::kCodeArray + (out_j / TC::kColsPerWord) * TC::kCodePitch + out_piece * 8);
-  volatile int* failed = &s_failed;
-  int stage = 0;
-  uint32_t it = 0;
-  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
-    const int buf = it & 1;
-    if (!mbar_wait(&full[stage], (it / TC::kStages) & 1u, failed)) *failed = 1;
-    if (*failed) break;                               // every thread sees the same outcome of the barrier, or the flag
+  const uint32_t out_j = tid >> 3, out_piece = tid & 7;
+  const uint32_t out_blk = out_j * bpc + out_piece;
+  const uint32_t out_staged = (out_j % TC::kColsPerWord) * TC::kCodeArray + (out_j / TC::kColsPerWord) * TC::kCodePitch + out_piece * 8;
+  constexpr uint32_t kAmaxAt = TC::kColsPerWord * TC::kCodeArray;               // staged maxima: [kRowBlocks][kCols]
 
-    const int64_t row0 = (int64_t)rt * TC::kRows, col0 = (int64_t)ct * TC::kCols;
-    const int live_rows = (int)min((int64_t)TC::kRows, rows - row0);            // of this tile
-    const int live_cols = (int)min((int64_t)TC::kCols, cols - col0);            // both multiples of 16 where that output exists
-    const uint32_t tile_smem = smem_base + stage * TC::kStageBytes;
-    uint8_t* staging = s_staging + buf * TC::kStagingBytes;
-    float* s_amax = reinterpret_cast<float*>(staging + TC::kColsPerWord * TC::kCodeArray);   // [kRowBlocks][kCols]
-    const float* mean = s_mean + buf * TC::kCols;
-
+  // The arithmetic of one tile.  kWhole: all of it lies inside the tensor; the tests of the edges are then not in the code
+  // (and the stores of a block not behind a branch).
+  auto quantize_tile = [&](auto whole, uint32_t tile_smem, uint32_t staging, uint32_t mean, int live_rows, int live_cols) {
+    constexpr bool kWhole = decltype(whole)::value;
     // ---- column phase: warp = row block, lane = 32-bit word of the row ----
-    if (kColsOut) {
+    if constexpr (kColsOut) {
       float v[TC::kColsPerWord][16];
-      const uint32_t row_base = tile_smem + col_smem;
+      float m[2] = {0.0f, 0.0f};
+      if constexpr (kMean) {
+        if constexpr (TC::kColsPerWord == 2) { const uint2 both = lds64(mean + lane * 8); m[0] = __uint_as_float(both.x); m[1] = __uint_as_float(both.y); }
+        else                                 { m[0] = __uint_as_float(lds32(mean + lane * 4)); }
+      }
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
-        const uint32_t w = lds32(row_base + r * 128 + ((word_chunk ^ (uint32_t)(r & 7)) << 4));
-        if constexpr (sizeof(T) == 2) { v[0][r] = bf16_lo(w); v[1][r] = bf16_hi(w); }
-        else                          { v[0][r] = __uint_as_float(w); }
+        const uint32_t w = lds32(tile_smem + word_at[r & 7] + (r >> 3) * 1024);
+        if constexpr (sizeof(T) == 4)  { v[0][r] = __uint_as_float(w); }
+        else if constexpr (kMean)      { add_bf16x2(w, m[0], m[1], v[0][r], v[1][r]); }
+        else                           { v[0][r] = bf16_lo(w); v[1][r] = bf16_hi(w); }
       }
-      if (kMean) {
+      if constexpr (kMean && sizeof(T) == 4) {
+        const f32x2 minus_m = pack2(m[0], m[0]);
 #pragma unroll
-        for (int c = 0; c < TC::kColsPerWord; ++c) {
-          const float m = mean[lane * TC::kColsPerWord + c];
-          const f32x2 minus_m = pack2(-m, -m);
-#pragma unroll
-          for (int r = 0; r < 16; r += 2) split2(add2(pack2(v[c][r], v[c][r + 1]), minus_m), v[c][r], v[c][r + 1]);
-        }
+        for (int r = 0; r < 16; r += 2) split2(add2(pack2(v[0][r], v[0][r + 1]), minus_m), v[0][r], v[0][r + 1]);
       }
-      const bool rows_live = warp * 16 < live_rows;
       float amax[TC::kColsPerWord];
 #pragma unroll
       for (int c = 0; c < TC::kColsPerWord; ++c) {
-        if (out.hadamard) hadamard16(v[c], out.hadamard & 0xFFFFu);           // uniform over the grid
+        if (!kPlain && out.hadamard) hadamard16(v[c], out.hadamard & 0xFFFFu);           // uniform over the grid
         const float a = abs_max16(v[c]);
         const float s = block_scale_from_amax(a);
         uint32_t packed[2];
-        if (kSR) {
-          const uint32_t b = (uint32_t)(col0 * bpc + (row0 >> 4)) + (uint32_t)(col_ctr + c * bpc);          // block index in Qt
-          const uint4 bits = rng(b, kRowsOut ? (offset ^ kColumnStream) : offset);                // alone: the transposed call's own stream
-          if (out.sr16) quantize16_sr(v[c], s, bits, packed);
+        if constexpr (kSR) {
+          const uint4 bits = philox4x32(keys, blk_t + col_blk + c * bpc, kRowsOut ? (offset ^ kColumnStream) : offset);   // alone: the transposed call's own stream
+          if (!kPlain && out.sr16) quantize16_sr(v[c], s, bits, packed);
           else quantize16_sr_hw(v[c], s, bits, packed);
         } else {
           quantize_rn<2>(v[c], s, packed);
         }
-        *reinterpret_cast<uint2*>(staging + c * TC::kCodeArray + lane * TC::kCodePitch + warp * 8) = make_uint2(packed[0], packed[1]);
+        sts64(staging + c * TC::kCodeArray + col_staged, packed[0], packed[1]);
         amax[c] = a;
-        if (rows_live && lane * TC::kColsPerWord + c < live_cols) running_t = fmaxf(running_t, a);
+        if (kWhole || (warp * 16 < live_rows && lane * TC::kColsPerWord + c < live_cols)) running_t = fmaxf(running_t, a);
       }
-      if constexpr (sizeof(T) == 2) *reinterpret_cast<float2*>(s_amax + warp * TC::kCols + 2 * lane) = make_float2(amax[0], amax[1]);
-      else                          s_amax[warp * TC::kCols + lane] = amax[0];
+      const uint32_t at = staging + kAmaxAt + (uint32_t)(warp * TC::kCols + lane * TC::kColsPerWord) * 4u;
+      if constexpr (TC::kColsPerWord == 2) sts64(at, __float_as_uint(amax[0]), __float_as_uint(amax[1]));
+      else                                 sts32(at, __float_as_uint(amax[0]));
     }
 
     // ---- row phase: a thread owns blocks (row, b) with b fixed, straight to global memory ----
-    if (kRowsOut) {
-      const bool cols_live = row_b * 16 < live_cols;
-      const int64_t tile_blk = row0 * bpr + (col0 >> 4);
-      float mb[16];
-      if (kMean) {
+    if constexpr (kRowsOut) {
+      [[maybe_unused]] float mb[16];
+      if constexpr (kMean) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 f = *reinterpret_cast<const float4*>(mean + row_b * 16 + 4 * i);
-          mb[4 * i] = f.x; mb[4 * i + 1] = f.y; mb[4 * i + 2] = f.z; mb[4 * i + 3] = f.w;
+          const uint4 f = lds128(mean + row_b * 64 + 16 * i);
+          mb[4 * i] = __uint_as_float(f.x); mb[4 * i + 1] = __uint_as_float(f.y); mb[4 * i + 2] = __uint_as_float(f.z); mb[4 * i + 3] = __uint_as_float(f.w);
         }
       }
 #pragma unroll
       for (int u = 0; u < TC::kRowUnits; ++u) {
-        const int r = row_r + u * kRowStep;
-        const uint32_t row_addr = tile_smem + (uint32_t)r * 128u;
-        const uint32_t swz = (uint32_t)(r & 7);
+        const uint32_t r = row_r + u * kRowStep;
+        const uint32_t row_addr = tile_smem + r * 128u;
+        const uint32_t swz = r & 7;
         RawBlock<T> raw;
         if constexpr (sizeof(T) == 2) {
-          raw.a = lds128(row_addr + (((uint32_t)(2 * row_b) ^ swz) << 4));
-          raw.b = lds128(row_addr + (((uint32_t)(2 * row_b + 1) ^ swz) << 4));
+          raw.a = lds128(row_addr + (((2 * row_b) ^ swz) << 4));
+          raw.b = lds128(row_addr + (((2 * row_b + 1) ^ swz) << 4));
         } else {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const uint4 w = lds128(row_addr + (((uint32_t)(4 * row_b + k) ^ swz) << 4));
+            const uint4 w = lds128(row_addr + (((4 * row_b + k) ^ swz) << 4));
             raw.q[k] = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
           }
         }
         float v[16];
-        raw.unpack(v);
-        if (kMean) subtract16(v, mb);
+        if constexpr (kMean) raw.unpack_plus(mb, v);
+        else raw.unpack(v);
         const float a = abs_max16(v);
         const float s = block_scale_from_amax(a);
-        const int64_t blk = tile_blk + row_blk + u * (kRowStep * bpr);
+        const uint32_t blk = blk_r + row_blk + u * (kRowStep * bpr);
         uint32_t packed[2];
-        if (kSR) {
-          if (out.sr16) quantize16_sr(v, s, rng((uint32_t)blk, offset), packed);
-          else quantize16_sr_hw(v, s, rng((uint32_t)blk, offset), packed);
+        if constexpr (kSR) {
+          const uint4 bits = philox4x32(keys, blk, offset);
+          if (!kPlain && out.sr16) quantize16_sr(v, s, bits, packed);
+          else quantize16_sr_hw(v, s, bits, packed);
+        } else {
+          quantize_rn<2>(v, s, packed);
         }
-        else     quantize_rn<2>(v, s, packed);
-        if (cols_live && r < live_rows) {
+        if (kWhole || (row_b * 16 < live_cols && r < live_rows)) {
           reinterpret_cast<uint2*>(out.codes_r)[blk] = make_uint2(packed[0], packed[1]);
           out.amax_r[blk] = a;
           running_r = fmaxf(running_r, a);
         }
       }
     }
-
-    uint32_t next_rt = rt, next_ct = ct;
-    advance(next_rt, next_ct);
-    if (tile + gridDim.x < tiles) fill_mean(next_ct, buf ^ 1);        // its last readers passed the previous barrier
-    __syncthreads();                                   // staging complete; this tile's stage is free
-    if (tid == 0) issue(stage);
-
-    // ---- write-out of Qt: out row j owns 64 contiguous code bytes and 8 maxima of this tile ----
-    if (kColsOut) {
-      uint8_t* tile_codes = out.codes_t + (col0 * pitch_t + (row0 >> 1));
-      const bool piece_live = out_piece * 16 < live_rows;
+  };
+  // Write-out of Qt: out row j owns 64 contiguous code bytes and 8 maxima of the tile whose first block in Qt is tile_t.
+  auto write_columns = [&](auto whole, uint32_t staging, uint32_t tile_t, int live_rows, int live_cols) {
+    constexpr bool kWhole = decltype(whole)::value;
 #pragma unroll
-      for (int k = 0; k < TC::kCols * 8 / kQuantThreads; ++k) {                 // 8-byte pieces: 8 per out row, 32 rows a trip
-        static_assert((kQuantThreads / 8) % TC::kColsPerWord == 0, "the staged array of a thread's pieces does not change");
-        if (piece_live && out_j + 32 * k < live_cols)
-          *reinterpret_cast<uint2*>(tile_codes + (out_off + 32 * k * pitch_t)) =
-              *reinterpret_cast<const uint2*>(staging + out_staged + (32 / TC::kColsPerWord) * TC::kCodePitch * k);
-      }
-      if (tid < TC::kCols * 2) {
-        const int j = tid & (TC::kCols - 1), h = tid / TC::kCols;               // half h: row blocks 4h .. 4h+3
-        if (j < live_cols) {
-          float* dst = out.amax_t + ((col0 + j) * bpc + (row0 >> 4) + 4 * h);
-          float a4[4];
+    for (int k = 0; k < TC::kCols * 8 / kQuantThreads; ++k) {                   // 8-byte pieces: 8 per out row, 32 rows a trip
+      static_assert((kQuantThreads / 8) % TC::kColsPerWord == 0, "the staged array of a thread's pieces does not change");
+      if (kWhole || (out_piece * 16 < live_rows && out_j + 32 * k < live_cols))
+        reinterpret_cast<uint2*>(out.codes_t)[tile_t + out_blk + 32 * k * bpc] = lds64(staging + out_staged + (32 / TC::kColsPerWord) * TC::kCodePitch * k);
+    }
+    if (tid < TC::kCols * 2) {
+      const uint32_t j = tid & (TC::kCols - 1), h = tid / TC::kCols;            // half h: row blocks 4h .. 4h+3
+      if (kWhole || j < live_cols) {
+        float* dst = out.amax_t + (tile_t + j * bpc + 4 * h);
+        float a4[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) a4[k] = s_amax[(4 * h + k) * TC::kCols + j];
-          if (live_rows == TC::kRows && (bpc & 3) == 0) {
-            *reinterpret_cast<float4*>(dst) = make_float4(a4[0], a4[1], a4[2], a4[3]);
-          } else {
+        for (int k = 0; k < 4; ++k) a4[k] = __uint_as_float(lds32(staging + kAmaxAt + ((4 * h + k) * TC::kCols + j) * 4));
+        if ((kWhole || live_rows == TC::kRows) && (bpc & 3) == 0) {
+          *reinterpret_cast<float4*>(dst) = make_float4(a4[0], a4[1], a4[2], a4[3]);
+        } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) if ((4 * h + k) * 16 < live_rows) dst[k] = a4[k];
-          }
+          for (int k = 0; k < 4; ++k) if (kWhole || (4 * h + k) * 16 < live_rows) dst[k] = a4[k];
         }
       }
     }
+  };
+
+  volatile int* failed = &s_failed;
+  int stage = 0;
+  uint32_t it = 0;
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+    const uint32_t buf = it & 1;
+    uint32_t next_rt = rt + walk.step_rows, next_ct = ct + walk.step_cols, next_r = blk_r + walk.step_r, next_t = blk_t + walk.step_t;
+    if (next_ct >= col_tiles) { next_ct -= col_tiles; ++next_rt; next_r += walk.wrap_r; next_t += walk.wrap_t; }
+    const bool more = tile + gridDim.x < tiles;
+    const float next_mean = more ? minus_mean(next_ct) : 0.0f;        // on its way while this tile is worked on
+
+    if (!mbar_wait(&full[stage], (it / TC::kStages) & 1u, failed)) *failed = 1;
+    if (lds32(failed_addr) != 0) break;               // every thread sees the same outcome of the barrier, or the flag
+
+    const uint32_t row0 = rt * TC::kRows, col0 = ct * TC::kCols;
+    const int live_rows = (int)min((int64_t)TC::kRows, rows - row0);            // of this tile
+    const int live_cols = (int)min((int64_t)TC::kCols, cols - col0);            // both multiples of 16 where that output exists
+    const bool whole = live_rows == TC::kRows && live_cols == TC::kCols;
+    const uint32_t tile_smem = smem_base + stage * TC::kStageBytes;
+    const uint32_t staging = staging_base + buf * TC::kStagingBytes;
+    const uint32_t mean = mean_base + buf * (TC::kCols * 4);
+    if (whole) quantize_tile(std::true_type{}, tile_smem, staging, mean, TC::kRows, TC::kCols);
+    else       quantize_tile(std::false_type{}, tile_smem, staging, mean, live_rows, live_cols);
+
+    if (kMean && more && tid < TC::kCols) s_mean[(buf ^ 1) * TC::kCols + tid] = next_mean;      // its last readers passed the previous barrier
+    __syncthreads();                                   // staging complete; this tile's stage is free
+    if (tid == 0) issue(stage);
+
+    if constexpr (kColsOut) {
+      if (whole) write_columns(std::true_type{}, staging, blk_t, TC::kRows, TC::kCols);
+      else       write_columns(std::false_type{}, staging, blk_t, live_rows, live_cols);
+    }
     rt = next_rt;
     ct = next_ct;
+    blk_r = next_r;
+    blk_t = next_t;
     if (++stage == TC::kStages) stage = 0;
   }
   if (s_failed) {
@@ -1024,7 +1049,7 @@ static int32_t launch_rows(const T* x, int64_t rows, int64_t cols, int64_t ld, c
     METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));       // running maximum and error word
   }
   METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)s.gx, (unsigned)s.gy), dim3((unsigned)s.bx, (unsigned)(kQuantThreads / s.bx)),
-                                  0, st, x, (int)rows, bpr, ld, mean, seed, offset, ctr, reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax,
+                                  0, st, x, (int)rows, bpr, ld, mean, PhiloxKeys(seed), offset, ctr, reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax,
                                   *records, sr16));
   return METIS_OK;
 }
@@ -1049,20 +1074,26 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
   int64_t grid = (int64_t)sm_count() * (split_lines ? 2 : 3);
   if (grid > tiles) grid = tiles;
   if (out.records && grid > kDualMaxCtas) grid = kDualMaxCtas;
-  const TileWalk walk = {(uint32_t)tiles, (uint32_t)col_tiles, (uint32_t)(grid / col_tiles), (uint32_t)(grid % col_tiles)};
+  const uint32_t bpr = (uint32_t)(cols >> 4), bpc = (uint32_t)(rows >> 4), step_rows = (uint32_t)(grid / col_tiles), step_cols = (uint32_t)(grid % col_tiles);
+  const TileWalk walk = {(uint32_t)tiles, (uint32_t)col_tiles, step_rows, step_cols, bpr, bpc,
+                         step_rows * TC::kRows * bpr + step_cols * TC::kBlocksPerRow, TC::kRows * bpr - (uint32_t)col_tiles * TC::kBlocksPerRow,
+                         step_cols * TC::kCols * bpc + step_rows * TC::kRowBlocks, TC::kRowBlocks - (uint32_t)col_tiles * TC::kCols * bpc};
+  const PhiloxKeys keys(seed);
+  const bool plain = !out.hadamard && !out.sr16;
   const bool with_rows = out.codes_r != nullptr, with_cols = out.codes_t != nullptr;
-#define METIS_LAUNCH_TILE(MEAN, SR, ROWS, COLS)                                                             \
+#define METIS_LAUNCH_TILE(MEAN, SR, ROWS, COLS, PLAIN)                                                      \
   do {                                                                                                      \
-    auto kern = quantize_tile_kernel<T, MEAN, SR, ROWS, COLS>;                                              \
+    auto kern = quantize_tile_kernel<T, MEAN, SR, ROWS, COLS, PLAIN>;                                       \
     METIS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC::kSmemBytes)); \
     METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)grid), dim3(kQuantThreads), TC::kSmemBytes, st, map, walk, rows, cols, \
-                                    mean, seed, offset, ctr, out));                                         \
+                                    mean, keys, offset, ctr, out));                                         \
   } while (0)
-#define METIS_LAUNCH_TILE_MS(MEAN, SR)                                  \
-  do {                                                                  \
-    if (with_rows && with_cols) METIS_LAUNCH_TILE(MEAN, SR, true, true); \
-    else if (with_cols) METIS_LAUNCH_TILE(MEAN, SR, false, true);       \
-    else METIS_LAUNCH_TILE(MEAN, SR, true, false);                      \
+#define METIS_LAUNCH_TILE_MS(MEAN, SR)                                                                      \
+  do {                                                                                                      \
+    if (with_rows && with_cols) { if (plain) METIS_LAUNCH_TILE(MEAN, SR, true, true, true); else METIS_LAUNCH_TILE(MEAN, SR, true, true, false); } \
+    else if (with_cols) { if (plain) METIS_LAUNCH_TILE(MEAN, SR, false, true, true); else METIS_LAUNCH_TILE(MEAN, SR, false, true, false); } \
+    else if (plain || !SR) METIS_LAUNCH_TILE(MEAN, SR, true, false, true);                                  \
+    else METIS_LAUNCH_TILE(MEAN, SR, true, false, !SR);                                                     \
   } while (0)
   if (mean) { if (sr) METIS_LAUNCH_TILE_MS(true, true); else METIS_LAUNCH_TILE_MS(true, false); }
   else      { if (sr) METIS_LAUNCH_TILE_MS(false, true); else METIS_LAUNCH_TILE_MS(false, false); }

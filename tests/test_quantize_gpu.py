@@ -107,6 +107,19 @@ def test_one_launch_path_for_small_tensors(rows, cols, dtype, layout):
         assert_packed_equal(q, x.float().numpy(), layout, mean=mean.numpy(), what=f"small centred {rows}x{cols}")
 
 
+# Tiles of 128 rows x 64 (bf16) or 32 (fp32) columns: whole ones take a path without tests of edges.  One tile, one block more and
+# one less in either direction, and enough of them that a CTA walks over whole ones and an edge; with a mean, which the edge's
+# missing rows must not bring into the unit.
+@pytest.mark.parametrize("rows,cols", [(128, 64), (112, 64), (128, 48), (144, 80), (16, 16), (8336, 2128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_whole_tiles_and_edges_of_both_orientations(rows, cols, dtype):
+    x = synthetic(rows, cols, "normal", seed=rows + cols, dtype=dtype)
+    mean = x.float().mean(0) + 3.0
+    q, qt = ops.nvfp4_quantize_dual(x.to(DEV), mean=mean.to(DEV))
+    assert_packed_equal(q, x.float().numpy(), cabi.SF_MMA, mean=mean.numpy(), what="rows")
+    assert_packed_equal(qt, np.ascontiguousarray((x.float().numpy() - mean.numpy()[None, :]).T), cabi.SF_MMA, what="columns")
+
+
 # Largest maxima that put other maxima of a bf16 tensor exactly on an E4M3 tie of the scale pass (19968 does with 117), and
 # one so large that most scales are E4M3 subnormals or zero; whole pieces of the tiled layout and edges of it.
 @pytest.mark.parametrize("rows,cols", [(256, 4096), (300, 4112)])
