@@ -6,6 +6,7 @@
 // lanes form a 16-element block exactly as in the stand-alone quantizer.  The E4M3 scale
 // bytes are produced by the shared finalisation pass (they need the tensor-wide maximum).
 #include "common.cuh"
+#include "tma.cuh"
 
 namespace metis {
 
@@ -217,20 +218,21 @@ __device__ __forceinline__ float norm_block(const float (&v)[16], float rs, cons
 
 // ---- long inputs, bf16 rows of up to 4096 elements: a warp per row --------------------------------------------
 // With a CTA per row two barriers stand between its parts (3.1 of 10.5 stalled warps waited there, issue slots 66 % busy,
-// 18 instructions per element).  A warp that owns its row needs none: the row stays in registers as loaded
-// (kM blocks of 16 elements per lane, block lane + 32 j), the sum of squares goes through shuffles.  The sums are added
-// in the order of the CTA-per-row kernel (16 squares of a block one after the other, lanes by butterfly, then the groups
-// of 32 blocks in order), so the results are its results; two blocks' chains share one packed instruction.  Measured at
-// 65536 x 3584 this pass 172 -> 150 us, 65536 x 1536 80 -> 64, 2048 x 2048 6.8 -> 4.8.  Loads that leave L2 first (to keep
-// the block maxima there for the scale pass) change nothing here and cost the tile kernels of quantize.cu 20 %; a prefetch
-// of the next row into L2 changes nothing either.
-constexpr int kNormRowThreads = 256;
+// 18 instructions per element).  A warp that owns its row needs none: the sum of squares goes through shuffles.  The sums are
+// added in the order of the CTA-per-row kernel (16 squares of a block one after the other, lanes by butterfly, then the groups
+// of 32 blocks in order), so the results are its results.  Loads that leave L2 first (to keep the block maxima there for the
+// scale pass) change nothing here and cost the tile kernels of quantize.cu 20 %; a prefetch of the next row into L2 changes
+// nothing either.
 // Fewer rows do not fill the SMs with a warp each (both launches, a CTA / a warp per row, us): 896 x 4096 7.6 / 9.2, 640 x 3584
 // 6.5 / 8.3, 640 x 2048 7.0 / 7.5, 800 x 2048 6.0 / 6.1; equal from 1024 x 3584 (9.5 / 9.6) on, and rows of 512 elements do not
 // care (896: 4.9 / 4.5).
 constexpr int64_t kNormRowsMinRows = 1024;
+
+// Narrow rows: the row stays in registers as loaded (kM blocks of 16 elements per lane, block lane + 32 j); two blocks' chains
+// of squares share one packed instruction.
+constexpr int kNormRowThreads = 256;
 template <typename TG, int kM, bool kWriteNorm>
-__global__ void __launch_bounds__(kNormRowThreads, kM <= 3 ? 3 : 2)
+__global__ void __launch_bounds__(kNormRowThreads, 3)
 rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
                              const TG* __restrict__ gamma, float eps, uint2* __restrict__ codes,
                              float* __restrict__ amax_out, unsigned int* __restrict__ gmax,
@@ -321,6 +323,212 @@ rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int 
     records[3 * blockIdx.x] = m;
     records[3 * blockIdx.x + 1] = 0u;
     records[3 * blockIdx.x + 2] = 0u;
+    if (blockIdx.x == 0) records[-1] = gridDim.x;
+  }
+}
+
+// Wider ones: one CTA per SM, whose lanes 0 fetch a warp's row into its part of shared memory by one bulk copy, and the next one
+// as soon as the row has been read for the second time.  (In registers such a row takes 128 of them a thread, which leaves 16
+// warps per SM, and a quarter of their time they waited for its loads.)  First reading: the sum of squares, by the
+// multiply-add that takes bf16 operands.  Second: norm and quantization, block by block, in 64 registers.  The butterflies of
+// the groups of 32 blocks share their shuffles.  Rows of whole 64-element groups are fetched with the 128-byte swizzle (one
+// box of 64 x cols/64), which keeps both readings free of bank conflicts; others as they lie, at two wavefronts for one.
+// Bound by issue (190 instructions per block of 16, 65 % of the slots) and close to memory.  Both launches, row in registers /
+// in shared memory, us: 65536 x 4096 191 / 150, x 3584 165 / 134, x 2048 101 / 78, x 1536 73 / 61, x 1024 52 / 44, 16384 x 3584
+// 45 / 40, 1024 x 4096 9.4 / 7.8.  Narrow rows gain less, and few of them lose what setting the copies up costs (x 1024: 1024
+// 5.3 / 5.5, 8192 9.6 / 10.1, 16384 17.7 / 16.8; x 768: 2048 6.0 / 6.3, 16384 17.5 / 16.0; x 512: 2048 4.8 / 5.2, 16384
+// 10.0 / 11.0, 65536 30.1 / 29.6), so up to 512 columns stay with the registers, and up to 1024 with fewer than 16384 rows.
+static bool norm_rows_staged(int64_t rows, int64_t blocks_per_row) { return blocks_per_row > 64 || (blocks_per_row > 32 && rows >= 16384); }
+constexpr int64_t kNormStagedSmem = 232448 - 2048;       // of a CTA for rows: less 1 KiB for the static part and 1 KiB for aligning
+constexpr int kNormStagedMaxWarps = 32;
+// acc + lo^2 + hi^2 for the two bf16 of a word, one rounding each
+__device__ __forceinline__ float add_squares(uint32_t w, float acc) {
+  asm("{ .reg .b16 l, h; mov.b32 {l, h}, %1; fma.rn.f32.bf16 %0, l, l, %0; fma.rn.f32.bf16 %0, h, h, %0; }" : "+f"(acc) : "r"(w));
+  return acc;
+}
+__device__ __forceinline__ uint4 norm_lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+// Sums over the 32 lanes of kN values (a power of two, at most 8) at once, each in the order of a butterfly over lane
+// distances 16, 8, 4, 2, 1: while there are several values a lane hands half of them to its partner and goes on with the other
+// half.  Value j ends up in the lanes whose upper bits are j (total_of picks it).
+template <int kN>
+__device__ __forceinline__ float butterfly_sums(float (&v)[kN], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int n = kN / 2; n >= 1; n >>= 1, o >>= 1) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + n], o);
+      v[i] = (upper ? v[i + n] : v[i]) + other;
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+template <typename TG, int kM, bool kWriteNorm>
+__global__ void __launch_bounds__(kNormStagedMaxWarps * 32, 1)
+rmsnorm_quantize_staged_kernel(const __grid_constant__ CUtensorMap map_x, const __nv_bfloat16* __restrict__ x, int rows, int blocks_per_row,
+                             int64_t ld, const TG* __restrict__ gamma, float eps, uint2* __restrict__ codes,
+                             float* __restrict__ amax_out, unsigned int* __restrict__ gmax,
+                             unsigned int* __restrict__ records, void* __restrict__ norm_out, int swizzled, int bufs) {
+  constexpr bool kProductBf16 = sizeof(TG) == 2;
+  constexpr int kPow = kM <= 1 ? 1 : kM <= 2 ? 2 : kM <= 4 ? 4 : 8;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full[2 * kNormStagedMaxWarps];
+  __shared__ unsigned s_top[kNormStagedMaxWarps];
+  __shared__ int s_failed[kNormStagedMaxWarps];             // by warp: gave up waiting for a row
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t row_bytes = (uint32_t)blocks_per_row * 32u, pitch = (row_bytes + 1023u) & ~1023u;
+  const uint32_t s_gamma = base, mine = base + (kProductBf16 ? pitch : 0u) + (uint32_t)(warp * bufs) * pitch;
+  uint64_t* my_full = full + 2 * warp;
+  if (lane == 0) {
+    for (int b = 0; b < bufs; ++b) mbar_init(&my_full[b], 1);
+    s_failed[warp] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  grid_dependency_wait();
+  __syncwarp();
+  const int row_step = gridDim.x * warps;
+  const int r_first = blockIdx.x * warps + warp;
+  auto fetch = [&](int r, int b) {                        // lane 0
+    mbar_expect_tx(&my_full[b], row_bytes);
+    if (swizzled) tma_load_3d_addr(mine + b * pitch, &map_x, 0, 0, r, smem_u32(&my_full[b]));
+    else          bulk_load_addr(mine + b * pitch, x + (int64_t)r * ld, row_bytes, smem_u32(&my_full[b]));
+  };
+  if (lane == 0) {
+    for (int b = 0; b < bufs; ++b) if (r_first + b * row_step < rows) fetch(r_first + b * row_step, b);
+  }
+  // gamma as 16-byte pieces, piece c of each 128-byte group g at c ^ (g & 7); the barrier behind it stands after the first sum
+  if constexpr (kProductBf16) {
+    for (int p = threadIdx.x; p < 2 * blocks_per_row; p += blockDim.x) {
+      const uint4 w = __ldg(reinterpret_cast<const uint4*>(gamma) + p);
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_gamma + (uint32_t)((p & ~7) | ((p ^ (p >> 3)) & 7)) * 16u), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+    }
+  }
+  bool gamma_there = !kProductBf16;
+  // this lane's pieces of group of 32 blocks j: at these offsets + 1024 j
+  const uint32_t group = (uint32_t)lane >> 2, swz0 = group * 128u + (((2u * (lane & 3u)) ^ (group & 7u)) << 4), swz1 = swz0 ^ 16u;
+  const uint32_t x0 = swizzled ? swz0 : (uint32_t)lane * 32u, x1 = swizzled ? swz1 : (uint32_t)lane * 32u + 16u;
+  const float n_cols = (float)(blocks_per_row * 16);
+  const bool last_live = lane + 32 * (kM - 1) < blocks_per_row;     // of the lane's kM blocks only the last may be missing
+  float running = 0.0f;
+  volatile int* failed = &s_failed[warp];
+  int b = 0;
+  uint32_t parity = 0;
+  bool gave_up = false;
+  for (int r = r_first; r < rows; r += row_step) {
+    const uint32_t row = mine + b * pitch;
+    if (!__all_sync(0xffffffffu, mbar_wait(&my_full[b], parity, failed))) {
+      gave_up = true;
+      break;
+    }
+    float ss[kPow];
+#pragma unroll
+    for (int j = 0; j < kPow; ++j) {
+      ss[j] = 0.0f;
+      if (j < kM - 1 || (j == kM - 1 && last_live)) {
+        const uint4 p = norm_lds128(row + x0 + 1024 * j), q = norm_lds128(row + x1 + 1024 * j);
+        const uint32_t w[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss[j] = add_squares(w[i], ss[j]);
+      }
+    }
+    const float sums = butterfly_sums<kPow>(ss, lane);
+    float tot = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kM; ++j) tot += __shfl_sync(0xffffffffu, sums, j * (32 / kPow));
+    const float rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, n_cols), eps)));   // llama.py:23-24
+    const f32x2 rs2 = pack2(rs, rs);
+    if (!gamma_there) {                                    // uniform over the CTA: every warp comes here or to the same barrier below
+      __syncthreads();
+      gamma_there = true;
+    }
+    const int64_t row_blk = (int64_t)r * blocks_per_row + lane;
+    uint2* row_codes = codes + row_blk;
+    float* row_amax = amax_out + row_blk;
+#pragma unroll
+    for (int j = 0; j < kM; ++j) {
+      if (j == kM - 1 && !last_live) break;
+      RawBlock<__nv_bfloat16> raw;
+      raw.a = norm_lds128(row + x0 + 1024 * j);
+      raw.b = norm_lds128(row + x1 + 1024 * j);
+      float v[16], y[16];
+      raw.unpack(v);
+      float a;
+      if constexpr (kProductBf16) {
+        const uint4 g0 = norm_lds128(s_gamma + swz0 + 1024 * j), g1 = norm_lds128(s_gamma + swz1 + 1024 * j);
+        const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {                     // both roundings of the reference, see rmsnorm_quantize_kernel
+          float n0, n1;
+          split2(mul2(pack2(v[2 * i], v[2 * i + 1]), rs2), n0, n1);
+          const __nv_bfloat162 n2 = __floats2bfloat162_rn(n0, n1);
+          const __nv_bfloat162 p2 = __hmul2(n2, *reinterpret_cast<const __nv_bfloat162*>(&gw[i]));
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
+          y[2 * i] = bf16_lo(w);
+          y[2 * i + 1] = bf16_hi(w);
+        }
+        a = abs_max16(y);
+      } else {
+        a = norm_block<__nv_bfloat16, TG>(v, rs, gamma + (lane + 32 * j) * 16, y);
+      }
+      uint32_t packed[2];
+      quantize_rn<2>(y, block_scale_from_amax(a), packed);
+      row_codes[32 * j] = make_uint2(packed[0], packed[1]);
+      row_amax[32 * j] = a;
+      running = fmaxf(running, a);
+      if (kWriteNorm) {
+        if (kProductBf16) {
+          __nv_bfloat162 o[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);   // exact: already bf16 values
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(norm_out) + (row_blk + 32 * j) * 16);
+          dst[0] = reinterpret_cast<uint4*>(o)[0];
+          dst[1] = reinterpret_cast<uint4*>(o)[1];
+        } else {
+          float4* dst = reinterpret_cast<float4*>(static_cast<float*>(norm_out) + (row_blk + 32 * j) * 16);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) dst[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+        }
+      }
+    }
+    __syncwarp();                                          // every lane has read the row: its place takes another one
+    const int next = r + bufs * row_step;
+    if (lane == 0 && next < rows) fetch(next, b);
+    if (++b == bufs) { b = 0; parity ^= 1u; }
+  }
+  if (!gamma_there) __syncthreads();
+  if (gave_up && lane == 0) {
+    *failed = 1;
+    if (!records) gmax[1] = 1u;                            // error word: the scale pass publishes NaN as the unit
+    // copies of this warp may still be in flight: give each a bounded chance to land before the CTA leaves
+    for (int k = 0; k < bufs; ++k) {
+      const uint64_t t0 = global_ns();
+      while (!mbar_try(&my_full[b], parity) && global_ns() - t0 < kWaitLimitNs) {}
+      if (++b == bufs) { b = 0; parity ^= 1u; }
+    }
+  }
+  const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(running));       // >= 0: the bits order like the value
+  if (!records) {
+    if (lane == 0 && top > 0u) atomicMax(gmax, top);
+    return;
+  }
+  if (lane == 0) s_top[warp] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned m = 0u, bad = 0u;
+    for (int w = 0; w < warps; ++w) { m = max(m, s_top[w]); bad |= (unsigned)s_failed[w]; }
+    records[3 * blockIdx.x] = m;
+    records[3 * blockIdx.x + 1] = 0u;
+    records[3 * blockIdx.x + 2] = bad;
     if (blockIdx.x == 0) records[-1] = gridDim.x;
   }
 }
@@ -531,7 +739,7 @@ static int32_t launch_norm(const TX* x, int64_t rows, int bpr, int bx, int64_t l
   return METIS_OK;
 }
 
-// The warp-per-row kernel for [rows, 16 bpr] bf16, 32 <= bpr <= 256 (512 to 4096 columns).
+// The warp-per-row kernels for [rows, 16 bpr] bf16, 32 <= bpr <= 256 (512 to 4096 columns): the row in registers,
 template <typename TG, int kM>
 static int32_t launch_norm_rows(const __nv_bfloat16* x, int64_t rows, int bpr, int64_t ld, const TG* gamma, float eps, uint32_t* codes,
                                 const WorkspaceView& ws, unsigned int** records, void* norm_out, int sms, cudaStream_t st) {
@@ -543,6 +751,33 @@ static int32_t launch_norm_rows(const __nv_bfloat16* x, int64_t rows, int bpr, i
   if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
   METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)blocks), dim3(kNormRowThreads), 0, st, x, (int)rows, bpr, ld, gamma, eps,
                                   reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, *records, norm_out));
+  return METIS_OK;
+}
+
+// and in shared memory: a CTA per SM, as many warps as
+// rows fit its shared memory (twice as many rows where there is room), no more than it takes to go round the same number of times.
+template <typename TG, int kM>
+static int32_t launch_norm_staged(const __nv_bfloat16* x, int64_t rows, int bpr, int64_t ld, const TG* gamma, float eps, uint32_t* codes,
+                                const WorkspaceView& ws, unsigned int** records, void* norm_out, int sms, cudaStream_t st) {
+  auto kern = norm_out ? rmsnorm_quantize_staged_kernel<TG, kM, true> : rmsnorm_quantize_staged_kernel<TG, kM, false>;
+  const int64_t pitch = ceil_div((int64_t)bpr * 32, 1024) * 1024, room = kNormStagedSmem - (sizeof(TG) == 2 ? pitch : 0);
+  int64_t warps = room / pitch;
+  if (warps > kNormStagedMaxWarps) warps = kNormStagedMaxWarps;
+  const int64_t rounds = ceil_div(rows, sms * warps);
+  warps = ceil_div(rows, sms * rounds);
+  const int64_t bufs = rounds > 1 && 2 * warps * pitch <= room ? 2 : 1;
+  const int64_t blocks = ceil_div(rows, warps * rounds) < sms ? ceil_div(rows, warps * rounds) : sms;
+  if (blocks > kMaxRecords) *records = nullptr;
+  if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
+  const bool swizzled = bpr % 4 == 0 && ld % 64 == 0;        // whole 64-element groups, a row a whole number of them from the next
+  CUtensorMap map = {};
+  if (swizzled) {
+    if (int32_t rc = make_row_map(&map, x, bpr / 4, rows, ld * 2, "x")) return rc;
+  }
+  const size_t smem = (size_t)((sizeof(TG) == 2 ? pitch : 0) + warps * bufs * pitch + 1024);
+  METIS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kNormStagedSmem + 1024)));
+  METIS_CUDA_OK(launch_overlapped(kLaunchStream, kern, dim3((unsigned)blocks), dim3((unsigned)warps * 32), smem, st, map, x, (int)rows, bpr, ld, gamma, eps,
+                                  reinterpret_cast<uint2*>(codes), ws.amax, ws.gmax, *records, norm_out, swizzled ? 1 : 0, (int)bufs));
   return METIS_OK;
 }
 
@@ -565,11 +800,14 @@ static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t 
     // a warp per row from kNormRowsMinRows on, and where a CTA per row has more CTAs than there are records
     if (bpr >= 32 && bpr <= 256 &&
         (rows >= kNormRowsMinRows || (*records && norm_ctas<TX, TG, 1>(rows, bx, norm_out != nullptr, sms) > kMaxRecords))) {
+      if (!norm_rows_staged(rows, bpr))
+        return bpr <= 32 ? launch_norm_rows<TG, 1>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
+                         : launch_norm_rows<TG, 2>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
       switch ((bpr + 31) / 32) {
-#define METIS_NORM_ROWS(M) case M: return launch_norm_rows<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
-        METIS_NORM_ROWS(1); METIS_NORM_ROWS(2); METIS_NORM_ROWS(3); METIS_NORM_ROWS(4);
-        METIS_NORM_ROWS(5); METIS_NORM_ROWS(6); METIS_NORM_ROWS(7); METIS_NORM_ROWS(8);
-#undef METIS_NORM_ROWS
+#define METIS_NORM_STAGED(M) case M: return launch_norm_staged<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
+        METIS_NORM_STAGED(2); METIS_NORM_STAGED(3); METIS_NORM_STAGED(4); METIS_NORM_STAGED(5);
+        METIS_NORM_STAGED(6); METIS_NORM_STAGED(7); METIS_NORM_STAGED(8);
+#undef METIS_NORM_STAGED
       }
     }
   }

@@ -67,6 +67,10 @@ __device__ __forceinline__ void tma_load_2d_addr(uint32_t dst, const CUtensorMap
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_addr(uint32_t dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void bulk_load_addr(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -134,5 +138,18 @@ static inline int32_t make_map(CUtensorMap* map, CUtensorMapDataType dt, int64_t
   return METIS_OK;
 }
 
+// Rows of whole 128-byte groups as [rows, groups, 64] bf16, one row to a box, each group swizzled over 128 bytes.
+static inline int32_t make_row_map(CUtensorMap* map, const void* base, int64_t groups, int64_t rows, int64_t pitch_bytes, const char* what) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(METIS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const cuuint64_t dims[3] = {64, (cuuint64_t)groups, (cuuint64_t)rows};
+  const cuuint64_t strides[2] = {128, (cuuint64_t)pitch_bytes};
+  const cuuint32_t box[3] = {64, (cuuint32_t)groups, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(METIS_ERR_CUDA, "cuTensorMapEncodeTiled(%s) failed with %d", what, (int)r);
+  return METIS_OK;
+}
 
 }  // namespace metis

@@ -65,6 +65,29 @@ def test_bf16_rows(rows, cols, gdtype):
     assert mism < 2e-3
 
 
+# Rows in shared memory: rows of whole 64-element groups (fetched swizzled) and others, one or two places per warp and several
+# rounds, rows further apart than they are long, and values whose squares are subnormal, infinite or NaN.  Every row has the bits that the
+# CTA-per-row kernel gives it in a call of 500 rows.
+@pytest.mark.parametrize("rows,cols,gap", [(16384, 1040, 0), (16397, 1024, 0), (9600, 1536, 8), (9500, 1536, 64), (5000, 4096, 0), (4900, 3568, 0), (1024, 2064, 24)])
+@pytest.mark.parametrize("gdtype", [torch.bfloat16, torch.float32])
+def test_rows_staged_in_shared_memory(rows, cols, gap, gdtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    wide = torch.randn(rows, cols + gap, generator=g, device=DEV).to(torch.bfloat16)
+    x = wide[:, :cols]
+    x[3] *= 1e-20
+    x[4] *= 1e-38
+    x[5, 7], x[6, 9] = float("inf"), float("nan")
+    gamma = (1.0 + 0.1 * torch.randn(cols, generator=g, device=DEV)).to(gdtype)
+    _, y = ops.rmsnorm_nvfp4_quantize(x, gamma, 1e-6, return_norm=True)
+    for r in list(range(0, rows - 500, 3100)) + [rows - 500]:
+        _, want = ops.rmsnorm_nvfp4_quantize(x[r:r + 500], gamma, 1e-6, return_norm=True)
+        same = torch.equal(y[r:r + 500].view(torch.int16 if y.dtype == torch.bfloat16 else torch.int32), want.view(torch.int16 if y.dtype == torch.bfloat16 else torch.int32))
+        assert same, (rows, cols, r)
+    q, y = ops.rmsnorm_nvfp4_quantize(x[8:], gamma, 1e-6, return_norm=True)
+    again = ops.nvfp4_quantize(y)                         # the quantizer's own tests compare it with the oracle
+    assert torch.equal(q.codes, again.codes) and torch.equal(q.scales, again.scales) and torch.equal(q.unit, again.unit)
+
+
 # The warp-per-row kernel: every number of blocks per lane, rows that end inside a round of 32 blocks and inside a CTA's
 # eight rows, and fewer than 1024 rows where a CTA per row would leave more records than there is room for (whether it
 # would depends on the type of gamma; both kernels have to pass).
