@@ -29,7 +29,6 @@ constexpr int kDebugNoMma = 2;
 constexpr int kDebugNoLoad = 4;
 constexpr int kDebugNoEpilogue = 16;     // accumulator chunks are read and dropped
 constexpr int kDebugNoStore = 32;        // everything but the global stores of the epilogue
-constexpr int kDebugLsuStore = 64;       // pair kernel: store D with ordinary store instructions instead of TMA
 constexpr int kDebugProfile = 128;       // pair kernel: CTA 0's issuer writes its cycle counts to status[2..6]
 constexpr int kDebugNoScaleCopy = 0x10000;   // pair kernel: the MMAs read whatever tensor memory holds as scales
 constexpr int kDebugGroupMask = 0xFF00;  // pair kernel: row tiles per band of the tile order (0 = the default)
@@ -38,14 +37,13 @@ constexpr int kDebugNoMma = 0;
 constexpr int kDebugNoLoad = 0;
 constexpr int kDebugNoEpilogue = 0;
 constexpr int kDebugNoStore = 0;
-constexpr int kDebugLsuStore = 0;
 constexpr int kDebugProfile = 0;
 constexpr int kDebugNoScaleCopy = 0;
 constexpr int kDebugGroupMask = 0;
 #endif
 // run the single-CTA kernel where the CTA-pair kernel would be chosen (tests cover both)
 constexpr int kDebugSingleCta = 8;
-constexpr int kDebugMask = kDebugDropFirstSfa | kDebugNoMma | kDebugNoLoad | kDebugSingleCta | kDebugNoEpilogue | kDebugNoStore | kDebugLsuStore | kDebugGroupMask | kDebugProfile | kDebugNoScaleCopy;
+constexpr int kDebugMask = kDebugDropFirstSfa | kDebugNoMma | kDebugNoLoad | kDebugSingleCta | kDebugNoEpilogue | kDebugNoStore | kDebugGroupMask | kDebugProfile | kDebugNoScaleCopy;
 
 template <int BN> struct GemmCfg {
   static constexpr int kStages = (BN == 256) ? 4 : 6;
@@ -184,13 +182,13 @@ __device__ __forceinline__ void report(int32_t* status, volatile int* abort_flag
 
 template <typename TD> struct EpilogueCtx {
   const GemmParams* p;
-  uint8_t* staging;      // 2 KiB of shared memory owned by this warp
+  uint8_t* staging;      // shared memory owned by this warp: buffers of 2 KiB
   int64_t row0;          // first of the warp's 32 rows; lane l holds row0 + l
   float g, c0, c1;
   float* partial = nullptr;   // split-K: raw fp32 partial sums [M, ldp] of this split go here instead of D
   int64_t ldp = 0;
   const CUtensorMap* dmap = nullptr;   // D as [M, N] with 32-row x 64-byte boxes, 64-byte swizzle: stores go through the TMA unit
-  uint32_t flip = 0;                   //   and `staging` is then two buffers of 2 KiB used in turn
+  uint32_t flip = 0;                   //   from the buffers in turn
 };
 
 // v[i] += c * rvec[col0 + i] for the 32 columns of a chunk (128-bit loads when the chunk is whole
@@ -200,13 +198,12 @@ __device__ __forceinline__ void add_rank1(float (&v)[32], const float* __restric
   if (!rvec) return;
   if (full_chunk && (reinterpret_cast<uintptr_t>(rvec) & 15u) == 0) {
     const float4* r4 = reinterpret_cast<const float4*>(rvec + col0);
+    const f32x2 c2 = pack2(c, c);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float4 f = __ldg(r4 + i);
-      v[4 * i] = fmaf(c, f.x, v[4 * i]);
-      v[4 * i + 1] = fmaf(c, f.y, v[4 * i + 1]);
-      v[4 * i + 2] = fmaf(c, f.z, v[4 * i + 2]);
-      v[4 * i + 3] = fmaf(c, f.w, v[4 * i + 3]);
+      split2(fma2(c2, pack2(f.x, f.y), pack2(v[4 * i], v[4 * i + 1])), v[4 * i], v[4 * i + 1]);
+      split2(fma2(c2, pack2(f.z, f.w), pack2(v[4 * i + 2], v[4 * i + 3])), v[4 * i + 2], v[4 * i + 3]);
     }
   } else {
 #pragma unroll
@@ -248,11 +245,11 @@ __device__ __forceinline__ void add_c(float (&v)[32], const TD* __restrict__ src
 // through shared memory: 64-byte rows, 16-byte pieces XOR-swizzled by the row (the 64-byte swizzle
 // pattern of the tensor maps), so that neither side has bank conflicts.
 //   with a tensor map of D (ctx.dmap): lane 0 hands each 32 x 64-byte piece to the TMA unit, which
-//     clips it at the edges of D.  The warp owns two such buffers and waits, before it refills one,
-//     until the store issued from it two pieces ago has read it; the stores never pass through
+//     clips it at the edges of D.  The warp owns kBuffers such buffers and waits, before it refills one,
+//     until the store issued from it has read it; the stores never pass through
 //     the load/store unit, which the operand feed of the tensor core needs
 //   without: every store instruction writes 64 contiguous bytes of 8 rows
-template <typename TD>
+template <typename TD, int kBuffers = 1>
 __device__ __forceinline__ void emit_chunk(EpilogueCtx<TD>& ctx, const uint32_t (&r)[32], int64_t col0) {
   const GemmParams& p = *ctx.p;
   const int lane = threadIdx.x & 31;
@@ -270,8 +267,9 @@ __device__ __forceinline__ void emit_chunk(EpilogueCtx<TD>& ctx, const uint32_t 
     return;
   }
   float v[32];
+  const f32x2 g2 = pack2(ctx.g, ctx.g);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ctx.g;
+  for (int i = 0; i < 32; i += 2) split2(mul2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), g2), v[i], v[i + 1]);
   const bool full_chunk = col0 + 32 <= p.N;
   add_rank1(v, p.rvec0, ctx.c0, col0, p.N, full_chunk);
   add_rank1(v, p.rvec1, ctx.c1, col0, p.N, full_chunk);
@@ -283,8 +281,8 @@ __device__ __forceinline__ void emit_chunk(EpilogueCtx<TD>& ctx, const uint32_t 
 #pragma unroll
     for (int h = 0; h < kPieces; ++h) {
       uint8_t* buf = ctx.staging + ctx.flip * 2048;
-      ctx.flip ^= 1u;
-      if (lane == 0) bulk_store_wait_read<1>();
+      if (kBuffers == 2) ctx.flip ^= 1u;
+      if (lane == 0) bulk_store_wait_read<kBuffers - 1>();
       __syncwarp();
 #pragma unroll
       for (int k = 0; k < 4; ++k) {

@@ -7,15 +7,16 @@
 // instead of the 54 KiB of the single-CTA kernel, for the same 512 tensor-pipe cycles: the operand
 // feed (L2 -> shared memory, and shared memory -> tensor core) is what bounds the single-CTA kernel.
 //
-// Roles per CTA (320 threads): warp 0 TMA producer, warp 1 tensor-core issuer (leader only),
-// warps 2-9 epilogue (two warps per 32-lane quarter of tensor memory, alternate column chunks).  The scale tiles travel shared memory -> tensor memory by tcgen05.cp issued
+// Roles per CTA (320 or 576 threads): warp 0 TMA producer, warp 1 tensor-core issuer (leader only),
+// warps 2-9 or 2-17 epilogue (two or four warps per 32-lane quarter of tensor memory, alternate column chunks;
+// epilogue_parts has the rule).  The scale tiles travel shared memory -> tensor memory by tcgen05.cp issued
 // by the leader in front of each stage's MMAs: one instruction copies in both CTAs, in pipe order
 // with the MMAs, so no cross-SM handshake sits inside the pipeline loop (a handshake through the
 // peer costs a cluster round trip of more than a thousand cycles per two stages).
 //   full[s]      leader's: all bytes of stage s of BOTH CTAs (the peer's TMA loads signal it remotely)
 //   empty[s]     local: stage s consumed (commit multicast by the leader to both CTAs)
 //   acc_full     local: accumulator complete (commit multicast)
-//   acc_release  leader's: 16 epilogue warps (8 remote arrivals) have drained the shared accumulator columns
+//   acc_release  leader's: the epilogue warps of both CTAs that read shared accumulator columns have drained them
 // No copy is multicast.  Every wait is bounded; both CTAs meet at a cluster barrier before they
 // free tensor memory, so neither exits while the other can still signal or read it.
 #include "gemm_common.cuh"
@@ -32,9 +33,9 @@ struct PairCfg {
   static constexpr int kSfaBytes = 4 * 512;               // scales of this CTA's rows of A
   static constexpr int kSfbBytes = 2 * 4 * 512;           // scales of all 256 rows of B
   static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;   // 38 KiB
-  static constexpr int kStagingBytes = 8 * 4096;           // epilogue: two buffers of 32 rows x 64 bytes for each of 8 warps
+  static constexpr int kStagingBytes = 16 * 2048;          // epilogue: 16 buffers of 32 rows x 64 bytes, two for each of 8 warps or one for each of 16
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
-  static constexpr int kThreads = 320;
+  static constexpr int threads(int parts) { return 64 + 128 * parts; }
 };
 
 // ---- cluster plumbing ------------------------------------------------------------------------------------
@@ -111,8 +112,9 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d, uint32_t a_lo, uint
 
 // ---- the kernel ---------------------------------------------------------------------------------------
 
-template <typename TD>
-__global__ void __launch_bounds__(PairCfg::kThreads, 1)
+// kParts: epilogue warps per 32-lane quarter, 2 or 4
+template <typename TD, int kParts>
+__global__ void __launch_bounds__(PairCfg::threads(kParts), 1)
 nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
                        const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_u,
@@ -120,6 +122,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   using Cfg = PairCfg;
   constexpr int kStages = Cfg::kStages;
   constexpr int BN = Cfg::BN;
+  constexpr int kReleasing = kParts < Cfg::kSharedChunks ? kParts : Cfg::kSharedChunks;     // warps of a quarter that read shared columns
 
   extern __shared__ uint8_t smem_raw[];
   // the dynamic window starts at the same offset in both CTAs, so this rounding gives both the
@@ -155,7 +158,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
-    mbar_init(acc_release, 16);
+    mbar_init(acc_release, 2 * 4 * kReleasing);
     mbar_init(drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -334,16 +337,16 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       __syncwarp();
     }
   } else {
-    // ===== epilogue (both CTAs): warps 2..9; warp w owns tensor-memory lanes 32*(w%4) .. +31 and,
-    // of the 8 column chunks taken in drain order, those with index (w-2)/4, +2, +4, +6 =====
+    // ===== epilogue (both CTAs): warps 2 and up; warp w owns tensor-memory lanes 32*(w%4) .. +31 and,
+    // of the 8 column chunks taken in drain order, those with index (w-2)/4, + kParts, ... =====
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int part = (warp - 2) >> 2;
     const uint32_t release_leader = map_to_cta(smem_u32(acc_release), 0);
     EpilogueCtx<TD> ctx;
     ctx.g = p.alpha * __ldg(p.a_unit) * __ldg(p.b_unit);
     ctx.p = &p;
-    ctx.staging = staging + (warp - 2) * 4096;
-    ctx.dmap = (p.debug & kDebugLsuStore) ? nullptr : &map_d;
+    ctx.staging = staging + (warp - 2) * (8192 / kParts);
+    ctx.dmap = &map_d;
     uint32_t local_tile = 0;
     for (int64_t tile = pair; tile < num_tiles; tile += num_pairs, ++local_tile) {
       int64_t tm, tn;
@@ -365,28 +368,42 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       // accumulator [0,256) they are its last chunks, for the odd one [160,416) its first ones.
       constexpr int kChunks = BN / 32;
       const int first_chunk = !odd ? kChunks - Cfg::kSharedChunks : 0;
-      int ch[4];
+      int ch[kChunks / kParts];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) ch[k] = (first_chunk + half + 2 * k) & (kChunks - 1);
-      // this warp's first two chunks cover its part of the shared columns (drain index 0 and 2,
-      // or 1): pull them into registers and hand the columns to the next tile's MMAs at once
-      uint32_t ra[32], rb[32];
-      tc_load32(t_row + ch[0] * 32, ra);
-      tc_load32(t_row + ch[1] * 32, rb);
-      tc_wait_ld(ra);
-      tc_wait_ld(rb);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(release_leader);
-      // the other two loads fly while the first two chunks are scaled and stored
-      emit_chunk<TD>(ctx, ra, n0 + ch[0] * 32);
-      tc_load32(t_row + ch[2] * 32, ra);
-      emit_chunk<TD>(ctx, rb, n0 + ch[1] * 32);
-      tc_load32(t_row + ch[3] * 32, rb);
-      tc_wait_ld(ra);
-      tc_wait_ld(rb);
-      emit_chunk<TD>(ctx, ra, n0 + ch[2] * 32);
-      emit_chunk<TD>(ctx, rb, n0 + ch[3] * 32);
+      for (int k = 0; k < kChunks / kParts; ++k) ch[k] = (first_chunk + part + kParts * k) & (kChunks - 1);
+      // this warp's first chunks cover its part of the shared columns (drain index 0 and 2 or 1; 0, 1 or 2):
+      // pull them into registers and hand the columns to the next tile's MMAs at once
+      constexpr int kBuffers = 4 / kParts;
+      uint32_t ra[32];
+      if constexpr (kParts == 2) {
+        uint32_t rb[32];
+        tc_load32(t_row + ch[0] * 32, ra);
+        tc_load32(t_row + ch[1] * 32, rb);
+        tc_wait_ld(ra);
+        tc_wait_ld(rb);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(release_leader);
+        // the other two loads fly while the first two chunks are scaled and stored
+        emit_chunk<TD, kBuffers>(ctx, ra, n0 + ch[0] * 32);
+        tc_load32(t_row + ch[2] * 32, ra);
+        emit_chunk<TD, kBuffers>(ctx, rb, n0 + ch[1] * 32);
+        tc_load32(t_row + ch[3] * 32, rb);
+        tc_wait_ld(ra);
+        tc_wait_ld(rb);
+        emit_chunk<TD, kBuffers>(ctx, ra, n0 + ch[2] * 32);
+        emit_chunk<TD, kBuffers>(ctx, rb, n0 + ch[3] * 32);
+      } else {
+        tc_load32(t_row + ch[0] * 32, ra);
+        tc_wait_ld(ra);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0 && part < kReleasing) mbar_arrive_cluster(release_leader);
+        emit_chunk<TD, kBuffers>(ctx, ra, n0 + ch[0] * 32);
+        tc_load32(t_row + ch[1] * 32, ra);
+        tc_wait_ld(ra);
+        emit_chunk<TD, kBuffers>(ctx, ra, n0 + ch[1] * 32);
+      }
       tc_fence_before();
     }
     if (lane == 0) bulk_store_wait_all();                    // shared memory stays until the TMA unit has read it
@@ -403,19 +420,25 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
 // ---- host side ----------------------------------------------------------------------------------------------
 
-template <typename TD>
-static int32_t launch_pair_t(const metis_gemm_args* a, const CUtensorMap* maps, const GemmParams& p) {
-  auto kern = nvfp4_gemm_pair_kernel<TD>;
+// Epilogue warps per lane quarter.  Four of them take half the time for a tile, which is what bounds short products (a tile
+// of 8192 x 8192 x 512: 3.3 -> 2.9 us, with a row vector 4.6 -> 3.4) and the last tile of every product.  With a row vector
+// (rvec0) and many rounds of long tiles two are faster: the vector's broadcast loads take shared-memory bandwidth that the
+// operands need, and four warps ask for it while the next tile starts.  Two / four, us: without one 8192 x 8192 x 1024
+// 51.1 / 48.4, x 2048 71.4 / 69.1, x 4096 114.2 / 112.9, 4096 x 14336 x 4096 128.2 / 124.9; with one 8192 x 8960 x 1536
+// 79.3 / 75.3, 1120 x 3584 x 3584 (one round) 14.2 / 13.0, 1024 x 18944 x 3584 (four) 36.9 / 36.5, but (14 to 16 rounds) 8192 x
+// 8192 x 2048 78.0 / 80.4, x 4096 122.9 / 127.2, 4096 x 18944 x 3584 131.5 / 135.6.
+static int epilogue_parts(const GemmParams& p, int64_t rounds) {
+  const int64_t stages = ceil_div(p.K, 256) + ceil_div(p.rank, 64);
+  return p.rvec0 && stages >= 10 && rounds > 4 ? 2 : 4;
+}
+
+template <typename TD, int kParts>
+static int32_t launch_pair_t(const metis_gemm_args* a, const CUtensorMap* maps, const GemmParams& p, int64_t pairs) {
+  auto kern = nvfp4_gemm_pair_kernel<TD, kParts>;
   METIS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kSmemBytes));
-  const int64_t tiles = ceil_div(a->M, 2 * kBM) * ceil_div(a->N, PairCfg::BN);
-  int64_t pairs = gemm_sm_budget(a->sm_limit) / 2;
-  if (pairs > tiles) pairs = tiles;
-  // the fewest pairs that still finish in the same number of rounds: 256 tiles take 4 rounds on 74 pairs
-  // and on 64, and the SMs left over are free for whatever runs beside this product
-  pairs = ceil_div(tiles, ceil_div(tiles, pairs));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-  cfg.blockDim = dim3(PairCfg::kThreads, 1, 1);
+  cfg.blockDim = dim3(PairCfg::threads(kParts), 1, 1);
   cfg.dynamicSmemBytes = PairCfg::kSmemBytes;
   cfg.stream = reinterpret_cast<cudaStream_t>(a->stream);
   cudaLaunchAttribute attr[2];
@@ -435,6 +458,14 @@ static int32_t launch_pair_t(const metis_gemm_args* a, const CUtensorMap* maps, 
 // of A and T), mb and mu too (this CTA's half of the 256 rows of B and U).
 int32_t launch_gemm_pair(const metis_gemm_args* a, const CUtensorMap& ma, const CUtensorMap& mb,
                          const CUtensorMap& mt, const CUtensorMap& mu, const GemmParams& p) {
+  const int64_t tiles = ceil_div(a->M, 2 * kBM) * ceil_div(a->N, PairCfg::BN);
+  int64_t pairs = gemm_sm_budget(a->sm_limit) / 2;
+  if (pairs > tiles) pairs = tiles;
+  // the fewest pairs that still finish in the same number of rounds: 256 tiles take 4 rounds on 74 pairs
+  // and on 64, and the SMs left over are free for whatever runs beside this product
+  const int64_t rounds = ceil_div(tiles, pairs);
+  pairs = ceil_div(tiles, rounds);
+  const bool four = epilogue_parts(p, rounds) == 4;
   // the scale arrays as [tiles, 512 bytes]: one box = the 4 tiles (2 KiB) of one stage and row block
   const int64_t sf_tiles_k = sf_tiles_per_row(a->K);
   CUtensorMap maps[7] = {ma, mb, {}, {}, mt, mu, {}};
@@ -445,10 +476,10 @@ int32_t launch_gemm_pair(const metis_gemm_args* a, const CUtensorMap& ma, const 
   // D in boxes of 32 rows x 64 bytes for the epilogue's TMA stores
   if (a->d_dtype == METIS_DTYPE_BF16) {
     if (int32_t rc = make_map(&maps[6], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->d, a->N, a->M, a->ldd * 2, 32, 32, "D", 64)) return rc;
-    return launch_pair_t<__nv_bfloat16>(a, maps, p);
+    return four ? launch_pair_t<__nv_bfloat16, 4>(a, maps, p, pairs) : launch_pair_t<__nv_bfloat16, 2>(a, maps, p, pairs);
   }
   if (int32_t rc = make_map(&maps[6], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d, a->N, a->M, a->ldd * 4, 16, 32, "D", 64)) return rc;
-  return launch_pair_t<float>(a, maps, p);
+  return four ? launch_pair_t<float, 4>(a, maps, p, pairs) : launch_pair_t<float, 2>(a, maps, p, pairs);
 }
 
 }  // namespace metis

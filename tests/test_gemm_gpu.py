@@ -63,6 +63,27 @@ def test_fused_low_rank_product(M, N, K, rank):
     assert rel_l2(got, want) <= 1e-5, rel_l2(got, want)
 
 
+# Two or four epilogue warps per lane quarter (pair kernel): with a row vector, ten pipeline stages and more than four rounds of
+# tiles two, else four.  Each side of the three lines, edges of D inside a 32-column chunk and a row block; few SMs give many rounds.
+@pytest.mark.parametrize("M,N,K,rank,row,sms", [(1300, 1096, 2560, 0, True, 8), (1300, 1096, 2304, 0, True, 8), (1300, 1096, 2304, 64, True, 8),
+                                                (1300, 1096, 2560, 0, False, 8), (1300, 1096, 2560, 0, True, 14), (1300, 1096, 2560, 0, True, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
+    qa, qb, da, db = operands(M, N, K, seed=K + rank)
+    g = torch.Generator(device=DEV).manual_seed(M + sms)
+    kw, want = dict(out_dtype=dtype, sm_limit=sms), O.gemm_reference(da, db).astype(np.float64)
+    if row:
+        v, w = (torch.randn(n, generator=g, device=DEV) for n in (N, M))
+        kw["rank1"] = ((None, v), (w, v))
+        want += (1 + w.double().cpu().numpy())[:, None] * v.double().cpu().numpy()[None, :]
+    if rank:
+        t, u = (torch.randn(n, rank, generator=g, device=DEV).to(torch.bfloat16) for n in (M, N))
+        kw["lowrank"] = (t, u)
+        want += float(qa.unit) * float(qb.unit) * (t.double() @ u.double().T).cpu().numpy()
+    got = run(qa, qb, **kw).float().cpu().numpy()
+    assert rel_l2(got, want) <= (1e-5 if dtype == torch.float32 else 2.0 ** -8)      # fp32 sums; one rounding to bf16
+
+
 # the projection shapes of the two decoder configurations (Qwen2-style 1.5B at rank 64, 7B at rank 128)
 DECODER_SHAPES = [(1536, 1536, 64), (256, 1536, 64), (8960, 1536, 64), (1536, 8960, 64),
                   (3584, 3584, 128), (512, 3584, 128), (18944, 3584, 128), (3584, 18944, 128)]
