@@ -150,6 +150,12 @@ __device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
   }
 }
 
+// eight floats by one 32-byte load
+__device__ __forceinline__ void load8_wide(const float* p, float* f) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p));
+}
+
 // The same product along the tiled scale layout.  A 16-byte piece of that layout holds the scales of the rows l, l + 32,
 // l + 64, l + 96 of a 128-row block for 4 blocks of 16 columns: a warp takes these four rows, lane k of it every 32nd block
 // from k on, so that one 16-byte read of scales (shared by four lanes) and the 16 floats of v (which stay in L1) serve
@@ -158,13 +164,17 @@ __device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
 // The additions are those of the other kernels, in the same order: 16 products of a block one after the other, a lane's
 // blocks one after the other, then the lanes pairwise, so which kernel runs does not show in the result (a sum that
 // differs in its last bit can flip the rounding of an activation, and a block of decoder layers makes 1 % of that).
-// Bound by issue and by the conversions (two codes become two halves with one, exactly): 18944 x 3584 takes 13.5 us, its
-// bytes 6.  Against the kernel it replaced there, six weights in turn, us: 18944 x 3584 20.5 -> 13.5, 3584 x 18944
-// 23.6 -> 17.4, 14336 x 4096 21.5 -> 13.1, 4096 x 14336 18.5 -> 14.6, 8960 x 1536 10.2 -> 4.4, 1536 x 8960 7.7 -> 5.7,
-// 4096 x 4096 6.4 -> 5.5.  Four warps in a CTA: with eight the last ones end less evenly (3584 x 18944 19.0); a warp per
-// two rows reads v and the scales twice (30).
+// Bound by issue, the conversions (two codes become two halves with one, exactly) and L1: a lane reads the 16 floats of its own
+// block of v, so a warp's load of them touches 16 lines whatever its width, and with 32-byte loads (v on such a boundary) it does
+// so twice instead of four times.  18944 x 3584 takes 11.9 us, its bytes 6.  Six weights in turn, us, gemv_staged_kernel or
+// gemv_kernel / 16-byte loads / 32-byte loads, two rows' additions packed: 18944 x 3584 20.5 / 13.5 / 11.9, 3584 x 18944
+// 23.6 / 17.8 / 17.0, 14336 x 4096 21.5 / 13.3 / 11.9, 4096 x 14336 18.5 / 14.5 / 13.2, 8960 x 1536 10.2 / 4.2 / 3.7,
+// 1536 x 8960 7.7 / 5.6 / 5.3, 4096 x 4096 6.4 / 5.6 / 5.3.  (Packed additions where warps share rows: 4096 x 14336 13.7; the next
+// round's codes in registers ahead of the work: 18944 x 3584 13.5.)  Four warps in a CTA: with eight the last ones end less evenly
+// (3584 x 18944 19.0); a warp per two rows reads v and the scales twice (30).
 constexpr int kGemvWarps = 4, kGemvCtasPerSm = 8;
-template <bool kSplit>
+// kWideV: v starts on a 32-byte boundary
+template <bool kSplit, bool kWideV>
 __global__ void __launch_bounds__(32 * kGemvWarps, kGemvCtasPerSm)
 gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, const float* __restrict__ unit_ptr,
                  int64_t R, int64_t C, int trips, int split, const float* __restrict__ v, float* __restrict__ out) {
@@ -192,25 +202,48 @@ gemv_quad_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ 
 #pragma unroll
       for (int c = 0; c < 4; ++c) w[c] = __ldg(row_codes[c] + k);
       float f[16];
-      const float4* v4 = reinterpret_cast<const float4*>(v) + 4 * (int64_t)k;
+      if constexpr (kWideV) {
+        load8_wide(v + 16 * (int64_t)k, f);
+        load8_wide(v + 16 * (int64_t)k + 8, f + 8);
+      } else {
+        const float4* v4 = reinterpret_cast<const float4*>(v) + 4 * (int64_t)k;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 q = __ldg(v4 + i);
-        f[4 * i] = q.x; f[4 * i + 1] = q.y; f[4 * i + 2] = q.z; f[4 * i + 3] = q.w;
+        for (int i = 0; i < 4; ++i) {
+          const float4 q = __ldg(v4 + i);
+          f[4 * i] = q.x; f[4 * i + 1] = q.y; f[4 * i + 2] = q.z; f[4 * i + 3] = q.w;
+        }
       }
       const uint32_t s4[4] = {sw.x >> byte, sw.y >> byte, sw.z >> byte, sw.w >> byte};
+      if constexpr (kSplit) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float e[16];
-        e2m1x8_to_float(w[c].x, e);
-        e2m1x8_to_float(w[c].y, e + 8);
-        float part = 0.0f;
+        for (int c = 0; c < 4; ++c) {
+          float e[16];
+          e2m1x8_to_float(w[c].x, e);
+          e2m1x8_to_float(w[c].y, e + 8);
+          float part = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) part = fmaf(e[i], f[i], part);
-        if (kSplit) sums[(c * trips + t) * 32] = __float_as_uint(part);
-        else acc[c] = fmaf(part, e4m3_to_float((uint8_t)s4[c]), acc[c]);
+          for (int i = 0; i < 16; ++i) part = fmaf(e[i], f[i], part);
+          sums[(c * trips + t) * 32] = __float_as_uint(part);
+        }
+        sums[(4 * trips + t) * 32] = __byte_perm(__byte_perm(s4[0], s4[1], 0x0040), __byte_perm(s4[2], s4[3], 0x0040), 0x5410);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {                    // two rows' chains to a packed instruction
+          f32x2 part = 0ull;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float e0[8], e1[8];
+            e2m1x8_to_float(h == 0 ? w[c].x : w[c].y, e0);
+            e2m1x8_to_float(h == 0 ? w[c + 1].x : w[c + 1].y, e1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) part = fma2(pack2(e0[i], e1[i]), pack2(f[8 * h + i], f[8 * h + i]), part);
+          }
+          float p[2];
+          split2(part, p[0], p[1]);
+          acc[c] = fmaf(p[0], e4m3_to_float((uint8_t)s4[c]), acc[c]);
+          acc[c + 1] = fmaf(p[1], e4m3_to_float((uint8_t)s4[c + 1]), acc[c + 1]);
+        }
       }
-      if (kSplit) sums[(4 * trips + t) * 32] = __byte_perm(__byte_perm(s4[0], s4[1], 0x0040), __byte_perm(s4[2], s4[3], 0x0040), 0x5410);
     }
   }
   const float unit = __ldg(unit_ptr);
@@ -457,11 +490,15 @@ static cudaError_t launch_gemv_quad(const uint8_t* codes, const uint8_t* scales,
   const int64_t quads = ceil_div(R, 128) * 32, trips = ceil_div(C, 512);
   const int split = gemv_split(R, C);
   const dim3 grid((unsigned)ceil_div(quads * split, kGemvWarps)), block(32 * kGemvWarps);
-  if (split == 1) return launch_overlapped(kLaunchShort, gemv_quad_kernel<false>, grid, block, 0, st, codes, scales, unit, R, C, (int)trips, 1, v, out);
+  const bool wide_v = (reinterpret_cast<uintptr_t>(v) & 31u) == 0;
+  if (split == 1)
+    return launch_overlapped(kLaunchShort, wide_v ? gemv_quad_kernel<false, true> : gemv_quad_kernel<false, false>, grid, block, 0, st, codes, scales,
+                             unit, R, C, (int)trips, 1, v, out);
   const size_t smem = (size_t)gemv_sum_bytes(C, split);
-  cudaError_t e = cudaFuncSetAttribute(gemv_quad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSumBytesMax);
+  auto kern = wide_v ? gemv_quad_kernel<true, true> : gemv_quad_kernel<true, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSumBytesMax);
   if (e != cudaSuccess) return e;
-  return launch_overlapped(kLaunchShort, gemv_quad_kernel<true>, grid, block, smem, st, codes, scales, unit, R, C, (int)trips, split, v, out);
+  return launch_overlapped(kLaunchShort, kern, grid, block, smem, st, codes, scales, unit, R, C, (int)trips, split, v, out);
 }
 
 // t = bf16( float(bf16(yv * s)) / (unit_a * unit_b) ), 8 elements per thread

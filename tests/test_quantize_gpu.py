@@ -578,3 +578,17 @@ def test_a_workspace_with_room_for_records_gives_the_same_bytes(rows, cols, tran
     xs = x.float().cpu().numpy()
     ocodes, oscales, ounit = oracle_packed(np.ascontiguousarray(xs.T) if transpose else xs, layout)
     assert np.array_equal(got[1][0].cpu().numpy(), ocodes) and np.array_equal(got[1][1].cpu().numpy(), oscales)
+
+
+# The vector on a 32-byte boundary takes wider loads than on a 16-byte one; rows alone and shared by warps, a last round of 32
+# blocks that is not full, rows missing in the last four.
+@pytest.mark.parametrize("rows,cols", [(14336, 1552), (2600, 768), (1033, 8208), (1024, 4096)])
+def test_vector_product_does_not_depend_on_the_vectors_alignment(rows, cols):
+    q = ops.nvfp4_quantize(synthetic(rows, cols, "weights", seed=rows, dtype=torch.bfloat16).to(DEV))
+    store = torch.randn(cols + 8, device=DEV, generator=torch.Generator(device=DEV).manual_seed(cols))
+    v = store[4:cols + 4]
+    assert v.data_ptr() % 32 == 16
+    got = ops.nvfp4_gemv(q, v)
+    assert torch.equal(got, ops.nvfp4_gemv(q, v.clone()))
+    want = q.dequantize(torch.float32).double() @ v.double()
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5
