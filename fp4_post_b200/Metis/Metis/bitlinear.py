@@ -105,8 +105,8 @@ class PackedOperand:
         return self._dense[dtype]
 
 
-def _packed_matmul(a, b, rank1=(), lowrank=None, c=None, out_dtype=torch.bfloat16, sm_limit=0, scaled=None):
-    return ops.nvfp4_gemm(a, b, rank1=rank1, lowrank=lowrank, c=c, out_dtype=out_dtype, sm_limit=sm_limit, scaled=scaled)
+def _packed_matmul(a, b, rank1=(), lowrank=None, c=None, out_dtype=torch.bfloat16, sm_limit=0, scaled=None, rows_ready=None):
+    return ops.nvfp4_gemm(a, b, rank1=rank1, lowrank=lowrank, c=c, out_dtype=out_dtype, sm_limit=sm_limit, scaled=scaled, rows_ready=rows_ready)
 
 
 def _backward_can_pack(shared) -> bool:
@@ -886,7 +886,7 @@ class MetisFusedFunction(torch.autograd.Function):
         N = rq.q.shape[0]
         act = xa.dtype if xa.dtype in (torch.bfloat16, torch.float32) else torch.float32
         rank1_v, rank1_r = [], []
-        join_residual = bias_row = None
+        v_ready = r_ready = bias_row = None
 
         def ready(op):
             if op.ready_event is not None:             # quantized on another stream: order this stream after it, once
@@ -897,8 +897,8 @@ class MetisFusedFunction(torch.autograd.Function):
             # quantization of x instead of after it
             # (weights from the cache, or quantized on the second stream itself: fresh ones made on this
             # stream are still being quantized here)
-            beside = vq.ready_event is not None and rq.ready_event is not None
-            overlap = MetisFusedFunction.concurrent_branches and (beside or (not vq.fresh and not rq.fresh))
+            elsewhere = vq.ready_event is not None and rq.ready_event is not None
+            overlap = MetisFusedFunction.concurrent_branches and xa.mean_event is not None and (elsewhere or (not vq.fresh and not rq.fresh))
             if not overlap:
                 ready(vq)
                 ready(rq)
@@ -911,20 +911,26 @@ class MetisFusedFunction(torch.autograd.Function):
                 with on_stream(side):
                     bias_row = bias.float()
                     bias_done = recorded_event(side)
-            with _beside(xa.mean_event if overlap else None, xa.mean.device) as join:
-                if overlap and vq.ready_event is not None:      # quantized on a stream of their own: order this one after each
-                    current_stream(xa.mean.device).wait_event(vq.ready_event)
-                row_v = ops.nvfp4_gemv(vq.q, xa.mean)
-                # the product with V needs only this one: the pass over the (much larger) residual
-                # weight stays off the critical path until the residual product
-                v_ready = recorded_event(current_stream(xa.mean.device)) if overlap else None
-                if overlap and rq.ready_event is not None:
-                    current_stream(xa.mean.device).wait_event(rq.ready_event)
-                row_r = ops.nvfp4_gemv(rq.q, xa.mean)
-            if v_ready is not None:
-                current_stream(xa.mean.device).wait_event(v_ready)
-                row_v.record_stream(current_stream(xa.mean.device))
-                join_residual = lambda: join(row_r)
+            if overlap:
+                # Each on a stream of its own: the pass over the (much larger) residual weight waits for nothing of the one over V.
+                # A product joins its row vector when it needs it (rows_ready), which a product split along K does at its end.
+                dev = xa.mean.device
+                main = current_stream(dev)
+
+                def beside(op, index):
+                    side = _aux_stream(dev, index)
+                    side.wait_event(xa.mean_event)
+                    if op.ready_event is not None:              # quantized on a stream of its own: order this one after it
+                        side.wait_event(op.ready_event)
+                    with on_stream(side):
+                        row = ops.nvfp4_gemv(op.q, xa.mean)
+                        done = recorded_event(side)
+                    row.record_stream(main)
+                    return row, done
+                row_v, v_ready = beside(vq, 0)
+                row_r, r_ready = beside(rq, 1)
+            else:
+                row_v, row_r = ops.nvfp4_gemv(vq.q, xa.mean), ops.nvfp4_gemv(rq.q, xa.mean)
             rank1_v.append((None, row_v))
             rank1_r.append((None, row_r))
         if bias is not None:
@@ -934,24 +940,22 @@ class MetisFusedFunction(torch.autograd.Function):
         if act == torch.bfloat16:
             if M <= 128:                            # decode-sized: the scaling comes out of the product's own last launch
                 ready(rq)                           # its unit
-                yv, t_acc = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, scaled=(s, xa.q.unit, rq.q.unit))     # [M, r]
+                yv, t_acc = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, scaled=(s, xa.q.unit, rq.q.unit), rows_ready=v_ready)     # [M, r]
             else:
-                yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act)
+                yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, rows_ready=v_ready)
                 ready(rq)
                 t_acc = ops.lowrank_scale(yv, s, xa.q.unit, rq.q.unit)
             lowrank = (t_acc, u_weight.detach().to(torch.bfloat16))
         else:
-            yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act)
+            yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, rows_ready=v_ready)
             ready(rq)
             ts = yv * s.to(act)
             lowrank = _bf16_factors(ts.float() / (xa.q.unit * rq.q.unit), u_weight.detach(), act)
-        if join_residual is not None:
-            join_residual()
         if bias_row is not None:
             here.wait_event(bias_done)
             bias_row.record_stream(here)
         ready(rq)
-        y = _packed_matmul(xa.q, rq.q, rank1=rank1_r, lowrank=lowrank, out_dtype=act)
+        y = _packed_matmul(xa.q, rq.q, rank1=rank1_r, lowrank=lowrank, out_dtype=act, rows_ready=r_ready)
         if (MetisFusedFunction.concurrent_branches and xa.q.codes.is_cuda and any(ctx.needs_input_grad)
                 and xa._qt is not None and LinearLowbitFunction._backward_centred()):
             _row_sums_beside(xa)        # queued behind the product: it runs as that one drains, not in front of it

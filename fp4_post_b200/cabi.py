@@ -28,7 +28,7 @@ EXPORTS = (
     "metis_query", "metis_last_error_string", "metis_nvfp4_sf_bytes",
     "metis_nvfp4_quantize_workspace_bytes", "metis_nvfp4_quantize", "metis_rmsnorm_nvfp4_quantize",
     "metis_nvfp4_dequantize", "metis_nvfp4_dequantize_ratio", "metis_col_mean_workspace_bytes", "metis_col_mean", "metis_nvfp4_gemv",
-    "metis_nvfp4_gemm", "metis_nvfp4_gemm_scaled", "metis_nvfp4_quantize_static", "metis_nvfp4_gemm_workspace_bytes",
+    "metis_nvfp4_gemm", "metis_nvfp4_gemm_scaled", "metis_nvfp4_gemm_joined", "metis_nvfp4_quantize_static", "metis_nvfp4_gemm_workspace_bytes",
     "metis_lowrank_scale",
     "metis_nvfp4_quantize_dual_workspace_bytes", "metis_nvfp4_quantize_dual", "metis_nvfp4_quantize_dual_finish",
     "metis_rmsnorm_mean_workspace_bytes", "metis_rmsnorm_mean",
@@ -114,6 +114,8 @@ def lib() -> C.CDLL:
     L.metis_nvfp4_gemm.restype = i32
     L.metis_nvfp4_gemm_scaled.argtypes = [C.POINTER(GemmArgs), vp, i32, vp, vp, vp]
     L.metis_nvfp4_gemm_scaled.restype = i32
+    L.metis_nvfp4_gemm_joined.argtypes = [C.POINTER(GemmArgs), vp, vp, i32, vp, vp, vp]
+    L.metis_nvfp4_gemm_joined.restype = i32
     L.metis_lowrank_scale.argtypes = [vp, i64, i64, i64, vp, i32, vp, vp, vp, vp]
     L.metis_lowrank_scale.restype = i32
     for name in ("metis_bf16_panel_gemm_workspace_bytes", "metis_lowrank_dts_workspace_bytes", "metis_lowrank_du_workspace_bytes"):

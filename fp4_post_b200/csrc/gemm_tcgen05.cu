@@ -429,7 +429,7 @@ static int tile_width(int64_t M, int64_t N, int sms) {
 
 template <int BN, typename TD>
 static int32_t launch_gemm(const metis_gemm_args* a, const CUtensorMap& ma, const CUtensorMap& mb,
-                           const CUtensorMap& mt, const CUtensorMap& mu, const GemmParams& p) {
+                           const CUtensorMap& mt, const CUtensorMap& mu, const GemmParams& p, cudaEvent_t rows_ready) {
   using Cfg = GemmCfg<BN>;
   auto kern = nvfp4_gemm_kernel<BN, TD>;
   // per device and cheap, so it is simply repeated on every launch
@@ -441,6 +441,7 @@ static int32_t launch_gemm(const metis_gemm_args* a, const CUtensorMap& ma, cons
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   METIS_CUDA_OK(launch_overlapped(kLaunchGemm, kern, dim3((unsigned)grid), dim3(kGemmThreads), Cfg::kSmemBytes, st, ma, mb, mt, mu, p));
   if (p.splits > 1) {
+    if (rows_ready) METIS_CUDA_OK(cudaStreamWaitEvent(st, rows_ready, 0));      // the partial sums know nothing of the row vectors
     const int64_t threads = a->M * ceil_div(a->N, 4);
     int64_t blocks = ceil_div(threads, 256);
     if (blocks > (int64_t)device_sm_count() * 8) blocks = (int64_t)device_sm_count() * 8;
@@ -475,7 +476,8 @@ struct ScaledOutput {
 };
 }  // namespace
 
-static int32_t run_gemm(const metis_gemm_args* a, const ScaledOutput* scaled) {
+// rows_ready: an event after which the row vectors are there (nullptr: they are when the stream gets here)
+static int32_t run_gemm(const metis_gemm_args* a, const ScaledOutput* scaled, cudaEvent_t rows_ready = nullptr) {
   if (!a) return fail(METIS_ERR_BAD_ARGUMENT, "args is null");
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return fail(METIS_ERR_BAD_SHAPE, "empty GEMM %lld x %lld x %lld", (long long)a->M, (long long)a->N, (long long)a->K);
   if (a->K % 32 != 0) return fail(METIS_ERR_BAD_SHAPE, "K = %lld must be a multiple of 32 (16-byte rows of packed codes)", (long long)a->K);
@@ -539,22 +541,35 @@ static int32_t run_gemm(const metis_gemm_args* a, const ScaledOutput* scaled) {
     p.scaled = static_cast<__nv_bfloat16*>(scaled->t);
   }
   const bool bf16 = a->d_dtype == METIS_DTYPE_BF16;
+  if (rows_ready && p.splits == 1) METIS_CUDA_OK(cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(a->stream), rows_ready, 0));
   int32_t rc;
   if (pair) rc = launch_gemm_pair(a, ma, mb, mt, mu, p);
-  else if (bn == 256) rc = bf16 ? launch_gemm<256, __nv_bfloat16>(a, ma, mb, mt, mu, p) : launch_gemm<256, float>(a, ma, mb, mt, mu, p);
-  else rc = bf16 ? launch_gemm<128, __nv_bfloat16>(a, ma, mb, mt, mu, p) : launch_gemm<128, float>(a, ma, mb, mt, mu, p);
+  else if (bn == 256) rc = bf16 ? launch_gemm<256, __nv_bfloat16>(a, ma, mb, mt, mu, p, rows_ready) : launch_gemm<256, float>(a, ma, mb, mt, mu, p, rows_ready);
+  else rc = bf16 ? launch_gemm<128, __nv_bfloat16>(a, ma, mb, mt, mu, p, rows_ready) : launch_gemm<128, float>(a, ma, mb, mt, mu, p, rows_ready);
   if (rc || !scale_behind) return rc;
   return metis_lowrank_scale(a->d, a->M, a->N, a->ldd, scaled->s, scaled->s_dtype, scaled->unit_a, scaled->unit_b, scaled->t, a->stream);
 }
 
 extern "C" int32_t metis_nvfp4_gemm(const metis_gemm_args* a) { return run_gemm(a, nullptr); }
 
-extern "C" int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* a, const void* s, int32_t s_dtype, const float* unit_a,
-                                           const float* unit_b, void* t) {
+static int32_t run_gemm_scaled(const metis_gemm_args* a, const void* s, int32_t s_dtype, const float* unit_a,
+                               const float* unit_b, void* t, cudaEvent_t rows_ready) {
   if (!a || !s || !unit_a || !unit_b || !t) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
   if (s_dtype != METIS_DTYPE_BF16 && s_dtype != METIS_DTYPE_F32) return fail(METIS_ERR_BAD_ARGUMENT, "unknown s_dtype %d", s_dtype);
   if (a->d_dtype != METIS_DTYPE_BF16 || a->N % 8 != 0 || a->ldd % 8 != 0) return fail(METIS_ERR_BAD_ARGUMENT, "the scaled copy is of a bf16 D whose width is a multiple of 8");
   if (!aligned16(t) || (reinterpret_cast<uintptr_t>(s) & 3u)) return fail(METIS_ERR_BAD_ALIGNMENT, "t must be 16-byte aligned");
   const ScaledOutput scaled = {s, s_dtype, unit_a, unit_b, t};
-  return run_gemm(a, &scaled);
+  return run_gemm(a, &scaled, rows_ready);
+}
+
+extern "C" int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* a, const void* s, int32_t s_dtype, const float* unit_a,
+                                           const float* unit_b, void* t) {
+  return run_gemm_scaled(a, s, s_dtype, unit_a, unit_b, t, nullptr);
+}
+
+extern "C" int32_t metis_nvfp4_gemm_joined(const metis_gemm_args* a, void* rows_ready, const void* s, int32_t s_dtype,
+                                           const float* unit_a, const float* unit_b, void* t) {
+  if (!rows_ready) return fail(METIS_ERR_BAD_ARGUMENT, "rows_ready is null");
+  const cudaEvent_t ev = static_cast<cudaEvent_t>(rows_ready);
+  return t ? run_gemm_scaled(a, s, s_dtype, unit_a, unit_b, t, ev) : run_gemm(a, nullptr, ev);
 }

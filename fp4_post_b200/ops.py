@@ -454,7 +454,7 @@ def lowrank_scale(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_
 def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Optional[torch.Tensor] = None,
                out_dtype: torch.dtype = torch.bfloat16, alpha: float = 1.0,
                status: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-               sm_limit: int = 0, scaled=None, _debug: int = 0):
+               sm_limit: int = 0, scaled=None, rows_ready: Optional["torch.cuda.Event"] = None, _debug: int = 0):
     """D = alpha*ua*ub * (A @ B^T + T @ U^T) + sum_i cvec_i (x) rvec_i (+ c), see metis_nvfp4_gemm.
 
     a: [M, K], b: [N, K] (both METIS_SF_MMA).  lowrank = (T [M, r] bf16, U [N, r] bf16), already in
@@ -462,7 +462,9 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
     Only the packed parts of a and b enter the product; their mean vectors do not.
     sm_limit > 0 caps the SMs this launch occupies (room for a collective's kernel beside it).
     scaled = (s, unit_a, unit_b), for a bf16 D: returns (D, lowrank_scale(D, s, unit_a, unit_b)); the second value costs
-    no launch of its own where the product is split along K."""
+    no launch of its own where the product is split along K.
+    rows_ready: an event recorded on another stream behind the launches that write the row vectors of rank1; the product's
+    stream waits for it as late as it can (a product split along K only in front of the launch that adds its splits)."""
     M, K = a.shape
     N, K2 = b.shape
     if K != K2:
@@ -519,7 +521,8 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
             keep.append(ws)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws_bytes
         if scaled is None:
-            rc = cabi.lib().metis_nvfp4_gemm(C.byref(args))
+            rc = cabi.lib().metis_nvfp4_gemm(C.byref(args)) if rows_ready is None else \
+                cabi.lib().metis_nvfp4_gemm_joined(C.byref(args), rows_ready.cuda_event, None, 0, None, None, None)
         else:
             s, unit_a, unit_b = scaled
             if s.dtype not in (torch.bfloat16, torch.float32):
@@ -527,8 +530,9 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
             s = s.reshape(-1).contiguous()
             assert s.numel() == N and s.device == dev
             t = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), s.data_ptr(), _dtype_code(s, "s"), _unit_ptr(unit_a, dev),
-                                                    _unit_ptr(unit_b, dev), t.data_ptr())
+            more = (s.data_ptr(), _dtype_code(s, "s"), _unit_ptr(unit_a, dev), _unit_ptr(unit_b, dev), t.data_ptr())
+            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), *more) if rows_ready is None else \
+                cabi.lib().metis_nvfp4_gemm_joined(C.byref(args), rows_ready.cuda_event, *more)
     cabi.check(rc, "metis_nvfp4_gemm")
     LAUNCHES["gemm"] += 2 if ws_bytes > 0 or scaled is not None else 1       # the sum of the splits, or the scaling
     return out if scaled is None else (out, t)

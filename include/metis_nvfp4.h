@@ -359,6 +359,14 @@ int32_t metis_nvfp4_gemm_scaled(const metis_gemm_args* args, const void* s, int3
                                 const float* unit_b, void* t);
 
 /*
+ * metis_nvfp4_gemm (t null: s, unit_a and unit_b are not read) or metis_nvfp4_gemm_scaled whose row vectors rvec0 and
+ * rvec1 another stream writes: they are complete once rows_ready (a cudaEvent_t recorded there) has happened.  A product
+ * split along K waits for it in front of the launch that adds its partial sums, any other in front of the product.
+ */
+int32_t metis_nvfp4_gemm_joined(const metis_gemm_args* args, void* rows_ready, const void* s, int32_t s_dtype,
+                                const float* unit_a, const float* unit_b, void* t);
+
+/*
  * Scratch that lets a decode-sized product (M <= 128: the rollout path, bitlinear.py:704-751,
  * and the weight gradients of the rank-r factors) split its K loop over otherwise idle SMs:
  * bytes of fp32 partial sums, 0 when the shape is not split.  Without the scratch the same

@@ -84,6 +84,42 @@ def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
     assert rel_l2(got, want) <= (1e-5 if dtype == torch.float32 else 2.0 ** -8)      # fp32 sums; one rounding to bf16
 
 
+# Row vectors that another stream writes late: split along K (waits in front of the sum of the splits) or not, with the scaled copy
+# and without, issued and captured.
+@pytest.mark.parametrize("M,N,K", [(16, 512, 2048), (16, 64, 512), (300, 264, 512)])
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("captured", [False, True])
+def test_row_vectors_from_another_stream(M, N, K, scaled, captured):
+    qa, qb, _, _ = operands(M, N, K, seed=M + N)
+    g = torch.Generator(device=DEV).manual_seed(N)
+    late = torch.randn(N, generator=g, device=DEV)
+    s = torch.rand(N, generator=g, device=DEV).to(torch.bfloat16)
+    kw = dict(scaled=(s, qa.unit, qb.unit)) if scaled else {}
+    want = ops.nvfp4_gemm(qa, qb, rank1=((None, late),), **kw)
+    side, row = torch.cuda.Stream(), torch.zeros(N, device=DEV)
+    torch.cuda.synchronize()
+
+    def call():
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(2_000_000)
+            row.copy_(late)
+            ev = torch.cuda.Event()
+            ev.record()
+        return ops.nvfp4_gemm(qa, qb, rank1=((None, row),), rows_ready=ev, **kw)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = call()
+        row.zero_()
+        graph.replay()
+    else:
+        got = call()
+    torch.cuda.synchronize()
+    for a, b in zip(got if scaled else (got,), want if scaled else (want,)):
+        assert torch.equal(a, b)
+
+
 # the projection shapes of the two decoder configurations (Qwen2-style 1.5B at rank 64, 7B at rank 128)
 DECODER_SHAPES = [(1536, 1536, 64), (256, 1536, 64), (8960, 1536, 64), (1536, 8960, 64),
                   (3584, 3584, 128), (512, 3584, 128), (18944, 3584, 128), (3584, 18944, 128)]
