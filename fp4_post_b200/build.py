@@ -2,7 +2,8 @@
 
     python -m fp4_post_b200.build        # or: from fp4_post_b200.build import build; build()
 
-Output: fp4_post_b200/_lib/libmetis_nvfp4.so.  nvcc cross-compiles without a GPU.
+Output: fp4_post_b200/_lib/libmetis_nvfp4.so, and _lib/metis_host.so, the native part of the tensor-level wrappers (g++ against
+the installed torch).  nvcc cross-compiles without a GPU.
 
     python -m fp4_post_b200.build --timing-knobs
 
@@ -18,6 +19,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -25,6 +27,8 @@ CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_lib"
 LIB = OUT_DIR / "libmetis_nvfp4.so"
 KNOBS_LIB = OUT_DIR / "libmetis_nvfp4_knobs.so"
+HOST_SOURCE = CSRC / "host_ops.cpp"
+HOST_MODULE = OUT_DIR / "metis_host.so"
 SOURCES = ["api.cu", "quantize.cu", "rmsnorm_quant.cu", "dequantize.cu", "gemm_tcgen05.cu", "gemm_tcgen05_pair.cu", "lowrank_bwd.cu", "decoder_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -48,6 +52,14 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _host_command() -> list[str]:
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *(f"-I{p}" for p in include), str(HOST_SOURCE), "-o", str(HOST_MODULE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
 def build(force: bool = False, verbose: bool = False, timing_knobs: bool = False) -> Path:
     """Compile every .cu file to an object and link the shared library. Returns its path."""
     nvcc = _nvcc()
@@ -68,6 +80,9 @@ def build(force: bool = False, verbose: bool = False, timing_knobs: bool = False
                 cmd.insert(1, "-Xptxas=-v")
                 print(" ".join(cmd), file=sys.stderr)
             procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    host = None
+    if not timing_knobs and (force or _stale(HOST_MODULE, [HOST_SOURCE, PKG.parent / "include" / "metis_nvfp4.h"])):
+        host = subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     failed = []
     for src, p in procs:
         out, _ = p.communicate()
@@ -75,6 +90,10 @@ def build(force: bool = False, verbose: bool = False, timing_knobs: bool = False
             print(out, file=sys.stderr)
         if p.returncode != 0:
             failed.append((src, out))
+    if host is not None:
+        out, _ = host.communicate()
+        if host.returncode != 0:
+            raise RuntimeError(f"g++ failed:\n--- {HOST_SOURCE.name} ---\n{out}")
     if failed:
         raise RuntimeError("nvcc failed:\n" + "\n".join(f"--- {s} ---\n{o}" for s, o in failed))
     if force or procs or _stale(lib, objs):

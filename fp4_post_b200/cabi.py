@@ -6,8 +6,12 @@ There is no CPU fallback: if the library is missing, `lib()` raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 from pathlib import Path
 
+import torch  # noqa: F401  (the native wrappers below link against it: it has to be loaded first)
+
+HOST_PATH = Path(__file__).resolve().parent / "_lib" / "metis_host.so"
 LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libmetis_nvfp4.so"
 
 DTYPE_BF16, DTYPE_F32 = 0, 1
@@ -59,6 +63,7 @@ class GemmArgs(C.Structure):
 
 
 _lib = None
+_host = None
 
 
 class MetisLibraryError(RuntimeError):
@@ -135,8 +140,29 @@ def lib() -> C.CDLL:
     L.metis_rope_pair.restype = i32
     L.metis_silu_mul.argtypes = [vp, vp, vp, i64, vp]
     L.metis_silu_mul.restype = i32
+    _bind_host(L)
     _lib = L
     return L
+
+
+def _bind_host(L: C.CDLL) -> None:
+    """Load the native part of the wrappers in ops.py once and give it the entry points of L."""
+    global _host
+    if _host is None:
+        if not HOST_PATH.exists():
+            raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build`")
+        spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    for name in EXPORTS:
+        _host.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
+
+
+def host():
+    """The native wrappers (csrc/host_ops.cpp): allocations and call in one; every function returns (status, tensors...)."""
+    if _host is None or _lib is None:
+        lib()
+    return _host
 
 
 def check(rc: int, what: str) -> None:

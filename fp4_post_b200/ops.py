@@ -1,10 +1,12 @@
 """Tensor-level wrappers over the C ABI: PyTorch supplies device memory and streams only.
 
-Every function needs CUDA tensors and the built library; nothing here computes on the CPU.
+Types and shapes are checked here; allocating outputs and workspace and making the call is one native call for the entry points
+that a forward or a step makes many of (csrc/host_ops.cpp; us per call from Python, before / now: fused norm 22.9 / 13.1,
+quantizer 21.0 / 11.6, both orientations 28.4 / 15.8, column mean 15.2 / 8.3, vector product 9.7 / 5.3, product 9.9 / 6.8, of
+which the launches take 3 to 6).  Every function needs CUDA tensors and the built library; nothing here computes on the CPU.
 """
 from __future__ import annotations
 
-import ctypes as C
 from dataclasses import dataclass
 from typing import Optional
 
@@ -117,23 +119,14 @@ def _sf_bytes(R: int, Cc: int, sf_layout: int) -> int:
     return cabi.lib().metis_nvfp4_sf_bytes(R, Cc, sf_layout)
 
 
-def _packed_buffers(L, R: int, Cc: int, sf_layout: int, dev):
-    """codes, scales and unit of one quantized tensor as views of a single allocation."""
-    half = Cc // 2
-    n_codes, n_scales = R * half, _sf_bytes(R, Cc, sf_layout)
-    o_scales = (n_codes + 255) & ~255
-    o_unit = (o_scales + n_scales + 255) & ~255
-    buf = torch.empty(o_unit + 16, dtype=torch.uint8, device=dev)
-    return (torch.as_strided(buf, (R, half), (half, 1)), torch.as_strided(buf, (n_scales,), (1,), o_scales),
-            torch.as_strided(buf, (4,), (1,), o_unit).view(torch.float32))
-
-
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
 def _rows2d(x: torch.Tensor) -> torch.Tensor:
     """View x as [rows, cols] with unit stride along cols (copy only if it has to)."""
+    if x.dim() == 2 and x.is_contiguous() and x.stride(0) == x.shape[1]:      # (a single row may have any stride)
+        return x
     x2 = x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) < x2.shape[1]):
         x2 = x2.contiguous()
@@ -170,15 +163,10 @@ def col_mean(x: torch.Tensor) -> torch.Tensor:
     """Column means of x viewed as [rows, cols], fp32 (input_flat.mean(dim=0), bitlinear.py:326)."""
     _need_cuda(x, "x")
     x2 = _rows2d(x)
-    rows, cols = x2.shape
-    L = cabi.lib()
     with _on_device(x2.device):
-        mean = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        ws_bytes = L.metis_col_mean_workspace_bytes(rows, cols)
-        ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=x2.device)
-        rc = L.metis_col_mean(x2.data_ptr(), _dtype_code(x2, "x"), rows, cols, x2.stride(0), mean.data_ptr(),
-                              ws.data_ptr(), ws.numel(), _stream())
-    cabi.check(rc, "metis_col_mean")
+        rc, mean = cabi.host().col_mean(x2, _dtype_code(x2, "x"), _stream())
+    if rc:
+        cabi.check(rc, "metis_col_mean")
     LAUNCHES["col_mean"] += 2
     return mean
 
@@ -199,6 +187,14 @@ def _sr_flags(stochastic: bool, sr_bits: int) -> int:
     return cabi.Q_SR16 if stochastic and sr_bits == 16 else 0
 
 
+def _mean_row(mean: torch.Tensor, cols: int) -> torch.Tensor:
+    _need_cuda(mean, "mean")
+    if mean.dim() != 1 or mean.dtype != torch.float32 or not mean.is_contiguous():
+        mean = mean.reshape(-1).to(torch.float32).contiguous()
+    assert mean.numel() == cols
+    return mean
+
+
 def nvfp4_quantize(x: torch.Tensor, *, transpose: bool = False, stochastic: bool = False, seed: int = 0,
                    offset: int = 0, sf_layout: int = cabi.SF_MMA,
                    mean: Optional[torch.Tensor] = None,
@@ -216,7 +212,6 @@ def nvfp4_quantize(x: torch.Tensor, *, transpose: bool = False, stochastic: bool
     R, Cc = (cols, rows) if transpose else (rows, cols)
     if Cc % 16 != 0 or R == 0:
         raise ValueError(f"NVFP4 block shape (1, 16) does not divide tensor shape {(R, Cc)}")
-    L = cabi.lib()
     flags = (cabi.Q_TRANSPOSE if transpose else 0) | (cabi.Q_STOCHASTIC if stochastic else 0) | _hadamard_flags(hadamard_signs)
     flags |= _sr_flags(stochastic, sr_bits)
     dev = x2.device
@@ -226,17 +221,12 @@ def nvfp4_quantize(x: torch.Tensor, *, transpose: bool = False, stochastic: bool
         flags |= cabi.Q_OFFSET_ON_DEVICE
         offset = offset_counter.data_ptr()
     if mean is not None:
-        _need_cuda(mean, "mean")
-        mean = mean.reshape(-1).to(torch.float32).contiguous()
-        assert mean.numel() == cols
+        mean = _mean_row(mean, cols)
     with _on_device(dev):
-        codes, scales, unit = _packed_buffers(L, R, Cc, sf_layout, dev)
-        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(R, Cc) + cabi.QUANTIZE_EXTRA_WORKSPACE, dtype=torch.uint8, device=dev)
-        rc = L.metis_nvfp4_quantize(x2.data_ptr(), _dtype_code(x2, "x"), rows, cols, x2.stride(0), _ptr(mean),
-                                    flags, seed & (2**64 - 1), offset & (2**64 - 1), sf_layout,
-                                    codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), ws.data_ptr(),
-                                    ws.numel(), _stream())
-    cabi.check(rc, "metis_nvfp4_quantize")
+        rc, codes, scales, unit = cabi.host().quantize(x2, _dtype_code(x2, "x"), transpose, flags, seed & (2**64 - 1), offset & (2**64 - 1), sf_layout,
+                                                       _sf_bytes(R, Cc, sf_layout), cabi.QUANTIZE_EXTRA_WORKSPACE, mean, _stream())
+    if rc:
+        cabi.check(rc, "metis_nvfp4_quantize")
     LAUNCHES["quantize"] += 2
     q = NVFP4Tensor(codes, scales, unit, (R, Cc), sf_layout)
     if mean is not None:
@@ -263,7 +253,6 @@ def nvfp4_quantize_dual(x: torch.Tensor, *, stochastic: bool = False, seed: int 
     rows, cols = x2.shape
     if rows % 16 != 0 or cols % 16 != 0 or rows == 0:
         raise ValueError(f"NVFP4 block shape (1, 16) does not divide both dimensions of tensor shape {(rows, cols)}")
-    L = cabi.lib()
     flags = (cabi.Q_STOCHASTIC if stochastic else 0) | _hadamard_flags(hadamard_signs)      # rotation: the transposed output only
     flags |= _sr_flags(stochastic, sr_bits)
     if defer not in (None, "rowmajor", "transposed"):
@@ -277,22 +266,14 @@ def nvfp4_quantize_dual(x: torch.Tensor, *, stochastic: bool = False, seed: int 
         flags |= cabi.Q_OFFSET_ON_DEVICE
         offset = offset_counter.data_ptr()
     if mean is not None:
-        _need_cuda(mean, "mean")
-        mean = mean.reshape(-1).to(torch.float32).contiguous()
-        assert mean.numel() == cols
+        mean = _mean_row(mean, cols)
+    host = cabi.host()
     with _on_device(dev):
-        codes, scales, unit = _packed_buffers(L, rows, cols, sf_layout, dev)
-        codes_t, scales_t, unit_t = _packed_buffers(L, cols, rows, sf_layout, dev)
-        ws = torch.empty(L.metis_nvfp4_quantize_dual_workspace_bytes(rows, cols), dtype=torch.uint8, device=dev)
-        sums = None
-        if token_sums and rows % 64 == 0 and hadamard_signs is None:
-            sums = torch.empty(cols, dtype=torch.float32, device=dev)
-        rc = L.metis_nvfp4_quantize_dual(x2.data_ptr(), _dtype_code(x2, "x"), rows, cols, x2.stride(0), _ptr(mean),
-                                         flags, seed & (2**64 - 1), offset & (2**64 - 1), sf_layout,
-                                         codes.data_ptr(), scales.data_ptr(), unit.data_ptr(),
-                                         codes_t.data_ptr(), scales_t.data_ptr(), unit_t.data_ptr(), _ptr(sums),
-                                         ws.data_ptr(), ws.numel(), _stream())
-    cabi.check(rc, "metis_nvfp4_quantize_dual")
+        rc, codes, scales, unit, codes_t, scales_t, unit_t, sums, ws = host.quantize_dual(
+            x2, _dtype_code(x2, "x"), flags, seed & (2**64 - 1), offset & (2**64 - 1), sf_layout, _sf_bytes(rows, cols, sf_layout),
+            _sf_bytes(cols, rows, sf_layout), mean, token_sums and rows % 64 == 0 and hadamard_signs is None, _stream())
+    if rc:
+        cabi.check(rc, "metis_nvfp4_quantize_dual")
     LAUNCHES["quantize"] += 2
     q = NVFP4Tensor(codes, scales, unit, (rows, cols), sf_layout)
     qt = NVFP4Tensor(codes_t, scales_t, unit_t, (cols, rows), sf_layout)
@@ -305,15 +286,11 @@ def nvfp4_quantize_dual(x: torch.Tensor, *, stochastic: bool = False, seed: int 
 
     def finish():
         with _on_device(dev):
-            rc2 = L.metis_nvfp4_quantize_dual_finish(rows, cols, deferred, sf_layout, scales.data_ptr(), unit.data_ptr(),
-                                                     codes_t.data_ptr(), scales_t.data_ptr(), unit_t.data_ptr(), _ptr(sums),
-                                                     ws.data_ptr(), ws.numel(), _stream())
-        cabi.check(rc2, "metis_nvfp4_quantize_dual_finish")
-        # the buffers were allocated on the quantizing call's stream and are now also used on this one
-        cur = current_stream(dev)
-        for t in (ws, scales, unit, codes_t, scales_t, unit_t, sums):
-            if t is not None:
-                t.record_stream(cur)
+            # the buffers were allocated on the quantizing call's stream and are now also used on this one
+            cur = torch._C._cuda_getCurrentStream(dev.index)
+            rc2, = host.quantize_dual_finish(rows, cols, deferred, sf_layout, scales, unit, codes_t, scales_t, unit_t, sums, ws, _stream(), *cur)
+        if rc2:
+            cabi.check(rc2, "metis_nvfp4_quantize_dual_finish")
         LAUNCHES["quantize"] += 1
     return q, qt, finish
 
@@ -330,20 +307,15 @@ def rmsnorm_nvfp4_quantize(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e
         raise ValueError(f"NVFP4 block shape (1, 16) does not divide tensor shape {(rows, cols)}")
     gamma = gamma.contiguous()
     assert gamma.numel() == cols
-    L = cabi.lib()
-    dev = x2.device
-    with _on_device(dev):
-        codes, scales, unit = _packed_buffers(L, rows, cols, sf_layout, dev)
-        ws = torch.empty(L.metis_nvfp4_quantize_workspace_bytes(rows, cols) + cabi.QUANTIZE_EXTRA_WORKSPACE, dtype=torch.uint8, device=dev)
-        norm = None
-        if return_norm:
-            out_dtype = torch.bfloat16 if (x2.dtype == torch.bfloat16 and gamma.dtype == torch.bfloat16) else torch.float32
-            norm = torch.empty((rows, cols), dtype=out_dtype, device=dev)
-        rc = L.metis_rmsnorm_nvfp4_quantize(x2.data_ptr(), _dtype_code(x2, "x"), rows, cols, x2.stride(0),
-                                            gamma.data_ptr(), _dtype_code(gamma, "gamma"), float(eps), sf_layout,
-                                            codes.data_ptr(), scales.data_ptr(), unit.data_ptr(), _ptr(norm),
-                                            ws.data_ptr(), ws.numel(), _stream())
-    cabi.check(rc, "metis_rmsnorm_nvfp4_quantize")
+    dtype, gamma_dtype = _dtype_code(x2, "x"), _dtype_code(gamma, "gamma")
+    norm_dtype = -1
+    if return_norm:
+        norm_dtype = cabi.DTYPE_BF16 if dtype == gamma_dtype == cabi.DTYPE_BF16 else cabi.DTYPE_F32
+    with _on_device(x2.device):
+        rc, codes, scales, unit, norm = cabi.host().rmsnorm_quantize(x2, dtype, gamma, gamma_dtype, float(eps), sf_layout, _sf_bytes(rows, cols, sf_layout),
+                                                                     cabi.QUANTIZE_EXTRA_WORKSPACE, norm_dtype, _stream())
+    if rc:
+        cabi.check(rc, "metis_rmsnorm_nvfp4_quantize")
     LAUNCHES["rmsnorm_quantize"] += 2
     q = NVFP4Tensor(codes, scales, unit, (rows, cols), sf_layout)
     return (q, norm.reshape(x.shape)) if return_norm else q
@@ -418,15 +390,14 @@ def nvfp4_dequantize_ratio(q: NVFP4Tensor, dtype: torch.dtype, unit0, unit1, ove
 def nvfp4_gemv(q: NVFP4Tensor, v: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[r] = sum_c v[c] * value(q)[r, c] (v None: row sums), fp32; the mean vectors of q are ignored."""
     R, Cc = q.shape
-    L = cabi.lib()
     if v is not None:
-        v = v.reshape(-1).to(torch.float32).contiguous()
+        if v.dim() != 1 or v.dtype != torch.float32 or not v.is_contiguous():
+            v = v.reshape(-1).to(torch.float32).contiguous()
         assert v.numel() == Cc
     with _on_device(q.device):
-        out = torch.empty(R, dtype=torch.float32, device=q.device)
-        rc = L.metis_nvfp4_gemv(q.codes.data_ptr(), q.scales.data_ptr(), q.unit.data_ptr(), q.sf_layout, R, Cc,
-                                _ptr(v), out.data_ptr(), _stream())
-    cabi.check(rc, "metis_nvfp4_gemv")
+        rc, out = cabi.host().gemv(q.codes, q.scales, q.unit, q.sf_layout, R, Cc, v, _stream())
+    if rc:
+        cabi.check(rc, "metis_nvfp4_gemv")
     LAUNCHES["gemv"] += 1
     return out
 
@@ -443,12 +414,18 @@ def lowrank_scale(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_
     M, r = yv.shape
     assert s.numel() == r and s.device == yv.device
     with _on_device(yv.device):
-        out = torch.empty((M, r), dtype=torch.bfloat16, device=yv.device)
-        rc = cabi.lib().metis_lowrank_scale(yv.data_ptr(), M, r, yv.stride(0), s.data_ptr(), _dtype_code(s, "s"),
-                                            unit_a.data_ptr(), unit_b.data_ptr(), out.data_ptr(), _stream())
-    cabi.check(rc, "metis_lowrank_scale")
+        rc, out = cabi.host().lowrank_scale(yv, s, _dtype_code(s, "s"), unit_a, unit_b, _stream())
+    if rc:
+        cabi.check(rc, "metis_lowrank_scale")
     LAUNCHES["gemv"] += 1
     return out
+
+
+def _fp32_vector(t: torch.Tensor, n: int) -> torch.Tensor:
+    if t.dim() != 1 or t.dtype != torch.float32 or not t.is_contiguous():
+        t = t.reshape(-1).to(torch.float32).contiguous()
+    assert t.numel() == n and t.is_cuda
+    return t
 
 
 def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Optional[torch.Tensor] = None,
@@ -472,12 +449,7 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
     if a.sf_layout != cabi.SF_MMA or b.sf_layout != cabi.SF_MMA:
         raise ValueError("GEMM operands need METIS_SF_MMA scales")
     dev = a.device
-    args = cabi.GemmArgs()
-    args.M, args.N, args.K = M, N, K
-    args.a_codes, args.a_scales, args.a_unit = a.codes.data_ptr(), a.scales.data_ptr(), a.unit.data_ptr()
-    args.b_codes, args.b_scales, args.b_unit = b.codes.data_ptr(), b.scales.data_ptr(), b.unit.data_ptr()
-    args.alpha = float(alpha)
-    keep = []
+    T = U = None
     if lowrank is not None:
         T, U = lowrank
         if T.dtype != torch.bfloat16 or U.dtype != torch.bfloat16:
@@ -485,55 +457,34 @@ def nvfp4_gemm(a: NVFP4Tensor, b: NVFP4Tensor, *, lowrank=None, rank1=(), c: Opt
         T, U = _rows2d(T), _rows2d(U)
         if T.shape[0] != M or U.shape[0] != N or T.shape[1] != U.shape[1]:
             raise ValueError(f"low-rank shapes {tuple(T.shape)} / {tuple(U.shape)} do not fit [{M}, r] / [{N}, r]")
-        keep += [T, U]
-        args.rank = T.shape[1]
-        args.lr_t, args.ldt = T.data_ptr(), T.stride(0)
-        args.lr_u, args.ldu = U.data_ptr(), U.stride(0)
     if len(rank1) > 2:
         raise ValueError("at most two rank-1 terms")
+    vectors = [None, None, None, None]                    # cvec0, rvec0, cvec1, rvec1
     for i, (cv, rv) in enumerate(rank1):
-        rv = rv.reshape(-1).to(torch.float32).contiguous()
-        assert rv.numel() == N and rv.is_cuda
-        keep.append(rv)
+        vectors[2 * i + 1] = _fp32_vector(rv, N)
         if cv is not None:
-            cv = cv.reshape(-1).to(torch.float32).contiguous()
-            assert cv.numel() == M and cv.is_cuda
-            keep.append(cv)
-        setattr(args, f"cvec{i}", _ptr(cv))
-        setattr(args, f"rvec{i}", rv.data_ptr())
+            vectors[2 * i] = _fp32_vector(cv, M)
+    if out is not None:
+        assert out.shape == (M, N) and out.dtype == out_dtype and out.stride(1) == 1
+    if c is not None:
+        assert c.shape == (M, N) and c.dtype == out_dtype and c.stride(1) == 1 and c.is_cuda
+    s = unit_a = unit_b = None
+    s_dtype = 0
+    if scaled is not None:
+        s, unit_a, unit_b = scaled
+        if s.dtype not in (torch.bfloat16, torch.float32):
+            s = s.float()
+        s = s.reshape(-1).contiguous()
+        assert s.numel() == N and s.device == dev
+        s_dtype = _dtype_code(s, "s")
+        _unit_ptr(unit_a, dev)
+        _unit_ptr(unit_b, dev)
     with _on_device(dev):
-        if out is None:
-            out = torch.empty((M, N), dtype=out_dtype, device=dev)
-        else:
-            assert out.shape == (M, N) and out.dtype == out_dtype and out.stride(1) == 1
-        if c is not None:
-            assert c.shape == (M, N) and c.dtype == out_dtype and c.stride(1) == 1 and c.is_cuda
-            args.c, args.ldc = c.data_ptr(), c.stride(0)
-        args.d, args.ldd = out.data_ptr(), out.stride(0)
-        args.d_dtype = _DTYPES[out_dtype]
-        args.reserved = int(_debug)
-        args.sm_limit = int(sm_limit)
-        args.status = _ptr(status)
-        args.stream = _stream()
-        ws_bytes = cabi.lib().metis_nvfp4_gemm_workspace_bytes(M, N, K) if M <= 128 else 0
-        if ws_bytes > 0:                      # decode-sized product: scratch for its split-K partial sums
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            keep.append(ws)
-            args.workspace, args.workspace_bytes = ws.data_ptr(), ws_bytes
-        if scaled is None:
-            rc = cabi.lib().metis_nvfp4_gemm(C.byref(args)) if rows_ready is None else \
-                cabi.lib().metis_nvfp4_gemm_joined(C.byref(args), rows_ready.cuda_event, None, 0, None, None, None)
-        else:
-            s, unit_a, unit_b = scaled
-            if s.dtype not in (torch.bfloat16, torch.float32):
-                s = s.float()
-            s = s.reshape(-1).contiguous()
-            assert s.numel() == N and s.device == dev
-            t = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-            more = (s.data_ptr(), _dtype_code(s, "s"), _unit_ptr(unit_a, dev), _unit_ptr(unit_b, dev), t.data_ptr())
-            rc = cabi.lib().metis_nvfp4_gemm_scaled(C.byref(args), *more) if rows_ready is None else \
-                cabi.lib().metis_nvfp4_gemm_joined(C.byref(args), rows_ready.cuda_event, *more)
-    cabi.check(rc, "metis_nvfp4_gemm")
+        rc, out, t, ws_bytes = cabi.host().gemm(M, N, K, float(alpha), a.codes, a.scales, a.unit, b.codes, b.scales, b.unit, T, U, *vectors, c, out,
+                                                _DTYPES[out_dtype], int(_debug), int(sm_limit), status, 0 if rows_ready is None else rows_ready.cuda_event,
+                                                s, s_dtype, unit_a, unit_b, _stream())
+    if rc:
+        cabi.check(rc, "metis_nvfp4_gemm")
     LAUNCHES["gemm"] += 2 if ws_bytes > 0 or scaled is not None else 1       # the sum of the splits, or the scaling
     return out if scaled is None else (out, t)
 

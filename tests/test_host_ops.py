@@ -1,0 +1,69 @@
+"""The native part of the tensor-level wrappers (csrc/host_ops.cpp): it takes positional arguments from ops.py only, and what does not
+fit is an exception, not a crash.  Its results are covered by every test of ops.py on a GPU."""
+import threading
+
+import pytest
+import torch
+
+from fp4_post_b200 import cabi, ops
+
+
+@pytest.fixture(scope="module")
+def host():
+    from fp4_post_b200.build import build
+    build()
+    return cabi.host()
+
+
+def test_arguments_that_do_not_fit_are_type_errors(host):
+    x = torch.zeros(16, 16)
+    for name in ("quantize", "quantize_dual", "quantize_dual_finish", "rmsnorm_quantize", "col_mean", "gemv", "lowrank_scale", "gemm"):
+        f = getattr(host, name)
+        with pytest.raises(TypeError):
+            f()
+        with pytest.raises(TypeError):
+            f(*["text"] * 40)
+    with pytest.raises(TypeError):
+        host.col_mean(x, 0)                        # no stream
+    with pytest.raises(TypeError):
+        host.col_mean(None, 0, 0)
+    with pytest.raises((TypeError, OverflowError)):
+        host.col_mean(x, 0, -1)
+
+
+def test_every_entry_point_it_knows_is_exported(host):
+    assert not host.bind("metis_no_such_entry", 0)
+    known = [n for n in cabi.EXPORTS if host.bind(n, cabi.C.cast(getattr(cabi.lib(), n), cabi.C.c_void_p).value)]
+    assert "metis_nvfp4_gemm" in known and len(known) == 14
+
+
+def test_rows_of_unusual_strides_get_a_leading_dimension():
+    one = torch.zeros(64).as_strided((1, 64), (1, 1))
+    assert one.is_contiguous() and ops._rows2d(one).stride(0) >= 64
+    wide = torch.zeros(4, 80)[:, :64]
+    assert ops._rows2d(wide).stride(0) == 80
+    assert ops._rows2d(torch.zeros(64, 4).T).stride(0) == 64
+
+
+@pytest.mark.gpu
+def test_calls_from_several_threads(host):
+    x = torch.randn(512, 1024, device="cuda").to(torch.bfloat16)
+    want = ops.nvfp4_quantize(x)
+    wrong = []
+
+    def work():
+        st = torch.cuda.Stream()
+        st.wait_stream(torch.cuda.default_stream())
+        with torch.cuda.stream(st):
+            for _ in range(50):
+                q = ops.nvfp4_quantize(x)
+                mean = ops.col_mean(x)
+                if not (torch.equal(q.codes, want.codes) and torch.equal(q.scales, want.scales) and mean.numel() == 1024):
+                    wrong.append(1)
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong
