@@ -114,18 +114,11 @@ def _backward_can_pack(shared) -> bool:
     return LinearLowbitFunction._packed_backward_ok(shared.source)
 
 
-def _bf16_factors(t32: torch.Tensor, u: torch.Tensor, act: torch.dtype):
-    """The rank-r factors as bf16 operands of the side product.  With bf16 activations they are
-    simply rounded (the reference computes them in bf16 too).  With fp32 activations each factor
-    is split into a bf16 head and tail and the product is issued as [Th Tl Th] [Uh Uh Ul]^T, which
-    keeps about 16 significant bits at three times the (small) rank."""
-    r = t32.shape[1]
-    if act != torch.float32 or 3 * r > 256:
-        return t32.to(torch.bfloat16), u.to(torch.bfloat16)
-    u32 = u.float()
-    t_hi, u_hi = t32.to(torch.bfloat16), u32.to(torch.bfloat16)
-    t_lo, u_lo = (t32 - t_hi.float()).to(torch.bfloat16), (u32 - u_hi.float()).to(torch.bfloat16)
-    return torch.cat([t_hi, t_lo, t_hi], dim=1), torch.cat([u_hi, u_hi, u_lo], dim=1)
+def _bf16_factors(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_b: torch.Tensor, u: torch.Tensor):
+    """The rank-r factors of an fp32 layer, (s . yv) / (unit_a * unit_b) and u, as bf16 operands of the side product.  Each is
+    split into a bf16 head and tail and the product is issued as [Th Tl Th] [Uh Uh Ul]^T, which keeps about 16 significant
+    bits at three times the (small) rank; where that is more than the product takes, they are rounded."""
+    return ops.lowrank_factors(yv, s, unit_a, unit_b, u.float().contiguous(), 1 if 3 * yv.shape[1] > 256 else 3)
 
 
 def _dual_ok(flat: torch.Tensor) -> bool:
@@ -949,8 +942,7 @@ class MetisFusedFunction(torch.autograd.Function):
         else:
             yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, rows_ready=v_ready)
             ready(rq)
-            ts = yv * s.to(act)
-            lowrank = _bf16_factors(ts.float() / (xa.q.unit * rq.q.unit), u_weight.detach(), act)
+            lowrank = _bf16_factors(yv, s.detach(), xa.q.unit, rq.q.unit, u_weight.detach())
         if bias_row is not None:
             here.wait_event(bias_done)
             bias_row.record_stream(here)

@@ -33,7 +33,7 @@ EXPORTS = (
     "metis_nvfp4_quantize_workspace_bytes", "metis_nvfp4_quantize", "metis_rmsnorm_nvfp4_quantize",
     "metis_nvfp4_dequantize", "metis_nvfp4_dequantize_ratio", "metis_col_mean_workspace_bytes", "metis_col_mean", "metis_nvfp4_gemv",
     "metis_nvfp4_gemm", "metis_nvfp4_gemm_scaled", "metis_nvfp4_gemm_joined", "metis_nvfp4_quantize_static", "metis_nvfp4_gemm_workspace_bytes",
-    "metis_lowrank_scale",
+    "metis_lowrank_scale", "metis_lowrank_factors",
     "metis_nvfp4_quantize_dual_workspace_bytes", "metis_nvfp4_quantize_dual", "metis_nvfp4_quantize_dual_finish",
     "metis_rmsnorm_mean_workspace_bytes", "metis_rmsnorm_mean",
     "metis_bf16_panel_gemm_workspace_bytes", "metis_bf16_panel_gemm",
@@ -123,6 +123,8 @@ def lib() -> C.CDLL:
     L.metis_nvfp4_gemm_joined.restype = i32
     L.metis_lowrank_scale.argtypes = [vp, i64, i64, i64, vp, i32, vp, vp, vp, vp]
     L.metis_lowrank_scale.restype = i32
+    L.metis_lowrank_factors.argtypes = [vp, i64, i64, i64, vp, i32, vp, vp, vp, vp, i64, i64, vp, i32, vp]
+    L.metis_lowrank_factors.restype = i32
     for name in ("metis_bf16_panel_gemm_workspace_bytes", "metis_lowrank_dts_workspace_bytes", "metis_lowrank_du_workspace_bytes"):
         getattr(L, name).argtypes = [i64, i64, i64]
         getattr(L, name).restype = i64

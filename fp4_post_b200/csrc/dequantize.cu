@@ -533,6 +533,39 @@ lowrank_scale_kernel(const __nv_bfloat16* __restrict__ yv, int64_t M, int64_t r,
   }
 }
 
+// The rank-r factors of an fp32 layer as bf16 operands of the side product, both in one launch: t32 = (yv * s) / (unit_a * unit_b)
+// and u, either rounded (kParts = 1) or split into a bf16 head and tail, [Th Tl Th] and [Uh Uh Ul] (kParts = 3).  One element
+// per thread and round: the operands are a few hundred KB, and what it replaced were a dozen launches of one operation
+// each (issued from Python 85 us of host time, 25 on the GPU at 2048 x 64; now 12 and 3).
+template <typename TS, int kParts>
+__global__ void __launch_bounds__(256)
+lowrank_factors_kernel(const float* __restrict__ yv, int64_t M, int64_t r, int64_t ldy, const TS* __restrict__ s, const float* __restrict__ unit_a,
+                       const float* __restrict__ unit_b, __nv_bfloat16* __restrict__ t, const float* __restrict__ u, int64_t N, int64_t ldu,
+                       __nv_bfloat16* __restrict__ u_out) {
+  grid_dependency_wait();
+  const float units = __fmul_rn(__ldg(unit_a), __ldg(unit_b));
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (M + N) * r; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t row = i / r, col = i - row * r;
+    const bool of_t = row < M;
+    float v;
+    if (of_t) {
+      float sv;
+      if constexpr (sizeof(TS) == 2) sv = __bfloat162float(s[col]); else sv = s[col];
+      v = __fdiv_rn(__fmul_rn(yv[row * ldy + col], sv), units);
+    } else {
+      v = u[(row - M) * ldu + col];
+    }
+    const __nv_bfloat16 head = __float2bfloat16_rn(v);
+    __nv_bfloat16* to = (of_t ? t + row * (kParts * r) : u_out + (row - M) * (kParts * r)) + col;
+    to[0] = head;
+    if constexpr (kParts == 3) {
+      const __nv_bfloat16 tail = __float2bfloat16_rn(__fsub_rn(v, __bfloat162float(head)));
+      to[r] = of_t ? tail : head;
+      to[2 * r] = of_t ? head : tail;
+    }
+  }
+}
+
 }  // namespace metis
 
 using namespace metis;
@@ -556,6 +589,27 @@ extern "C" int32_t metis_lowrank_scale(const void* yv, int64_t M, int64_t r, int
   else
     launch_overlapped(kLaunchShort, lowrank_scale_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, st, y, M, r, ld, static_cast<const float*>(s), unit_a, unit_b, o);
   METIS_CUDA_OK(cudaGetLastError());
+  return METIS_OK;
+}
+
+extern "C" int32_t metis_lowrank_factors(const float* yv, int64_t M, int64_t r, int64_t ldy, const void* s, int32_t s_dtype,
+                                         const float* unit_a, const float* unit_b, void* t, const float* u, int64_t N, int64_t ldu,
+                                         void* u_out, int32_t parts, void* stream) {
+  if (!yv || !s || !unit_a || !unit_b || !t || !u || !u_out) return fail(METIS_ERR_BAD_ARGUMENT, "null pointer");
+  if (M <= 0 || N <= 0 || r <= 0 || ldy < r || ldu < r) return fail(METIS_ERR_BAD_SHAPE, "bad shape [%lld, %lld], [%lld, %lld]", (long long)M, (long long)r, (long long)N, (long long)r);
+  if (s_dtype != METIS_DTYPE_BF16 && s_dtype != METIS_DTYPE_F32) return fail(METIS_ERR_BAD_ARGUMENT, "unknown s_dtype %d", s_dtype);
+  if (parts != 1 && parts != 3) return fail(METIS_ERR_BAD_ARGUMENT, "parts must be 1 or 3");
+  int64_t blocks = ceil_div((M + N) * r, 256);
+  if (blocks > (int64_t)device_sm_count() * 16) blocks = (int64_t)device_sm_count() * 16;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto run = [&](auto kern, auto* sv) {
+    return launch_overlapped(kLaunchShort, kern, dim3((unsigned)blocks), dim3(256), 0, st, yv, M, r, ldy, sv, unit_a, unit_b, static_cast<__nv_bfloat16*>(t), u, N,
+                             ldu, static_cast<__nv_bfloat16*>(u_out));
+  };
+  const __nv_bfloat16* s16 = static_cast<const __nv_bfloat16*>(s);
+  const float* s32 = static_cast<const float*>(s);
+  METIS_CUDA_OK(s_dtype == METIS_DTYPE_BF16 ? (parts == 3 ? run(lowrank_factors_kernel<__nv_bfloat16, 3>, s16) : run(lowrank_factors_kernel<__nv_bfloat16, 1>, s16))
+                                            : (parts == 3 ? run(lowrank_factors_kernel<float, 3>, s32) : run(lowrank_factors_kernel<float, 1>, s32)));
   return METIS_OK;
 }
 

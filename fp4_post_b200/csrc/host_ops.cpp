@@ -25,7 +25,7 @@ namespace {
   X(metis_nvfp4_quantize) X(metis_nvfp4_quantize_workspace_bytes) X(metis_nvfp4_quantize_dual)                                  \
   X(metis_nvfp4_quantize_dual_workspace_bytes) X(metis_nvfp4_quantize_dual_finish) X(metis_rmsnorm_nvfp4_quantize)              \
   X(metis_col_mean) X(metis_col_mean_workspace_bytes) X(metis_nvfp4_gemv) X(metis_nvfp4_gemm) X(metis_nvfp4_gemm_scaled)       \
-  X(metis_nvfp4_gemm_joined) X(metis_nvfp4_gemm_workspace_bytes) X(metis_lowrank_scale)
+  X(metis_nvfp4_gemm_joined) X(metis_nvfp4_gemm_workspace_bytes) X(metis_lowrank_scale) X(metis_lowrank_factors)
 struct Entries {
 #define X(name) decltype(&::name) name = nullptr;
   METIS_HOST_ENTRIES(X)
@@ -286,6 +286,28 @@ PyObject* lowrank_scale(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   METIS_HOST_END
 }
 
+// yv [M, r] fp32, s, its dtype code, unit_a, unit_b, u [N, r] fp32, parts, stream -> t, u as bf16
+PyObject* lowrank_factors(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  METIS_HOST_BEGIN(args, nargs)
+  const at::Tensor &yv = a.tensor(), &s = a.tensor();
+  const int32_t s_dtype = (int32_t)a.i64();
+  const at::Tensor &unit_a = a.tensor(), &unit_b = a.tensor(), &u = a.tensor();
+  const int64_t parts = a.i64();
+  void* stream = a.address();
+  const int64_t M = yv.size(0), r = yv.size(1), N = u.size(0);
+  at::Tensor t, u_out;
+  int32_t rc;
+  {
+    NoGil free_;
+    t = at::empty({M, parts * r}, yv.options().dtype(at::kBFloat16));
+    u_out = at::empty({N, parts * r}, yv.options().dtype(at::kBFloat16));
+    rc = lib.metis_lowrank_factors(ptr<float>(yv), M, r, yv.stride(0), s.data_ptr(), s_dtype, ptr<float>(unit_a), ptr<float>(unit_b), t.data_ptr(),
+                                   ptr<float>(u), N, u.stride(0), u_out.data_ptr(), (int32_t)parts, stream);
+  }
+  return result(rc, {t, u_out});
+  METIS_HOST_END
+}
+
 // M, N, K, alpha, codes, scales, unit of A, of B, T or None, U or None, cvec0, rvec0, cvec1, rvec1 (None where there is none), C or None,
 // D or None, dtype code of D, debug bits, SM limit, status or None, rows_ready (address or 0), s or None, its dtype code, unit_a, unit_b,
 // stream -> D, scaled copy or None, bytes of workspace the product was given (as a number behind the tensors)
@@ -362,7 +384,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 #define METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {METHOD(quantize), METHOD(quantize_dual), METHOD(quantize_dual_finish), METHOD(rmsnorm_quantize), METHOD(col_mean),
-                         METHOD(gemv), METHOD(lowrank_scale), METHOD(gemm), METHOD(bind), {nullptr, nullptr, 0, nullptr}};
+                         METHOD(gemv), METHOD(lowrank_scale), METHOD(lowrank_factors), METHOD(gemm), METHOD(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "metis_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

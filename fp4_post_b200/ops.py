@@ -421,6 +421,28 @@ def lowrank_scale(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_
     return out
 
 
+def lowrank_factors(yv: torch.Tensor, s: torch.Tensor, unit_a: torch.Tensor, unit_b: torch.Tensor, u: torch.Tensor, parts: int):
+    """(yv * s) / (unit_a * unit_b) [M, r] and u [N, r] as bf16 operands of the side product, for fp32 yv and u: rounded (parts = 1)
+    or split into head and tail (parts = 3: [Th Tl Th] and [Uh Uh Ul], [M, 3r] and [N, 3r])."""
+    _need_cuda(yv, "yv")
+    _need_cuda(u, "u")
+    for name, t in (("yv", yv), ("u", u)):
+        if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1 or (t.shape[0] > 1 and t.stride(0) < t.shape[1]):
+            raise TypeError(f"{name} must be an fp32 matrix with contiguous rows")
+    if s.dtype not in (torch.bfloat16, torch.float32):
+        s = s.float()
+    s = s.reshape(-1).contiguous()
+    assert s.numel() == yv.shape[1] == u.shape[1] and s.device == yv.device == u.device
+    _unit_ptr(unit_a, yv.device)
+    _unit_ptr(unit_b, yv.device)
+    with _on_device(yv.device):
+        rc, t, u_out = cabi.host().lowrank_factors(yv, s, _dtype_code(s, "s"), unit_a, unit_b, u, parts, _stream())
+    if rc:
+        cabi.check(rc, "metis_lowrank_factors")
+    LAUNCHES["gemv"] += 1
+    return t, u_out
+
+
 def _fp32_vector(t: torch.Tensor, n: int) -> torch.Tensor:
     if t.dim() != 1 or t.dtype != torch.float32 or not t.is_contiguous():
         t = t.reshape(-1).to(torch.float32).contiguous()

@@ -305,6 +305,16 @@ int32_t metis_lowrank_scale(const void* yv, int64_t M, int64_t r, int64_t ld, co
                             void* stream);
 
 /*
+ * Both factors of the side product of an fp32 layer: t32 = (yv * s) / (unit_a * unit_b) for yv [M, r] fp32 (row pitch ldy)
+ * and u [N, r] fp32 (row pitch ldu), as bf16.  parts = 1: rounded, [M, r] and [N, r].  parts = 3: split into a bf16 head and
+ * tail, rows [Th Tl Th] of t [M, 3r] and [Uh Uh Ul] of u_out [N, 3r], which keeps about 16 significant bits.  s is bf16
+ * or fp32 [r]; t and u_out are dense.
+ */
+int32_t metis_lowrank_factors(const float* yv, int64_t M, int64_t r, int64_t ldy, const void* s, int32_t s_dtype,
+                              const float* unit_a, const float* unit_b, void* t, const float* u, int64_t N, int64_t ldu,
+                              void* u_out, int32_t parts, void* stream);
+
+/*
  * D[M,N] = g * ( sum_k A[m,k] B[n,k]  +  sum_j T[m,j] U[n,j] )
  *          + cvec0[m]*rvec0[n] + cvec1[m]*rvec1[n]  ( + C[m,n] )
  * with g = alpha * (*a_unit) * (*b_unit).

@@ -17,7 +17,7 @@ def host():
 
 def test_arguments_that_do_not_fit_are_type_errors(host):
     x = torch.zeros(16, 16)
-    for name in ("quantize", "quantize_dual", "quantize_dual_finish", "rmsnorm_quantize", "col_mean", "gemv", "lowrank_scale", "gemm"):
+    for name in ("quantize", "quantize_dual", "quantize_dual_finish", "rmsnorm_quantize", "col_mean", "gemv", "lowrank_scale", "lowrank_factors", "gemm"):
         f = getattr(host, name)
         with pytest.raises(TypeError):
             f()
@@ -34,7 +34,7 @@ def test_arguments_that_do_not_fit_are_type_errors(host):
 def test_every_entry_point_it_knows_is_exported(host):
     assert not host.bind("metis_no_such_entry", 0)
     known = [n for n in cabi.EXPORTS if host.bind(n, cabi.C.cast(getattr(cabi.lib(), n), cabi.C.c_void_p).value)]
-    assert "metis_nvfp4_gemm" in known and len(known) == 14
+    assert "metis_nvfp4_gemm" in known and len(known) == 15
 
 
 def test_rows_of_unusual_strides_get_a_leading_dimension():

@@ -112,3 +112,22 @@ def test_dequantized_in_a_ratio_of_units():
     got = ops.nvfp4_dequantize_ratio(q, torch.bfloat16, *units)
     want = ops.nvfp4_dequantize(q, torch.bfloat16, unit=(units[0] * units[1]) / (units[2] * units[3]))
     assert torch.equal(got, want)
+
+
+# Bit for bit the torch expressions: more elements than one round of the grid, a row and a half, subnormal tails, a pitch.
+@pytest.mark.parametrize("M,N,r,parts", [(2048, 2048, 64, 3), (16384, 8960, 64, 3), (1, 16, 8, 3), (300, 50, 128, 1)])
+@pytest.mark.parametrize("s_dtype", [torch.bfloat16, torch.float32])
+def test_factors_of_an_fp32_layer(M, N, r, parts, s_dtype):
+    g = torch.Generator(device=DEV).manual_seed(M + r)
+    store = torch.randn(M, r + 8, generator=g, device=DEV) * torch.exp(8 * torch.randn(M, 1, generator=g, device=DEV))
+    yv = store[:, :r]
+    u, s = torch.randn(N, r, generator=g, device=DEV), torch.rand(r, generator=g, device=DEV).to(s_dtype)
+    ua, ub = torch.tensor([0.37], device=DEV), torch.tensor([1.9e-3], device=DEV)
+    t, u_out = ops.lowrank_factors(yv, s, ua, ub, u, parts)
+    t32 = (yv * s.float()) / (ua * ub)
+
+    def split(v, order):
+        head = v.to(torch.bfloat16)
+        pieces = (head, (v - head.float()).to(torch.bfloat16))
+        return torch.cat([pieces[i] for i in order], dim=1) if parts == 3 else head
+    assert torch.equal(t, split(t32, (0, 1, 0))) and torch.equal(u_out, split(u, (0, 0, 1)))
