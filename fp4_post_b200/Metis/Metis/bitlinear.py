@@ -558,9 +558,9 @@ _BRANCH = 0          # which member of a projection group is being issued (forwa
 
 
 def _aux_stream(device: torch.device, index: int = 0) -> "torch.cuda.Stream":
-    """A side stream of `device` for work that may overlap the current stream's.  Index 0: the low-rank branch and
-    the mean's row vectors; 1: the mean row of the input gradient, the cast of the bias; 2, 4: deferred scale passes (activations and
-    gradients, weights); 3: members of a projection group (forward_group); 5: the weights' quantization."""
+    """A side stream of `device` for work that may overlap the current stream's.  Index 0: the low-rank branch, the mean's
+    row vector with V, the cast of the bias; 1: the mean's row vectors with the residual weight (both directions); 2, 4: deferred
+    scale passes (activations and gradients, weights); 3: members of a projection group (forward_group); 5: the weights' quantization."""
     # the streams of deferred scale passes (2, 4) yield to everything else: their results are wanted last.  Not in a
     # data-parallel step: the collectives' kernel (default priority) would queue behind every side stream for the
     # SMs the capped GEMM leaves it
@@ -895,33 +895,38 @@ class MetisFusedFunction(torch.autograd.Function):
             if not overlap:
                 ready(vq)
                 ready(rq)
-            if overlap and bias is not None and bias.dtype != torch.float32:
-                # The bias is cast beside the product too, on a stream of its own: `mean_event` says nothing about it (a
-                # grouped activation's event is that of the call that quantized it, and the bias may have been written
-                # since), so an event of this call orders the cast behind whatever the current stream has queued.
-                here, side = current_stream(xa.mean.device), _aux_stream(xa.mean.device, 1)
-                side.wait_event(recorded_event(here))
-                with on_stream(side):
-                    bias_row = bias.float()
-                    bias_done = recorded_event(side)
             if overlap:
                 # Each on a stream of its own: the pass over the (much larger) residual weight waits for nothing of the one over V.
                 # A product joins its row vector when it needs it (rows_ready), which a product split along K does at its end.
                 dev = xa.mean.device
                 main = current_stream(dev)
 
-                def beside(op, index):
+                def beside(op, index, also=None):
                     side = _aux_stream(dev, index)
                     side.wait_event(xa.mean_event)
                     if op.ready_event is not None:              # quantized on a stream of its own: order this one after it
                         side.wait_event(op.ready_event)
                     with on_stream(side):
                         row = ops.nvfp4_gemv(op.q, xa.mean)
+                        if also is not None:
+                            side.wait_event(also)
                         done = recorded_event(side)
                     row.record_stream(main)
                     return row, done
                 row_v, v_ready = beside(vq, 0)
-                row_r, r_ready = beside(rq, 1)
+                bias_done = None
+                if bias is not None and bias.dtype != torch.float32:
+                    # The bias is cast beside the product too, behind the pass over V (not in front of the long one over the
+                    # residual weight: a decoder block of 64 tokens takes 188.7 us, 191.1 with it there).  `mean_event` says
+                    # nothing about it (a grouped activation's event is that of the call that quantized it, and the bias may have
+                    # been written since), so an event of this call orders the cast behind whatever the current stream has queued.
+                    side = _aux_stream(dev, 0)
+                    side.wait_event(recorded_event(main))
+                    with on_stream(side):
+                        bias_row = bias.float()
+                        bias_done = recorded_event(side)
+                    bias_row.record_stream(main)
+                row_r, r_ready = beside(rq, 1, bias_done)       # r_ready: both vectors of the residual product
             else:
                 row_v, row_r = ops.nvfp4_gemv(vq.q, xa.mean), ops.nvfp4_gemv(rq.q, xa.mean)
             rank1_v.append((None, row_v))
@@ -943,9 +948,6 @@ class MetisFusedFunction(torch.autograd.Function):
             yv = _packed_matmul(xa.q, vq.q, rank1=rank1_v, out_dtype=act, rows_ready=v_ready)
             ready(rq)
             lowrank = _bf16_factors(yv, s.detach(), xa.q.unit, rq.q.unit, u_weight.detach())
-        if bias_row is not None:
-            here.wait_event(bias_done)
-            bias_row.record_stream(here)
         ready(rq)
         y = _packed_matmul(xa.q, rq.q, rank1=rank1_r, lowrank=lowrank, out_dtype=act, rows_ready=r_ready)
         if (MetisFusedFunction.concurrent_branches and xa.q.codes.is_cuda and any(ctx.needs_input_grad)
