@@ -586,7 +586,7 @@ __device__ __noinline__ void finish_edge(const float* from, int64_t row_pitch, i
 // the row (the whole of it where its sum is wanted); a CTA takes 64 / tx items at once.
 // Bound by issue: edges, padding and divisions stay out of the unrolled path (62 instructions per block with them and with
 // scalar arithmetic, 27 with packed arithmetic alone).  One output / both / both with token sums, us: 16384 x 4096
-// 11.2 / 21.0 / 28.2 before that, 5.8 / 10.4 / 21.2 now; 65536 x 4096 32 / 62 / 79 and 16 / 30 / 67 (the bytes alone take
+// 11.2 / 21.0 / 28.2 before that, 6.6 / 10.4 / 19.7 now; 65536 x 4096 32 / 62 / 79 and 17 / 30 / 67 (the bytes alone take
 // 13 / 26 / 46); 64 x 18944, one output, 4.0 and 2.8.
 constexpr int kFinThreads = 128;
 // What the jobs of a launch want: no row sums, every row made of whole groups of four blocks; no row sums; sums, four rows to
