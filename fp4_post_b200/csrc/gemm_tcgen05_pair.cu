@@ -16,18 +16,19 @@
 //   full[s]      leader's: all bytes of stage s of BOTH CTAs (the peer's TMA loads signal it remotely)
 //   empty[s]     local: stage s consumed (commit multicast by the leader to both CTAs)
 //   acc_full     local: accumulator complete (commit multicast)
-//   acc_release  leader's: the epilogue warps of both CTAs that read shared accumulator columns have drained them
+//   acc_release  leader's: every epilogue warp of both CTAs has drained its shared accumulator columns of this tile, and all of the
+//                tile before (pair_drain.cuh has the whole condition)
 // No copy is multicast.  Every wait is bounded; both CTAs meet at a cluster barrier before they
 // free tensor memory, so neither exits while the other can still signal or read it.
 #include "gemm_common.cuh"
+#include "pair_drain.cuh"
 
 namespace metis {
 
 struct PairCfg {
   static constexpr int BN = 256;
   static constexpr int kStages = 5;
-  static constexpr int kAccStride = 160;
-  static constexpr int kSharedChunks = 3;
+  static constexpr int kAccStride = PairDrain::kStride;
   static constexpr int kABytes = kBM * kBKBytes;          // 16 KiB: this CTA's 128 rows of A
   static constexpr int kBBytes = 128 * kBKBytes;          // 16 KiB: this CTA's 128 rows of B
   static constexpr int kSfaBytes = 4 * 512;               // scales of this CTA's rows of A
@@ -122,7 +123,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   using Cfg = PairCfg;
   constexpr int kStages = Cfg::kStages;
   constexpr int BN = Cfg::BN;
-  constexpr int kReleasing = kParts < Cfg::kSharedChunks ? kParts : Cfg::kSharedChunks;     // warps of a quarter that read shared columns
+  static_assert(PairDrain::kChunks * 32 == BN);
 
   extern __shared__ uint8_t smem_raw[];
   // the dynamic window starts at the same offset in both CTAs, so this rounding gives both the
@@ -158,7 +159,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
-    mbar_init(acc_release, 2 * 4 * kReleasing);
+    mbar_init(acc_release, PairDrain::arrivals(kParts));
     mbar_init(drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -364,18 +365,14 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       tc_fence_after();
       const uint32_t odd = local_tile & 1u;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + odd * Cfg::kAccStride;
-      // drain order: the 3 chunks shared with the other accumulator first.  For the even
-      // accumulator [0,256) they are its last chunks, for the odd one [160,416) its first ones.
-      constexpr int kChunks = BN / 32;
-      const int first_chunk = !odd ? kChunks - Cfg::kSharedChunks : 0;
-      int ch[kChunks / kParts];
+      int ch[PairDrain::kChunks / kParts];
 #pragma unroll
-      for (int k = 0; k < kChunks / kParts; ++k) ch[k] = (first_chunk + part + kParts * k) & (kChunks - 1);
-      // this warp's first chunks cover its part of the shared columns (drain index 0 and 2 or 1; 0, 1 or 2):
-      // pull them into registers and hand the columns to the next tile's MMAs at once
+      for (int k = 0; k < PairDrain::kChunks / kParts; ++k) ch[k] = PairDrain::chunk(kParts, part, k, odd);
+      // this warp's first chunks cover its part of the shared columns: pull them into registers and hand the columns
+      // to the next tile's MMAs at once
       constexpr int kBuffers = 4 / kParts;
       uint32_t ra[32];
-      if constexpr (kParts == 2) {
+      if constexpr (PairDrain::before_release(kParts) == 2) {
         uint32_t rb[32];
         tc_load32(t_row + ch[0] * 32, ra);
         tc_load32(t_row + ch[1] * 32, rb);
@@ -398,7 +395,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         tc_wait_ld(ra);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0 && part < kReleasing) mbar_arrive_cluster(release_leader);
+        if (lane == 0) mbar_arrive_cluster(release_leader);
         emit_chunk<TD, kBuffers>(ctx, ra, n0 + ch[0] * 32);
         tc_load32(t_row + ch[1] * 32, ra);
         tc_wait_ld(ra);
