@@ -9,7 +9,7 @@
 //
 // Roles per CTA (320 or 576 threads): warp 0 TMA producer, warp 1 tensor-core issuer (leader only),
 // warps 2-9 or 2-17 epilogue (two or four warps per 32-lane quarter of tensor memory, alternate column chunks;
-// epilogue_parts has the rule).  The scale tiles travel shared memory -> tensor memory by tcgen05.cp issued
+// pair_epilogue_parts has the rule).  The scale tiles travel shared memory -> tensor memory by tcgen05.cp issued
 // by the leader in front of each stage's MMAs: one instruction copies in both CTAs, in pipe order
 // with the MMAs, so no cross-SM handshake sits inside the pipeline loop (a handshake through the
 // peer costs a cluster round trip of more than a thousand cycles per two stages).
@@ -417,18 +417,6 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
 // ---- host side ----------------------------------------------------------------------------------------------
 
-// Epilogue warps per lane quarter.  Four of them take half the time for a tile, which is what bounds short products (a tile
-// of 8192 x 8192 x 512: 3.3 -> 2.9 us, with a row vector 4.6 -> 3.4) and the last tile of every product.  With a row vector
-// (rvec0) and many rounds of long tiles two are faster: the vector's broadcast loads take shared-memory bandwidth that the
-// operands need, and four warps ask for it while the next tile starts.  Two / four, us: without one 8192 x 8192 x 1024
-// 51.1 / 48.4, x 2048 71.4 / 69.1, x 4096 114.2 / 112.9, 4096 x 14336 x 4096 128.2 / 124.9; with one 8192 x 8960 x 1536
-// 79.3 / 75.3, 1120 x 3584 x 3584 (one round) 14.2 / 13.0, 1024 x 18944 x 3584 (four) 36.9 / 36.5, but (14 to 16 rounds) 8192 x
-// 8192 x 2048 78.0 / 80.4, x 4096 122.9 / 127.2, 4096 x 18944 x 3584 131.5 / 135.6.
-static int epilogue_parts(const GemmParams& p, int64_t rounds) {
-  const int64_t stages = ceil_div(p.K, 256) + ceil_div(p.rank, 64);
-  return p.rvec0 && stages >= 10 && rounds > 4 ? 2 : 4;
-}
-
 template <typename TD, int kParts>
 static int32_t launch_pair_t(const metis_gemm_args* a, const CUtensorMap* maps, const GemmParams& p, int64_t pairs) {
   auto kern = nvfp4_gemm_pair_kernel<TD, kParts>;
@@ -462,7 +450,8 @@ int32_t launch_gemm_pair(const metis_gemm_args* a, const CUtensorMap& ma, const 
   // and on 64, and the SMs left over are free for whatever runs beside this product
   const int64_t rounds = ceil_div(tiles, pairs);
   pairs = ceil_div(tiles, rounds);
-  const bool four = epilogue_parts(p, rounds) == 4;
+  const int64_t stages = ceil_div(p.K, 256) + ceil_div(p.rank, 64);
+  const bool four = pair_epilogue_parts(stages, rounds, (p.rvec0 != nullptr) + (p.rvec1 != nullptr), p.c != nullptr, a->d_dtype == METIS_DTYPE_F32) == 4;
   // the scale arrays as [tiles, 512 bytes]: one box = the 4 tiles (2 KiB) of one stage and row block
   const int64_t sf_tiles_k = sf_tiles_per_row(a->K);
   CUtensorMap maps[7] = {ma, mb, {}, {}, mt, mu, {}};

@@ -63,10 +63,11 @@ def test_fused_low_rank_product(M, N, K, rank):
     assert rel_l2(got, want) <= 1e-5, rel_l2(got, want)
 
 
-# Two or four epilogue warps per lane quarter (pair kernel): with a row vector, ten pipeline stages and more than four rounds of
-# tiles two, else four.  Each side of the three lines, edges of D inside a 32-column chunk and a row block; few SMs give many rounds.
+# Two or four epilogue warps per lane quarter (pair kernel), by stages, rounds of tiles and vectors (test_pair_drain.py has the lines): two and four
+# with row vectors and without, edges of D inside a 32-column chunk and a row block; few SMs give many rounds.
 @pytest.mark.parametrize("M,N,K,rank,row,sms", [(1300, 1096, 2560, 0, True, 8), (1300, 1096, 2304, 0, True, 8), (1300, 1096, 2304, 64, True, 8),
-                                                (1300, 1096, 2560, 0, False, 8), (1300, 1096, 2560, 0, True, 14), (1300, 1096, 2560, 0, True, 0)])
+                                                (1300, 1096, 2560, 0, False, 8), (1300, 1096, 2560, 0, True, 14), (1300, 1096, 2560, 0, True, 0),
+                                                (1300, 1096, 4096, 0, True, 8), (1300, 1096, 3840, 64, True, 8), (1300, 1096, 1280, 0, False, 8)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
     qa, qb, da, db = operands(M, N, K, seed=K + rank)
