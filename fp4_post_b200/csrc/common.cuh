@@ -296,7 +296,7 @@ struct PhiloxKeys {
     }
   }
 };
-// Counter words {block, 0, offset}: block indexes stay below 2^32 (the entry points refuse more, kMaxStochasticElements;
+// Counter words {block, 0, offset}: block indexes stay below 2^32 (the entry points refuse more, kMaxElements;
 // this GPU's memory does not hold such a tensor and its codes), and with the second word known to be zero the first
 // round's product with c2 and the second round's with c0 are the same for the whole launch: the compiler takes them
 // out of the loop.  (One wide multiplication in place of each pair of high and low products was measured slower:

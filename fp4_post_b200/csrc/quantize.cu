@@ -139,7 +139,7 @@ template <typename T> struct TileCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 2 * kCols * 4 + 64 + 1024;
 };
 constexpr int64_t kTileRowsMinElements = 1 << 20;          // row-major tensors from this size on go through the tile kernel
-constexpr int64_t kMaxStochasticElements = (int64_t)1 << 36;   // blocks are counted in 32 bits (struct Philox)
+constexpr int64_t kMaxElements = (int64_t)1 << 36;         // blocks are counted in 32 bits (TileWalk, philox4x32)
 constexpr uint64_t kColumnStream = 1ull << 63;             // Philox counter space of the transposed output in dual mode
 
 // Workspace of the dual quantizer: word 63 = number of CTA records, records from word 64 on (3 words per CTA),
@@ -150,7 +150,7 @@ constexpr int kDualHeaderBytes = 256 + ((kDualMaxCtas * 3 * 4 + 255) / 256) * 25
 // How a CTA walks the tiles: their number, those along a row of x, and gridDim.x split into whole rows of tiles
 // and a remainder; blocks per row of Q (bpr) and of Qt (bpc), and what a step and the wrap to the next row of tiles add to the index
 // of a tile's first block in Q (_r) and in Qt (_t).  Block indexes are counted modulo 2^32 and a tensor has fewer blocks
-// (launch_tile), so the additions end in the right place whichever way they wrap.
+// (kMaxElements), so the additions end in the right place whichever way they wrap.
 struct TileWalk {
   uint32_t tiles, col_tiles, step_rows, step_cols;
   uint32_t bpr, bpc, step_r, wrap_r, step_t, wrap_t;
@@ -1228,7 +1228,7 @@ extern "C" int32_t metis_nvfp4_quantize(const void* x, int32_t x_dtype, int64_t 
     return fail(METIS_ERR_BAD_ALIGNMENT, "x must be 16-byte aligned with cols and ld multiples of %lld", (long long)need);
   if (col_mean && !aligned16(col_mean)) return fail(METIS_ERR_BAD_ALIGNMENT, "col_mean must be 16-byte aligned");
   if (rows >= ((int64_t)1 << 31) || cols >= ((int64_t)1 << 31)) return fail(METIS_ERR_TOO_LARGE, "tensor too large");
-  if (sr && rows * cols >= kMaxStochasticElements) return fail(METIS_ERR_TOO_LARGE, "stochastic rounding of 2^36 elements or more");
+  if (rows * cols >= kMaxElements) return fail(METIS_ERR_TOO_LARGE, "tensor of 2^36 elements or more");
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // With METIS_QUANTIZE_EXTRA_WORKSPACE bytes more than it needs the workspace also holds a record per CTA of the first
@@ -1328,7 +1328,7 @@ extern "C" int32_t metis_nvfp4_quantize_dual(const void* x, int32_t x_dtype, int
     return fail(METIS_ERR_WORKSPACE, "workspace of %lld bytes, need %lld", (long long)workspace_bytes,
                 (long long)metis_nvfp4_quantize_dual_workspace_bytes(rows, cols));
   if (rows >= ((int64_t)1 << 31) || cols >= ((int64_t)1 << 31)) return fail(METIS_ERR_TOO_LARGE, "tensor too large");
-  if (sr && rows * cols >= kMaxStochasticElements) return fail(METIS_ERR_TOO_LARGE, "stochastic rounding of 2^36 elements or more");
+  if (rows * cols >= kMaxElements) return fail(METIS_ERR_TOO_LARGE, "tensor of 2^36 elements or more");
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // every CTA of the first pass leaves its maxima and its error word in a record of its own: nothing to zero first

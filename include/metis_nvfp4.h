@@ -130,9 +130,9 @@ int64_t metis_nvfp4_quantize_workspace_bytes(int64_t R, int64_t C);
  * By default the hardware conversion cvt.rs.satfinite.e2m1x4.f32 does it: 8 random bits per element, up with
  * probability floor(256 p) / 256.  METIS_Q_SR16 selects the software form with 16 random bits per element
  * (floor(index + U), U in steps of 2^-16), about 8 more instructions per element.  The random bits are
- * Philox4x32-10(seed; block index, offset), one call per block of 16; the block index has 32 bits, and stochastic
- * calls with 2^36 elements or more are rejected with METIS_ERR_TOO_LARGE.  With METIS_Q_OFFSET_ON_DEVICE the offset is not
- * the argument's value but the content of the device uint64 it points to (8-byte aligned),
+ * Philox4x32-10(seed; block index, offset), one call per block of 16.  Block indexes have 32 bits: calls with 2^36
+ * elements or more are rejected with METIS_ERR_TOO_LARGE (with its codes and scales a bf16 tensor of that size takes 193 GB, more
+ * than the device has).  With METIS_Q_OFFSET_ON_DEVICE the offset is not the argument's value but the content of the device uint64 it points to (8-byte aligned),
  * and the call adds 1 to that counter when its kernels have read it: successive calls on one
  * stream draw fresh bits although their arguments are identical, which is what a captured
  * CUDA graph needs when it is replayed (the reference's torch.rand advances a device-side
