@@ -64,6 +64,7 @@ class GemmArgs(C.Structure):
 
 _lib = None
 _host = None
+_host_lib = None            # the library whose entry points _host has
 
 
 class MetisLibraryError(RuntimeError):
@@ -142,28 +143,26 @@ def lib() -> C.CDLL:
     L.metis_rope_pair.restype = i32
     L.metis_silu_mul.argtypes = [vp, vp, vp, i64, vp]
     L.metis_silu_mul.restype = i32
-    _bind_host(L)
     _lib = L
     return L
 
 
-def _bind_host(L: C.CDLL) -> None:
-    """Load the native part of the wrappers in ops.py once and give it the entry points of L."""
-    global _host
-    if _host is None:
-        if not HOST_PATH.exists():
-            raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build`")
-        spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
-        _host = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(_host)
-    for name in EXPORTS:
-        _host.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
-
-
 def host():
-    """The native wrappers (csrc/host_ops.cpp): allocations and call in one; every function returns (status, tensors...)."""
-    if _host is None or _lib is None:
-        lib()
+    """The native part of the wrappers in ops.py (csrc/host_ops.cpp), with the entry points of lib(): allocations and call in one; every
+    function returns (status, tensors...).  Callers of the C entry points alone do without it."""
+    global _host, _host_lib
+    L = lib()
+    if _host_lib is not L:
+        if _host is None:
+            if not HOST_PATH.exists():
+                raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build`")
+            spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _host = module
+        for name in EXPORTS:
+            _host.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
+        _host_lib = L
     return _host
 
 

@@ -37,6 +37,15 @@ def test_every_entry_point_it_knows_is_exported(host):
     assert "metis_nvfp4_gemm" in known and len(known) == 15
 
 
+def test_the_c_entry_points_do_without_it(host, monkeypatch, tmp_path):
+    for name in ("_lib", "_host", "_host_lib"):
+        monkeypatch.setattr(cabi, name, None, raising=False)
+    monkeypatch.setattr(cabi, "HOST_PATH", tmp_path / "nothing.so")
+    assert cabi.lib().metis_nvfp4_sf_bytes(128, 64, cabi.SF_MMA) > 0
+    with pytest.raises(cabi.MetisLibraryError):
+        cabi.host()
+
+
 def test_rows_of_unusual_strides_get_a_leading_dimension():
     one = torch.zeros(64).as_strided((1, 64), (1, 1))
     assert one.is_contiguous() and ops._rows2d(one).stride(0) >= 64
