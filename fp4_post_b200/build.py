@@ -2,8 +2,8 @@
 
     python -m fp4_post_b200.build        # or: from fp4_post_b200.build import build; build()
 
-Output: fp4_post_b200/_lib/libmetis_nvfp4.so, and _lib/metis_host.so, the native part of the tensor-level wrappers (g++ against
-the installed torch).  nvcc cross-compiles without a GPU.
+Output: fp4_post_b200/_lib/libmetis_nvfp4.so, and cabi.HOST_PATH, the native part of the tensor-level wrappers (g++ against the
+installed torch and Python, whose versions are in its name).  nvcc cross-compiles without a GPU.
 
     python -m fp4_post_b200.build --timing-knobs
 
@@ -22,13 +22,14 @@ import sys
 import sysconfig
 from pathlib import Path
 
+from .cabi import HOST_PATH
+
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_lib"
 LIB = OUT_DIR / "libmetis_nvfp4.so"
 KNOBS_LIB = OUT_DIR / "libmetis_nvfp4_knobs.so"
 HOST_SOURCE = CSRC / "host_ops.cpp"
-HOST_MODULE = OUT_DIR / "metis_host.so"
 SOURCES = ["api.cu", "quantize.cu", "rmsnorm_quant.cu", "dequantize.cu", "gemm_tcgen05.cu", "gemm_tcgen05_pair.cu", "lowrank_bwd.cu", "decoder_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -57,7 +58,7 @@ def _host_command() -> list[str]:
     root = Path(torch.__file__).resolve().parent
     include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            *(f"-I{p}" for p in include), str(HOST_SOURCE), "-o", str(HOST_MODULE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+            *(f"-I{p}" for p in include), str(HOST_SOURCE), "-o", str(HOST_PATH), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
 
 
 def build(force: bool = False, verbose: bool = False, timing_knobs: bool = False) -> Path:
@@ -81,7 +82,7 @@ def build(force: bool = False, verbose: bool = False, timing_knobs: bool = False
                 print(" ".join(cmd), file=sys.stderr)
             procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     host = None
-    if not timing_knobs and (force or _stale(HOST_MODULE, [HOST_SOURCE, PKG.parent / "include" / "metis_nvfp4.h"])):
+    if not timing_knobs and (force or _stale(HOST_PATH, [HOST_SOURCE, PKG.parent / "include" / "metis_nvfp4.h"])):
         host = subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     failed = []
     for src, p in procs:

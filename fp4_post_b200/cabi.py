@@ -7,11 +7,14 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib.util
+import sysconfig
 from pathlib import Path
 
-import torch  # noqa: F401  (the native wrappers below link against it: it has to be loaded first)
+import torch                # the native wrappers below link against it: it has to be loaded first
 
-HOST_PATH = Path(__file__).resolve().parent / "_lib" / "metis_host.so"
+# The native part of the wrappers is compiled against one torch and one Python: their versions are in its name, so that no other
+# loads it and build.py makes one for each.
+HOST_PATH = Path(__file__).resolve().parent / "_lib" / f"metis_host-{sysconfig.get_config_var('SOABI')}-torch-{torch.__version__}.so"
 LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libmetis_nvfp4.so"
 
 DTYPE_BF16, DTYPE_F32 = 0, 1
@@ -155,7 +158,7 @@ def host():
     if _host_lib is not L:
         if _host is None:
             if not HOST_PATH.exists():
-                raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build`")
+                raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build` under this Python and torch")
             spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
             module = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(module)

@@ -1,6 +1,9 @@
 """The native part of the tensor-level wrappers (csrc/host_ops.cpp): it takes positional arguments from ops.py only, and what does not
 fit is an exception, not a crash.  Its results are covered by every test of ops.py on a GPU."""
+import subprocess
+import sys
 import threading
+from pathlib import Path
 
 import pytest
 import torch
@@ -44,6 +47,20 @@ def test_the_c_entry_points_do_without_it(host, monkeypatch, tmp_path):
     assert cabi.lib().metis_nvfp4_sf_bytes(128, 64, cabi.SF_MMA) > 0
     with pytest.raises(cabi.MetisLibraryError):
         cabi.host()
+
+
+def test_another_torch_or_python_does_not_load_it(host):
+    """A module of another ABI is not found under the name that this one asks for, and build() makes the right one."""
+    code = ("import sys, sysconfig, torch\n"
+            "{change}\n"
+            "from fp4_post_b200 import build, cabi\n"
+            "assert not cabi.HOST_PATH.exists(), cabi.HOST_PATH\n"
+            "cabi.lib()\n"
+            "try:\n    cabi.host()\n"
+            "except cabi.MetisLibraryError:\n    print('refused', str(cabi.HOST_PATH) in build._host_command())\n")
+    for change in ("torch.__version__ = '0.0.1+other'", "real = sysconfig.get_config_var\nsysconfig.get_config_var = lambda n: 'cpython-000' if n == 'SOABI' else real(n)"):
+        out = subprocess.run([sys.executable, "-c", code.format(change=change)], capture_output=True, text=True, cwd=Path(__file__).resolve().parents[1])
+        assert out.stdout.split() == ["refused", "True"], out.stderr
 
 
 def test_rows_of_unusual_strides_get_a_leading_dimension():
