@@ -69,6 +69,11 @@ struct Args {
     if (x == -1 && PyErr_Occurred()) throw BadArguments();
     return x;
   }
+  bool truth() {
+    const int x = PyObject_IsTrue(next());
+    if (x < 0) throw BadArguments();
+    return x != 0;
+  }
   uint64_t u64() {
     const unsigned long long x = PyLong_AsUnsignedLongLong(next());
     if (x == (unsigned long long)-1 && PyErr_Occurred()) throw BadArguments();
@@ -118,7 +123,7 @@ PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   METIS_HOST_BEGIN(args, nargs)
   const at::Tensor& x = a.tensor();
   const int32_t dtype = (int32_t)a.i64();
-  const bool transposed = a.i64() != 0;
+  const bool transposed = a.truth();
   const uint32_t flags = (uint32_t)a.i64();
   const uint64_t seed = a.u64(), offset = a.u64();
   const int32_t layout = (int32_t)a.i64();
@@ -150,7 +155,7 @@ PyObject* quantize_dual(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int32_t layout = (int32_t)a.i64();
   const int64_t sf_bytes = a.i64(), sf_bytes_t = a.i64();
   const at::Tensor mean = a.optional();
-  const bool want_sums = a.i64() != 0;
+  const bool want_sums = a.truth();
   void* stream = a.address();
   const int64_t rows = x.size(0), cols = x.size(1);
   Packed q, qt;

@@ -34,6 +34,14 @@ def test_arguments_that_do_not_fit_are_type_errors(host):
         host.col_mean(x, 0, -1)
 
 
+@pytest.mark.parametrize("no", [None, False, 0, ""])
+def test_switches_are_truth_values(host, no):
+    x = torch.zeros(16, 8)                         # blocks of 16 do not divide it: refused before anything is launched
+    assert host.quantize(x, cabi.DTYPE_F32, no, 0, 0, 0, cabi.SF_MMA, 0, 0, None, 0)[0] == -2
+    rc, *tensors = host.quantize_dual(x, cabi.DTYPE_F32, 0, 0, 0, cabi.SF_MMA, 0, 0, None, no, 0)
+    assert rc == -2 and tensors[6] is None         # no token sums
+
+
 def test_every_entry_point_it_knows_is_exported(host):
     assert not host.bind("metis_no_such_entry", 0)
     known = [n for n in cabi.EXPORTS if host.bind(n, cabi.C.cast(getattr(cabi.lib(), n), cabi.C.c_void_p).value)]
