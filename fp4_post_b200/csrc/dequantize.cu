@@ -150,9 +150,9 @@ __device__ __forceinline__ void e2m1x8_to_float(uint32_t w, float* f) {
   }
 }
 
-// eight floats by one 32-byte load
+// eight floats by one 32-byte load (volatile: behind the wait for the kernel that writes them)
 __device__ __forceinline__ void load8_wide(const float* p, float* f) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p));
 }
 
