@@ -378,7 +378,7 @@ __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w 
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 // The two bf16 of a word plus c0 and c1, in fp32 (mixed-precision additions: the operands are not converted first).
 __device__ __forceinline__ void add_bf16x2(uint32_t w, float c0, float c1, float& lo, float& hi) {
-  asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; add.rn.f32.bf16 %0, l, %3; add.rn.f32.bf16 %1, h, %4; }" : "=f"(lo), "=f"(hi) : "r"(w), "f"(c0), "f"(c1));
+  asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; add.rn.f32.bf16 %0, l, %3; add.rn.f32.bf16 %1, h, %4; }" : "=&f"(lo), "=f"(hi) : "r"(w), "f"(c0), "f"(c1));
 }
 
 // 8 consecutive elements starting at p (16-byte aligned for bf16, 32-byte for fp32).

@@ -1,5 +1,6 @@
 """Inline assembly in fp4_post_b200/csrc against the contract that the compiler holds it to: a statement that reads or writes memory is
-volatile (else it may move in front of the wait for the kernel that wrote that memory, or of a barrier)."""
+volatile (else it may move in front of the wait for the kernel that wrote that memory, or of a barrier), and an output that is written
+before the last input is read is marked (else it may get that input's register)."""
 import re
 from pathlib import Path
 
@@ -60,3 +61,18 @@ def test_memory_is_touched_by_volatile_statements_only():
         seen += touches
         assert volatile or not touches, f"{where}: {template!r}"
     assert seen > 30
+
+
+def test_outputs_written_before_the_last_input_is_read_are_marked():
+    seen = 0
+    for where, _, text in statements():
+        template, outputs, inputs = parts(text)
+        steps = [s for s in template.replace("%%", "").split(";") if re.search(r"%\d", s)]
+        if len(steps) < 2:
+            continue
+        seen += 1
+        last_read = max((i for i, s in enumerate(steps) for n in re.findall(r"%(\d+)", s) if int(n) >= len(outputs)), default=-1)
+        for n, constraint in enumerate(outputs):
+            first_write = min((i for i, s in enumerate(steps) if re.search(rf"%{n}\b", s)), default=len(steps))
+            assert "&" in constraint or "+" in constraint or first_write >= last_read, f"{where}: output {n} of {template!r}"
+    assert seen >= 5
