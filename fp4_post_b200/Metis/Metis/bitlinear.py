@@ -616,35 +616,6 @@ def forward_group(layers, x: torch.Tensor):
     return outs
 
 
-class _beside:
-    """`with _beside(event, device) as join: ...` issues the body on the device's second stream once
-    `event` has happened; `join(*tensors)` afterwards makes the current stream wait for it and hands
-    the tensors over.  With event None the body simply runs on the current stream."""
-
-    def __init__(self, event, device):
-        self.event, self.device, self.ctx = event, device, None
-
-    def __enter__(self):
-        if self.event is None:
-            return lambda *tensors: None
-        self.main, self.aux = current_stream(self.device), _aux_stream(self.device)
-        self.aux.wait_event(self.event)
-        self.ctx = on_stream(self.aux)
-        self.ctx.__enter__()
-
-        def join(*tensors):
-            self.main.wait_stream(self.aux)
-            for t in tensors:
-                if t is not None:
-                    t.record_stream(self.main)
-        return join
-
-    def __exit__(self, *exc):
-        if self.ctx is not None:
-            self.ctx.__exit__(*exc)
-        return False
-
-
 # fp4_post_b200.dp.GradientReducer installs itself here: the fused backward hands it every weight
 # gradient the moment it is final (data-parallel training); None = single process.
 GRADIENT_REDUCER = None
