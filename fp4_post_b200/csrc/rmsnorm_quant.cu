@@ -333,7 +333,7 @@ rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int 
 // multiply-add that takes bf16 operands.  Second: norm and quantization, block by block, in 64 registers.  The butterflies of
 // the groups of 32 blocks share their shuffles.  Rows of whole 64-element groups are fetched with the 128-byte swizzle (one
 // box of 64 x cols/64), which keeps both readings free of bank conflicts; others as they lie, at two wavefronts for one.
-// Bound by issue (190 instructions per block of 16, 65 % of the slots) and close to memory.  Both launches, row in registers /
+// Bound by issue (190 instructions per block of 16, 67 % of the slots at 65536 x 3584, 30 warps) and close to memory.  Both launches, row in registers /
 // in shared memory, us: 65536 x 4096 191 / 150, x 3584 165 / 134, x 2048 101 / 78, x 1536 73 / 61, x 1024 52 / 44, 16384 x 3584
 // 45 / 40, 1024 x 4096 9.4 / 7.8.  Narrow rows gain less, and few of them lose what setting the copies up costs (x 1024: 1024
 // 5.3 / 5.5, 8192 9.6 / 10.1, 16384 17.7 / 16.8; x 768: 2048 6.0 / 6.3, 16384 17.5 / 16.0; x 512: 2048 4.8 / 5.2, 16384
