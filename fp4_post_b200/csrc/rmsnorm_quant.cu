@@ -466,6 +466,7 @@ rmsnorm_quantize_staged_kernel(const __grid_constant__ CUtensorMap map_x, const 
       if constexpr (kProductBf16) {
         const uint4 g0 = norm_lds128(s_gamma + swz0 + 1024 * j), g1 = norm_lds128(s_gamma + swz1 + 1024 * j);
         const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        a = 0.0f;                                         // what a block of NaN has, as norm_block gives it
 #pragma unroll
         for (int i = 0; i < 8; ++i) {                     // both roundings of the reference, see rmsnorm_quantize_kernel
           float n0, n1;
@@ -475,8 +476,8 @@ rmsnorm_quantize_staged_kernel(const __grid_constant__ CUtensorMap map_x, const 
           const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
           y[2 * i] = bf16_lo(w);
           y[2 * i + 1] = bf16_hi(w);
+          a = max3(a, fabsf(y[2 * i]), fabsf(y[2 * i + 1]));
         }
-        a = abs_max16(y);
       } else {
         a = norm_block<__nv_bfloat16, TG>(v, rs, gamma + (lane + 32 * j) * 16, y);
       }

@@ -88,6 +88,22 @@ def test_rows_staged_in_shared_memory(rows, cols, gap, gdtype):
     assert torch.equal(q.codes, again.codes) and torch.equal(q.scales, again.scales) and torch.equal(q.unit, again.unit)
 
 
+# A row that is NaN throughout (one NaN in it, or an infinity whose square meets gamma 0): its scales have the bytes that the kernels
+# for fewer rows give it, with the row in shared memory and in registers.
+@pytest.mark.parametrize("rows,cols", [(1200, 3104), (1200, 1040), (1200, 4096), (1200, 512)])
+@pytest.mark.parametrize("gdtype", [torch.bfloat16, torch.float32])
+def test_scales_of_a_row_that_is_not_a_number(rows, cols, gdtype):
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    x = torch.randn(rows, cols, generator=g, device=DEV).to(torch.bfloat16)
+    x[6, 9], x[7, 3] = float("nan"), float("inf")
+    gamma = (1.0 + 0.1 * torch.randn(cols, generator=g, device=DEV)).to(gdtype)
+    gamma[16:32] = 0
+    got, want = (ops.rmsnorm_nvfp4_quantize(t, gamma, 1e-6, sf_layout=cabi.SF_ROWMAJOR) for t in (x, x[:500]))
+    for q in (got, want):
+        q.by_row = q.scales.reshape(-1, cols // 16)[6:8]
+    assert torch.equal(got.by_row, want.by_row) and torch.equal(got.codes[6:8], want.codes[6:8])
+
+
 # The warp-per-row kernel: every number of blocks per lane, rows that end inside a round of 32 blocks and inside a CTA's
 # eight rows, and fewer than 1024 rows where a CTA per row would leave more records than there is room for (whether it
 # would depends on the type of gamma; both kernels have to pass).
