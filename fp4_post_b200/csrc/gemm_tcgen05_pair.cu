@@ -451,7 +451,7 @@ int32_t launch_gemm_pair(const metis_gemm_args* a, const CUtensorMap& ma, const 
   const int64_t rounds = ceil_div(tiles, pairs);
   pairs = ceil_div(tiles, rounds);
   const int64_t stages = ceil_div(p.K, 256) + ceil_div(p.rank, 64);
-  const bool four = pair_epilogue_parts(stages, rounds, (p.rvec0 != nullptr) + (p.rvec1 != nullptr), p.c != nullptr, a->d_dtype == METIS_DTYPE_F32) == 4;
+  const bool four = pair_epilogue_parts(p.N, stages, rounds, (p.rvec0 != nullptr) + (p.rvec1 != nullptr), p.c != nullptr, a->d_dtype == METIS_DTYPE_F32) == 4;
   // the scale arrays as [tiles, 512 bytes]: one box = the 4 tiles (2 KiB) of one stage and row block
   const int64_t sf_tiles_k = sf_tiles_per_row(a->K);
   CUtensorMap maps[7] = {ma, mb, {}, {}, mt, mu, {}};

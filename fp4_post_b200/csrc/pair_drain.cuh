@@ -25,9 +25,9 @@ struct PairDrain {
   static constexpr int arrivals(int parts) { return 2 * 4 * parts; }
 };
 
-// Epilogue warps per lane quarter of a product of `stages` pipeline stages a tile, `rounds` tiles a pair, with `vectors` row vectors and
-// perhaps an addend C.  Four take half the time for a tile, which is what bounds a product while its epilogue takes longer than the
-// MMAs of the next tile, and they end the last tile sooner.  Once the MMAs cover the epilogue, two are faster: what four
+// Epilogue warps per lane quarter of a product [., N] of `stages` pipeline stages a tile, `rounds` tiles a pair, with `vectors` row
+// vectors and perhaps an addend C.  Four take half the time for a tile, which is what bounds a product while its epilogue takes
+// longer than the MMAs of the next tile, and they end the last tile sooner.  Once the MMAs cover the epilogue, two are faster: what four
 // read and store at once takes bandwidth that the operands need, while the next tile starts.  Both sides, us, two / four, L2 cold,
 // 14 rounds (8192 x 8192, bf16 D) by stages:
 //   nothing        2: 50.1 / 46.0    5: 57.4 / 57.4     6: 62.4 / 66.3     8: 74.6 / 75.9    14: 101.0 / 103.0
@@ -38,14 +38,20 @@ struct PairDrain {
 //   C, two         20: 163.9 / 153.7 24: 174.0 / 174.1  32: 218.1 / 228.4
 // Fewer rounds weigh the last tile more: 9 stages and a vector 23.5 / 22.6 (2 rounds), 27.6 / 27.5 (3), 36.1 / 36.9 (5), 45.5 / 47.2
 // (7); 8 stages 35.7 / 35.0 (5), 50.1 / 50.0 (8); 6 stages and nothing 21.5 / 21.5 (2), 25.6 / 27.6 (3); 16 stages and two vectors
-// 44.0 / 42.0 (4), 49.3 / 48.7 (5), 71.8 / 71.7 (8), 20 stages 40.8 / 39.6 (3), 53.9 / 55.3 (5).  Stages of the side product count
-// like the others, and an fp32 D has the same lines (both rows of a weight gradient: 16 stages 133.2 / 136.2, 10 stages 125.1 / 113.6),
-// but its addend is twice as long: four lose at every length (2 stages 151.6 / 166.8, 16 stages 169.2 / 194.6, with a vector 191.5 /
-// 198.6) until two vectors make up for it (12 stages 207.5 / 198.9, 24 227.2 / 226.1, 32 255.0 / 272.3).
-static inline int pair_epilogue_parts(int64_t stages, int64_t rounds, int vectors, bool addend, bool fp32) {
-  if (fp32 && addend && vectors < 2) return 2;
-  constexpr int kTwoFrom[2][3] = {{6, 9, 16}, {16, 20, 24}};
-  return stages >= kTwoFrom[addend][vectors] && rounds > (vectors == 2 ? 4 : 2) ? 2 : 4;
+// 44.0 / 42.0 (4), 49.3 / 48.7 (5), 71.8 / 71.7 (8), 20 stages 40.8 / 39.6 (3), 53.9 / 55.3 (5).  Back to back with operands in L2 the
+// lines lie a stage lower: a vector and 8 stages 41.6 / 43.0 (8 rounds), two and 14 61.4 / 63.3 (8), C and 14 54.9 / 57.6 (6), C, two and 32
+// 60.4 / 63.3 (3).  Stages of the side product count like the others, and an fp32 D has the same lines (both rows of a weight gradient: 16
+// stages 133.2 / 136.2, 10 stages 125.1 / 113.6), but its stores and its addend are twice as long: without a vector four gain 1 % at
+// most and lose up to 5 (2304 x 4096, 6 stages, 14.8 / 15.6), with C they lose at every length (2 stages 151.6 / 166.8, 16 stages 169.2 /
+// 194.6, with a vector 191.5 / 198.6) until two vectors make up for it (12 stages 207.5 / 198.9, 24 227.2 / 226.1, 32 255.0 / 272.3).
+// A single column of tiles with chunks outside D gives four warps as many chunks as two have: 1634 x 144 x 1024 5.5 / 5.9, 14842 x 176 x 1280
+// with C 9.8 / 10.4; from 200 columns on they are not slower (14842 x 192 x 2304 with a vector 1.02, x 256 1.09 as fast).  One round with an addend alone
+// ends with its reads either way (163 x 5296 x 512 7.8 / 8.4, 825 x 416 x 1952 10.9 / 11.3).  300 products drawn from 129 to 16384 rows, 136 to
+// 16384 columns and K of 256 to 16384 take 0.96 of their time with two, back to back and L2 cold.
+static inline int pair_epilogue_parts(int64_t N, int64_t stages, int64_t rounds, int vectors, bool addend, bool fp32) {
+  if (N <= 192 || (fp32 && vectors < (addend ? 2 : 1)) || (addend && vectors == 0 && rounds == 1)) return 2;
+  constexpr int kTwoFrom[2][3] = {{6, 9, 16}, {14, 20, 24}};
+  return stages + (rounds > 7) >= kTwoFrom[addend][vectors] && rounds > (vectors == 2 && !addend ? 4 : 2) ? 2 : 4;
 }
 
 }  // namespace metis

@@ -89,15 +89,20 @@ def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
 # chunks inside D and the others of its lane quarter one: every launch gives the bits of the first (test_pair_drain.py has the order).
 @pytest.mark.parametrize("K", [32, 256, 1024])
 @pytest.mark.parametrize("sms", [2, 4, 8])
-@pytest.mark.parametrize("addend", [False, True])
+@pytest.mark.parametrize("terms", ["none", "addend", "rows"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-def test_many_short_tiles_per_pair(K, sms, addend, dtype):
+def test_many_short_tiles_per_pair(K, sms, terms, dtype):
     M, N = 1300, 4 * 256 + 144
     qa, qb, da, db = operands(M, N, K, seed=K + sms)
     kw, want = dict(out_dtype=dtype, sm_limit=sms), O.gemm_reference(da, db).astype(np.float64)
-    if addend:
-        kw["c"] = torch.randn(M, N, generator=torch.Generator(device=DEV).manual_seed(K), device=DEV).to(dtype)
+    g = torch.Generator(device=DEV).manual_seed(K)
+    if terms == "addend":
+        kw["c"] = torch.randn(M, N, generator=g, device=DEV).to(dtype)
         want += kw["c"].double().cpu().numpy()
+    if terms == "rows":
+        v, w = (torch.randn(n, generator=g, device=DEV) for n in (N, M))
+        kw["rank1"] = ((None, v), (w, v))
+        want += (1 + w.double().cpu().numpy())[:, None] * v.double().cpu().numpy()[None, :]
     first = run(qa, qb, **kw)
     assert rel_l2(first.float().cpu().numpy(), want) <= (1e-5 if dtype == torch.float32 else 2.0 ** -8)      # fp32 sums; one rounding to bf16
     for _ in range(100):

@@ -16,8 +16,8 @@ extern "C" int stride() { return PairDrain::kStride; }
 extern "C" int chunk(int parts, int part, int k, int odd) { return PairDrain::chunk(parts, part, k, odd); }
 extern "C" int before_release(int parts) { return PairDrain::before_release(parts); }
 extern "C" int arrivals(int parts) { return PairDrain::arrivals(parts); }
-extern "C" int epilogue_parts(int stages, int rounds, int vectors, int addend, int fp32) {
-  return metis::pair_epilogue_parts(stages, rounds, vectors, addend != 0, fp32 != 0);
+extern "C" int epilogue_parts(int N, int stages, int rounds, int vectors, int addend, int fp32) {
+  return metis::pair_epilogue_parts(N, stages, rounds, vectors, addend != 0, fp32 != 0);
 }
 """
 
@@ -61,11 +61,13 @@ def test_a_warp_that_falls_behind_loses_nothing(drain, parts):
                     assert what != "read" or not cols & columns(later), (parts, part, at, tile, later)
 
 
-# Both sides of each line as it was timed: stages, rounds, row vectors, addend, fp32 -> the faster of two and four.
-@pytest.mark.parametrize("shape,parts", [((5, 14, 0, 0, 0), 4), ((6, 14, 0, 0, 0), 2), ((16, 14, 0, 0, 0), 2), ((6, 2, 0, 0, 0), 4), ((6, 3, 0, 0, 0), 2),
-                                         ((7, 14, 1, 0, 0), 4), ((9, 14, 1, 0, 0), 2), ((18, 4, 1, 0, 0), 2), ((9, 2, 1, 0, 1), 4),
-                                         ((14, 7, 2, 0, 0), 4), ((16, 14, 2, 0, 0), 2), ((20, 3, 2, 0, 1), 4), ((12, 14, 0, 1, 0), 4), ((16, 14, 0, 1, 0), 2),
-                                         ((16, 14, 1, 1, 0), 4), ((20, 14, 1, 1, 0), 2), ((20, 14, 2, 1, 0), 4), ((32, 14, 2, 1, 0), 2),
-                                         ((2, 14, 0, 1, 1), 2), ((32, 2, 0, 1, 1), 2), ((16, 8, 1, 1, 1), 2), ((12, 14, 2, 1, 1), 4), ((32, 14, 2, 1, 1), 2)])
+# Both sides of each line as it was timed: columns, stages, rounds, row vectors, addend, fp32 -> the faster of two and four.
+@pytest.mark.parametrize("shape,parts", [((8192, 4, 14, 0, 0, 0), 4), ((8192, 6, 14, 0, 0, 0), 2), ((8192, 16, 14, 0, 0, 0), 2), ((8192, 6, 2, 0, 0, 0), 4), ((8192, 6, 3, 0, 0, 0), 2),
+                                         ((8192, 7, 14, 1, 0, 0), 4), ((8192, 8, 14, 1, 0, 0), 2), ((8192, 8, 5, 1, 0, 0), 4), ((8192, 18, 4, 1, 0, 0), 2),
+                                         ((8192, 9, 2, 1, 0, 1), 4), ((8192, 14, 7, 2, 0, 0), 4), ((8192, 16, 14, 2, 0, 0), 2), ((8192, 20, 3, 2, 0, 1), 4),
+                                         ((8192, 12, 14, 0, 1, 0), 4), ((8192, 16, 14, 0, 1, 0), 2), ((8192, 14, 6, 0, 1, 0), 2), ((8192, 16, 14, 1, 1, 0), 4),
+                                         ((8192, 20, 14, 1, 1, 0), 2), ((8192, 20, 14, 2, 1, 0), 4), ((8192, 32, 3, 2, 1, 0), 2),
+                                         ((4096, 6, 2, 0, 0, 1), 2), ((8192, 2, 14, 0, 1, 1), 2), ((8192, 32, 2, 0, 1, 1), 2), ((8192, 16, 8, 1, 1, 1), 2),
+                                         ((8192, 12, 14, 2, 1, 1), 4), ((8192, 32, 14, 2, 1, 1), 2), ((144, 4, 1, 0, 0, 0), 2), ((176, 5, 1, 0, 1, 0), 2), ((5296, 2, 1, 0, 1, 0), 2), ((256, 4, 1, 0, 0, 0), 4)])
 def test_the_faster_number_of_warps(drain, shape, parts):
     assert drain.epilogue_parts(*shape) == parts
