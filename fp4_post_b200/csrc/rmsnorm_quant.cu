@@ -228,11 +228,11 @@ __device__ __forceinline__ float norm_block(const float (&v)[16], float rs, cons
 // care (896: 4.9 / 4.5).
 constexpr int64_t kNormRowsMinRows = 1024;
 
-// Narrow rows: the row stays in registers as loaded (kM blocks of 16 elements per lane, block lane + 32 j); two blocks' chains
+// Narrow rows, and wide ones where norm_rows_staged says so: the row stays in registers as loaded (kM blocks of 16 elements per lane, block lane + 32 j); two blocks' chains
 // of squares share one packed instruction.
 constexpr int kNormRowThreads = 256;
 template <typename TG, int kM, bool kWriteNorm>
-__global__ void __launch_bounds__(kNormRowThreads, 3)
+__global__ void __launch_bounds__(kNormRowThreads, kM <= 3 ? 3 : 2)
 rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int blocks_per_row, int64_t ld,
                              const TG* __restrict__ gamma, float eps, uint2* __restrict__ codes,
                              float* __restrict__ amax_out, unsigned int* __restrict__ gmax,
@@ -337,8 +337,9 @@ rmsnorm_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int rows, int 
 // in shared memory, us: 65536 x 4096 191 / 150, x 3584 165 / 134, x 2048 101 / 78, x 1536 73 / 61, x 1024 52 / 44, 16384 x 3584
 // 45 / 40, 1024 x 4096 9.4 / 7.8.  Narrow rows gain less, and few of them lose what setting the copies up costs (x 1024: 1024
 // 5.3 / 5.5, 8192 9.6 / 10.1, 16384 17.7 / 16.8; x 768: 2048 6.0 / 6.3, 16384 17.5 / 16.0; x 512: 2048 4.8 / 5.2, 16384
-// 10.0 / 11.0, 65536 30.1 / 29.6), so up to 512 columns stay with the registers, and up to 1024 with fewer than 16384 rows.
-static bool norm_rows_staged(int64_t rows, int64_t blocks_per_row) { return blocks_per_row > 64 || (blocks_per_row > 32 && rows >= 16384); }
+// 10.0 / 11.0, 65536 30.1 / 29.6), so up to 512 columns stay with the registers, and up to 1024 with fewer than 16384 rows; so do calls that
+// write the normalised tensor or read an fp32 gamma, by size (norm_rows_staged in rows_shape.cuh has the rule).
+static bool norm_rows_swizzled(int64_t bpr, int64_t ld) { return bpr % 4 == 0 && ld % 64 == 0; }      // whole 64-element groups, a row a whole number of them from the next
 constexpr int64_t kNormStagedSmem = 232448 - 2048;       // of a CTA for rows: less 1 KiB for the static part and 1 KiB for aligning
 constexpr int kNormStagedMaxWarps = 32;
 // acc + lo^2 + hi^2 for the two bf16 of a word, one rounding each
@@ -770,7 +771,7 @@ static int32_t launch_norm_staged(const __nv_bfloat16* x, int64_t rows, int bpr,
   const int64_t blocks = ceil_div(rows, warps * rounds) < sms ? ceil_div(rows, warps * rounds) : sms;
   if (blocks > kMaxRecords) *records = nullptr;
   if (!*records) METIS_CUDA_OK(cudaMemsetAsync(ws.gmax, 0, 2 * sizeof(unsigned int), st));   // running maximum and error word
-  const bool swizzled = bpr % 4 == 0 && ld % 64 == 0;        // whole 64-element groups, a row a whole number of them from the next
+  const bool swizzled = norm_rows_swizzled(bpr, ld);
   CUtensorMap map = {};
   if (swizzled) {
     if (int32_t rc = make_row_map(&map, x, bpr / 4, rows, ld * 2, "x")) return rc;
@@ -801,14 +802,15 @@ static int32_t dispatch_chunks(const TX* x, int64_t rows, int64_t cols, int64_t 
     // a warp per row from kNormRowsMinRows on, and where a CTA per row has more CTAs than there are records
     if (bpr >= 32 && bpr <= 256 &&
         (rows >= kNormRowsMinRows || (*records && norm_ctas<TX, TG, 1>(rows, bx, norm_out != nullptr, sms) > kMaxRecords))) {
-      if (!norm_rows_staged(rows, bpr))
-        return bpr <= 32 ? launch_norm_rows<TG, 1>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
-                         : launch_norm_rows<TG, 2>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+      const bool staged = norm_rows_staged(rows, bpr, sizeof(TG) == 4, norm_out != nullptr, norm_rows_swizzled(bpr, ld));
       switch ((bpr + 31) / 32) {
-#define METIS_NORM_STAGED(M) case M: return launch_norm_staged<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
-        METIS_NORM_STAGED(2); METIS_NORM_STAGED(3); METIS_NORM_STAGED(4); METIS_NORM_STAGED(5);
-        METIS_NORM_STAGED(6); METIS_NORM_STAGED(7); METIS_NORM_STAGED(8);
-#undef METIS_NORM_STAGED
+        case 1: return launch_norm_rows<TG, 1>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st);
+#define METIS_NORM_ROWS(M)                                                                                                     \
+  case M: return staged ? launch_norm_staged<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)       \
+                        : launch_norm_rows<TG, M>(x, rows, bpr, ld, gamma, eps, codes, ws, records, norm_out, sms, st)
+        METIS_NORM_ROWS(2); METIS_NORM_ROWS(3); METIS_NORM_ROWS(4); METIS_NORM_ROWS(5);
+        METIS_NORM_ROWS(6); METIS_NORM_ROWS(7); METIS_NORM_ROWS(8);
+#undef METIS_NORM_ROWS
       }
     }
   }

@@ -1,4 +1,4 @@
-// Launch shape of the row-major quantizer that feeds registers (quantize_rows_kernel): plain host arithmetic, no CUDA.
+// Launch shapes and rules of the quantizers and the fused norm: plain host arithmetic, no CUDA.
 #pragma once
 
 #include <stdint.h>
@@ -9,6 +9,7 @@ constexpr int kQuantThreads = 256;
 // Per-CTA records that a quantizer's scratch holds (see workspace_records).
 constexpr int kMaxRecords = 640;
 
+// Of the row-major quantizer that feeds registers (quantize_rows_kernel).
 struct RowsShape {
   int bx;              // threads along a row; kQuantThreads / bx rows per CTA and round
   int64_t gx, gy;      // CTAs along a row, CTAs along the rows (which each of them strides over)
@@ -36,6 +37,25 @@ static inline RowsShape rows_shape(int64_t rows, int64_t blocks_per_row, int64_t
   if (s.gy > 65535) s.gy = 65535;
   if (s.gy < 1) s.gy = 1;
   return s;
+}
+
+// Fused norm of bf16 rows of 16 bpr elements by a warp per row: the row in shared memory, or in registers.
+// Staging rows keeps more warps on an SM, which is what the codes alone of long inputs need; a normalised tensor written beside them, or gamma
+// read from global memory in fp32, asks for bandwidth instead, and what staging costs is no longer hidden.  Below 1600 rows staged ones
+// go once round, where registers hold too few of them.  Both launches, inputs not in L2, in registers / staged, us (rmsnorm_quant.cu has more):
+//   bf16 gamma, codes alone   1300 x 2576 1.05 as fast staged, 2048 x 1552 0.92, 3000 x 2560 0.98, 8192 x 2560 1.01, 65536 x 3584 165 / 137
+//   bf16 gamma, norm written  3000 x 2560 12.0 / 12.6, 4096 x 2576 15.7 / 17.4, 16384 x 2048 34.1 / 36.2, 65536 x 2560 146 / 162, 8192 x 3584
+//                             33.8 / 35.6, 12000 x 4096 52.8 / 53.7; but 16384 x 1088 23.8 / 22.9, 4096 x 3600 22.1 / 20.6
+//   fp32 gamma, codes alone   6000 x 2048 15.4 / 16.8, 12000 x 1552 22.8 / 24.7; but 1300 x 2048 7.9 / 7.5, 4096 x 2576 17.0 / 16.8, and where
+//                             rows are fetched swizzled 32768 x 2048 1.05 as fast staged
+//   fp32 gamma, norm written  not swizzled 32768 x 2064 121 / 132, 16384 x 4080 125 / 139; but 8192 x 2064 37.2 / 35.8, and swizzled
+//                             32768 x 2048 113 / 109
+static inline bool norm_rows_staged(int64_t rows, int64_t bpr, bool fp32_gamma, bool norm, bool swizzled) {
+  if (bpr <= 32 || (bpr <= 64 && rows < 16384)) return false;
+  if (rows < 1600) return true;
+  if (fp32_gamma) return norm ? swizzled || rows < 12000 || bpr <= 80 : bpr > 144 || (swizzled && rows >= 16384);
+  if (norm) return (bpr <= 72 && rows >= 16384) || rows < (bpr > 224 ? 12000 : bpr > 192 ? 8192 : 0);
+  return bpr > 176 || rows >= 3400;
 }
 
 }  // namespace metis

@@ -195,3 +195,26 @@ def test_norm_with_column_mean(rows, cols, gdtype):
     # second pass: the quantizer on y with that mean, against the oracle
     q = ops.nvfp4_quantize(y, mean=mean, sf_layout=cabi.SF_ROWMAJOR)
     assert_packed_equal(q, y.float().cpu().numpy(), cabi.SF_ROWMAJOR, mean=mean.cpu().numpy(), what="norm + mean -> quant")
+
+
+# A warp per row with the row in registers, where it is the faster one of the two (norm_rows_staged): each number of blocks per lane,
+# beside the smallest and largest sizes that take it, against the CTA-per-row kernel's rows of a call of 500.
+@pytest.mark.parametrize("rows,cols,gdtype", [(1600, 1296, torch.bfloat16), (1605, 1552, torch.bfloat16), (1602, 2560, torch.bfloat16), (2561, 3072, torch.bfloat16),
+                                              (8192, 3584, torch.bfloat16), (12003, 4096, torch.bfloat16), (12001, 3600, torch.float32), (12000, 1296, torch.float32),
+                                              (1600, 1040, torch.float32), (1610, 2304, torch.float32), (16390, 528, torch.float32)])
+def test_rows_in_registers(rows, cols, gdtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=g, device=DEV).to(torch.bfloat16)
+    x[3] *= 1e-38
+    x[4, 7], x[5, 9] = float("inf"), float("nan")
+    gamma = (1.0 + 0.1 * torch.randn(cols, generator=g, device=DEV)).to(gdtype)
+    as_bits = torch.int16 if gdtype == torch.bfloat16 else torch.int32
+    _, y = ops.rmsnorm_nvfp4_quantize(x, gamma, 1e-6, return_norm=True)
+    for r in (0, rows - 500):
+        _, want = ops.rmsnorm_nvfp4_quantize(x[r:r + 500], gamma, 1e-6, return_norm=True)
+        assert torch.equal(y[r:r + 500].view(as_bits), want.view(as_bits))
+    x[3:6] = 1                                            # finite from here on: codes, scales and unit of both forms
+    (q, y), plain = ops.rmsnorm_nvfp4_quantize(x, gamma, 1e-6, return_norm=True), ops.rmsnorm_nvfp4_quantize(x, gamma, 1e-6)
+    again = ops.nvfp4_quantize(y)                         # the quantizer's own tests compare it with the oracle
+    for p in (q, plain):
+        assert torch.equal(p.codes, again.codes) and torch.equal(p.scales, again.scales) and torch.equal(p.unit, again.unit)
