@@ -1064,14 +1064,9 @@ static int32_t launch_tile(const T* x, int64_t rows, int64_t cols, int64_t ld, c
     return rc;
   const int64_t col_tiles = ceil_div(cols, TC::kCols), tiles = col_tiles * ceil_div(rows, TC::kRows);
   if (tiles >= (int64_t)1 << 31) return fail(METIS_ERR_TOO_LARGE, "tensor of more than 2^31 tiles");
-  // Three CTAs of ~63 KiB per SM.  Two for tensors of several hundred MB whose rows do not start on 128-byte lines: there the
-  // kernel is bound by memory, a tile's rows end in the middle of lines that the tile to the right begins with, and with more
-  // tiles in flight those lines come from memory twice (us, three / two CTAs, one output: 24576 x 8304 183 / 137, 65536 x 4128
-  // 221 / 162; both: 65536 x 8304 890 / 662, 98304 x 4112 668 / 551; but both at 131072 x 2064 317 / 364, 20480 x 8304
-  // 229 / 237, and with stochastic rounding, which is bound by issue, 98304 x 4112 574 / 587).
-  const int64_t split_lines_from = (int64_t)(out.codes_r && out.codes_t ? 768 : 384) * 1000 * 1000;
-  const bool split_lines = !sr && (ld * (int64_t)sizeof(T)) % 128 != 0 && rows * ld * (int64_t)sizeof(T) >= split_lines_from;
-  int64_t grid = (int64_t)sm_count() * (split_lines ? 2 : 3);
+  const bool split_lines = (ld * (int64_t)sizeof(T)) % 128 != 0;
+  int64_t grid = (int64_t)sm_count() * tile_ctas_per_sm(rows * ld * (int64_t)sizeof(T), split_lines, mean != nullptr, sizeof(T) == 4,
+                                                          out.codes_r != nullptr, out.codes_t != nullptr);
   if (grid > tiles) grid = tiles;
   if (out.records && grid > kDualMaxCtas) grid = kDualMaxCtas;
   const uint32_t bpr = (uint32_t)(cols >> 4), bpc = (uint32_t)(rows >> 4), step_rows = (uint32_t)(grid / col_tiles), step_cols = (uint32_t)(grid % col_tiles);

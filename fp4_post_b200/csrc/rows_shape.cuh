@@ -39,6 +39,24 @@ static inline RowsShape rows_shape(int64_t rows, int64_t blocks_per_row, int64_t
   return s;
 }
 
+// CTAs per SM of the tile quantizer for a tensor of `bytes` (whole rows as they lie).  Three fit (~63 KiB each).  Two, or one, where rows do
+// not start on 128-byte lines (split_lines) and the tensor is larger than L2: a tile's rows end in the middle of lines that the tile to the
+// right begins with, and with more tiles in flight those lines come from memory twice.  The more work there is on a tile (the mean above all,
+// stochastic rounding little) the further off the line.  First pass and scale pass, us, bf16 unless stated:
+//   three / two CTAs   one output 15568 x 4112 44.6 / 39.6, 21088 x 8304 138 / 98, stochastic 54192 x 8304 424 / 299; centred 23360 x 4112
+//                      63.1 / 62.7, 31136 x 4112 86.6 / 81.4, stochastic 30112 x 8304 200 / 143, fp32 30400 x 4112 149 / 114; transposed
+//                      15568 x 4112 57.8 / 57.2, 21088 x 8304 189 / 163, centred 31136 x 4112 120 / 106 (but 15424 x 8304 79.4 / 83.0), fp32 and
+//                      centred 7712 x 8304 68.7 / 69.2, 15056 x 8304 146 / 132 (but 8736 x 14320 125 / 141); both 15568 x 4112 103 / 95.7,
+//                      centred and stochastic 23360 x 4112 113 / 103, 31136 x 4112 230 / 171, fp32 15568 x 4112 132 / 114
+//   two / one          both, not centred 42560 x 4112 207 / 193, 21088 x 8304 302 / 218, 54192 x 8304 1011 / 553, fp32 15056 x 8304 251 / 190 (but stochastic
+//                      60800 x 4112 267 / 272); centred 60800 x 4112 247 / 321
+static inline int tile_ctas_per_sm(int64_t bytes, bool split_lines, bool mean, bool fp32, bool rows_out, bool cols_out) {
+  const int64_t mb = split_lines ? bytes / 1000000 : 0;
+  const bool both = rows_out && cols_out;
+  if (both && !mean && mb >= 350) return 1;
+  return mb >= (!mean || both ? 128 : fp32 && cols_out ? 384 : 256) ? 2 : 3;
+}
+
 // Fused norm of bf16 rows of 16 bpr elements by a warp per row: the row in shared memory, or in registers.
 // Staging rows keeps more warps on an SM, which is what the codes alone of long inputs need; a normalised tensor written beside them, or gamma
 // read from global memory in fp32, asks for bandwidth instead, and what staging costs is no longer hidden.  Below 1600 rows staged ones

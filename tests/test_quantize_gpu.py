@@ -122,6 +122,29 @@ def test_whole_tiles_and_edges_of_both_orientations(rows, cols, dtype):
 
 # Largest maxima that put other maxima of a bf16 tensor exactly on an E4M3 tie of the scale pass (19968 does with 117), and
 # one so large that most scales are E4M3 subnormals or zero; whole pieces of the tiled layout and edges of it.
+# Tensors larger than L2 whose rows do not start on 128-byte lines go by two CTAs per SM or one (tile_ctas_per_sm): every output is that of
+# a call with fewer rows or columns, which holds the largest maximum too and goes by three.
+@pytest.mark.parametrize("rows,cols,dtype,centred", [(16400, 4112, torch.bfloat16, False), (8192, 9744, torch.float32, True), (21088, 8304, torch.bfloat16, False)])
+@pytest.mark.parametrize("stochastic", [False, True])
+def test_large_tensors_whose_rows_split_lines(rows, cols, dtype, centred, stochastic):
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    x = torch.randn(rows, cols, generator=g, device=DEV).to(dtype)
+    x[0, 0] = 100.0
+    mean = torch.randn(cols, generator=g, device=DEV) if centred else None
+    kw = dict(sf_layout=cabi.SF_ROWMAJOR, **(dict(stochastic=True, seed=3, offset=5) if stochastic else {}))
+
+    def same(p, part):
+        n = part.codes.shape[0]
+        assert torch.equal(p.codes[:n], part.codes) and torch.equal(p.scales[:part.scales.numel()], part.scales) and torch.equal(p.unit, part.unit)
+    q = ops.nvfp4_quantize(x, mean=mean, **kw)
+    same(q, ops.nvfp4_quantize(x[:2048], mean=mean, **kw))
+    same(ops.nvfp4_quantize(x, transpose=True, mean=mean, **kw), ops.nvfp4_quantize(x[:, :512], transpose=True, mean=mean[:512] if centred else None, **kw))
+    both, both_t = ops.nvfp4_quantize_dual(x, mean=mean, **kw)
+    same(q, both)
+    if not stochastic:                                    # each output of a stochastic pass for both has bits of its own
+        same(ops.nvfp4_quantize(x, transpose=True, mean=mean, **kw), both_t)
+
+
 @pytest.mark.parametrize("rows,cols", [(256, 4096), (300, 4112)])
 @pytest.mark.parametrize("top", [19968.0, 1.5, 3.0e6])
 @pytest.mark.parametrize("layout", [cabi.SF_ROWMAJOR, cabi.SF_MMA])
