@@ -44,14 +44,18 @@ struct PairDrain {
 // stages 133.2 / 136.2, 10 stages 125.1 / 113.6), but its stores and its addend are twice as long: without a vector four gain 1 % at
 // most and lose up to 5 (2304 x 4096, 6 stages, 14.8 / 15.6), with C they lose at every length (2 stages 151.6 / 166.8, 16 stages 169.2 /
 // 194.6, with a vector 191.5 / 198.6) until two vectors make up for it (12 stages 207.5 / 198.9, 24 227.2 / 226.1, 32 255.0 / 272.3).
+// Products of 2018 and 4096 rows have the lines up to two stages lower, and the rule follows them, since the others lose 2 % at most by that: a vector
+// and 8 stages 31.6 / 34.2 and 28.0 / 29.5 (5 rounds), 37.5 / 39.0 (7); two vectors and 14 33.9 / 35.1 (4), 38.7 / 39.6 (5); C and 13
+// 32.2 / 34.0 (3), 40.5 / 42.7 (4), 60.8 / 62.2 (7), C and 18 26.6 / 29.1 and 25.2 / 26.4 (2); C, a vector and 18 48.2 / 50.8 and 45.3 / 46.1 (4).
 // A single column of tiles with chunks outside D gives four warps as many chunks as two have: 1634 x 144 x 1024 5.5 / 5.9, 14842 x 176 x 1280
 // with C 9.8 / 10.4; from 200 columns on they are not slower (14842 x 192 x 2304 with a vector 1.02, x 256 1.09 as fast).  One round with an addend alone
 // ends with its reads either way (163 x 5296 x 512 7.8 / 8.4, 825 x 416 x 1952 10.9 / 11.3).  300 products drawn from 129 to 16384 rows, 136 to
 // 16384 columns and K of 256 to 16384 take 0.96 of their time with two, back to back and L2 cold.
 static inline int pair_epilogue_parts(int64_t N, int64_t stages, int64_t rounds, int vectors, bool addend, bool fp32) {
   if (N <= 192 || (fp32 && vectors < (addend ? 2 : 1)) || (addend && vectors == 0 && rounds == 1)) return 2;
-  constexpr int kTwoFrom[2][3] = {{6, 9, 16}, {14, 20, 24}};
-  return stages + (rounds > 7) >= kTwoFrom[addend][vectors] && rounds > (vectors == 2 && !addend ? 4 : 2) ? 2 : 4;
+  constexpr int kTwoFrom[2][3] = {{6, 8, 14}, {13, 18, 24}};
+  const int fewest = addend && vectors == 0 ? 2 : fp32 && vectors == 2 && !addend ? 5 : 3;         // rounds
+  return stages >= kTwoFrom[addend][vectors] && rounds >= fewest ? 2 : 4;
 }
 
 }  // namespace metis

@@ -63,8 +63,8 @@ def test_a_warp_that_falls_behind_loses_nothing(drain, parts):
 
 # Both sides of each line as it was timed: columns, stages, rounds, row vectors, addend, fp32 -> the faster of two and four.
 @pytest.mark.parametrize("shape,parts", [((8192, 4, 14, 0, 0, 0), 4), ((8192, 6, 14, 0, 0, 0), 2), ((8192, 16, 14, 0, 0, 0), 2), ((8192, 6, 2, 0, 0, 0), 4), ((8192, 6, 3, 0, 0, 0), 2),
-                                         ((8192, 7, 14, 1, 0, 0), 4), ((8192, 8, 14, 1, 0, 0), 2), ((8192, 8, 5, 1, 0, 0), 4), ((8192, 18, 4, 1, 0, 0), 2),
-                                         ((8192, 9, 2, 1, 0, 1), 4), ((8192, 14, 7, 2, 0, 0), 4), ((8192, 16, 14, 2, 0, 0), 2), ((8192, 20, 3, 2, 0, 1), 4),
+                                         ((8192, 7, 14, 1, 0, 0), 4), ((8192, 8, 14, 1, 0, 0), 2), ((8192, 8, 5, 1, 0, 0), 2), ((8192, 18, 4, 1, 0, 0), 2),
+                                         ((8192, 9, 2, 1, 0, 1), 4), ((8192, 14, 7, 2, 0, 0), 2), ((8192, 13, 3, 0, 1, 0), 2), ((8192, 18, 2, 0, 1, 0), 2), ((8192, 18, 4, 1, 1, 0), 2), ((8192, 16, 14, 2, 0, 0), 2), ((8192, 20, 3, 2, 0, 1), 4),
                                          ((8192, 12, 14, 0, 1, 0), 4), ((8192, 16, 14, 0, 1, 0), 2), ((8192, 14, 6, 0, 1, 0), 2), ((8192, 16, 14, 1, 1, 0), 4),
                                          ((8192, 20, 14, 1, 1, 0), 2), ((8192, 20, 14, 2, 1, 0), 4), ((8192, 32, 3, 2, 1, 0), 2),
                                          ((4096, 6, 2, 0, 0, 1), 2), ((8192, 2, 14, 0, 1, 1), 2), ((8192, 32, 2, 0, 1, 1), 2), ((8192, 16, 8, 1, 1, 1), 2),
