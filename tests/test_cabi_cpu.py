@@ -81,19 +81,32 @@ def test_quantize_rejects_bad_arguments_without_a_device(L):
     assert L.metis_nvfp4_quantize(p, 1, 0, 32, 32, None, 0, 0, 0, 0, p, p, p, p, 4096, None) == -2   # empty
 
 
-def test_calls_with_more_blocks_than_32_bits_count_are_refused(L):
-    # two blocks would share their random bits or their place in the outputs from there on; nothing is read or launched
+def test_stochastic_calls_with_more_blocks_than_the_counter_has_are_refused(L):
+    # two blocks would share their random bits from there on; nothing is read or launched
     from fp4_post_b200 import cabi
     buf = (C.c_uint8 * 4096)()
     p = C.addressof(buf)
     p += (-p) % 256
     rows, cols, room = 1 << 20, 1 << 16, 1 << 60
-    for flags in (cabi.Q_STOCHASTIC, cabi.Q_STOCHASTIC | cabi.Q_TRANSPOSE, cabi.Q_STOCHASTIC | cabi.Q_SR16, 0, cabi.Q_TRANSPOSE):
+    for flags in (cabi.Q_STOCHASTIC, cabi.Q_STOCHASTIC | cabi.Q_TRANSPOSE, cabi.Q_STOCHASTIC | cabi.Q_SR16):
         assert L.metis_nvfp4_quantize(p, 0, rows, cols, cols, None, flags, 0, 0, 1, p, p, p, p, room, None) == -7
         assert b"2^36" in L.metis_last_error_string()
-    for flags in (cabi.Q_STOCHASTIC, 0):
-        assert L.metis_nvfp4_quantize_dual(p, 0, rows, cols, cols, None, flags, 0, 0, 1, p, p, p, p, p, p, None, p, room, None) == -7
+    assert L.metis_nvfp4_quantize_dual(p, 0, rows, cols, cols, None, cabi.Q_STOCHASTIC, 0, 0, 1, p, p, p, p, p, p, None, p, room, None) == -7
+    assert b"2^36" in L.metis_last_error_string()
+
+
+def test_calls_with_more_blocks_than_32_bits_count_are_refused(L):
+    # round to nearest: two blocks would share their place in the outputs from there on; nothing is read or launched
+    from fp4_post_b200 import cabi
+    buf = (C.c_uint8 * 4096)()
+    p = C.addressof(buf)
+    p += (-p) % 256
+    rows, cols, room = 1 << 20, 1 << 16, 1 << 60
+    for flags in (0, cabi.Q_TRANSPOSE):
+        assert L.metis_nvfp4_quantize(p, 0, rows, cols, cols, None, flags, 0, 0, 1, p, p, p, p, room, None) == -7
         assert b"2^36" in L.metis_last_error_string()
+    assert L.metis_nvfp4_quantize_dual(p, 0, rows, cols, cols, None, 0, 0, 0, 1, p, p, p, p, p, p, None, p, room, None) == -7
+    assert b"2^36" in L.metis_last_error_string()
 
 
 def test_dual_quantizer_rejects_bad_arguments_without_a_device(L):

@@ -66,8 +66,7 @@ def test_fused_low_rank_product(M, N, K, rank):
 # Two or four epilogue warps per lane quarter (pair kernel), by stages, rounds of tiles and vectors (test_pair_drain.py has the lines): two and four
 # with row vectors and without, edges of D inside a 32-column chunk and a row block; few SMs give many rounds.
 @pytest.mark.parametrize("M,N,K,rank,row,sms", [(1300, 1096, 2560, 0, True, 8), (1300, 1096, 2304, 0, True, 8), (1300, 1096, 2304, 64, True, 8),
-                                                (1300, 1096, 2560, 0, False, 8), (1300, 1096, 2560, 0, True, 14), (1300, 1096, 2560, 0, True, 0),
-                                                (1300, 1096, 4096, 0, True, 8), (1300, 1096, 3840, 64, True, 8), (1300, 1096, 1280, 0, False, 8)])
+                                                (1300, 1096, 2560, 0, False, 8), (1300, 1096, 2560, 0, True, 14), (1300, 1096, 2560, 0, True, 0)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
     qa, qb, da, db = operands(M, N, K, seed=K + rank)
@@ -83,6 +82,12 @@ def test_epilogue_warps(M, N, K, rank, row, sms, dtype):
         want += float(qa.unit) * float(qb.unit) * (t.double() @ u.double().T).cpu().numpy()
     got = run(qa, qb, **kw).float().cpu().numpy()
     assert rel_l2(got, want) <= (1e-5 if dtype == torch.float32 else 2.0 ** -8)      # fp32 sums; one rounding to bf16
+
+
+@pytest.mark.parametrize("M,N,K,rank,row,sms", [(1300, 1096, 4096, 0, True, 8), (1300, 1096, 3840, 64, True, 8), (1300, 1096, 1280, 0, False, 8), (1300, 1096, 1536, 0, False, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_epilogue_warps_on_both_sides_of_each_line(M, N, K, rank, row, sms, dtype):
+    test_epilogue_warps(M, N, K, rank, row, sms, dtype)
 
 
 # Many short tiles per pair, where the epilogue bounds the product, and a last column of tiles of which one epilogue warp has two
