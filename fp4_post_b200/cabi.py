@@ -150,22 +150,26 @@ def lib() -> C.CDLL:
     return L
 
 
+def _bind_host() -> None:
+    global _host, _host_lib
+    L = lib()
+    if _host is None:
+        if not HOST_PATH.exists():
+            raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build` under this Python and torch")
+        spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    for name in EXPORTS:
+        _host.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
+    _host_lib = L
+
+
 def host():
     """The native part of the wrappers in ops.py (csrc/host_ops.cpp), with the entry points of lib(): allocations and call in one; every
     function returns (status, tensors...).  Callers of the C entry points alone do without it."""
-    global _host, _host_lib
-    L = lib()
-    if _host_lib is not L:
-        if _host is None:
-            if not HOST_PATH.exists():
-                raise MetisLibraryError(f"{HOST_PATH} is missing: build it with `python -m fp4_post_b200.build` under this Python and torch")
-            spec = importlib.util.spec_from_file_location("metis_host", HOST_PATH)
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
-            _host = module
-        for name in EXPORTS:
-            _host.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
-        _host_lib = L
+    if _host_lib is None or _host_lib is not _lib:
+        _bind_host()
     return _host
 
 
